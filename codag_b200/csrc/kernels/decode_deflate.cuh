@@ -1,23 +1,28 @@
-// Warp decoder for one Deflate (RFC 1951) chunk.
+// Team decoder for one Deflate (RFC 1951) chunk: two scan warps, a token warp, an expander warp.
 //
-// CODAG's decoder (include/zlib/zlib.h:807-902) decodes with 5-bit literal/length and 8-bit
-// distance lookup tables, walks code lengths 6..15 serially on a miss, copies
-// back-references with 4-byte pieces and ignores stored blocks.  This decoder keeps the
-// same one-warp-per-chunk shape but:
-//   - builds per-block lookup tables in shared memory of LB (9..11) bits for literals and
-//     lengths and 8 bits for distances, in parallel over the warp (canonical codes are
-//     tiled in MSB-first order, so each table slot finds its code by walking lengths);
-//   - keeps a 64-bit bit buffer refilled 32 bits at a time from the TMA input ring;
-//   - decodes a length or distance code together with its extra bits (one table entry
-//     gives both widths) and two literals per step where the table slot holds both codes;
-//   - expands back-references warp-cooperatively out of a shared-memory window of the
-//     output (the OUT ring: 1 or 2 KiB in the kernels here); older sources are read back
-//     from the chunk's already-written output, and such a load (length <= 32) is left in
-//     flight while the next symbols decode;
-//   - drains output in quarter-window pieces with vector stores;
-//   - decodes stored blocks.
-// Every lane runs the same symbol loop on the same data (shared-memory reads broadcast), so
-// control flow stays uniform and only the stores are lane-specific.
+// CODAG's decoder (include/zlib/zlib.h:807-902) runs one symbol at a time on all 32 lanes
+// of a warp.  So did the first kernels here, and they spent about 140 warp instructions on every
+// symbol.  This decoder puts the lanes to work on different symbols, in three stages:
+//
+//   - Scan (two warps, 64 lanes).  A Huffman bit stream read from a wrong bit falls into step with
+//     the right symbol boundaries after a while (text compressed by zlib at level 6: after 106 bits
+//     on average, in 99% of the cases within 512).  The lanes cut the next stretch of a block into
+//     64 pieces.  Each warms up kWarmBits before its piece to guess where the piece's first symbol
+//     starts, decodes the piece from there, and notes where every kCell-th symbol begins.  A lane
+//     whose start turns out not to be the end of the lane below decodes once more, until the chain
+//     from lane 0, whose start is known, holds.  So the result is the serial decoder's, whatever
+//     the guesses were.
+//   - Tokens (one warp).  Decodes the noted cells again, 32 at a time, this time from known starts,
+//     into a dense list of tokens.  Decoding twice is cheaper than keeping every lane's tokens:
+//     their number varies too much from piece to piece to give each lane room of its own.
+//   - Expand (one warp).  Places 32 tokens at a time by a prefix sum of their lengths and writes 32
+//     consecutive output bytes per step: each lane finds the token that covers its byte, then takes
+//     the literal or the byte `distance` before from a 32 KiB shared-memory window (the largest
+//     distance Deflate has, so no source is ever read back from global memory).  A source inside the
+//     same 32 bytes is followed lane to lane.
+//
+// The stages run as a pipeline, each handing over in two buffers with a named barrier, so no warp
+// spins.
 #pragma once
 #include "device_common.cuh"
 
@@ -34,16 +39,16 @@ __constant__ uint8_t kDistExtra[30] = {0, 0, 0, 0, 1, 1, 2, 2,  3,  3,  4,  4,  
                                        6, 7, 7, 8, 8, 9, 9, 10, 10, 11, 11, 12, 12, 13, 13};
 __constant__ uint8_t kCodeLenOrder[19] = {16, 17, 18, 0, 8, 7, 9, 6, 10, 5, 11, 4, 12, 3, 13, 2, 14, 1, 15};
 
-constexpr uint32_t kDistLB = 8;
+constexpr uint32_t kLitLB = 10;  // codes of 11 and more bits: 0.02-0.3% of the symbols measured
+constexpr uint32_t kDistLB = 9;
 constexpr uint32_t kCodeLenLB = 7;
 
 // Table entry (32 bits):
-//   [0,5)   bits consumed in all: code length + extra bits, or both codes of a literal pair
-//   [5,9)   code length of the (first) symbol
-//   [9,11)  kind: literal(s), length, end of block, other (invalid, or not in the table)
-//   [11]    a second literal follows in [24,32) (literal/length tables only)
+//   [0,5)   bits consumed in all: code length + extra bits
+//   [5,9)   code length of the symbol
+//   [9,11)  kind: literal, length, end of block, other (invalid, or not in the table)
 //   [12]    the code is longer than the table: decode it with slow_entry
-//   [16,32) literal byte in [16,24) / length or distance base / code-length symbol
+//   [16,32) literal byte / length or distance base / code-length symbol
 enum : uint32_t {
   kKindShift = 9,
   kKindMask = 3u << kKindShift,
@@ -51,7 +56,6 @@ enum : uint32_t {
   kKindLenBits = 1u << kKindShift,
   kKindEndBits = 2u << kKindShift,
   kKindBadBits = 3u << kKindShift,
-  kPairFlag = 1u << 11,
   kSlowFlag = 1u << 12,
   kSlowEntry = kKindBadBits | kSlowFlag,
 };
@@ -84,18 +88,18 @@ __device__ __forceinline__ uint32_t bfe32(uint32_t x, uint32_t pos, uint32_t n) 
 }
 
 struct HuffTable {
-  uint32_t* lut;     // 1 << lb entries
+  uint32_t* lut;     // 1 << LB entries
   uint16_t* sorted;  // symbols ordered by (code length, symbol)
   uint32_t* cnt;     // [16] codes per length
   uint32_t* first;   // [16] first canonical code per length
   uint32_t* index;   // [16] position of the first code of each length in `sorted`
-  uint32_t lb;
 };
 
 // Builds `t` from code lengths lens[0..nsym).  False when the lengths over-subscribe the
 // code space.  Incomplete codes are accepted; their unused codes decode as invalid.
-__device__ bool build_table(const uint8_t* lens, uint32_t nsym, const HuffTable& t, int alpha,
-                            uint32_t* fill, uint32_t lane) {
+template <uint32_t LB, int ALPHA>
+__device__ __noinline__ bool build_table(const uint8_t* lens, uint32_t nsym, HuffTable t, uint32_t* fill,
+                                         uint32_t lane) {
   if (lane < 16) t.cnt[lane] = 0;
   __syncwarp();
   for (uint32_t s = lane; s < nsym; s += 32) {
@@ -130,556 +134,692 @@ __device__ bool build_table(const uint8_t* lens, uint32_t nsym, const HuffTable&
     if (l && rank == 0) fill[l] += __popc(grp);
     __syncwarp();
   }
-  const uint32_t n = 1u << t.lb;
-  for (uint32_t x = lane; x < n; x += 32) {
-    const uint32_t v = __brev(x) >> (32 - t.lb);  // MSB-first code prefix of table slot x
-    uint32_t entry = kSlowEntry;
-    for (uint32_t l = 1; l <= t.lb; l++) {
-      const uint32_t k = (v >> (t.lb - l)) - t.first[l];
-      if (k < t.cnt[l]) {
-        entry = make_entry(t.sorted[t.index[l] + k], l, alpha);
-        break;
+  // canonical codes tiled in MSB-first order: slot x finds its code by comparing its prefix of
+  // every length with that length's range of codes (ranges of two lengths never both match)
+  uint32_t first[LB], cnt[LB];
+#pragma unroll
+  for (uint32_t l = 1; l <= LB; l++) {
+    first[l - 1] = t.first[l];
+    cnt[l - 1] = t.cnt[l];
+  }
+  for (uint32_t x = lane; x < (1u << LB); x += 32) {
+    const uint32_t v = __brev(x) >> (32 - LB);  // MSB-first code prefix of table slot x
+    uint32_t len = 0, k = 0;
+#pragma unroll
+    for (uint32_t l = 1; l <= LB; l++) {
+      const uint32_t d = (v >> (LB - l)) - first[l - 1];
+      if (d < cnt[l - 1]) {
+        len = l;
+        k = d;
       }
     }
-    t.lut[x] = entry;
+    t.lut[x] = len ? make_entry(t.sorted[t.index[len] + k], len, ALPHA) : static_cast<uint32_t>(kSlowEntry);
   }
   __syncwarp();
-  if (alpha == kAlphaLitLen) {
-    // literal pairs: when the bits of slot x after its literal code hold a whole literal
-    // code too, the entry carries both.  Only the first-literal fields of the other slot
-    // are read, and a pair rewrite leaves those fields unchanged, so lanes need no order.
-    for (uint32_t x = lane; x < n; x += 32) {
-      const uint32_t e1 = t.lut[x];
-      const uint32_t l1 = (e1 >> 5) & 15u;
-      if ((e1 & kKindMask) != kKindLitBits || l1 >= t.lb) continue;
-      const uint32_t e2 = t.lut[x >> l1];
-      const uint32_t l2 = (e2 >> 5) & 15u;
-      if ((e2 & kKindMask) != kKindLitBits || l1 + l2 > t.lb) continue;
-      t.lut[x] = (e1 & ~31u & 0x00ffffffu) | (l1 + l2) | kPairFlag | ((e2 & 0x00ff0000u) << 8);
-    }
-    __syncwarp();
-  }
   return true;
 }
 
-// Codes longer than the table width: walk lengths lb+1..15 (zlib.h:459-527 does 6..15).
-__device__ __forceinline__ uint32_t slow_entry(uint64_t bb, const HuffTable& t, int alpha) {
-  const uint32_t rev = __brev(static_cast<uint32_t>(bb));
-  for (uint32_t l = t.lb + 1; l < 16; l++) {
+// Codes longer than the table width: walk lengths LB+1..15 (zlib.h:459-527 does 6..15).
+template <uint32_t LB>
+__device__ __noinline__ uint32_t slow_entry(uint32_t bits, HuffTable t, int alpha) {
+  const uint32_t rev = __brev(bits);
+  for (uint32_t l = LB + 1; l < 16; l++) {
     const uint32_t k = (rev >> (32 - l)) - t.first[l];
     if (k < t.cnt[l]) return make_entry(t.sorted[t.index[l] + k], l, alpha);
   }
   return 0;
 }
 
-// Per-warp shared memory of the Deflate decoder: the current block's canonical codes, and
-// (InflateScratch) its lookup tables.  The batched kernel can keep the lookup tables in
-// global memory instead (read through L1), which frees 3-9 KiB of shared memory per warp.
-struct InflateCodes {
+// Tables of one block.
+struct InflateTables {
+  uint32_t lit_lut[1u << kLitLB];
+  uint32_t dist_lut[1u << kDistLB];
   uint32_t lit_cnt[16], lit_first[16], lit_index[16];
   uint32_t dist_cnt[16], dist_first[16], dist_index[16];
-  uint32_t fill[16];
   uint16_t lit_sorted[288];
   uint16_t dist_sorted[32];
-  uint8_t lens[320];
+  __device__ __forceinline__ HuffTable lit() { return {lit_lut, lit_sorted, lit_cnt, lit_first, lit_index}; }
+  __device__ __forceinline__ HuffTable dist() { return {dist_lut, dist_sorted, dist_cnt, dist_first, dist_index}; }
 };
-template <int LB>
-struct InflateScratch : InflateCodes {
-  uint32_t lit_lut[1u << LB];
-  uint32_t dist_lut[1u << kDistLB];
-};
-// entries of the global-memory tables of one warp
-template <int LB>
-constexpr uint32_t kLutEntries = (1u << LB) + (1u << kDistLB);
 
-// table entry i: a shared-memory table (saddr) or a global one (p)
-template <bool GT>
-__device__ __forceinline__ uint32_t lut_ld(const uint32_t* p, uint32_t saddr, uint32_t i) {
-  if constexpr (GT) return p[i];
-  else return ld_s32(saddr + 4u * i);
+constexpr uint32_t kPieces = 64;
+constexpr uint32_t kCell = 8;          // symbols from one noted start to the next
+constexpr uint32_t kCells = 28;        // noted starts of one piece
+constexpr uint32_t kRow = kCells + 1;  // an odd stride spreads the lanes' rows over the banks
+// A piece aims at kPieceTokens symbols (by the last stretch's bits per symbol), well below the
+// kCell * kCells it may hold, and is at most kMaxSpan words long, so that 64 pieces fit the 15 KiB of
+// the input ring that are resident behind any read position.  Spans are odd numbers of words: the
+// lanes' first words lie in different banks.
+constexpr uint32_t kPieceTokens = 150;
+constexpr uint32_t kMinSpan = 13, kMaxSpan = 47;
+constexpr uint32_t kWarmBits = 640;
+
+enum : uint32_t { kBatchTokens = 0, kBatchStored = 1, kBatchDone = 2 };
+struct ScanBatch {
+  uint16_t row[kPieces * kRow];  // bit offset of each cell from its piece's first bit
+  uint16_t cnt[kPieces];         // symbols of each piece
+  uint32_t kind;
+  uint32_t base;   // first bit (kBatchTokens), first byte (kBatchStored), in ring coordinates
+  uint32_t size;   // bits per piece, or bytes
+  uint32_t table;
+  int32_t status;  // with kBatchDone
+};
+
+// Token: bit 31 set = a literal in bits 0-7; clear = a match, length in bits 0-8 and distance in
+// bits 9-24.
+constexpr uint32_t kTokens = 32 * kCell;
+constexpr uint32_t kLastTokens = 0x80000000u;
+constexpr uint32_t kStageWords = 400;  // 32 cells of 8 symbols of 48 bits, and the words around them
+
+using InflateRing = InRing<16>;
+using InflateWin = OutRing<15, 11, true>;  // 32 KiB window, 2 KiB drains by TMA bulk stores
+constexpr uint32_t kTeamWarps = 4;
+
+// Shared memory of one team; three teams fit an SM.
+struct InflateTeam {
+  alignas(128) uint8_t win[InflateWin::kBytes];
+  alignas(128) uint8_t ring[InflateRing::kBytes];
+  InflateTables tab[2];  // the scan warps build the next block's while the token warp reads the last's
+  ScanBatch batch[2];
+  alignas(16) uint32_t tok[2][kTokens];
+  uint32_t tok_cnt[2];  // tokens in the buffer; kLastTokens with the chunk's last one
+  uint32_t stage[kStageWords];
+  uint16_t cell_end[kPieces];
+  uint8_t lens[320];
+  uint32_t fill[2][16];
+  uint32_t last[kPieces];  // scan warps: where each piece ended, and how
+  uint8_t how[kPieces];
+  uint32_t redo[2], stop_at[2], sum[2], header_ok;
+  int32_t scan_st;
+  int32_t status;      // the scan's, with the last token buffer
+  uint32_t stop;       // set by the expander: the output is full or a distance is bad
+  uint32_t stopped[2]; // `stop` as the token warp saw it, one word per batch buffer
+  uint32_t job;     // batched kernel: the team's current job
+  uint64_t bar[16];
+};
+static_assert(sizeof(InflateTeam) <= 76458, "three teams per SM: 227 KiB / 3 less 1 KiB each");
+
+template <uint32_t ID, uint32_t THREADS>
+__device__ __forceinline__ void team_barrier() {
+  asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(THREADS) : "memory");
+}
+__device__ __forceinline__ void scan_barrier() { team_barrier<1, 64>(); }      // the scan warps
+__device__ __forceinline__ void batch_barrier() { team_barrier<2, 96>(); }     // scan -> tokens
+__device__ __forceinline__ void token_barrier() { team_barrier<3, 64>(); }     // tokens -> expander
+__device__ __forceinline__ void job_barrier() { team_barrier<4, 32 * kTeamWarps>(); }
+
+// One symbol (with its distance) at bit offset `sh` of w0: returns its kind, the bits it takes in
+// `used` and its token.
+__device__ __forceinline__ uint32_t symbol(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t sh, uint32_t s_lit,
+                                           uint32_t s_dist, InflateTables& tab, uint32_t& used, uint32_t& tok) {
+  const uint32_t lo = __funnelshift_r(w0, w1, sh);
+  uint32_t e = ld_s32(s_lit + 4u * (lo & ((1u << kLitLB) - 1u)));
+  if (e & kSlowFlag) e = slow_entry<kLitLB>(lo, tab.lit(), kAlphaLitLen);
+  used = e & 31u;
+  tok = 0x80000000u | ((e >> 16) & 0xffu);
+  uint32_t kind = used ? e & kKindMask : static_cast<uint32_t>(kKindBadBits);
+  if (kind == kKindLenBits) {
+    const uint32_t ln = (e >> 5) & 15u;
+    const uint32_t len = (e >> 16) + bfe32(lo, ln, used - ln);
+    const uint32_t x = __funnelshift_r(lo, __funnelshift_r(w1, w2, sh), used);
+    uint32_t d = ld_s32(s_dist + 4u * (x & ((1u << kDistLB) - 1u)));
+    if (d & kSlowFlag) d = slow_entry<kDistLB>(x, tab.dist(), kAlphaDist);
+    const uint32_t dt = d & 31u, dn = (d >> 5) & 15u;
+    if (!dt || (d & kKindMask)) kind = kKindBadBits;
+    tok = len | (((d >> 16) + bfe32(x, dn, dt - dn)) << 9);
+    used += dt;
+  }
+  return kind;
 }
 
-template <int NSLOT>
-struct BitReader {
-  uint64_t bb;    // pending bits, next bit in bit 0
-  uint32_t bc;    // number of pending bits
-  uint32_t wpos;  // ring position of the next 32-bit word (multiple of 4)
+// ---------------------------------------------------------------------------------------
+// scan warps
+// ---------------------------------------------------------------------------------------
+enum : uint32_t { kRun = 0, kEob = 1, kBad = 2, kFull = 3 };  // how a lane's piece ended
 
-  // append one word; returns a status (corruption = read far beyond the stream)
-  __device__ __forceinline__ int refill(InRing<NSLOT>& in) {
-    if (wpos < in.hi) {
-      const uint32_t end = min(wpos + 4, in.hi);
-      if (end > (in.waited << kSlotLog2)) {
-        // the buffer holds at most 8 bytes before wpos; everything older is consumed
-        if (!in.release(wpos >= 8 ? wpos - 8 : 0)) return CODAG_ETIMEOUT;
-        const int st = in.ensure(end);
-        if (st) return st;
-      }
-    } else if (wpos > in.hi + 16) {
-      return CODAG_ECORRUPT;
+struct InflateScan {
+  InflateRing in;  // warp 0 of the two fills it
+  InflateTeam& sm;
+  uint32_t warp, lane, id;
+  uint32_t pos;    // next bit of the stream, in ring coordinates (streams are < 2^28 bytes)
+  uint32_t hi8;    // first bit past the stream
+  uint32_t span;   // words per piece
+  uint32_t k;      // batch buffer
+  uint32_t tab, handed;  // tables of this block, and of the batch handed over last
+  uint32_t fixed;  // bit t: tab[t] holds the fixed codes
+
+  // 32 stream bits at bit p (they must be resident, or beyond the stream's end)
+  __device__ __forceinline__ uint32_t peek(uint32_t p) const {
+    const uint32_t a = (p >> 5) << 2;
+    return __funnelshift_r(in.rd32(a), in.rd32(a + 4), p & 31u);
+  }
+
+  // makes `bits` bits from pos resident (as far as the stream goes); both warps are done reading
+  // what lies below pos
+  __device__ __forceinline__ int need(uint32_t bits) {
+    scan_barrier();
+    if (warp == 0) {
+      const uint32_t p = pos >> 3, end = ((pos + bits) >> 3) + 8u;
+      const int st = in.release(p < in.hi ? p : in.hi) ? in.ensure(end < in.hi ? end : in.hi) : CODAG_ETIMEOUT;
+      if (lane == 0) sm.scan_st = st;
     }
-    bb |= static_cast<uint64_t>(in.rd32(wpos)) << bc;
-    bc += 32;
-    wpos += 4;
+    scan_barrier();
+    return sm.scan_st;
+  }
+
+  // hands batch buffer k to the token warp; false when the expander wants no more
+  __device__ __forceinline__ bool handoff(uint32_t kind, uint32_t base, uint32_t size, int status) {
+    if (id == 0) {
+      ScanBatch& b = sm.batch[k];
+      b.kind = kind;
+      b.base = base;
+      b.size = size;
+      b.table = tab;
+      b.status = status;
+    }
+    batch_barrier();
+    const bool go = sm.stopped[k] == 0;
+    k ^= 1u;
+    handed = tab;
+    return go;
+  }
+
+  // Where the first symbol that ends at or past `end` ends, decoding from bit p, a guess; what the
+  // stream does not allow is stepped over.
+  __device__ __forceinline__ uint32_t warm_up(uint32_t p, uint32_t end, bool go, uint32_t s_lit, uint32_t s_dist) {
+    uint32_t n = 0;
+    while (__any_sync(FULL, go)) {
+      if (go) {
+        const uint32_t a = (p >> 5) << 2;
+        uint32_t used, tok;
+        const uint32_t kind =
+            symbol(in.rd32(a), in.rd32(a + 4), in.rd32(a + 8), p & 31u, s_lit, s_dist, sm.tab[tab], used, tok);
+        p += kind == kKindBadBits ? 1u : used;
+        go = p < end && ++n < 2u * kWarmBits;
+      }
+    }
+    return p;
+  }
+
+  // The symbols of one piece from bit p until one ends at or past `end`, as the serial decoder would
+  // read them; every kCell-th start is noted in `row` as an offset from bit `from`.  Every turn brings
+  // the lanes back together.
+  __device__ __forceinline__ uint32_t piece(uint32_t p, uint32_t end, uint32_t from, bool on, uint16_t* row,
+                                            uint32_t s_lit, uint32_t s_dist, uint32_t& cnt, uint32_t& how) {
+    uint32_t n = 0, h = kRun;
+    bool go = on && p < end;
+    while (__any_sync(FULL, go)) {
+      if (go) {
+        const uint32_t a = (p >> 5) << 2;
+        uint32_t used, tok;
+        const uint32_t kind =
+            symbol(in.rd32(a), in.rd32(a + 4), in.rd32(a + 8), p & 31u, s_lit, s_dist, sm.tab[tab], used, tok);
+        const uint32_t at = p;
+        p += used;
+        if (kind == kKindBadBits || p > hi8) {
+          h = kBad;
+          go = false;
+        } else if (kind == kKindEndBits) {
+          h = kEob;
+          go = false;
+        } else {
+          if ((n & (kCell - 1u)) == 0) row[n / kCell] = static_cast<uint16_t>(at - from);
+          n++;
+          go = p < end;
+          if (go && n == kCell * kCells) {
+            h = kFull;
+            go = false;
+          }
+        }
+      }
+    }
+    cnt = n;
+    how = h;
+    return p;
+  }
+
+  // The symbols of one block, stretch by stretch, up to and including its end-of-block code.
+  __device__ __forceinline__ int symbols() {
+    const uint32_t s_lit = smem_u32(sm.tab[tab].lit_lut), s_dist = smem_u32(sm.tab[tab].dist_lut);
+    for (;;) {
+      // no longer than the rest of the stream needs, so that short streams use all lanes
+      const uint32_t rest = (hi8 - pos) / (32u * kPieces);
+      const uint32_t words = (span < rest ? span : rest > kMinSpan ? rest : kMinSpan) | 1u;
+      const uint32_t bits = words * 32u;
+      int st = need(kPieces * bits + 64u);
+      if (st) return st;
+      const uint32_t from = pos + id * bits, end = from + bits;
+      uint16_t* row = sm.batch[k].row + id * kRow;
+      const bool inside = from < hi8;
+      uint32_t start = warm_up(id * bits > kWarmBits ? from - kWarmBits : pos, from, inside && id, s_lit, s_dist);
+      if (!inside) start = from;
+      bool redo = start < hi8;
+      uint32_t last = start, cnt = 0, how = redo ? kRun : kBad;
+      uint64_t stop;
+      for (;;) {
+        uint32_t c, h;
+        const uint32_t l = piece(start, end, from, redo, row, s_lit, s_dist, c, h);
+        if (redo) {
+          last = l;
+          cnt = c;
+          how = h;
+        }
+        sm.last[id] = last;
+        sm.how[id] = static_cast<uint8_t>(how);
+        scan_barrier();
+        // lanes whose start is not where the lane below ended; only those below the first lane that
+        // ended the stretch matter
+        const uint32_t below = id ? sm.last[id - 1] : 0u, bhow = id ? sm.how[id - 1] : static_cast<uint32_t>(kBad);
+        redo = bhow == kRun && below != start;
+        const uint32_t rm = __ballot_sync(FULL, redo), sp = __ballot_sync(FULL, how != kRun);
+        if (lane == 0) {
+          sm.redo[warp] = rm;
+          sm.stop_at[warp] = sp;
+        }
+        scan_barrier();
+        const uint64_t m = (static_cast<uint64_t>(sm.redo[1]) << 32) | sm.redo[0];
+        stop = (static_cast<uint64_t>(sm.stop_at[1]) << 32) | sm.stop_at[0];
+        if (!m || (stop && __ffsll(stop) < __ffsll(m))) break;
+        if (redo) {
+          start = last = below;
+          cnt = 0;
+          redo = start < hi8;
+          how = redo ? kRun : kBad;
+        }
+      }
+      const uint32_t top = stop ? static_cast<uint32_t>(__ffsll(stop)) - 1u : kPieces - 1u;  // last piece that counts
+      if (id > top) cnt = 0;
+      sm.batch[k].cnt[id] = static_cast<uint16_t>(cnt);
+      const uint32_t s = __reduce_add_sync(FULL, cnt);
+      if (lane == 0) sm.sum[warp] = s;
+      const uint32_t next = sm.last[top], end_how = sm.how[top];
+      scan_barrier();
+      const uint32_t total = sm.sum[0] + sm.sum[1];
+      if (total && !handoff(kBatchTokens, pos, bits, CODAG_OK)) return CODAG_ECORRUPT;
+      if (end_how == kBad) return CODAG_ECORRUPT;
+      if (total) {
+        const uint32_t w = (next - pos) * kPieceTokens / (32u * total);
+        span = w < kMaxSpan ? w : kMaxSpan;
+      }
+      pos = next;
+      if (end_how == kEob) return CODAG_OK;
+    }
+  }
+
+  // Stored block: the token warp reads its bytes itself.
+  __device__ __forceinline__ int stored() {
+    pos = (pos + 7u) & ~7u;
+    int st = need(64);
+    if (st) return st;
+    const uint32_t v = peek(pos);
+    pos += 32;
+    const uint32_t len = v & 0xffffu;
+    if (len != (~(v >> 16) & 0xffffu)) return CODAG_ECORRUPT;
+    if ((pos >> 3) + len > in.hi) return CODAG_ECORRUPT;
+    if (len && !handoff(kBatchStored, pos >> 3, len, CODAG_OK)) return CODAG_ECORRUPT;
+    // the ring goes on in steps it can hold
+    for (uint32_t left = len * 8u; left;) {
+      const uint32_t step = left < 8192u * 8u ? left : 8192u * 8u;
+      st = need(step);
+      if (st) return st;
+      pos += step;
+      left -= step;
+    }
     return CODAG_OK;
   }
 
-  __device__ __forceinline__ void start(InRing<NSLOT>& in, uint32_t p) {
-    wpos = p & ~3u;
-    bb = 0;
-    bc = 0;
-    (void)in;
+  // Code lengths and tables of a dynamic block (zlib.h:607-707); both warps read the code lengths,
+  // then one builds the literal/length table and the other the distance table.
+  __device__ __forceinline__ int dynamic_header() {
+    int st = need(2400);  // the largest header: 14 + 19 * 3 + 316 * 7 bits
+    if (st) return st;
+    const uint32_t v = peek(pos);
+    const uint32_t hlit = (v & 31u) + 257u, hdist = ((v >> 5) & 31u) + 1u, hclen = ((v >> 10) & 15u) + 4u;
+    pos += 14;
+    if (hlit > 286 || hdist > 30) return CODAG_ECORRUPT;
+    const HuffTable cl = sm.tab[tab].dist();
+    const uint32_t s_cl = smem_u32(sm.tab[tab].dist_lut);
+    if (warp == 0) {
+      if (lane < 19)  // code length code lengths, 3 bits each in kCodeLenOrder order
+        sm.lens[kCodeLenOrder[lane]] = lane < hclen ? static_cast<uint8_t>(peek(pos + 3u * lane) & 7u) : 0;
+      __syncwarp();
+      const bool ok = build_table<kCodeLenLB, kAlphaCodeLen>(sm.lens, 19, cl, sm.fill[0], lane);
+      __syncwarp();
+      for (uint32_t s = lane; s < 80; s += 32) reinterpret_cast<uint32_t*>(sm.lens)[s] = 0;
+      if (lane == 0) sm.header_ok = ok;
+    }
+    pos += 3u * hclen;
+    scan_barrier();
+    if (!sm.header_ok) return CODAG_ECORRUPT;
+    // literal/length and distance code lengths, run-length coded with symbols 16..18.  Lane l decodes
+    // at bit l of a 32-bit stretch; the warp then steps from symbol to symbol by shuffles.
+    uint32_t idx = 0, prev = 0;
+    const uint32_t total = hlit + hdist;
+    uint32_t at = 0;
+    while (idx < total) {
+      pos += at;
+      at = 0;
+      if (pos > hi8) return CODAG_ECORRUPT;
+      const uint32_t bits = peek(pos + lane);
+      const uint32_t e = ld_s32(s_cl + 4u * (bits & ((1u << kCodeLenLB) - 1u)));
+      const uint32_t n = e & 31u, sym = e >> 16, x = bits >> n;
+      // the run this symbol stands for: value (or 255: the previous one), repeats, bits
+      const uint32_t rep = sym < 16 ? 1u : sym == 16 ? 3u + (x & 3u) : sym == 17 ? 3u + (x & 7u) : 11u + (x & 127u);
+      const uint32_t took = n + (sym < 16 ? 0u : sym == 16 ? 2u : sym == 17 ? 3u : 7u);
+      const uint32_t val = sym < 16 ? sym : sym == 16 ? 255u : 0u;
+      const uint32_t run = (e & kSlowFlag) ? 0u : rep | (took << 8) | (val << 16);  // code lengths are at most 7 bits
+      while (at < 32 && idx < total) {
+        const uint32_t r = __shfl_sync(FULL, run, at);
+        if (!r) return CODAG_ECORRUPT;
+        const uint32_t rr = r & 0xffu;
+        uint32_t vv = r >> 16;
+        if (vv == 255u) {
+          if (idx == 0) return CODAG_ECORRUPT;
+          vv = prev;
+        }
+        if (idx + rr > total) return CODAG_ECORRUPT;
+        if (warp == 0 && vv && lane < rr) sm.lens[idx + lane] = static_cast<uint8_t>(vv);  // a repeat of 7 or more is zeros
+        prev = vv;
+        idx += rr;
+        at += (r >> 8) & 0xffu;
+      }
+    }
+    pos += at;
+    scan_barrier();
+    if (sm.lens[256] == 0) return CODAG_ECORRUPT;
+    bool ok;
+    if (warp == 0) ok = build_table<kLitLB, kAlphaLitLen>(sm.lens, hlit, sm.tab[tab].lit(), sm.fill[0], lane);
+    else ok = build_table<kDistLB, kAlphaDist>(sm.lens + hlit, hdist, sm.tab[tab].dist(), sm.fill[1], lane);
+    if (lane == 0) sm.sum[warp] = ok;
+    scan_barrier();
+    return sm.sum[0] & sm.sum[1] ? CODAG_OK : CODAG_ECORRUPT;
   }
-  __device__ __forceinline__ void drop(uint32_t n) {
-    bb >>= n;
-    bc -= n;
+
+  // fixed Huffman codes (RFC 1951 3.2.6)
+  __device__ __forceinline__ void fixed_tables() {
+    for (uint32_t s = id; s < 320; s += 64) sm.lens[s] = s < 144 ? 8 : s < 256 ? 9 : s < 280 ? 7 : s < 288 ? 8 : 5;
+    scan_barrier();
+    if (warp == 0) build_table<kLitLB, kAlphaLitLen>(sm.lens, 288, sm.tab[tab].lit(), sm.fill[0], lane);
+    else build_table<kDistLB, kAlphaDist>(sm.lens + 288, 30, sm.tab[tab].dist(), sm.fill[1], lane);
+    scan_barrier();
   }
-  // stream position (ring coordinates) of the next unread bit, times 8
-  __device__ __forceinline__ uint64_t bitpos() const { return static_cast<uint64_t>(wpos) * 8u - bc; }
+
+  // The stream bound to `in`, `wrapper` header bytes first.
+  __device__ __forceinline__ int run(uint32_t wrapper) {
+    if (in.lo + wrapper > in.hi) return CODAG_ECORRUPT;
+    pos = (in.lo + wrapper) * 8u;
+    hi8 = in.hi * 8u;
+    span = 41;
+    bool last = false;
+    while (!last) {
+      if (pos >= hi8) return CODAG_ECORRUPT;
+      int st = need(64);
+      if (st) return st;
+      const uint32_t h = peek(pos);
+      last = h & 1u;
+      const uint32_t btype = (h >> 1) & 3u;
+      pos += 3;
+      tab = handed ^ 1u;  // the token warp may still read the tables of the last batch
+      if (btype == 0) {
+        st = stored();
+      } else if (btype == 1) {
+        if (!((fixed >> tab) & 1u)) fixed_tables();
+        fixed |= 1u << tab;
+      } else if (btype == 2) {
+        fixed &= ~(1u << tab);
+        st = dynamic_header();
+      } else {
+        st = CODAG_ECORRUPT;
+      }
+      if (!st && btype) st = symbols();
+      if (st) return st;
+    }
+    return pos > hi8 ? CODAG_ECORRUPT : CODAG_OK;
+  }
 };
 
-// ---------------------------------------------------------------------------------------
-// Decoder/expander pairs (one CTA of two warps per chunk)
-// ---------------------------------------------------------------------------------------
-// The decoder warp runs the block and symbol loops below but emits tokens instead of bytes; the
-// expander warp turns the tokens into output through the usual window.  Tokens travel in two
-// shared-memory batches handed over with a named barrier of the pair's 64 threads: after
-// barrier k the decoder fills one batch while the expander drains the other, and each side
-// reaches barrier k+1 only when done with its batch, so neither ever spins.
-// Token: bit 31 set = one or two literals (bits 0-7, 8-15; bit 16 = two); clear = a match,
-// length in bits 0-8 and distance in bits 9-24.
-// 496 tokens a batch: the two batches and their counters fit in 4 KiB (the batched kernel keeps
-// them in the expander warp's idle input ring)
-constexpr uint32_t kTokBatch = 496;
-struct TokenShared {
-  uint32_t tok[2][kTokBatch];
-  uint32_t cnt[2];
-  uint32_t done;
-  int32_t status;
-  uint32_t job;  // batched kernel: the pair's current job
-};
-static_assert(sizeof(TokenShared) <= 4096, "token batches must fit a 4 KiB ring");
-
-__device__ __forceinline__ void pair_barrier(uint32_t id) {
-  asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory");
+// Binds a team's input ring (barriers initialised) and its window.
+__device__ __forceinline__ void inflate_ring(InflateRing& in, InflateTeam& sm, uint64_t wait_cycles, uint32_t lane,
+                                             bool init) {
+  in.buf = sm.ring;
+  in.sbuf = smem_u32(sm.ring);
+  in.bar = sm.bar;
+  in.phase = 0;
+  in.wait_cycles = wait_cycles;
+  in.lane = lane;
+  if (init) init_ring_barriers<16>(sm.bar, lane);
+}
+__device__ __forceinline__ void inflate_window(InflateWin& o, InflateTeam& sm, uint32_t lane) {
+  o.buf = sm.win;
+  o.sbuf = smem_u32(sm.win);
+  o.lane = lane;
 }
 
-struct NoTokens {  // single-warp decode: bytes go straight to the window
-  static constexpr bool kOn = false;
-  __device__ __forceinline__ void literal(uint32_t, uint32_t) {}
-  __device__ __forceinline__ void match(uint32_t, uint32_t) {}
-};
+// Scan warps (0 and 1 of the team): the stream bound to `in`.
+__device__ __forceinline__ void inflate_scan(InflateRing& in, InflateTeam& sm, uint32_t wrapper, uint32_t warp,
+                                             uint32_t lane) {
+  InflateScan d{in, sm, warp, lane, warp * 32u + lane, 0, 0, 0, 0, 0, 1, 0};
+  int st = d.run(wrapper);
+  if (warp == 0) {
+    if (!d.in.drain()) st = CODAG_ETIMEOUT;
+    in.phase = d.in.phase;  // the next stream through this ring goes on from here
+  }
+  d.handoff(kBatchDone, 0, 0, st);
+}
 
-struct TokenPipe {
-  static constexpr bool kOn = true;
-  TokenShared* sh;
-  uint32_t bar, k, n, lane;
-  __device__ __forceinline__ void handoff() {
+// ---------------------------------------------------------------------------------------
+// token warp
+// ---------------------------------------------------------------------------------------
+// Word w of the stream in ring coordinates, straight from global memory; bytes outside [lo, hi)
+// are not read.
+__device__ __forceinline__ uint32_t stream_word(const uint8_t* gbase, uint32_t w, uint32_t lo, uint32_t hi) {
+  const uint32_t a = 4u * w;
+  if (a >= lo && a + 4u <= hi) return __ldg(reinterpret_cast<const uint32_t*>(gbase + a));
+  uint32_t v = 0;
+  for (uint32_t i = 0; i < 4; i++)
+    if (a + i >= lo && a + i < hi) v |= static_cast<uint32_t>(__ldg(gbase + a + i)) << (8u * i);
+  return v;
+}
+
+__device__ __forceinline__ void inflate_tokens(InflateTeam& sm, const uint8_t* gbase, uint32_t lo, uint32_t hi,
+                                               uint32_t lane) {
+  uint32_t kb = 0, k = 0;
+  // hands the token buffer with n tokens to the expander
+  const auto handoff = [&](uint32_t n) {
+    if (lane == 0) sm.tok_cnt[k] = n;
     __syncwarp();
-    if (lane == 0) sh->cnt[k] = n;
-    pair_barrier(bar);
+    token_barrier();
     k ^= 1u;
-    n = 0;
-  }
-  __device__ __forceinline__ void push(uint32_t t) {
-    // lane 0 writes the token: a predicated store, no branch on the lane
-    const uint32_t a = smem_u32(&sh->tok[k][n]);
-    asm volatile("{ .reg .pred p; setp.eq.u32 p, %0, 0; @p st.shared.u32 [%1], %2; }" ::"r"(lane), "r"(a), "r"(t)
-                 : "memory");
-    if (++n == kTokBatch) handoff();
-  }
-  // one literal, or two (second in bits 8-15 when `two`)
-  __device__ __forceinline__ void literal(uint32_t bytes, uint32_t two) { push(0x80000000u | (two << 16) | bytes); }
-  __device__ __forceinline__ void match(uint32_t len, uint32_t dist) { push(len | (dist << 9)); }
-  // the last batch, with the decoder's status
-  __device__ __forceinline__ void finish(int st) {
-    __syncwarp();
-    if (lane == 0) {
-      sh->cnt[k] = n;
-      sh->status = st;
-      sh->done = 1;
+  };
+  // the expander's word, the same for every lane
+  const auto stopped = [&]() { return __shfl_sync(FULL, *static_cast<volatile uint32_t*>(&sm.stop), 0) != 0; };
+  for (;;) {
+    const bool drop = stopped();
+    if (lane == 0) sm.stopped[kb] = drop;  // both scan warps read the word of their batch's buffer
+    batch_barrier();
+    ScanBatch& b = sm.batch[kb];
+    kb ^= 1u;
+    const uint32_t kind = b.kind;
+    if (kind == kBatchDone) {
+      if (lane == 0) sm.status = b.status;
+      handoff(kLastTokens);
+      return;
     }
-    pair_barrier(bar);
-  }
-};
-
-// Output stand-in for the decoder warp of a pair, which writes no bytes itself.
-struct NullOut {
-  static constexpr uint32_t kBytes = 4096, kFlush = 1024;
-  uint32_t flushed = 0, store = 0;
-  uint8_t* gdst = nullptr;
-  __device__ __forceinline__ void put8(uint32_t, uint32_t) {}
-  __device__ __forceinline__ uint32_t get8(uint32_t) const { return 0; }
-  __device__ __forceinline__ void flush_to(uint32_t) {}
-  __device__ __forceinline__ void finish(uint32_t) {}
-};
-
-// GT: lit_lut / dist_lut are global memory (else shared memory, e.g. InflateScratch's).
-template <int NSLOT, int LB, class OUT, class TOK = NoTokens, bool GT = false>
-__device__ int decode_deflate_chunk(InRing<NSLOT>& in, OUT& out, InflateCodes& sc, uint32_t* lit_lut,
-                                    uint32_t* dist_lut, uint64_t chunk_bytes, uint32_t wrapper, TOK* tok = nullptr) {
-  // Before each symbol fewer than kFlush bytes of the window are unflushed; what is written
-  // until the next flush (a match of up to 258 bytes, a piece of a stored block) must not wrap
-  // onto them.
-  static_assert(OUT::kBytes - OUT::kFlush >= 258, "window too small for a match");
-  constexpr uint32_t kStoredPiece = OUT::kBytes - OUT::kFlush < 1024u ? OUT::kBytes - OUT::kFlush : 1024u;
-  const uint32_t lane = in.lane;
-  const uint32_t cap = static_cast<uint32_t>(chunk_bytes);
-  const HuffTable lit{lit_lut, sc.lit_sorted, sc.lit_cnt, sc.lit_first, sc.lit_index, LB};
-  const HuffTable dst{dist_lut, sc.dist_sorted, sc.dist_cnt, sc.dist_first, sc.dist_index, kDistLB};
-  const HuffTable cl{dist_lut, sc.dist_sorted, sc.dist_cnt, sc.dist_first, sc.dist_index, kCodeLenLB};
-  const uint32_t s_lit = GT ? 0u : smem_u32(lit_lut), s_dist = GT ? 0u : smem_u32(dist_lut);
-
-  uint32_t op = 0;  // bytes produced (chunks are < 2 GiB)
-  int st = CODAG_OK;
-  BitReader<NSLOT> br;
-  const uint32_t lit_sh = 16u + 8u * (lane & 1u);  // first literal in bits 16-23, second in 24-31
-  bool fixed_ready = false;
-
-  if (in.lo + wrapper > in.hi) st = CODAG_ECORRUPT;
-  if (!st && !in.release(in.lo)) st = CODAG_ETIMEOUT;
-  const uint32_t start = in.lo + wrapper;
-  br.start(in, start);
-  if (!st) st = br.refill(in);
-  if (!st) br.drop((start & 3u) * 8u);
-
-#define CODAG_REFILL()                   \
-  if (br.bc < 32) {                      \
-    st = br.refill(in);                  \
-    if (st) break;                       \
-  }
-  // one deferred far copy: pend_len bytes for [pend_op, pend_end), byte `lane` in pend_val
-  uint32_t pend_op = 0, pend_len = 0, pend_end = 0, pend_val = 0;
-#define CODAG_COMPLETE()                                              \
-  if (pend_len) {                                                     \
-    if (lane < pend_len) out.put8(pend_op + lane, pend_val);          \
-    pend_len = 0;                                                     \
-    pend_end = 0;                                                     \
-  }
-#define CODAG_FLUSH()   \
-  {                     \
-    CODAG_COMPLETE();   \
-    out.flush_to(op);   \
-  }
-
-  bool last = false;
-  while (!st && !last) {
-    if (br.bitpos() > static_cast<uint64_t>(in.hi) * 8u) { st = CODAG_ECORRUPT; break; }
-    CODAG_REFILL();
-    last = br.bb & 1u;
-    const uint32_t btype = static_cast<uint32_t>(br.bb >> 1) & 3u;
-    br.drop(3);
-    if (btype == 0) {  // stored block
-      br.drop(br.bc & 7u);
-      CODAG_REFILL();
-      const uint32_t len = static_cast<uint32_t>(br.bb) & 0xffffu;
-      const uint32_t nlen = static_cast<uint32_t>(br.bb >> 16) & 0xffffu;
-      br.drop(32);
-      if (len != (~nlen & 0xffffu)) { st = CODAG_ECORRUPT; break; }
-      uint32_t p = br.wpos - br.bc / 8u;
-      if (p + len > in.hi || op + len > cap) { st = CODAG_ECORRUPT; break; }
-      uint32_t left = len;
-      while (left) {
-        const uint32_t piece = left < kStoredPiece ? left : kStoredPiece;
-        if (!in.release(p)) { st = CODAG_ETIMEOUT; break; }
-        st = in.ensure(p + piece);
-        if (st) break;
-        if constexpr (TOK::kOn) {  // two bytes per literal token
-          for (uint32_t t = 0; t < piece; t += 2) {
-            const uint32_t two = t + 1 < piece ? 1u : 0u;
-            tok->literal(in.rd8(p + t) | (two ? in.rd8(p + t + 1) << 8 : 0u), two);
-          }
-        } else {
-          for (uint32_t t = lane; t < piece; t += 32) out.put8(op + t, in.rd8(p + t));
-        }
-        op += piece;
-        p += piece;
-        left -= piece;
-        __syncwarp();
-        CODAG_FLUSH();
+    if (drop) continue;
+    if (kind == kBatchStored) {
+      const uint32_t at = b.base, len = b.size;
+      for (uint32_t i = 0; i < len && !stopped(); i += kTokens) {
+        const uint32_t n = len - i < kTokens ? len - i : kTokens;
+        for (uint32_t q = lane; q < n; q += 32) sm.tok[k][q] = 0x80000000u | __ldg(gbase + at + i + q);
+        handoff(n);
       }
-      if (st) break;
-      br.start(in, p);
-      st = br.refill(in);
-      if (st) break;
-      br.drop((p & 3u) * 8u);
       continue;
     }
-    if (btype == 3) { st = CODAG_ECORRUPT; break; }
-    if (btype == 1) {  // fixed Huffman codes (RFC 1951 3.2.6)
-      if (!fixed_ready) {
-        for (uint32_t s = lane; s < 320; s += 32)
-          sc.lens[s] = s < 144 ? 8 : s < 256 ? 9 : s < 280 ? 7 : s < 288 ? 8 : 5;
-        __syncwarp();
-        build_table(sc.lens, 288, lit, kAlphaLitLen, sc.fill, lane);
-        build_table(sc.lens + 288, 30, dst, kAlphaDist, sc.fill, lane);
-        fixed_ready = true;
+    // cells of the pieces, as running totals
+    const uint32_t c0 = b.cnt[lane], c1 = b.cnt[32 + lane];
+    uint32_t e0 = (c0 + kCell - 1u) / kCell, e1 = (c1 + kCell - 1u) / kCell;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t o0 = __shfl_up_sync(FULL, e0, d), o1 = __shfl_up_sync(FULL, e1, d);
+      if (lane >= static_cast<uint32_t>(d)) {
+        e0 += o0;
+        e1 += o1;
       }
-    } else {  // dynamic Huffman codes (zlib.h:607-707)
-      fixed_ready = false;
-      CODAG_REFILL();
-      const uint32_t hlit = (static_cast<uint32_t>(br.bb) & 31u) + 257u;
-      const uint32_t hdist = (static_cast<uint32_t>(br.bb >> 5) & 31u) + 1u;
-      const uint32_t hclen = (static_cast<uint32_t>(br.bb >> 10) & 15u) + 4u;
-      br.drop(14);
-      if (hlit > 286 || hdist > 30) { st = CODAG_ECORRUPT; break; }
-      // code length code lengths, 3 bits each in kCodeLenOrder order
-      for (uint32_t i0 = 0; i0 < 19; i0 += 10) {
-        CODAG_REFILL();
-        const uint32_t i = i0 + lane;
-        if (lane < 10 && i < 19) {
-          const uint32_t v = i < hclen ? static_cast<uint32_t>(br.bb >> (3 * lane)) & 7u : 0u;
-          sc.lens[kCodeLenOrder[i]] = static_cast<uint8_t>(v);
-        }
-        const uint32_t took = hclen > i0 ? min(hclen - i0, 10u) : 0u;
-        br.drop(3 * took);
-      }
-      if (st) break;
-      __syncwarp();
-      if (!build_table(sc.lens, 19, cl, kAlphaCodeLen, sc.fill, lane)) { st = CODAG_ECORRUPT; break; }
-      // literal/length and distance code lengths, run-length coded with symbols 16..18
-      uint32_t idx = 0, prev = 0;
-      const uint32_t total = hlit + hdist;
-      while (idx < total) {
-        CODAG_REFILL();
-        const uint32_t e = lut_ld<GT>(dist_lut, s_dist, static_cast<uint32_t>(br.bb & ((1u << kCodeLenLB) - 1u)));
-        if (e & kSlowFlag) { st = CODAG_ECORRUPT; break; }  // code lengths are at most 7 bits
-        br.drop(e & 31u);
-        const uint32_t sym = e >> 16;
-        if (sym < 16) {
-          if (lane == 0) sc.lens[idx] = static_cast<uint8_t>(sym);
-          prev = sym;
-          idx++;
-          continue;
-        }
-        uint32_t rep, val = 0;
-        if (sym == 16) {
-          if (idx == 0) { st = CODAG_ECORRUPT; break; }
-          val = prev;
-          rep = 3u + (static_cast<uint32_t>(br.bb) & 3u);
-          br.drop(2);
-        } else if (sym == 17) {
-          rep = 3u + (static_cast<uint32_t>(br.bb) & 7u);
-          br.drop(3);
-        } else {
-          rep = 11u + (static_cast<uint32_t>(br.bb) & 127u);
-          br.drop(7);
-        }
-        if (idx + rep > total) { st = CODAG_ECORRUPT; break; }
-        for (uint32_t t = lane; t < rep; t += 32) sc.lens[idx + t] = static_cast<uint8_t>(val);
-        prev = val;
-        idx += rep;
-      }
-      if (st) break;
-      __syncwarp();
-      if (sc.lens[256] == 0) { st = CODAG_ECORRUPT; break; }
-      // the distance lengths follow the literal/length lengths; move them to their slot
-      uint8_t dl = 0;
-      if (lane < hdist) dl = sc.lens[hlit + lane];
-      __syncwarp();
-      for (uint32_t s = hlit + lane; s < 288; s += 32) sc.lens[s] = 0;
-      __syncwarp();
-      if (lane < 32) sc.lens[288 + lane] = lane < hdist ? dl : 0;
-      __syncwarp();
-      if (!build_table(sc.lens, hlit, lit, kAlphaLitLen, sc.fill, lane)) { st = CODAG_ECORRUPT; break; }
-      if (!build_table(sc.lens + 288, hdist, dst, kAlphaDist, sc.fill, lane)) { st = CODAG_ECORRUPT; break; }
     }
-
-    // symbol loop (zlib.h:712-805)
-    for (;;) {
-      CODAG_REFILL();
-      uint32_t e = lut_ld<GT>(lit_lut, s_lit, static_cast<uint32_t>(br.bb) & ((1u << LB) - 1u));
-      if ((e & kKindMask) == kKindLitBits) {  // one literal or a pair
-        const uint32_t pair = (e >> 11) & 1u;
-        br.drop(e & 31u);
-        if constexpr (TOK::kOn) {
-          tok->literal(((e >> 16) & 0xffu) | ((e >> 16) & 0xff00u), pair);
-          op += 1u + pair;
-          continue;
-        } else {
-          // lane 0 stores the literal, lane 1 the second of a pair: one predicated byte store
-          // of the entry shifted by lit_sh, with no branch on the lane
-          const uint32_t a = out.sbuf + ((op + lane) & OUT::kMask);
-          asm volatile("{ .reg .pred p; setp.le.u32 p, %0, %1; @p st.shared.u8 [%2], %3; }" ::"r"(lane), "r"(pair),
-                       "r"(a), "r"(e >> lit_sh)
-                       : "memory");
-          op += 1u + pair;
-          if (op - out.flushed >= OUT::kFlush) CODAG_FLUSH();
-          continue;
+    e1 += __shfl_sync(FULL, e0, 31);
+    const uint32_t cells = __shfl_sync(FULL, e1, 31);
+    sm.cell_end[lane] = static_cast<uint16_t>(e0);
+    sm.cell_end[32 + lane] = static_cast<uint16_t>(e1);
+    __syncwarp();
+    InflateTables& tab = sm.tab[b.table];
+    const uint32_t s_lit = smem_u32(tab.lit_lut), s_dist = smem_u32(tab.dist_lut), s_stage = smem_u32(sm.stage);
+    const uint32_t base = b.base, bits = b.size;
+    for (uint32_t c = 0; c < cells && !stopped(); c += 32) {
+      const uint32_t x = c + lane < cells ? c + lane : cells - 1u;  // lanes past the end repeat the last cell
+      uint32_t q = 0;  // its piece: as many as end at or before it
+#pragma unroll
+      for (uint32_t step = kPieces / 2; step; step >>= 1)
+        if (sm.cell_end[q + step - 1u] <= x) q += step;
+      const uint32_t first = q ? sm.cell_end[q - 1u] : 0u, j = x - first;
+      uint32_t p = base + q * bits + b.row[q * kRow + j];
+      const uint32_t left = b.cnt[q] - j * kCell;
+      const uint32_t n = c + lane < cells ? (left < kCell ? left : kCell) : 0u;
+      // the words of all cells: they follow one another
+      const uint32_t w_lo = __shfl_sync(FULL, p, 0) >> 5;
+      const uint32_t w_n = ((__shfl_sync(FULL, p, 31) + 48u * kCell) >> 5) + 3u - w_lo;
+      for (uint32_t i = lane; i < w_n && i < kStageWords; i += 32) sm.stage[i] = stream_word(gbase, w_lo + i, lo, hi);
+      uint32_t t = n;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t o = __shfl_up_sync(FULL, t, d);
+        if (lane >= static_cast<uint32_t>(d)) t += o;
+      }
+      const uint32_t total = __shfl_sync(FULL, t, 31);
+      uint32_t* dst = sm.tok[k] + (t - n);
+      __syncwarp();
+      p -= 32u * w_lo;
+      for (uint32_t i = 0; i < kCell; i++) {
+        if (i < n) {
+          const uint32_t a = s_stage + ((p >> 5) << 2);
+          uint32_t used, tok;
+          symbol(ld_s32(a), ld_s32(a + 4), ld_s32(a + 8), p & 31u, s_lit, s_dist, tab, used, tok);
+          dst[i] = tok;
+          p += used;
         }
-      }
-      if (e & kSlowFlag) {
-        e = slow_entry(br.bb, lit, kAlphaLitLen);
-        if (!e) { st = CODAG_ECORRUPT; break; }
-        if ((e & kKindMask) == kKindLitBits) {
-          br.drop(e & 31u);
-          if constexpr (TOK::kOn) {
-            tok->literal((e >> 16) & 0xffu, 0u);
-            op++;
-            continue;
-          }
-          if (lane == 0) out.put8(op, (e >> 16) & 0xffu);
-          op++;
-          if (op - out.flushed >= OUT::kFlush) CODAG_FLUSH();
-          continue;
-        }
-      }
-      if ((e & kKindMask) == kKindEndBits) {
-        br.drop(e & 31u);
-        break;
-      }
-      if ((e & kKindMask) != kKindLenBits) { st = CODAG_ECORRUPT; break; }
-      // length: code and extra bits in one step (at most 20 bits; 32 are buffered)
-      const uint32_t ln = (e >> 5) & 15u, lt = e & 31u;
-      const uint32_t len = (e >> 16) + bfe32(static_cast<uint32_t>(br.bb), ln, lt - ln);
-      br.drop(lt);
-      if (br.bc < 28) {  // distance code and extra bits take at most 28 bits
-        st = br.refill(in);
-        if (st) break;
-      }
-      uint32_t d = lut_ld<GT>(dist_lut, s_dist, static_cast<uint32_t>(br.bb) & ((1u << kDistLB) - 1u));
-      if (d & kSlowFlag) {
-        d = slow_entry(br.bb, dst, kAlphaDist);
-        if (!d) { st = CODAG_ECORRUPT; break; }
-      }
-      if (d & kKindMask) { st = CODAG_ECORRUPT; break; }
-      const uint32_t dn = (d >> 5) & 15u, dt = d & 31u;
-      const uint32_t dist = (d >> 16) + bfe32(static_cast<uint32_t>(br.bb), dn, dt - dn);
-      br.drop(dt);
-      if (dist > op || op + len > cap) { st = CODAG_ECORRUPT; break; }
-      if constexpr (TOK::kOn) {
-        tok->match(len, dist);
-        op += len;
-        continue;
-      }
-      const uint32_t src = op - dist;
-      if (dist + len <= OUT::kBytes) {  // source still in the shared-memory window
-        if (src < pend_end) CODAG_COMPLETE();
         __syncwarp();
-        if (dist >= len) {
-          for (uint32_t t = lane; t < len; t += 32) out.put8(op + t, out.get8(src + t));
-        } else {
-          uint32_t r = lane % dist;
-          const uint32_t step = 32u % dist;
-          for (uint32_t t = lane; t < len; t += 32) {
-            out.put8(op + t, out.get8(src + r));
-            r += step;
-            if (r >= dist) r -= dist;
-          }
-        }
-      } else if (len <= 32) {
-        // older than the window: the bytes were flushed to the chunk's output already.  The
-        // load is issued now and its bytes enter the window later (CODAG_COMPLETE), so the
-        // memory latency overlaps the next symbols.
-        CODAG_COMPLETE();
-        pend_val = (lane < len && src + lane < out.store) ? static_cast<uint32_t>(out.gdst[src + lane]) : 0u;
-        pend_op = op;
-        pend_len = len;
-        pend_end = op + len;
-      } else {
-        CODAG_COMPLETE();
-        const uint32_t r0 = dist >= len ? lane : lane % dist;
-        const uint32_t step = dist >= len ? 32u : 32u % dist;
-        uint32_t r = r0;
-        for (uint32_t t = lane; t < len; t += 32) {
-          const uint32_t sp = src + r;
-          out.put8(op + t, sp < out.store ? out.gdst[sp] : 0u);  // unstored bytes are never stored either
-          r += step;
-          if (dist < len && r >= dist) r -= dist;
-        }
       }
-      op += len;
-      if (op - out.flushed >= OUT::kFlush) CODAG_FLUSH();
+      handoff(total);
     }
   }
-  CODAG_COMPLETE();
-#undef CODAG_FLUSH
-#undef CODAG_COMPLETE
-#undef CODAG_REFILL
-  if (!in.drain() && st == CODAG_OK) st = CODAG_ETIMEOUT;
-  out.finish(op);
-  if (st == CODAG_OK && (op < out.store || op > cap || br.bitpos() > static_cast<uint64_t>(in.hi) * 8u))
-    st = CODAG_ECORRUPT;
-  return st;
 }
 
-// Expander warp of a pair: drains the decoder's token batches into `out` (the window and far
-// copies of decode_deflate_chunk).  Returns CODAG_OK or CODAG_ECORRUPT (fewer bytes than the
-// stored part); the decoder's status arrives in sh->status.
+// ---------------------------------------------------------------------------------------
+// expander warp
+// ---------------------------------------------------------------------------------------
+// Up to 32 output bytes at out position b0 + lane (lanes below n): w is the lane's token word
+// (literal with bit 31, else a distance).
 template <class OUT>
-__device__ int expand_tokens(TokenShared* sh, uint32_t bar, OUT& out, uint32_t lane) {
-  static_assert(OUT::kBytes - OUT::kFlush >= 258, "window too small for a match");
-  uint32_t op = 0, k = 0;
-  const uint32_t tok_sh = 8u * (lane & 1u);  // a literal token: first byte in bits 0-7, second in 8-15
-  uint32_t pend_op = 0, pend_len = 0, pend_end = 0, pend_val = 0;
-#define CODAG_COMPLETE()                                     \
-  if (pend_len) {                                            \
-    if (lane < pend_len) out.put8(pend_op + lane, pend_val); \
-    pend_len = 0;                                            \
-    pend_end = 0;                                            \
+__device__ __forceinline__ void expand_step(OUT& out, uint32_t b0, uint32_t n, uint32_t w, uint32_t lane) {
+  const bool copy = !(w >> 31), on = lane < n;
+  uint32_t v = w;
+  if (__any_sync(FULL, on && copy && w <= lane)) {
+    // some sources lie in these 32 bytes: follow each to a lane that starts outside or is a literal
+    uint32_t root = copy && w <= lane ? lane - w : lane;
+    for (;;) {
+      const uint32_t up = __shfl_sync(FULL, root, root);
+      if (!__any_sync(FULL, up != root)) break;
+      root = up;
+    }
+    if (on && copy && w > lane) v = out.get8(b0 + lane - w);
+    v = __shfl_sync(FULL, v, root);
+  } else if (on && copy) {
+    v = out.get8(b0 + lane - w);
   }
-  for (;;) {
-    pair_barrier(bar);
-    const uint32_t cnt = sh->cnt[k], done = sh->done;
-    const uint32_t s_tok = smem_u32(sh->tok[k]);
-    for (uint32_t i = 0; i < cnt; i++) {
-      const uint32_t t = ld_s32(s_tok + 4u * i);
-      if (t >> 31) {  // literals: lane 0 stores the first, lane 1 the second (predicated)
-        const uint32_t two = (t >> 16) & 1u;
-        const uint32_t a = out.sbuf + ((op + lane) & OUT::kMask);
-        asm volatile("{ .reg .pred p; setp.le.u32 p, %0, %1; @p st.shared.u8 [%2], %3; }" ::"r"(lane), "r"(two),
-                     "r"(a), "r"(t >> tok_sh)
-                     : "memory");
-        op += 1u + two;
-      } else {
-        const uint32_t len = t & 0x1ffu, dist = (t >> 9) & 0xffffu;
-        const uint32_t src = op - dist;
-        if (dist + len <= OUT::kBytes) {  // source still in the shared-memory window
-          if (src < pend_end) CODAG_COMPLETE();
-          __syncwarp();
-          if (dist >= len) {
-            for (uint32_t q = lane; q < len; q += 32) out.put8(op + q, out.get8(src + q));
-          } else {
-            uint32_t r = lane % dist;
-            const uint32_t step = 32u % dist;
-            for (uint32_t q = lane; q < len; q += 32) {
-              out.put8(op + q, out.get8(src + r));
-              r += step;
-              if (r >= dist) r -= dist;
-            }
-          }
-        } else if (len <= 32) {  // flushed already: load now, write into the window later
-          CODAG_COMPLETE();
-          pend_val = (lane < len && src + lane < out.store) ? static_cast<uint32_t>(out.gdst[src + lane]) : 0u;
-          pend_op = op;
-          pend_len = len;
-          pend_end = op + len;
-        } else {
-          CODAG_COMPLETE();
-          const uint32_t r0 = dist >= len ? lane : lane % dist;
-          const uint32_t step = dist >= len ? 32u : 32u % dist;
-          uint32_t r = r0;
-          for (uint32_t q = lane; q < len; q += 32) {
-            const uint32_t sp = src + r;
-            out.put8(op + q, sp < out.store ? out.gdst[sp] : 0u);
-            r += step;
-            if (dist < len && r >= dist) r -= dist;
-          }
-        }
-        op += len;
+  if (on) out.put8(b0 + lane, v);
+  __syncwarp();
+}
+
+// Tokens [0, total) at s_tok.  False when the output would pass `cap` or a distance reaches before
+// the chunk.
+template <class OUT>
+__device__ __forceinline__ bool expand_batch(uint32_t s_tok, uint32_t total, OUT& out, uint32_t& op, uint32_t cap,
+                                             uint32_t lane) {
+  constexpr uint32_t kSteps = 6;  // 32-byte steps whose tokens are found, and bytes moved, side by side
+  const uint32_t le = 0xffffffffu >> (31u - lane);
+  for (uint32_t g = 0; g < total; g += 32) {
+    const uint32_t tok = g + lane < total ? ld_s32(s_tok + 4u * (g + lane)) : 0u;
+    const bool lit = tok >> 31;
+    const uint32_t len = lit ? 1u : tok & 0x1ffu;  // 0 past the batch
+    const uint32_t word = lit ? tok : tok >> 9;
+    uint32_t s = len;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t o = __shfl_up_sync(FULL, s, d);
+      if (lane >= static_cast<uint32_t>(d)) s += o;
+    }
+    const uint32_t bytes = __shfl_sync(FULL, s, 31);
+    s -= len;
+    if (__any_sync(FULL, len && !lit && word > op + s) || bytes > cap - op) return false;
+    uint32_t before = 0;  // tokens that start below the step's bytes
+    for (uint32_t q = 0; q < bytes; q += 32 * kSteps) {
+      uint32_t w[kSteps];
+      bool near = false;
+#pragma unroll
+      for (uint32_t i = 0; i < kSteps; i++) {
+        const uint32_t r = s - q - 32u * i;
+        const uint32_t starts = __reduce_or_sync(FULL, (len && r < 32u) ? 1u << r : 0u);
+        w[i] = __shfl_sync(FULL, word, before + __popc(starts & le) - 1u);
+        before += __popc(starts);
+        near |= w[i] <= 32u * i + lane && q + 32u * i + lane < bytes;
       }
-      if (op - out.flushed >= OUT::kFlush) {
-        CODAG_COMPLETE();
-        out.flush_to(op);
+      if (!__any_sync(FULL, near)) {  // every source lies before these steps
+        uint32_t v[kSteps];
+#pragma unroll
+        for (uint32_t i = 0; i < kSteps; i++) {
+          const uint32_t at = q + 32u * i + lane;
+          v[i] = w[i];
+          if (at < bytes && !(w[i] >> 31)) v[i] = out.get8(op + at - w[i]);
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < kSteps; i++) {
+          const uint32_t at = q + 32u * i + lane;
+          if (at < bytes) out.put8(op + at, v[i]);
+        }
+        __syncwarp();
+      } else {
+#pragma unroll
+        for (uint32_t i = 0; i < kSteps; i++) {
+          if (q + 32u * i < bytes) expand_step(out, op + q + 32u * i, bytes - q - 32u * i, w[i], lane);
+        }
       }
     }
-    k ^= 1u;
-    if (done) break;
+    op += bytes;
+    out.flush_to(op);
   }
-  CODAG_COMPLETE();
-#undef CODAG_COMPLETE
+  return true;
+}
+
+// Drains the token buffers into `out` and returns the chunk's status.
+template <class OUT>
+__device__ __forceinline__ int inflate_expander(InflateTeam& sm, OUT& out, uint64_t chunk_bytes, uint32_t lane) {
+  const uint32_t cap = static_cast<uint32_t>(chunk_bytes);
+  uint32_t op = 0, k = 0;
+  bool ok = true;
+  for (;;) {
+    token_barrier();
+    const uint32_t cnt = sm.tok_cnt[k];
+    if (ok) {
+      ok = expand_batch(smem_u32(sm.tok[k]), cnt & ~kLastTokens, out, op, cap, lane);
+      if (!ok && lane == 0) sm.stop = 1;
+      __syncwarp();
+    }
+    k ^= 1u;
+    if (cnt & kLastTokens) break;
+  }
   out.finish(op);
-  return op < out.store ? CODAG_ECORRUPT : CODAG_OK;
+  const int st = sm.status;
+  if (st != CODAG_OK) return st;
+  return ok && op >= out.store ? CODAG_OK : CODAG_ECORRUPT;
 }
 
 }  // namespace codag_dev
