@@ -80,8 +80,9 @@ __device__ __forceinline__ void team_jobs(const BatchArgs& a, uint64_t n, uint32
                                           uint64_t wait_cycles, uint32_t warp, uint32_t lane, RleRing& rle) {
   InflateTeam& sm = sh.team;
   InflateRing in;
+  TokenRing tin;
   InflateWin o;
-  inflate_ring(in, sm, wait_cycles, lane, warp == 0);
+  inflate_rings(in, tin, sm, wait_cycles, warp, lane);
   inflate_window(o, sm, lane);
   for (;;) {
     if (warp == 0 && lane == 0) {
@@ -106,11 +107,12 @@ __device__ __forceinline__ void team_jobs(const BatchArgs& a, uint64_t n, uint32
     } else if (!job_in_bounds(a, d)) {
       if (a.status && warp == 0 && lane == 0) a.status[i] = CODAG_ECORRUPT;
     } else {
-      in.begin(a.comp + d.comp_off, d.comp_len);
       if (warp < 2) {
+        in.begin(a.comp + d.comp_off, d.comp_len);
         inflate_scan(in, sm, d.wrapper_bytes, warp, lane);
       } else if (warp == 2) {
-        inflate_tokens(sm, in.gbase, in.lo, in.hi, lane);
+        tin.begin(a.comp + d.comp_off, d.comp_len);
+        inflate_tokens(tin, sm, lane);
       } else {
         o.begin(a.out + d.out_off, d.out_len);
         const int st = inflate_expander(sm, o, d.out_len, lane);

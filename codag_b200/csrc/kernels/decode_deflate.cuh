@@ -15,11 +15,12 @@
 //   - Tokens (one warp).  Decodes the noted cells again, 32 at a time, this time from known starts,
 //     into a dense list of tokens.  Decoding twice is cheaper than keeping every lane's tokens:
 //     their number varies too much from piece to piece to give each lane room of its own.
-//   - Expand (one warp).  Places 32 tokens at a time by a prefix sum of their lengths and writes 32
-//     consecutive output bytes per step: each lane finds the token that covers its byte, then takes
-//     the literal or the byte `distance` before from a 32 KiB shared-memory window (the largest
-//     distance Deflate has, so no source is ever read back from global memory).  A source inside the
-//     same 32 bytes is followed lane to lane.
+//     The warp also marks the byte each token starts at in a bit map.
+//   - Expand (one warp).  Writes 32 consecutive output bytes per step, four steps side by side: each
+//     lane finds the token that covers its byte by counting the bits up to it, then takes the
+//     literal or the byte `distance` before from a 32 KiB shared-memory window (the largest distance
+//     Deflate has, so no source is ever read back from global memory).  A source inside the same 32
+//     bytes is followed lane to lane.
 //
 // The stages run as a pipeline, each handing over in two buffers with a named barrier, so no warp
 // spins.
@@ -40,7 +41,7 @@ __constant__ uint8_t kDistExtra[30] = {0, 0, 0, 0, 1, 1, 2, 2,  3,  3,  4,  4,  
 __constant__ uint8_t kCodeLenOrder[19] = {16, 17, 18, 0, 8, 7, 9, 6, 10, 5, 11, 4, 12, 3, 13, 2, 14, 1, 15};
 
 constexpr uint32_t kLitLB = 10;  // codes of 11 and more bits: 0.02-0.3% of the symbols measured
-constexpr uint32_t kDistLB = 9;
+constexpr uint32_t kDistLB = 8;   // of 9 and more bits: 0.2-0.8% of the distances
 constexpr uint32_t kCodeLenLB = 7;
 
 // Table entry (32 bits):
@@ -167,7 +168,7 @@ __device__ __noinline__ uint32_t slow_entry(uint32_t bits, HuffTable t, int alph
     const uint32_t k = (rev >> (32 - l)) - t.first[l];
     if (k < t.cnt[l]) return make_entry(t.sorted[t.index[l] + k], l, alpha);
   }
-  return 0;
+  return kKindBadBits;
 }
 
 // Tables of one block.
@@ -183,20 +184,19 @@ struct InflateTables {
 };
 
 constexpr uint32_t kPieces = 64;
-constexpr uint32_t kCell = 8;          // symbols from one noted start to the next
-constexpr uint32_t kCells = 28;        // noted starts of one piece
-constexpr uint32_t kRow = kCells + 1;  // an odd stride spreads the lanes' rows over the banks
-// A piece aims at kPieceTokens symbols (by the last stretch's bits per symbol), well below the
-// kCell * kCells it may hold, and is at most kMaxSpan words long, so that 64 pieces fit the 15 KiB of
+constexpr uint32_t kCell = 16;         // symbols from one noted start to the next
+constexpr uint32_t kCells = 13;        // noted starts of one piece: an odd row spreads over the banks
+// A piece aims at kPieceTokens symbols (by the last stretch's bits per symbol), so far below the
+// kCell * kCells it may hold that few stretches end early at a full row, and is at most kMaxSpan words long, so that 64 pieces fit the 15 KiB of
 // the input ring that are resident behind any read position.  Spans are odd numbers of words: the
 // lanes' first words lie in different banks.
-constexpr uint32_t kPieceTokens = 150;
+constexpr uint32_t kPieceTokens = 110;
 constexpr uint32_t kMinSpan = 13, kMaxSpan = 47;
 constexpr uint32_t kWarmBits = 640;
 
 enum : uint32_t { kBatchTokens = 0, kBatchStored = 1, kBatchDone = 2 };
 struct ScanBatch {
-  uint16_t row[kPieces * kRow];  // bit offset of each cell from its piece's first bit
+  uint16_t row[kPieces * kCells];  // bit offset of each cell from its piece's first bit
   uint16_t cnt[kPieces];         // symbols of each piece
   uint32_t kind;
   uint32_t base;   // first bit (kBatchTokens), first byte (kBatchStored), in ring coordinates
@@ -208,22 +208,29 @@ struct ScanBatch {
 // Token: bit 31 set = a literal in bits 0-7; clear = a match, length in bits 0-8 and distance in
 // bits 9-24.
 constexpr uint32_t kTokens = 32 * kCell;
-constexpr uint32_t kLastTokens = 0x80000000u;
-constexpr uint32_t kStageWords = 400;  // 32 cells of 8 symbols of 48 bits, and the words around them
+constexpr uint32_t kRange = 4096;  // output bytes of one token batch
+struct TokenBatch {
+  uint32_t starts[kRange / 32];  // bit b: a token starts at byte b of the range
+  uint32_t list;    // which token list
+  uint32_t before;  // its tokens that start before the range
+  uint32_t bytes;   // bytes of the range
+  uint32_t last;    // the chunk's last batch
+};
 
-using InflateRing = InRing<16>;
+using InflateRing = InRing<16, true>;  // the scan's input
+using TokenRing = InRing<4, true>;     // the token warp's, which lags by up to two stretches
 using InflateWin = OutRing<15, 11, true>;  // 32 KiB window, 2 KiB drains by TMA bulk stores
 constexpr uint32_t kTeamWarps = 4;
 
 // Shared memory of one team; three teams fit an SM.
 struct InflateTeam {
   alignas(128) uint8_t win[InflateWin::kBytes];
-  alignas(128) uint8_t ring[InflateRing::kBytes];
+  alignas(128) uint8_t ring[InflateRing::kAlloc];
+  alignas(128) uint8_t token_ring[TokenRing::kAlloc];
   InflateTables tab[2];  // the scan warps build the next block's while the token warp reads the last's
   ScanBatch batch[2];
   alignas(16) uint32_t tok[2][kTokens];
-  uint32_t tok_cnt[2];  // tokens in the buffer; kLastTokens with the chunk's last one
-  uint32_t stage[kStageWords];
+  TokenBatch out[2];
   uint16_t cell_end[kPieces];
   uint8_t lens[320];
   uint32_t fill[2][16];
@@ -231,11 +238,11 @@ struct InflateTeam {
   uint8_t how[kPieces];
   uint32_t redo[2], stop_at[2], sum[2], header_ok;
   int32_t scan_st;
-  int32_t status;      // the scan's, with the last token buffer
+  int32_t status;      // the scan's, with the last token batch
   uint32_t stop;       // set by the expander: the output is full or a distance is bad
   uint32_t stopped[2]; // `stop` as the token warp saw it, one word per batch buffer
   uint32_t job;     // batched kernel: the team's current job
-  uint64_t bar[16];
+  uint64_t bar[16], token_bar[4];
 };
 static_assert(sizeof(InflateTeam) <= 76458, "three teams per SM: 227 KiB / 3 less 1 KiB each");
 
@@ -248,28 +255,54 @@ __device__ __forceinline__ void batch_barrier() { team_barrier<2, 96>(); }     /
 __device__ __forceinline__ void token_barrier() { team_barrier<3, 64>(); }     // tokens -> expander
 __device__ __forceinline__ void job_barrier() { team_barrier<4, 32 * kTeamWarps>(); }
 
-// One symbol (with its distance) at bit offset `sh` of w0: returns its kind, the bits it takes in
-// `used` and its token.
-__device__ __forceinline__ uint32_t symbol(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t sh, uint32_t s_lit,
-                                           uint32_t s_dist, InflateTables& tab, uint32_t& used, uint32_t& tok) {
-  const uint32_t lo = __funnelshift_r(w0, w1, sh);
-  uint32_t e = ld_s32(s_lit + 4u * (lo & ((1u << kLitLB) - 1u)));
-  if (e & kSlowFlag) e = slow_entry<kLitLB>(lo, tab.lit(), kAlphaLitLen);
-  used = e & 31u;
-  tok = 0x80000000u | ((e >> 16) & 0xffu);
-  uint32_t kind = used ? e & kKindMask : static_cast<uint32_t>(kKindBadBits);
-  if (kind == kKindLenBits) {
+// One symbol, with its distance if it is a length.
+struct Symbol {
+  uint32_t e, d;   // table entries; d is 0 unless e is a length
+  uint32_t used;   // bits taken in all
+  uint32_t lo, x;  // stream bits of the literal/length and of the distance code
+  // end of block, or not a symbol: the table entry's kind has its upper bit set
+  __device__ __forceinline__ bool special() const { return ((e | d) & kKindEndBits) != 0; }
+  __device__ __forceinline__ bool end() const { return (e & kKindMask) == kKindEndBits; }
+  __device__ __forceinline__ bool literal() const { return (e & kKindMask) == kKindLitBits; }
+  __device__ __forceinline__ uint32_t length() const {
     const uint32_t ln = (e >> 5) & 15u;
-    const uint32_t len = (e >> 16) + bfe32(lo, ln, used - ln);
-    const uint32_t x = __funnelshift_r(lo, __funnelshift_r(w1, w2, sh), used);
-    uint32_t d = ld_s32(s_dist + 4u * (x & ((1u << kDistLB) - 1u)));
-    if (d & kSlowFlag) d = slow_entry<kDistLB>(x, tab.dist(), kAlphaDist);
-    const uint32_t dt = d & 31u, dn = (d >> 5) & 15u;
-    if (!dt || (d & kKindMask)) kind = kKindBadBits;
-    tok = len | (((d >> 16) + bfe32(x, dn, dt - dn)) << 9);
-    used += dt;
+    return (e >> 16) + bfe32(lo, ln, (e & 31u) - ln);
   }
-  return kind;
+  __device__ __forceinline__ uint32_t distance() const {
+    const uint32_t dn = (d >> 5) & 15u;
+    return (d >> 16) + bfe32(x, dn, (d & 31u) - dn);
+  }
+};
+
+// Table entries of a symbol with a code longer than its table (or no code: kKindBadBits).
+static __device__ __noinline__ uint2 slow_symbol(uint32_t lo, uint32_t hi, InflateTables* tab) {
+  uint32_t e = tab->lit_lut[lo & ((1u << kLitLB) - 1u)], d = 0;
+  if (e & kSlowFlag) e = slow_entry<kLitLB>(lo, tab->lit(), kAlphaLitLen);
+  if ((e & kKindMask) == kKindLenBits) {
+    const uint32_t x = __funnelshift_r(lo, hi, e & 31u);
+    d = tab->dist_lut[x & ((1u << kDistLB) - 1u)];
+    if (d & kSlowFlag) d = slow_entry<kDistLB>(x, tab->dist(), kAlphaDist);
+  }
+  return make_uint2(e, d);
+}
+
+// The symbol whose bits begin `lo`, `hi`.  The distance is looked up whether or not the symbol is a
+// length: nearly every time some lane has one, and without a branch several symbols overlap.
+__device__ __forceinline__ Symbol symbol(uint32_t lo, uint32_t hi, uint32_t s_lit, uint32_t s_dist, InflateTables& tab) {
+  Symbol y;
+  y.lo = lo;
+  y.e = ld_s32(s_lit + 4u * (lo & ((1u << kLitLB) - 1u)));
+  y.x = __funnelshift_r(lo, hi, y.e & 31u);
+  const uint32_t d = ld_s32(s_dist + 4u * (y.x & ((1u << kDistLB) - 1u)));
+  y.d = (y.e & kKindMask) == kKindLenBits ? d : 0u;
+  if ((y.e | y.d) & kSlowFlag) {
+    const uint2 z = slow_symbol(lo, hi, &tab);
+    y.e = z.x;
+    y.d = z.y;
+    y.x = __funnelshift_r(lo, hi, y.e & 31u);
+  }
+  y.used = (y.e & 31u) + (y.d & 31u);
+  return y;
 }
 
 // ---------------------------------------------------------------------------------------
@@ -324,18 +357,20 @@ struct InflateScan {
     return go;
   }
 
+  __device__ __forceinline__ Symbol at(uint32_t p, uint32_t s_lit, uint32_t s_dist) const {
+    const uint32_t a = in.sbuf + ((p >> 3) & (InflateRing::kMask & ~3u));
+    const uint32_t w0 = ld_s32(a), w1 = ld_s32(a + 4), w2 = ld_s32(a + 8), sh = p & 31u;
+    return symbol(__funnelshift_r(w0, w1, sh), __funnelshift_r(w1, w2, sh), s_lit, s_dist, sm.tab[tab]);
+  }
+
   // Where the first symbol that ends at or past `end` ends, decoding from bit p, a guess; what the
   // stream does not allow is stepped over.
   __device__ __forceinline__ uint32_t warm_up(uint32_t p, uint32_t end, bool go, uint32_t s_lit, uint32_t s_dist) {
-    uint32_t n = 0;
     while (__any_sync(FULL, go)) {
       if (go) {
-        const uint32_t a = (p >> 5) << 2;
-        uint32_t used, tok;
-        const uint32_t kind =
-            symbol(in.rd32(a), in.rd32(a + 4), in.rd32(a + 8), p & 31u, s_lit, s_dist, sm.tab[tab], used, tok);
-        p += kind == kKindBadBits ? 1u : used;
-        go = p < end && ++n < 2u * kWarmBits;
+        const Symbol y = at(p, s_lit, s_dist);
+        p += y.special() ? 1u : y.used;
+        go = p < end;
       }
     }
     return p;
@@ -350,24 +385,16 @@ struct InflateScan {
     bool go = on && p < end;
     while (__any_sync(FULL, go)) {
       if (go) {
-        const uint32_t a = (p >> 5) << 2;
-        uint32_t used, tok;
-        const uint32_t kind =
-            symbol(in.rd32(a), in.rd32(a + 4), in.rd32(a + 8), p & 31u, s_lit, s_dist, sm.tab[tab], used, tok);
-        const uint32_t at = p;
-        p += used;
-        if (kind == kKindBadBits || p > hi8) {
-          h = kBad;
-          go = false;
-        } else if (kind == kKindEndBits) {
-          h = kEob;
+        const Symbol y = at(p, s_lit, s_dist);
+        if ((n & (kCell - 1u)) == 0) row[n / kCell] = static_cast<uint16_t>(p - from);
+        p += y.used;
+        if (y.special() || p > hi8) {
+          h = y.end() && p <= hi8 ? kEob : kBad;
           go = false;
         } else {
-          if ((n & (kCell - 1u)) == 0) row[n / kCell] = static_cast<uint16_t>(at - from);
           n++;
-          go = p < end;
-          if (go && n == kCell * kCells) {
-            h = kFull;
+          if (p >= end || n == kCell * kCells) {
+            h = p >= end ? kRun : kFull;
             go = false;
           }
         }
@@ -389,7 +416,7 @@ struct InflateScan {
       int st = need(kPieces * bits + 64u);
       if (st) return st;
       const uint32_t from = pos + id * bits, end = from + bits;
-      uint16_t* row = sm.batch[k].row + id * kRow;
+      uint16_t* row = sm.batch[k].row + id * kCells;
       const bool inside = from < hi8;
       uint32_t start = warm_up(id * bits > kWarmBits ? from - kWarmBits : pos, from, inside && id, s_lit, s_dist);
       if (!inside) start = from;
@@ -578,16 +605,22 @@ struct InflateScan {
   }
 };
 
-// Binds a team's input ring (barriers initialised) and its window.
-__device__ __forceinline__ void inflate_ring(InflateRing& in, InflateTeam& sm, uint64_t wait_cycles, uint32_t lane,
-                                             bool init) {
-  in.buf = sm.ring;
-  in.sbuf = smem_u32(sm.ring);
-  in.bar = sm.bar;
+// Binds the rings (the warps that fill them initialise the barriers) and the window of a team.
+template <class RING>
+__device__ __forceinline__ void bind_ring(RING& in, uint8_t* buf, uint64_t* bar, uint64_t wait_cycles, uint32_t lane) {
+  in.buf = buf;
+  in.sbuf = smem_u32(buf);
+  in.bar = bar;
   in.phase = 0;
   in.wait_cycles = wait_cycles;
   in.lane = lane;
-  if (init) init_ring_barriers<16>(sm.bar, lane);
+}
+__device__ __forceinline__ void inflate_rings(InflateRing& in, TokenRing& tin, InflateTeam& sm, uint64_t wait_cycles,
+                                              uint32_t warp, uint32_t lane) {
+  bind_ring(in, sm.ring, sm.bar, wait_cycles, lane);
+  bind_ring(tin, sm.token_ring, sm.token_bar, wait_cycles, lane);
+  if (warp == 0) init_ring_barriers<16>(sm.bar, lane);
+  if (warp == 2) init_ring_barriers<4>(sm.token_bar, lane);
 }
 __device__ __forceinline__ void inflate_window(InflateWin& o, InflateTeam& sm, uint32_t lane) {
   o.buf = sm.win;
@@ -610,29 +643,44 @@ __device__ __forceinline__ void inflate_scan(InflateRing& in, InflateTeam& sm, u
 // ---------------------------------------------------------------------------------------
 // token warp
 // ---------------------------------------------------------------------------------------
-// Word w of the stream in ring coordinates, straight from global memory; bytes outside [lo, hi)
-// are not read.
-__device__ __forceinline__ uint32_t stream_word(const uint8_t* gbase, uint32_t w, uint32_t lo, uint32_t hi) {
-  const uint32_t a = 4u * w;
-  if (a >= lo && a + 4u <= hi) return __ldg(reinterpret_cast<const uint32_t*>(gbase + a));
-  uint32_t v = 0;
-  for (uint32_t i = 0; i < 4; i++)
-    if (a + i >= lo && a + i < hi) v |= static_cast<uint32_t>(__ldg(gbase + a + i)) << (8u * i);
+// inclusive prefix sum over the lanes
+__device__ __forceinline__ uint32_t warp_scan_add(uint32_t v, uint32_t lane) {
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t o = __shfl_up_sync(FULL, v, d);
+    if (lane >= static_cast<uint32_t>(d)) v += o;
+  }
   return v;
 }
 
-__device__ __forceinline__ void inflate_tokens(InflateTeam& sm, const uint8_t* gbase, uint32_t lo, uint32_t hi,
-                                               uint32_t lane) {
-  uint32_t kb = 0, k = 0;
-  // hands the token buffer with n tokens to the expander
-  const auto handoff = [&](uint32_t n) {
-    if (lane == 0) sm.tok_cnt[k] = n;
+__device__ __forceinline__ uint32_t token_len(uint32_t tok) { return tok >> 31 ? 1u : tok & 0x1ffu; }
+
+// Token warp (2 of the team); `in` is bound to the stream.
+__device__ __forceinline__ void inflate_tokens(TokenRing& in, InflateTeam& sm, uint32_t lane) {
+  uint32_t kb = 0, k = 0, list = 0;
+  bool dead = false;  // a wait for the input ran out
+  // hands token batch k to the expander
+  const auto handoff = [&](uint32_t before, uint32_t bytes, uint32_t last) {
+    if (lane == 0) {
+      TokenBatch& o = sm.out[k];
+      o.list = list;
+      o.before = before;
+      o.bytes = bytes;
+      o.last = last;
+    }
     __syncwarp();
     token_barrier();
     k ^= 1u;
   };
   // the expander's word, the same for every lane
-  const auto stopped = [&]() { return __shfl_sync(FULL, *static_cast<volatile uint32_t*>(&sm.stop), 0) != 0; };
+  const auto stopped = [&]() {
+    return dead || __shfl_sync(FULL, *static_cast<volatile uint32_t*>(&sm.stop), 0) != 0;
+  };
+  // bytes [at, end) resident
+  const auto need = [&](uint32_t at, uint32_t end) {
+    dead = dead || !in.release(at) || in.ensure(end < in.hi ? end : in.hi) != CODAG_OK;
+    return !dead;
+  };
   for (;;) {
     const bool drop = stopped();
     if (lane == 0) sm.stopped[kb] = drop;  // both scan warps read the word of their batch's buffer
@@ -641,8 +689,9 @@ __device__ __forceinline__ void inflate_tokens(InflateTeam& sm, const uint8_t* g
     kb ^= 1u;
     const uint32_t kind = b.kind;
     if (kind == kBatchDone) {
-      if (lane == 0) sm.status = b.status;
-      handoff(kLastTokens);
+      if (!in.drain()) dead = true;
+      if (lane == 0) sm.status = dead ? CODAG_ETIMEOUT : b.status;
+      handoff(0, 0, 1);
       return;
     }
     if (drop) continue;
@@ -650,65 +699,83 @@ __device__ __forceinline__ void inflate_tokens(InflateTeam& sm, const uint8_t* g
       const uint32_t at = b.base, len = b.size;
       for (uint32_t i = 0; i < len && !stopped(); i += kTokens) {
         const uint32_t n = len - i < kTokens ? len - i : kTokens;
-        for (uint32_t q = lane; q < n; q += 32) sm.tok[k][q] = 0x80000000u | __ldg(gbase + at + i + q);
-        handoff(n);
+        if (!need(at + i, at + i + n)) break;
+        for (uint32_t q = lane; q < n; q += 32) sm.tok[list][q] = 0x80000000u | in.rd8(at + i + q);
+        if (32u * lane < n) sm.out[k].starts[lane] = n - 32u * lane >= 32u ? FULL : (1u << (n - 32u * lane)) - 1u;
+        handoff(0, n, 0);
+        list ^= 1u;
       }
       continue;
     }
     // cells of the pieces, as running totals
-    const uint32_t c0 = b.cnt[lane], c1 = b.cnt[32 + lane];
-    uint32_t e0 = (c0 + kCell - 1u) / kCell, e1 = (c1 + kCell - 1u) / kCell;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const uint32_t o0 = __shfl_up_sync(FULL, e0, d), o1 = __shfl_up_sync(FULL, e1, d);
-      if (lane >= static_cast<uint32_t>(d)) {
-        e0 += o0;
-        e1 += o1;
-      }
-    }
-    e1 += __shfl_sync(FULL, e0, 31);
+    const uint32_t e0 = warp_scan_add((b.cnt[lane] + kCell - 1u) / kCell, lane);
+    const uint32_t e1 = warp_scan_add((b.cnt[32 + lane] + kCell - 1u) / kCell, lane) + __shfl_sync(FULL, e0, 31);
     const uint32_t cells = __shfl_sync(FULL, e1, 31);
     sm.cell_end[lane] = static_cast<uint16_t>(e0);
     sm.cell_end[32 + lane] = static_cast<uint16_t>(e1);
     __syncwarp();
     InflateTables& tab = sm.tab[b.table];
-    const uint32_t s_lit = smem_u32(tab.lit_lut), s_dist = smem_u32(tab.dist_lut), s_stage = smem_u32(sm.stage);
+    const uint32_t s_lit = smem_u32(tab.lit_lut), s_dist = smem_u32(tab.dist_lut);
     const uint32_t base = b.base, bits = b.size;
-    for (uint32_t c = 0; c < cells && !stopped(); c += 32) {
+    for (uint32_t c = 0, m; c < cells && !stopped(); c += m) {
       const uint32_t x = c + lane < cells ? c + lane : cells - 1u;  // lanes past the end repeat the last cell
       uint32_t q = 0;  // its piece: as many as end at or before it
 #pragma unroll
       for (uint32_t step = kPieces / 2; step; step >>= 1)
         if (sm.cell_end[q + step - 1u] <= x) q += step;
       const uint32_t first = q ? sm.cell_end[q - 1u] : 0u, j = x - first;
-      uint32_t p = base + q * bits + b.row[q * kRow + j];
+      uint32_t p = base + q * bits + b.row[q * kCells + j];
+      // as many of the cells, which follow one another, as the ring holds for certain
+      const uint32_t p0 = __shfl_sync(FULL, p, 0);
+      constexpr uint32_t kCellBits = 48u * kCell + 96u;
+      m = __popc(__ballot_sync(FULL, p - p0 + kCellBits <= 8u * 3u * kSlotBytes));
+      if (m > cells - c) m = cells - c;
       const uint32_t left = b.cnt[q] - j * kCell;
-      const uint32_t n = c + lane < cells ? (left < kCell ? left : kCell) : 0u;
-      // the words of all cells: they follow one another
-      const uint32_t w_lo = __shfl_sync(FULL, p, 0) >> 5;
-      const uint32_t w_n = ((__shfl_sync(FULL, p, 31) + 48u * kCell) >> 5) + 3u - w_lo;
-      for (uint32_t i = lane; i < w_n && i < kStageWords; i += 32) sm.stage[i] = stream_word(gbase, w_lo + i, lo, hi);
-      uint32_t t = n;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t o = __shfl_up_sync(FULL, t, d);
-        if (lane >= static_cast<uint32_t>(d)) t += o;
-      }
-      const uint32_t total = __shfl_sync(FULL, t, 31);
-      uint32_t* dst = sm.tok[k] + (t - n);
-      __syncwarp();
-      p -= 32u * w_lo;
+      const uint32_t n = lane < m ? (left < kCell ? left : kCell) : 0u;
+      if (!need(p0 >> 3, (__shfl_sync(FULL, p, static_cast<int>(m) - 1) + kCellBits) >> 3)) break;
+      uint32_t* dst = sm.tok[list] + (warp_scan_add(n, lane) - n);
+      uint32_t len = 0;  // bytes of this lane's tokens
       for (uint32_t i = 0; i < kCell; i++) {
         if (i < n) {
-          const uint32_t a = s_stage + ((p >> 5) << 2);
-          uint32_t used, tok;
-          symbol(ld_s32(a), ld_s32(a + 4), ld_s32(a + 8), p & 31u, s_lit, s_dist, tab, used, tok);
+          const uint32_t a = in.sbuf + ((p >> 3) & (TokenRing::kMask & ~3u));
+          const uint32_t w0 = ld_s32(a), w1 = ld_s32(a + 4), w2 = ld_s32(a + 8), sh = p & 31u;
+          const Symbol y =
+              symbol(__funnelshift_r(w0, w1, sh), __funnelshift_r(w1, w2, sh), s_lit, s_dist, tab);
+          const uint32_t tok = y.literal() ? 0x80000000u | (y.e >> 16) : y.length() | (y.distance() << 9);
           dst[i] = tok;
-          p += used;
+          len += token_len(tok);
+          p += y.used;
         }
         __syncwarp();
       }
-      handoff(total);
+      uint32_t s0 = warp_scan_add(len, lane);
+      const uint32_t total = __shfl_sync(FULL, s0, 31);
+      s0 -= len;
+      // the tokens' bytes in ranges the bit map covers: one, unless there are long matches
+      for (uint32_t r = 0; r < total; r += kRange) {
+        uint32_t* starts = sm.out[k].starts;
+        for (uint32_t i = lane; i < kRange / 32u; i += 32) starts[i] = 0;
+        __syncwarp();
+        uint32_t s = s0, before = 0;
+        if (total <= kRange) {
+#pragma unroll 4
+          for (uint32_t i = 0; i < n; i++) {
+            const uint32_t tok = dst[i];
+            atomicOr(&starts[s >> 5], 1u << (s & 31u));
+            s += token_len(tok);
+          }
+        } else {
+          for (uint32_t i = 0; i < n; i++) {
+            const uint32_t tok = dst[i];
+            if (s < r) before++;
+            else if (s - r < kRange) atomicOr(&starts[(s - r) >> 5], 1u << (s & 31u));
+            s += token_len(tok);
+          }
+          before = __reduce_add_sync(FULL, before);
+        }
+        handoff(before, total - r < kRange ? total - r : kRange, 0);
+      }
+      list ^= 1u;
     }
   }
 }
@@ -720,86 +787,103 @@ __device__ __forceinline__ void inflate_tokens(InflateTeam& sm, const uint8_t* g
 // (literal with bit 31, else a distance).
 template <class OUT>
 __device__ __forceinline__ void expand_step(OUT& out, uint32_t b0, uint32_t n, uint32_t w, uint32_t lane) {
-  const bool copy = !(w >> 31), on = lane < n;
+  const bool near = w <= lane;  // a copy whose source lies in these 32 bytes
   uint32_t v = w;
-  if (__any_sync(FULL, on && copy && w <= lane)) {
-    // some sources lie in these 32 bytes: follow each to a lane that starts outside or is a literal
-    uint32_t root = copy && w <= lane ? lane - w : lane;
-    for (;;) {
-      const uint32_t up = __shfl_sync(FULL, root, root);
-      if (!__any_sync(FULL, up != root)) break;
-      root = up;
-    }
-    if (on && copy && w > lane) v = out.get8(b0 + lane - w);
+  if (__any_sync(FULL, near)) {
+    // follow each to a lane that starts outside or is a literal: chains of up to 31 links, halved five times
+    uint32_t root = near ? lane - w : lane;
+#pragma unroll
+    for (int i = 0; i < 5; i++) root = __shfl_sync(FULL, root, root);
+    if (!near && !(w >> 31)) v = out.get8(b0 + lane - w);
     v = __shfl_sync(FULL, v, root);
-  } else if (on && copy) {
+  } else if (!(w >> 31)) {
     v = out.get8(b0 + lane - w);
   }
-  if (on) out.put8(b0 + lane, v);
+  if (lane < n) out.put8(b0 + lane, v);
   __syncwarp();
 }
 
-// Tokens [0, total) at s_tok.  False when the output would pass `cap` or a distance reaches before
-// the chunk.
+// 128 bytes at out position b0 (n of them wanted): lane l's byte of step i, at 32 i + l, is token word
+// w[i], of token t[i]; the first `before` tokens start before them.
 template <class OUT>
-__device__ __forceinline__ bool expand_batch(uint32_t s_tok, uint32_t total, OUT& out, uint32_t& op, uint32_t cap,
-                                             uint32_t lane) {
-  constexpr uint32_t kSteps = 6;  // 32-byte steps whose tokens are found, and bytes moved, side by side
-  const uint32_t le = 0xffffffffu >> (31u - lane);
-  for (uint32_t g = 0; g < total; g += 32) {
-    const uint32_t tok = g + lane < total ? ld_s32(s_tok + 4u * (g + lane)) : 0u;
-    const bool lit = tok >> 31;
-    const uint32_t len = lit ? 1u : tok & 0x1ffu;  // 0 past the batch
-    const uint32_t word = lit ? tok : tok >> 9;
-    uint32_t s = len;
+__device__ __forceinline__ void expand_steps(OUT& out, uint32_t b0, uint32_t n, uint32_t* w, const uint32_t* t,
+                                             uint32_t before, uint32_t lane) {
+  bool near = false;
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const uint32_t o = __shfl_up_sync(FULL, s, d);
-      if (lane >= static_cast<uint32_t>(d)) s += o;
+  for (uint32_t i = 0; i < 4; i++) near |= w[i] <= 32u * i + lane;
+  if (__any_sync(FULL, near)) {
+    // A match that goes on from before these bytes repeats itself with any multiple of its
+    // distance: one that reaches before them.
+    near = false;
+#pragma unroll
+    for (uint32_t i = 0; i < 4; i++) {
+      const uint32_t at = 32u * i + lane;
+      if (w[i] <= at && t[i] < before) w[i] *= at / w[i] + 1u;
+      near |= w[i] <= at;
     }
-    const uint32_t bytes = __shfl_sync(FULL, s, 31);
-    s -= len;
-    if (__any_sync(FULL, len && !lit && word > op + s) || bytes > cap - op) return false;
-    uint32_t before = 0;  // tokens that start below the step's bytes
-    for (uint32_t q = 0; q < bytes; q += 32 * kSteps) {
-      uint32_t w[kSteps];
-      bool near = false;
+    if (__any_sync(FULL, near)) {
+#pragma unroll
+      for (uint32_t i = 0; i < 4; i++)
+        if (32u * i < n) expand_step(out, b0 + 32u * i, n - 32u * i, w[i], lane);
+      return;
+    }
+  }
+  uint32_t v[4];
+#pragma unroll
+  for (uint32_t i = 0; i < 4; i++) {
+    v[i] = w[i];
+    if (!(w[i] >> 31)) v[i] = out.get8(b0 + 32u * i + lane - w[i]);
+  }
+#pragma unroll
+  for (uint32_t i = 0; i < 4; i++)
+    if (32u * i + lane < n) out.put8(b0 + 32u * i + lane, v[i]);
+  __syncwarp();
+}
+
+// The bytes of one token batch.  False when the output would pass `cap` or a distance reaches
+// before the chunk.
+template <class OUT>
+__device__ __forceinline__ bool expand_batch(InflateTeam& sm, const TokenBatch& b, OUT& out, uint32_t& op, uint32_t cap,
+                                             uint32_t lane) {
+  constexpr uint32_t kSteps = 8;  // 32-byte steps whose tokens are found side by side
+  const uint32_t le = 0xffffffffu >> (31u - lane);
+  const uint32_t bytes = b.bytes, s_tok = smem_u32(sm.tok[b.list]);
+  if (bytes > cap - op) return false;
+  uint32_t count = b.before;  // tokens that start before the 1 KiB at c
+  for (uint32_t c = 0; c < bytes; c += 1024) {
+    // lane l: the starts in the 32 bytes at c + 32 l, and how many tokens start before them
+    const uint32_t word = c + 32u * lane < bytes ? b.starts[c / 32u + lane] : 0u;
+    const uint32_t upto = warp_scan_add(__popc(word), lane) + count, pre = upto - __popc(word);
+    count = __shfl_sync(FULL, upto, 31);
+    const uint32_t end = bytes - c < 1024u ? bytes - c : 1024u;
+    for (uint32_t q = 0; q < end; q += 32 * kSteps) {
+      const uint32_t b0 = op + c + q, n = end - q;
+      uint32_t w[kSteps], t[kSteps];
 #pragma unroll
       for (uint32_t i = 0; i < kSteps; i++) {
-        const uint32_t r = s - q - 32u * i;
-        const uint32_t starts = __reduce_or_sync(FULL, (len && r < 32u) ? 1u << r : 0u);
-        w[i] = __shfl_sync(FULL, word, before + __popc(starts & le) - 1u);
-        before += __popc(starts);
-        near |= w[i] <= 32u * i + lane && q + 32u * i + lane < bytes;
+        const uint32_t starts = __shfl_sync(FULL, word, q / 32u + i);
+        t[i] = __shfl_sync(FULL, pre, q / 32u + i) + __popc(starts & le) - 1u;
+        const uint32_t tok = ld_s32(s_tok + 4u * t[i]);
+        // bytes past the end are taken for literals
+        w[i] = 32u * i + lane < n ? (tok >> 31 ? tok : tok >> 9) : 0x80000000u;
       }
-      if (!__any_sync(FULL, near)) {  // every source lies before these steps
-        uint32_t v[kSteps];
+      if (b0 < 32768u) {
+        bool bad = false;
 #pragma unroll
-        for (uint32_t i = 0; i < kSteps; i++) {
-          const uint32_t at = q + 32u * i + lane;
-          v[i] = w[i];
-          if (at < bytes && !(w[i] >> 31)) v[i] = out.get8(op + at - w[i]);
-        }
-#pragma unroll
-        for (uint32_t i = 0; i < kSteps; i++) {
-          const uint32_t at = q + 32u * i + lane;
-          if (at < bytes) out.put8(op + at, v[i]);
-        }
-        __syncwarp();
-      } else {
-#pragma unroll
-        for (uint32_t i = 0; i < kSteps; i++) {
-          if (q + 32u * i < bytes) expand_step(out, op + q + 32u * i, bytes - q - 32u * i, w[i], lane);
-        }
+        for (uint32_t i = 0; i < kSteps; i++) bad |= !(w[i] >> 31) && w[i] > b0 + 32u * i + lane;
+        if (__any_sync(FULL, bad)) return false;
       }
+      expand_steps(out, b0, n, w, t, __shfl_sync(FULL, pre, q / 32u), lane);
+      if (n > 128u)
+        expand_steps(out, b0 + 128u, n - 128u, w + 4, t + 4, __shfl_sync(FULL, pre, q / 32u + 4u), lane);
     }
-    op += bytes;
-    out.flush_to(op);
   }
+  op += bytes;
+  out.flush_to(op);
   return true;
 }
 
-// Drains the token buffers into `out` and returns the chunk's status.
+// Drains the token batches into `out` and returns the chunk's status.
 template <class OUT>
 __device__ __forceinline__ int inflate_expander(InflateTeam& sm, OUT& out, uint64_t chunk_bytes, uint32_t lane) {
   const uint32_t cap = static_cast<uint32_t>(chunk_bytes);
@@ -807,14 +891,15 @@ __device__ __forceinline__ int inflate_expander(InflateTeam& sm, OUT& out, uint6
   bool ok = true;
   for (;;) {
     token_barrier();
-    const uint32_t cnt = sm.tok_cnt[k];
+    const TokenBatch& b = sm.out[k];
+    const uint32_t last = b.last;
     if (ok) {
-      ok = expand_batch(smem_u32(sm.tok[k]), cnt & ~kLastTokens, out, op, cap, lane);
+      ok = expand_batch(sm, b, out, op, cap, lane);
       if (!ok && lane == 0) sm.stop = 1;
       __syncwarp();
     }
     k ^= 1u;
-    if (cnt & kLastTokens) break;
+    if (last) break;
   }
   out.finish(op);
   const int st = sm.status;

@@ -173,10 +173,14 @@ __device__ __forceinline__ uint32_t lanemask_lt(uint32_t lane) { return (1u << l
 constexpr uint32_t kSlotLog2 = 10;
 constexpr uint32_t kSlotBytes = 1u << kSlotLog2;
 
-template <int NSLOT>
+// MIRROR: the buffer is kMirror bytes longer and repeats its first bytes behind its end, so that a
+// few words that follow one another in the stream can be read from one masked address.
+template <int NSLOT, bool MIRROR = false>
 struct InRing {
   static constexpr uint32_t kBytes = NSLOT * kSlotBytes;
   static constexpr uint32_t kMask = kBytes - 1;
+  static constexpr uint32_t kMirror = 16;
+  static constexpr uint32_t kAlloc = kBytes + (MIRROR ? kMirror : 0u);
   static_assert((NSLOT & (NSLOT - 1)) == 0, "ring depth must be a power of two");
 
   uint8_t* buf;            // kBytes of shared memory, 16-byte aligned
@@ -228,12 +232,18 @@ struct InRing {
     const uint32_t tail_lo = body_hi > body_lo ? body_hi : body_lo;
     if (tail_lo < hi && s == ((hi - 1) >> kSlotLog2) && lane < 16) {
       const uint32_t p = tail_lo + lane;
-      if (p < hi) st_s8(sbuf + (p & kMask), gbase[p]);
+      if (p < hi) {
+        st_s8(sbuf + (p & kMask), gbase[p]);
+        if (MIRROR && (p & kMask) < kMirror) st_s8(sbuf + kBytes + (p & kMask), gbase[p]);
+      }
     }
     if (lane == 0) {
       fence_proxy_async_smem();
-      mbar_arrive_expect_tx(&bar[r], bytes);
+      // a slot that wraps to the buffer's start (never the stream's first, so its body starts with it)
+      const bool again = MIRROR && r == 0 && s != 0 && bytes >= kMirror;
+      mbar_arrive_expect_tx(&bar[r], again ? bytes + kMirror : bytes);
       if (bytes) bulk_g2s(buf + (a & kMask), gbase + a, bytes, &bar[r]);
+      if (again) bulk_g2s(buf + kBytes, gbase + a, kMirror, &bar[r]);
     }
   }
 

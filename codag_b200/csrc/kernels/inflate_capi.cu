@@ -24,12 +24,14 @@ __global__ void __launch_bounds__(32 * kTeamWarps, 3)
   if (threadIdx.x == 0) sm.stop = 0;
   __syncthreads();
   InflateRing in;
-  inflate_ring(in, sm, wait_cycles, lane, warp == 0);
-  in.begin(comp + off, static_cast<uint32_t>(next - off));
+  TokenRing tin;
+  inflate_rings(in, tin, sm, wait_cycles, warp, lane);
   if (warp < 2) {
+    in.begin(comp + off, static_cast<uint32_t>(next - off));
     inflate_scan(in, sm, wrapper, warp, lane);
   } else if (warp == 2) {
-    inflate_tokens(sm, in.gbase, in.lo, in.hi, lane);
+    tin.begin(comp + off, static_cast<uint32_t>(next - off));
+    inflate_tokens(tin, sm, lane);
   } else {
     const uint64_t base = chunk * chunk_bytes;
     InflateWin o;
