@@ -16,7 +16,7 @@ using namespace codag_capi;
 
 namespace {
 
-constexpr uint32_t kWarps = 8;       // warps per CTA: a Deflate team uses four, the RLE files all
+constexpr uint32_t kWarps = 8;       // warps per CTA: a Deflate team uses six, the RLE files all
 constexpr uint32_t kRleFirst = 3;    // with both kinds of work, every 3rd CTA takes RLE files first
 using RleRing = InRing<4>;
 struct BatchShared {
@@ -27,7 +27,7 @@ struct BatchShared {
   uint64_t bar[kWarps][4];  // the RLE rings' barriers (the team has its own)
 };
 static_assert(kWarps * RleRing::kBytes <= sizeof(InflateTeam::win), "the team's barriers keep their place");
-static_assert(sizeof(BatchShared) <= 76458, "three CTAs per SM");
+static_assert(sizeof(BatchShared) <= 76800, "three CTAs per SM");
 
 struct BatchArgs {
   const codag_chunk_desc* descs;
@@ -74,7 +74,7 @@ __device__ __forceinline__ void rle_ring(RleRing& in, BatchShared& sh, uint64_t 
   init_ring_barriers<4>(in.bar, lane);
 }
 
-// Entries [0, n) of the order, taken by the CTA's first four warps together: a Deflate stream by the
+// Entries [0, n) of the order, taken by the CTA's first six warps together: a Deflate stream by the
 // team, anything else by its first warp alone (in the window's memory, which is idle then).
 __device__ __forceinline__ void team_jobs(const BatchArgs& a, uint64_t n, uint32_t* queue, BatchShared& sh,
                                           uint64_t wait_cycles, uint32_t warp, uint32_t lane, RleRing& rle) {
@@ -87,7 +87,7 @@ __device__ __forceinline__ void team_jobs(const BatchArgs& a, uint64_t n, uint32
   for (;;) {
     if (warp == 0 && lane == 0) {
       sm.job = atomicAdd(queue, 1u);
-      sm.stop = 0;
+      sm.stop = sm.dead = 0;
       sm.status = CODAG_OK;
     }
     job_barrier();
@@ -110,17 +110,19 @@ __device__ __forceinline__ void team_jobs(const BatchArgs& a, uint64_t n, uint32
       if (warp < 2) {
         in.begin(a.comp + d.comp_off, d.comp_len);
         inflate_scan(in, sm, d.wrapper_bytes, warp, lane);
-      } else if (warp == 2) {
+      } else if (warp < 4) {
         tin.begin(a.comp + d.comp_off, d.comp_len);
-        inflate_tokens(tin, sm, lane);
+        inflate_tokens(tin, sm, warp - 2u, lane);
+      } else if (warp == 4) {
+        inflate_place(sm, d.out_len, lane);
       } else {
         o.begin(a.out + d.out_off, d.out_len);
-        const int st = inflate_expander(sm, o, d.out_len, lane);
+        const int st = inflate_copy(sm, o, lane);
         if (a.status && lane == 0) a.status[i] = st;
       }
     }
     job_barrier();
-    const bool timed_out = sm.status == CODAG_ETIMEOUT;
+    const bool timed_out = sm.status == CODAG_ETIMEOUT || sm.dead;
     job_barrier();  // every warp has looked before the next job resets it
     if (timed_out) break;  // ring state unknown: the team stops
   }

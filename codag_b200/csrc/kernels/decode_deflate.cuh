@@ -1,8 +1,8 @@
-// Team decoder for one Deflate (RFC 1951) chunk: two scan warps, a token warp, an expander warp.
+// Team decoder for one Deflate (RFC 1951) chunk: six warps in four stages.
 //
 // CODAG's decoder (include/zlib/zlib.h:807-902) runs one symbol at a time on all 32 lanes
 // of a warp.  So did the first kernels here, and they spent about 140 warp instructions on every
-// symbol.  This decoder puts the lanes to work on different symbols, in three stages:
+// symbol.  This decoder puts the lanes to work on different symbols:
 //
 //   - Scan (two warps, 64 lanes).  A Huffman bit stream read from a wrong bit falls into step with
 //     the right symbol boundaries after a while (text compressed by zlib at level 6: after 106 bits
@@ -12,18 +12,19 @@
 //     whose start turns out not to be the end of the lane below decodes once more, until the chain
 //     from lane 0, whose start is known, holds.  So the result is the serial decoder's, whatever
 //     the guesses were.
-//   - Tokens (one warp).  Decodes the noted cells again, 32 at a time, this time from known starts,
-//     into a dense list of tokens.  Decoding twice is cheaper than keeping every lane's tokens:
-//     their number varies too much from piece to piece to give each lane room of its own.
-//     The warp also marks the byte each token starts at in a bit map.
-//   - Expand (one warp).  Writes 32 consecutive output bytes per step, four steps side by side: each
-//     lane finds the token that covers its byte by counting the bits up to it, then takes the
-//     literal or the byte `distance` before from a 32 KiB shared-memory window (the largest distance
-//     Deflate has, so no source is ever read back from global memory).  A source inside the same 32
-//     bytes is followed lane to lane.
+//   - Tokens (two warps, taking turns).  Decodes the noted cells again, 32 at a time, this time from
+//     known starts, into a dense list of tokens, and marks the byte each token starts at in a bit
+//     map.  Decoding twice is cheaper than keeping every lane's tokens: their number varies too much
+//     from piece to piece to give each lane room of its own.
+//   - Place (one warp).  Finds the token that covers each output byte by counting the marks up to it,
+//     32 bytes per step and eight steps side by side.
+//   - Copy (one warp).  Takes each byte's literal, or the byte `distance` before it from a 32 KiB
+//     shared-memory window (the largest distance Deflate has, so no source is ever read back from
+//     global memory).  A source inside the same 32 bytes is followed lane to lane.
 //
-// The stages run as a pipeline, each handing over in two buffers with a named barrier, so no warp
-// spins.
+// The stages run as a pipeline, handing over in buffers guarded by named barriers, so no warp spins.
+// Each stage is one or two warps' chain of dependent instructions, about six cycles each, which is
+// why the work is spread over as many warps as it is.
 #pragma once
 #include "device_common.cuh"
 
@@ -45,11 +46,12 @@ constexpr uint32_t kDistLB = 8;   // of 9 and more bits: 0.2-0.8% of the distanc
 constexpr uint32_t kCodeLenLB = 7;
 
 // Table entry (32 bits):
-//   [0,5)   bits consumed in all: code length + extra bits
-//   [5,9)   code length of the symbol
+//   [0,5)   bits consumed in all: code length + extra bits, or both codes of a literal pair
+//   [5,9)   code length of the (first) symbol
 //   [9,11)  kind: literal, length, end of block, other (invalid, or not in the table)
+//   [11]    a second literal follows in [24,32) (literal/length tables only)
 //   [12]    the code is longer than the table: decode it with slow_entry
-//   [16,32) literal byte / length or distance base / code-length symbol
+//   [16,32) literal byte in [16,24) / length base / distance base less one / code-length symbol
 enum : uint32_t {
   kKindShift = 9,
   kKindMask = 3u << kKindShift,
@@ -57,6 +59,7 @@ enum : uint32_t {
   kKindLenBits = 1u << kKindShift,
   kKindEndBits = 2u << kKindShift,
   kKindBadBits = 3u << kKindShift,
+  kPairFlag = 1u << 11,
   kSlowFlag = 1u << 12,
   kSlowEntry = kKindBadBits | kSlowFlag,
 };
@@ -75,7 +78,7 @@ __device__ __forceinline__ uint32_t make_entry(uint32_t sym, uint32_t len, int a
     return entry_bits(len, len) | kKindBadBits;
   }
   if (alpha == kAlphaDist) {
-    if (sym < 30) return entry_bits(len + kDistExtra[sym], len) | (static_cast<uint32_t>(kDistBase[sym]) << 16);
+    if (sym < 30) return entry_bits(len + kDistExtra[sym], len) | (static_cast<uint32_t>(kDistBase[sym] - 1u) << 16);
     return entry_bits(len, len) | kKindBadBits;
   }
   return entry_bits(len, len) | (sym << 16);
@@ -157,6 +160,20 @@ __device__ __noinline__ bool build_table(const uint8_t* lens, uint32_t nsym, Huf
     t.lut[x] = len ? make_entry(t.sorted[t.index[len] + k], len, ALPHA) : static_cast<uint32_t>(kSlowEntry);
   }
   __syncwarp();
+  if (ALPHA == kAlphaLitLen) {
+    // literal pairs: when the bits of slot x after its literal code hold a whole literal
+    // code too, the entry carries both.  Only the first-literal fields of the other slot
+    // are read, and a pair rewrite leaves those fields unchanged, so lanes need no order.
+    for (uint32_t x = lane; x < (1u << LB); x += 32) {
+      const uint32_t e1 = t.lut[x];
+      const uint32_t l1 = (e1 >> 5) & 15u;
+      const uint32_t e2 = t.lut[x >> l1];
+      const uint32_t l2 = (e2 >> 5) & 15u;
+      if (((e1 | e2) & (kKindMask | kSlowFlag)) == kKindLitBits && l1 + l2 <= LB)
+        t.lut[x] = (e1 & ~31u & 0x00ffffffu) | (l1 + l2) | kPairFlag | ((e2 & 0x00ff0000u) << 8);
+    }
+    __syncwarp();
+  }
   return true;
 }
 
@@ -184,7 +201,8 @@ struct InflateTables {
 };
 
 constexpr uint32_t kPieces = 64;
-constexpr uint32_t kCell = 16;         // symbols from one noted start to the next
+constexpr uint32_t kCell = 15;         // symbols from one noted start to the next, or one more or less
+constexpr uint32_t kCellMax = 16;      // where two literals were read at once
 constexpr uint32_t kCells = 13;        // noted starts of one piece: an odd row spreads over the banks
 // A piece aims at kPieceTokens symbols (by the last stretch's bits per symbol), so far below the
 // kCell * kCells it may hold that few stretches end early at a full row, and is at most kMaxSpan words long, so that 64 pieces fit the 15 KiB of
@@ -196,8 +214,10 @@ constexpr uint32_t kWarmBits = 640;
 
 enum : uint32_t { kBatchTokens = 0, kBatchStored = 1, kBatchDone = 2 };
 struct ScanBatch {
-  uint16_t row[kPieces * kCells];  // bit offset of each cell from its piece's first bit
-  uint16_t cnt[kPieces];         // symbols of each piece
+  // bit offset of each cell from its piece's first bit; cell j starts with symbol kCell * j, or the
+  // next where bit 15 is set
+  uint16_t row[kPieces * kCells];
+  uint16_t cnt[kPieces];  // of each piece: symbols in bits 0-7, noted starts above
   uint32_t kind;
   uint32_t base;   // first bit (kBatchTokens), first byte (kBatchStored), in ring coordinates
   uint32_t size;   // bits per piece, or bytes
@@ -205,33 +225,47 @@ struct ScanBatch {
   int32_t status;  // with kBatchDone
 };
 
-// Token: bit 31 set = a literal in bits 0-7; clear = a match, length in bits 0-8 and distance in
-// bits 9-24.
-constexpr uint32_t kTokens = 32 * kCell;
-constexpr uint32_t kRange = 4096;  // output bytes of one token batch
+// Token: where its bytes come from in the low half (bit 15 set: the literal in bits 0-7; clear: the
+// distance less one), how many they are in the high half.
+constexpr uint32_t kLiteral = 0x8000u, kLiteralToken = 0x18000u;
+constexpr uint32_t kTokens = 32 * kCellMax;
+constexpr uint32_t kRange = 3072;  // output bytes of one token batch
 struct TokenBatch {
   uint32_t starts[kRange / 32];  // bit b: a token starts at byte b of the range
-  uint32_t list;    // which token list
-  uint32_t before;  // its tokens that start before the range
+  uint32_t before;  // tokens of the list that start before the range
   uint32_t bytes;   // bytes of the range
-  uint32_t last;    // the chunk's last batch
+  uint32_t what;    // kMore: another range of the same list follows; kLast: the chunk's last batch
 };
+enum : uint32_t { kMore = 1, kLast = 2 };
+
+// 256 output bytes: word 32 i + l is the low half of byte 32 i + l's token.
+constexpr uint32_t kSteps = 8;
+struct ByteBatch {
+  uint16_t word[32 * kSteps];
+  uint32_t bytes;
+  uint32_t near;  // 0: every source lies before the batch; else one more than the bytes before the
+                  // first token that starts in the batch
+  uint32_t last;  // the chunk's last batch; kBadChunk with it if the tokens were not sound
+};
+constexpr uint32_t kBadChunk = 2;
 
 using InflateRing = InRing<16, true>;  // the scan's input
-using TokenRing = InRing<4, true>;     // the token warp's, which lags by up to two stretches
+using TokenRing = InRing<2, true>;     // a token warp's, which lags by up to two stretches
+constexpr uint32_t align16(uint32_t v) { return (v + 15u) & ~15u; }
 using InflateWin = OutRing<15, 11, true>;  // 32 KiB window, 2 KiB drains by TMA bulk stores
-constexpr uint32_t kTeamWarps = 4;
+constexpr uint32_t kTeamWarps = 6;
 
 // Shared memory of one team; three teams fit an SM.
 struct InflateTeam {
   alignas(128) uint8_t win[InflateWin::kBytes];
-  alignas(128) uint8_t ring[InflateRing::kAlloc];
-  alignas(128) uint8_t token_ring[TokenRing::kAlloc];
-  InflateTables tab[2];  // the scan warps build the next block's while the token warp reads the last's
+  alignas(16) uint8_t ring[align16(InflateRing::kAlloc)];
+  alignas(16) uint8_t token_ring[2][align16(TokenRing::kAlloc)];
+  InflateTables tab[2];  // the scan warps build the next block's while the token warps read the last's
   ScanBatch batch[2];
-  alignas(16) uint32_t tok[2][kTokens];
+  alignas(16) uint32_t tok[2][kTokens];  // one list and one batch per token warp
   TokenBatch out[2];
-  uint16_t cell_end[kPieces];
+  ByteBatch place[2];
+  uint16_t cell_end[2][kPieces];
   uint8_t lens[320];
   uint32_t fill[2][16];
   uint32_t last[kPieces];  // scan warps: where each piece ended, and how
@@ -239,23 +273,34 @@ struct InflateTeam {
   uint32_t redo[2], stop_at[2], sum[2], header_ok;
   int32_t scan_st;
   int32_t status;      // the scan's, with the last token batch
-  uint32_t stop;       // set by the expander: the output is full or a distance is bad
-  uint32_t stopped[2]; // `stop` as the token warp saw it, one word per batch buffer
+  uint32_t stop;       // set by the place warp: the output is full or a distance is bad
+  uint32_t dead;       // a token warp's wait for its input ran out
+  uint32_t stopped[2]; // `stop` as the first token warp saw it, one word per batch buffer
   uint32_t job;     // batched kernel: the team's current job
-  uint64_t bar[16], token_bar[4];
+  uint64_t bar[16], token_bar[2][2];
 };
-static_assert(sizeof(InflateTeam) <= 76458, "three teams per SM: 227 KiB / 3 less 1 KiB each");
+static_assert(sizeof(InflateTeam) <= 76800, "three teams per SM: 228 KiB / 3 less 1 KiB each");
 
 template <uint32_t ID, uint32_t THREADS>
 __device__ __forceinline__ void team_barrier() {
   asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(THREADS) : "memory");
 }
-__device__ __forceinline__ void scan_barrier() { team_barrier<1, 64>(); }      // the scan warps
-__device__ __forceinline__ void batch_barrier() { team_barrier<2, 96>(); }     // scan -> tokens
-__device__ __forceinline__ void token_barrier() { team_barrier<3, 64>(); }     // tokens -> expander
-__device__ __forceinline__ void job_barrier() { team_barrier<4, 32 * kTeamWarps>(); }
+template <uint32_t THREADS>
+__device__ __forceinline__ void team_wait(uint32_t id) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(THREADS) : "memory");
+}
+template <uint32_t THREADS>
+__device__ __forceinline__ void team_signal(uint32_t id) {  // arrives without waiting
+  __threadfence_block();
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(THREADS) : "memory");
+}
+__device__ __forceinline__ void scan_barrier() { team_barrier<1, 64>(); }                    // the scan warps
+__device__ __forceinline__ void batch_barrier() { team_barrier<2, 128>(); }                  // scan -> tokens
+__device__ __forceinline__ void job_barrier() { team_barrier<3, 32 * kTeamWarps>(); }
+// buffer k of a producer and a consumer warp is full (the producer signals) or free (the consumer does)
+enum : uint32_t { kTokensFull = 4, kTokensFree = 6, kBytesFull = 8, kBytesFree = 10 };
 
-// One symbol, with its distance if it is a length.
+// One symbol, with its distance if it is a length, or two literals.
 struct Symbol {
   uint32_t e, d;   // table entries; d is 0 unless e is a length
   uint32_t used;   // bits taken in all
@@ -264,13 +309,11 @@ struct Symbol {
   __device__ __forceinline__ bool special() const { return ((e | d) & kKindEndBits) != 0; }
   __device__ __forceinline__ bool end() const { return (e & kKindMask) == kKindEndBits; }
   __device__ __forceinline__ bool literal() const { return (e & kKindMask) == kKindLitBits; }
-  __device__ __forceinline__ uint32_t length() const {
-    const uint32_t ln = (e >> 5) & 15u;
-    return (e >> 16) + bfe32(lo, ln, (e & 31u) - ln);
-  }
-  __device__ __forceinline__ uint32_t distance() const {
-    const uint32_t dn = (d >> 5) & 15u;
-    return (d >> 16) + bfe32(x, dn, (d & 31u) - dn);
+  __device__ __forceinline__ uint32_t count() const { return (e & kPairFlag) ? 2u : 1u; }
+  // token of a length and its distance
+  __device__ __forceinline__ uint32_t match() const {
+    const uint32_t ln = (e >> 5) & 15u, dn = (d >> 5) & 15u;
+    return (e & 0xffff0000u) + (bfe32(lo, ln, (e & 31u) - ln) << 16) + (d >> 16) + bfe32(x, dn, (d & 31u) - dn);
   }
 };
 
@@ -340,7 +383,7 @@ struct InflateScan {
     return sm.scan_st;
   }
 
-  // hands batch buffer k to the token warp; false when the expander wants no more
+  // hands batch buffer k to the token warps; false when the place warp wants no more
   __device__ __forceinline__ bool handoff(uint32_t kind, uint32_t base, uint32_t size, int status) {
     if (id == 0) {
       ScanBatch& b = sm.batch[k];
@@ -381,26 +424,35 @@ struct InflateScan {
   // the lanes back together.
   __device__ __forceinline__ uint32_t piece(uint32_t p, uint32_t end, uint32_t from, bool on, uint16_t* row,
                                             uint32_t s_lit, uint32_t s_dist, uint32_t& cnt, uint32_t& how) {
-    uint32_t n = 0, h = kRun;
+    uint32_t noted = 0, h = kRun;
+    int32_t due = 0;  // symbols before the next start to note
     bool go = on && p < end;
     while (__any_sync(FULL, go)) {
       if (go) {
         const Symbol y = at(p, s_lit, s_dist);
-        if ((n & (kCell - 1u)) == 0) row[n / kCell] = static_cast<uint16_t>(p - from);
+        if (due <= 0) {
+          row[noted++] = static_cast<uint16_t>((p - from) | (due < 0 ? 0x8000u : 0u));
+          due += kCell;
+        }
         p += y.used;
-        if (y.special() || p > hi8) {
-          h = y.end() && p <= hi8 ? kEob : kBad;
+        if (y.special()) {
+          h = y.end() ? kEob : kBad;
           go = false;
         } else {
-          n++;
-          if (p >= end || n == kCell * kCells) {
-            h = p >= end ? kRun : kFull;
+          due -= y.count();
+          go = p < end;
+          if (go && due <= 0 && noted == kCells) {
+            h = kFull;
             go = false;
           }
         }
       }
     }
-    cnt = n;
+    cnt = (noted * kCell - due) | (noted << 8);
+    if (p > hi8) {  // ran past the end of the stream: no symbol of this piece is taken
+      h = kBad;
+      cnt = 0;
+    }
     how = h;
     return p;
   }
@@ -457,7 +509,7 @@ struct InflateScan {
       const uint32_t top = stop ? static_cast<uint32_t>(__ffsll(stop)) - 1u : kPieces - 1u;  // last piece that counts
       if (id > top) cnt = 0;
       sm.batch[k].cnt[id] = static_cast<uint16_t>(cnt);
-      const uint32_t s = __reduce_add_sync(FULL, cnt);
+      const uint32_t s = __reduce_add_sync(FULL, cnt & 0xffu);
       if (lane == 0) sm.sum[warp] = s;
       const uint32_t next = sm.last[top], end_how = sm.how[top];
       scan_barrier();
@@ -473,7 +525,7 @@ struct InflateScan {
     }
   }
 
-  // Stored block: the token warp reads its bytes itself.
+  // Stored block: the token warps read its bytes themselves.
   __device__ __forceinline__ int stored() {
     pos = (pos + 7u) & ~7u;
     int st = need(64);
@@ -586,7 +638,7 @@ struct InflateScan {
       last = h & 1u;
       const uint32_t btype = (h >> 1) & 3u;
       pos += 3;
-      tab = handed ^ 1u;  // the token warp may still read the tables of the last batch
+      tab = handed ^ 1u;  // the token warps may still read the tables of the last batch
       if (btype == 0) {
         st = stored();
       } else if (btype == 1) {
@@ -605,22 +657,23 @@ struct InflateScan {
   }
 };
 
-// Binds the rings (the warps that fill them initialise the barriers) and the window of a team.
-template <class RING>
-__device__ __forceinline__ void bind_ring(RING& in, uint8_t* buf, uint64_t* bar, uint64_t wait_cycles, uint32_t lane) {
+// Binds a warp's input ring (it initialises the barriers) and the window of a team.
+template <int NSLOT>
+__device__ __forceinline__ void bind_ring(InRing<NSLOT, true>& in, uint8_t* buf, uint64_t* bar, uint64_t wait_cycles,
+                                          uint32_t lane, bool init) {
   in.buf = buf;
   in.sbuf = smem_u32(buf);
   in.bar = bar;
   in.phase = 0;
   in.wait_cycles = wait_cycles;
   in.lane = lane;
+  if (init) init_ring_barriers<NSLOT>(bar, lane);
 }
 __device__ __forceinline__ void inflate_rings(InflateRing& in, TokenRing& tin, InflateTeam& sm, uint64_t wait_cycles,
                                               uint32_t warp, uint32_t lane) {
-  bind_ring(in, sm.ring, sm.bar, wait_cycles, lane);
-  bind_ring(tin, sm.token_ring, sm.token_bar, wait_cycles, lane);
-  if (warp == 0) init_ring_barriers<16>(sm.bar, lane);
-  if (warp == 2) init_ring_barriers<4>(sm.token_bar, lane);
+  bind_ring(in, sm.ring, sm.bar, wait_cycles, lane, warp == 0);
+  const uint32_t w = warp & 1u;
+  bind_ring(tin, sm.token_ring[w], sm.token_bar[w], wait_cycles, lane, (warp >> 1) == 1);
 }
 __device__ __forceinline__ void inflate_window(InflateWin& o, InflateTeam& sm, uint32_t lane) {
   o.buf = sm.win;
@@ -641,7 +694,7 @@ __device__ __forceinline__ void inflate_scan(InflateRing& in, InflateTeam& sm, u
 }
 
 // ---------------------------------------------------------------------------------------
-// token warp
+// token warps
 // ---------------------------------------------------------------------------------------
 // inclusive prefix sum over the lanes
 __device__ __forceinline__ uint32_t warp_scan_add(uint32_t v, uint32_t lane) {
@@ -653,258 +706,330 @@ __device__ __forceinline__ uint32_t warp_scan_add(uint32_t v, uint32_t lane) {
   return v;
 }
 
-__device__ __forceinline__ uint32_t token_len(uint32_t tok) { return tok >> 31 ? 1u : tok & 0x1ffu; }
-
-// Token warp (2 of the team); `in` is bound to the stream.
-__device__ __forceinline__ void inflate_tokens(TokenRing& in, InflateTeam& sm, uint32_t lane) {
-  uint32_t kb = 0, k = 0, list = 0;
-  bool dead = false;  // a wait for the input ran out
-  // hands token batch k to the expander
-  const auto handoff = [&](uint32_t before, uint32_t bytes, uint32_t last) {
+// Token warps (2 and 3 of the team: `me` 0 and 1), taking turns at 32 cells or kTokens stored bytes; `in`
+// is bound to the stream.  Every turn ends in a batch, an empty one when no more are wanted, so the
+// place warp knows whose turn it is.
+__device__ __forceinline__ void inflate_tokens(TokenRing& in, InflateTeam& sm, uint32_t me, uint32_t lane) {
+  uint32_t kb = 0, turn = 0;
+  bool used = false;  // the list and the batch have been handed over before
+  TokenBatch& o = sm.out[me];
+  const auto reuse = [&]() {  // waits until the place warp is done with them
+    if (used) team_wait<64>(kTokensFree + me);
+    used = true;
+  };
+  const auto handoff = [&](uint32_t before, uint32_t bytes, uint32_t what) {
     if (lane == 0) {
-      TokenBatch& o = sm.out[k];
-      o.list = list;
       o.before = before;
       o.bytes = bytes;
-      o.last = last;
+      o.what = what;
     }
     __syncwarp();
-    token_barrier();
-    k ^= 1u;
+    team_signal<64>(kTokensFull + me);
   };
-  // the expander's word, the same for every lane
+  // the place warp's word, the same for every lane
   const auto stopped = [&]() {
-    return dead || __shfl_sync(FULL, *static_cast<volatile uint32_t*>(&sm.stop), 0) != 0;
+    const uint32_t v = *static_cast<volatile uint32_t*>(&sm.stop) | *static_cast<volatile uint32_t*>(&sm.dead);
+    return __shfl_sync(FULL, v, 0) != 0;
   };
   // bytes [at, end) resident
   const auto need = [&](uint32_t at, uint32_t end) {
-    dead = dead || !in.release(at) || in.ensure(end < in.hi ? end : in.hi) != CODAG_OK;
-    return !dead;
+    const bool ok = in.release(at) && in.ensure(end < in.hi ? end : in.hi) == CODAG_OK;
+    if (!ok && lane == 0) sm.dead = 1;
+    return ok;
   };
   for (;;) {
-    const bool drop = stopped();
-    if (lane == 0) sm.stopped[kb] = drop;  // both scan warps read the word of their batch's buffer
+    if (me == 0) {
+      const bool drop = stopped();
+      if (lane == 0) sm.stopped[kb] = drop;  // both scan warps read the word of their batch's buffer
+    }
     batch_barrier();
     ScanBatch& b = sm.batch[kb];
     kb ^= 1u;
     const uint32_t kind = b.kind;
     if (kind == kBatchDone) {
-      if (!in.drain()) dead = true;
-      if (lane == 0) sm.status = dead ? CODAG_ETIMEOUT : b.status;
-      handoff(0, 0, 1);
+      const bool drained = in.drain();
+      if (!drained && lane == 0) sm.dead = 1;
+      if ((turn & 1u) == me) {
+        if (lane == 0) sm.status = b.status;
+        reuse();
+        handoff(0, 0, kLast);
+      }
+      if (used) team_wait<64>(kTokensFree + me);
       return;
     }
-    if (drop) continue;
     if (kind == kBatchStored) {
       const uint32_t at = b.base, len = b.size;
-      for (uint32_t i = 0; i < len && !stopped(); i += kTokens) {
+      for (uint32_t i = 0; i < len; i += kTokens, turn++) {
+        if ((turn & 1u) != me) continue;
         const uint32_t n = len - i < kTokens ? len - i : kTokens;
-        if (!need(at + i, at + i + n)) break;
-        for (uint32_t q = lane; q < n; q += 32) sm.tok[list][q] = 0x80000000u | in.rd8(at + i + q);
-        if (32u * lane < n) sm.out[k].starts[lane] = n - 32u * lane >= 32u ? FULL : (1u << (n - 32u * lane)) - 1u;
+        reuse();
+        if (stopped() || !need(at + i, at + i + n)) {
+          handoff(0, 0, 0);
+          continue;
+        }
+        for (uint32_t q = lane; q < n; q += 32) sm.tok[me][q] = kLiteralToken | in.rd8(at + i + q);
+        if (32u * lane < n) o.starts[lane] = n - 32u * lane >= 32u ? FULL : (1u << (n - 32u * lane)) - 1u;
         handoff(0, n, 0);
-        list ^= 1u;
       }
       continue;
     }
     // cells of the pieces, as running totals
-    const uint32_t e0 = warp_scan_add((b.cnt[lane] + kCell - 1u) / kCell, lane);
-    const uint32_t e1 = warp_scan_add((b.cnt[32 + lane] + kCell - 1u) / kCell, lane) + __shfl_sync(FULL, e0, 31);
+    uint16_t* cell_end = sm.cell_end[me];
+    const uint32_t e0 = warp_scan_add(b.cnt[lane] >> 8, lane);
+    const uint32_t e1 = warp_scan_add(b.cnt[32 + lane] >> 8, lane) + __shfl_sync(FULL, e0, 31);
     const uint32_t cells = __shfl_sync(FULL, e1, 31);
-    sm.cell_end[lane] = static_cast<uint16_t>(e0);
-    sm.cell_end[32 + lane] = static_cast<uint16_t>(e1);
+    cell_end[lane] = static_cast<uint16_t>(e0);
+    cell_end[32 + lane] = static_cast<uint16_t>(e1);
     __syncwarp();
     InflateTables& tab = sm.tab[b.table];
     const uint32_t s_lit = smem_u32(tab.lit_lut), s_dist = smem_u32(tab.dist_lut);
     const uint32_t base = b.base, bits = b.size;
-    for (uint32_t c = 0, m; c < cells && !stopped(); c += m) {
-      const uint32_t x = c + lane < cells ? c + lane : cells - 1u;  // lanes past the end repeat the last cell
+    for (uint32_t c = 0; c < cells; c += 32, turn++) {
+      if ((turn & 1u) != me) continue;
+      const uint32_t count = cells - c < 32u ? cells - c : 32u;
+      const uint32_t x = c + (lane < count ? lane : count - 1u);  // lanes past the end repeat the last cell
       uint32_t q = 0;  // its piece: as many as end at or before it
 #pragma unroll
       for (uint32_t step = kPieces / 2; step; step >>= 1)
-        if (sm.cell_end[q + step - 1u] <= x) q += step;
-      const uint32_t first = q ? sm.cell_end[q - 1u] : 0u, j = x - first;
-      uint32_t p = base + q * bits + b.row[q * kCells + j];
-      // as many of the cells, which follow one another, as the ring holds for certain
-      const uint32_t p0 = __shfl_sync(FULL, p, 0);
-      constexpr uint32_t kCellBits = 48u * kCell + 96u;
-      m = __popc(__ballot_sync(FULL, p - p0 + kCellBits <= 8u * 3u * kSlotBytes));
-      if (m > cells - c) m = cells - c;
-      const uint32_t left = b.cnt[q] - j * kCell;
-      const uint32_t n = lane < m ? (left < kCell ? left : kCell) : 0u;
-      if (!need(p0 >> 3, (__shfl_sync(FULL, p, static_cast<int>(m) - 1) + kCellBits) >> 3)) break;
-      uint32_t* dst = sm.tok[list] + (warp_scan_add(n, lane) - n);
+        if (cell_end[q + step - 1u] <= x) q += step;
+      const uint32_t first = q ? cell_end[q - 1u] : 0u, j = x - first;
+      const uint16_t* row = b.row + q * kCells + j;
+      uint32_t p = base + q * bits + (row[0] & 0x7fffu);
+      const uint32_t next = j + 1u < b.cnt[q] >> 8 ? kCell * (j + 1u) + (row[1] >> 15) : b.cnt[q] & 0xffu;
+      const uint32_t n = lane < count ? next - (kCell * j + (row[0] >> 15)) : 0u;
+      uint32_t* dst = sm.tok[me] + (warp_scan_add(n, lane) - n);
       uint32_t len = 0;  // bytes of this lane's tokens
-      for (uint32_t i = 0; i < kCell; i++) {
-        if (i < n) {
-          const uint32_t a = in.sbuf + ((p >> 3) & (TokenRing::kMask & ~3u));
-          const uint32_t w0 = ld_s32(a), w1 = ld_s32(a + 4), w2 = ld_s32(a + 8), sh = p & 31u;
-          const Symbol y =
-              symbol(__funnelshift_r(w0, w1, sh), __funnelshift_r(w1, w2, sh), s_lit, s_dist, tab);
-          const uint32_t tok = y.literal() ? 0x80000000u | (y.e >> 16) : y.length() | (y.distance() << 9);
-          dst[i] = tok;
-          len += token_len(tok);
-          p += y.used;
+      reuse();
+      bool ok = !stopped();
+      // as many of the cells, which follow one another, at a time as the ring holds for certain:
+      // mostly all
+      for (uint32_t l0 = 0; ok && l0 < count;) {
+        constexpr uint32_t kCellBits = 48u * kCellMax + 96u;
+        const uint32_t p0 = __shfl_sync(FULL, p, static_cast<int>(l0));
+        const uint32_t fit = __ballot_sync(FULL, lane >= l0 && p - p0 + kCellBits <= 8u * kSlotBytes);
+        const uint32_t l1 = fit ? 32u - __clz(fit) : l0;  // [l0, l1): the cells that fit
+        const uint32_t last = __shfl_sync(FULL, p, static_cast<int>(l1) - 1);
+        ok = l1 > l0 && need(p0 >> 3, (last + kCellBits) >> 3);
+        if (!ok) break;
+        const bool mine = lane >= l0 && lane < l1;
+        for (uint32_t i = 0; __any_sync(FULL, mine && i < n);) {
+          if (mine && i < n) {
+            const uint32_t a = in.sbuf + ((p >> 3) & (TokenRing::kMask & ~3u));
+            const uint32_t w0 = ld_s32(a), w1 = ld_s32(a + 4), w2 = ld_s32(a + 8), sh = p & 31u;
+            const Symbol y = symbol(__funnelshift_r(w0, w1, sh), __funnelshift_r(w1, w2, sh), s_lit, s_dist, tab);
+            const uint32_t tok = y.literal() ? kLiteralToken | ((y.e >> 16) & 0xffu) : y.match();
+            dst[i] = tok;
+            if (y.e & kPairFlag) dst[i + 1u] = kLiteralToken | (y.e >> 24);
+            len += (tok >> 16) + y.count() - 1u;
+            i += y.count();
+            p += y.used;
+          }
         }
-        __syncwarp();
+        l0 = l1;
+      }
+      if (!ok) {
+        handoff(0, 0, 0);
+        continue;
       }
       uint32_t s0 = warp_scan_add(len, lane);
       const uint32_t total = __shfl_sync(FULL, s0, 31);
       s0 -= len;
+      if (total == 0) {  // a single cell noted just before the end of its block
+        handoff(0, 0, 0);
+        continue;
+      }
       // the tokens' bytes in ranges the bit map covers: one, unless there are long matches
       for (uint32_t r = 0; r < total; r += kRange) {
-        uint32_t* starts = sm.out[k].starts;
-        for (uint32_t i = lane; i < kRange / 32u; i += 32) starts[i] = 0;
+        if (r) reuse();
+        for (uint32_t i = lane; i < kRange / 32u; i += 32) o.starts[i] = 0;
         __syncwarp();
         uint32_t s = s0, before = 0;
         if (total <= kRange) {
 #pragma unroll 4
           for (uint32_t i = 0; i < n; i++) {
             const uint32_t tok = dst[i];
-            atomicOr(&starts[s >> 5], 1u << (s & 31u));
-            s += token_len(tok);
+            atomicOr(&o.starts[s >> 5], 1u << (s & 31u));
+            s += tok >> 16;
           }
         } else {
           for (uint32_t i = 0; i < n; i++) {
             const uint32_t tok = dst[i];
             if (s < r) before++;
-            else if (s - r < kRange) atomicOr(&starts[(s - r) >> 5], 1u << (s & 31u));
-            s += token_len(tok);
+            else if (s - r < kRange) atomicOr(&o.starts[(s - r) >> 5], 1u << (s & 31u));
+            s += tok >> 16;
           }
           before = __reduce_add_sync(FULL, before);
         }
-        handoff(before, total - r < kRange ? total - r : kRange, 0);
+        const bool more = total - r > kRange;
+        handoff(before, more ? kRange : total - r, more ? kMore : 0u);
       }
-      list ^= 1u;
     }
   }
 }
 
 // ---------------------------------------------------------------------------------------
-// expander warp
+// place warp
 // ---------------------------------------------------------------------------------------
-// Up to 32 output bytes at out position b0 + lane (lanes below n): w is the lane's token word
-// (literal with bit 31, else a distance).
-template <class OUT>
-__device__ __forceinline__ void expand_step(OUT& out, uint32_t b0, uint32_t n, uint32_t w, uint32_t lane) {
-  const bool near = w <= lane;  // a copy whose source lies in these 32 bytes
-  uint32_t v = w;
-  if (__any_sync(FULL, near)) {
-    // follow each to a lane that starts outside or is a literal: chains of up to 31 links, halved five times
-    uint32_t root = near ? lane - w : lane;
-#pragma unroll
-    for (int i = 0; i < 5; i++) root = __shfl_sync(FULL, root, root);
-    if (!near && !(w >> 31)) v = out.get8(b0 + lane - w);
-    v = __shfl_sync(FULL, v, root);
-  } else if (!(w >> 31)) {
-    v = out.get8(b0 + lane - w);
-  }
-  if (lane < n) out.put8(b0 + lane, v);
-  __syncwarp();
-}
-
-// 128 bytes at out position b0 (n of them wanted): lane l's byte of step i, at 32 i + l, is token word
-// w[i], of token t[i]; the first `before` tokens start before them.
-template <class OUT>
-__device__ __forceinline__ void expand_steps(OUT& out, uint32_t b0, uint32_t n, uint32_t* w, const uint32_t* t,
-                                             uint32_t before, uint32_t lane) {
-  bool near = false;
-#pragma unroll
-  for (uint32_t i = 0; i < 4; i++) near |= w[i] <= 32u * i + lane;
-  if (__any_sync(FULL, near)) {
-    // A match that goes on from before these bytes repeats itself with any multiple of its
-    // distance: one that reaches before them.
-    near = false;
-#pragma unroll
-    for (uint32_t i = 0; i < 4; i++) {
-      const uint32_t at = 32u * i + lane;
-      if (w[i] <= at && t[i] < before) w[i] *= at / w[i] + 1u;
-      near |= w[i] <= at;
-    }
-    if (__any_sync(FULL, near)) {
-#pragma unroll
-      for (uint32_t i = 0; i < 4; i++)
-        if (32u * i < n) expand_step(out, b0 + 32u * i, n - 32u * i, w[i], lane);
-      return;
-    }
-  }
-  uint32_t v[4];
-#pragma unroll
-  for (uint32_t i = 0; i < 4; i++) {
-    v[i] = w[i];
-    if (!(w[i] >> 31)) v[i] = out.get8(b0 + 32u * i + lane - w[i]);
-  }
-#pragma unroll
-  for (uint32_t i = 0; i < 4; i++)
-    if (32u * i + lane < n) out.put8(b0 + 32u * i + lane, v[i]);
-  __syncwarp();
-}
-
-// The bytes of one token batch.  False when the output would pass `cap` or a distance reaches
-// before the chunk.
-template <class OUT>
-__device__ __forceinline__ bool expand_batch(InflateTeam& sm, const TokenBatch& b, OUT& out, uint32_t& op, uint32_t cap,
-                                             uint32_t lane) {
-  constexpr uint32_t kSteps = 8;  // 32-byte steps whose tokens are found side by side
-  const uint32_t le = 0xffffffffu >> (31u - lane);
-  const uint32_t bytes = b.bytes, s_tok = smem_u32(sm.tok[b.list]);
-  if (bytes > cap - op) return false;
-  uint32_t count = b.before;  // tokens that start before the 1 KiB at c
-  for (uint32_t c = 0; c < bytes; c += 1024) {
-    // lane l: the starts in the 32 bytes at c + 32 l, and how many tokens start before them
-    const uint32_t word = c + 32u * lane < bytes ? b.starts[c / 32u + lane] : 0u;
-    const uint32_t upto = warp_scan_add(__popc(word), lane) + count, pre = upto - __popc(word);
-    count = __shfl_sync(FULL, upto, 31);
-    const uint32_t end = bytes - c < 1024u ? bytes - c : 1024u;
-    for (uint32_t q = 0; q < end; q += 32 * kSteps) {
-      const uint32_t b0 = op + c + q, n = end - q;
-      uint32_t w[kSteps], t[kSteps];
-#pragma unroll
-      for (uint32_t i = 0; i < kSteps; i++) {
-        const uint32_t starts = __shfl_sync(FULL, word, q / 32u + i);
-        t[i] = __shfl_sync(FULL, pre, q / 32u + i) + __popc(starts & le) - 1u;
-        const uint32_t tok = ld_s32(s_tok + 4u * t[i]);
-        // bytes past the end are taken for literals
-        w[i] = 32u * i + lane < n ? (tok >> 31 ? tok : tok >> 9) : 0x80000000u;
-      }
-      if (b0 < 32768u) {
-        bool bad = false;
-#pragma unroll
-        for (uint32_t i = 0; i < kSteps; i++) bad |= !(w[i] >> 31) && w[i] > b0 + 32u * i + lane;
-        if (__any_sync(FULL, bad)) return false;
-      }
-      expand_steps(out, b0, n, w, t, __shfl_sync(FULL, pre, q / 32u), lane);
-      if (n > 128u)
-        expand_steps(out, b0 + 128u, n - 128u, w + 4, t + 4, __shfl_sync(FULL, pre, q / 32u + 4u), lane);
-    }
-  }
-  op += bytes;
-  out.flush_to(op);
-  return true;
-}
-
-// Drains the token batches into `out` and returns the chunk's status.
-template <class OUT>
-__device__ __forceinline__ int inflate_expander(InflateTeam& sm, OUT& out, uint64_t chunk_bytes, uint32_t lane) {
+// Warp 4 of the team: the token word of every output byte.  Stops the chunk when its output would pass
+// `cap` or a distance reaches before its first byte.
+__device__ __forceinline__ void inflate_place(InflateTeam& sm, uint64_t chunk_bytes, uint32_t lane) {
   const uint32_t cap = static_cast<uint32_t>(chunk_bytes);
-  uint32_t op = 0, k = 0;
+  const uint32_t le = 0xffffffffu >> (31u - lane);
+  uint32_t op = 0, me = 0, k = 0, handed = 0;
   bool ok = true;
-  for (;;) {
-    token_barrier();
-    const TokenBatch& b = sm.out[k];
-    const uint32_t last = b.last;
-    if (ok) {
-      ok = expand_batch(sm, b, out, op, cap, lane);
-      if (!ok && lane == 0) sm.stop = 1;
-      __syncwarp();
+  const auto handoff = [&](uint32_t bytes, uint32_t near, uint32_t last) {
+    if (lane == 0) {
+      sm.place[k].bytes = bytes;
+      sm.place[k].near = near;
+      sm.place[k].last = last;
     }
+    __syncwarp();
+    team_signal<64>(kBytesFull + k);
     k ^= 1u;
-    if (last) break;
+    handed++;
+  };
+  for (;;) {
+    team_wait<64>(kTokensFull + me);
+    const TokenBatch& b = sm.out[me];
+    const uint32_t bytes = b.bytes, what = b.what, s_tok = smem_u32(sm.tok[me]);
+    if (bytes > cap - op) ok = false;
+    uint32_t count = b.before;  // tokens that start before the 1 KiB at c
+    for (uint32_t c = 0; ok && c < bytes; c += 1024) {
+      // lane l: the starts in the 32 bytes at c + 32 l, and how many tokens start before them
+      const uint32_t word = c + 32u * lane < bytes ? b.starts[c / 32u + lane] : 0u;
+      const uint32_t upto = warp_scan_add(__popc(word), lane) + count, pre = upto - __popc(word);
+      count = __shfl_sync(FULL, upto, 31);
+      const uint32_t end = bytes - c < 1024u ? bytes - c : 1024u;
+      for (uint32_t q = 0; q < end; q += 32 * kSteps) {
+        const uint32_t b0 = op + c + q, n = end - q;
+        uint32_t w[kSteps], t[kSteps];
+        bool near = false;
+#pragma unroll
+        for (uint32_t i = 0; i < kSteps; i++) {
+          const uint32_t starts = __shfl_sync(FULL, word, q / 32u + i);
+          t[i] = __shfl_sync(FULL, pre, q / 32u + i) + __popc(starts & le) - 1u;
+          // bytes past the end are taken for literals
+          w[i] = 32u * i + lane < n ? ld_s16(s_tok + 4u * t[i]) : kLiteral;
+          near |= w[i] < 32u * i + lane;
+        }
+        if (b0 < 32768u) {
+          bool bad = false;
+#pragma unroll
+          for (uint32_t i = 0; i < kSteps; i++) bad |= !(w[i] >> 15) && w[i] >= b0 + 32u * i + lane;
+          if (__any_sync(FULL, bad)) {
+            ok = false;
+            break;
+          }
+        }
+        uint32_t lead = 0;
+        if (__any_sync(FULL, near)) {
+          const uint32_t some = __ballot_sync(FULL, word != 0) & (FULL << (q / 32u));
+          const uint32_t f = some ? __ffs(some) - 1u : 32u;  // the first 32 bytes with a start
+          lead = f - q / 32u < kSteps ? 32u * (f - q / 32u) + __ffs(__shfl_sync(FULL, word, f & 31u)) - 1u : 32u * kSteps;
+          lead++;
+        }
+        if (handed >= 2u) team_wait<64>(kBytesFree + k);
+#pragma unroll
+        for (uint32_t i = 0; i < kSteps; i++) sm.place[k].word[32u * i + lane] = static_cast<uint16_t>(w[i]);
+        handoff(n < 32u * kSteps ? n : 32u * kSteps, lead, 0);
+      }
+    }
+    team_signal<64>(kTokensFree + me);
+    if (ok) op += bytes;
+    else if (lane == 0) sm.stop = 1;
+    __syncwarp();
+    if (what & kLast) break;
+    if (!(what & kMore)) me ^= 1u;
   }
+  if (handed >= 2u) team_wait<64>(kBytesFree + k);
+  handoff(0, 0, ok ? 1u : 1u | kBadChunk);
+  // the copy warp's last two signals
+  if (handed >= 2u) team_wait<64>(kBytesFree + k);
+  team_wait<64>(kBytesFree + (k ^ 1u));
+}
+
+// ---------------------------------------------------------------------------------------
+// copy warp
+// ---------------------------------------------------------------------------------------
+// Warp 5 of the team: writes the bytes through `out` and returns the chunk's status.
+template <class OUT>
+__device__ __forceinline__ int inflate_copy(InflateTeam& sm, OUT& out, uint32_t lane) {
+  uint32_t op = 0, k = 0, last;
+  do {
+    team_wait<64>(kBytesFull + k);
+    const ByteBatch& b = sm.place[k];
+    const uint32_t n = b.bytes, near = b.near;
+    last = b.last;
+    if (!near) {  // every source lies before the batch: all bytes at once
+      uint32_t v[kSteps];
+#pragma unroll
+      for (uint32_t i = 0; i < kSteps; i++) v[i] = b.word[32u * i + lane];
+#pragma unroll
+      for (uint32_t i = 0; i < kSteps; i++)
+        if (!(v[i] >> 15) && 32u * i < n) v[i] = out.get8(op + 32u * i + lane - 1u - v[i]);
+#pragma unroll
+      for (uint32_t i = 0; i < kSteps; i++)
+        if (32u * i + lane < n) out.put8(op + 32u * i + lane, v[i]);
+      __syncwarp();
+    } else if (near > n) {  // one match, repeating itself
+      const uint32_t d = b.word[0] + 1u, step = 32u % d;
+      uint32_t r = lane % d;
+#pragma unroll 4
+      for (uint32_t at = lane; at - lane < n; at += 32) {
+        const uint32_t v = out.get8(op - d + r);
+        if (at < n) out.put8(op + at, v);
+        r += step;
+        if (r >= d) r -= d;
+      }
+      __syncwarp();
+    } else {
+#pragma unroll 1
+      for (uint32_t h = 0; h < n; h += 128) {
+        uint32_t v[4];
+        bool inside = false;
+#pragma unroll
+        for (uint32_t i = 0; i < 4; i++) {
+          v[i] = b.word[h + 32u * i + lane];
+          inside |= v[i] < 32u * i + lane;
+        }
+        if (!__any_sync(FULL, inside)) {  // every source lies before these 128 bytes
+#pragma unroll
+          for (uint32_t i = 0; i < 4; i++)
+            if (!(v[i] >> 15) && h + 32u * i < n) v[i] = out.get8(op + h + 32u * i + lane - 1u - v[i]);
+#pragma unroll
+          for (uint32_t i = 0; i < 4; i++)
+            if (h + 32u * i + lane < n) out.put8(op + h + 32u * i + lane, v[i]);
+          __syncwarp();
+          continue;
+        }
+#pragma unroll 1
+        for (uint32_t i = h; i < n && i < h + 128u; i += 32) {
+          const uint32_t w = b.word[i + lane];
+          uint32_t x = w;
+          if (w >= lane && !(w >> 15)) x = out.get8(op + i + lane - 1u - w);
+          if (__any_sync(FULL, w < lane)) {
+            // follow sources among the 32 to a lane that starts outside or is a literal: chains of up
+            // to 31 links, halved five times
+            uint32_t root = w < lane ? lane - 1u - w : lane;
+#pragma unroll
+            for (int j = 0; j < 5; j++) root = __shfl_sync(FULL, root, root);
+            x = __shfl_sync(FULL, x, root);
+          }
+          if (i + lane < n) out.put8(op + i + lane, x);
+          __syncwarp();
+        }
+      }
+    }
+    team_signal<64>(kBytesFree + k);
+    k ^= 1u;
+    op += n;
+    out.flush_to(op);
+  } while (!last);
   out.finish(op);
+  if (sm.dead) return CODAG_ETIMEOUT;
   const int st = sm.status;
   if (st != CODAG_OK) return st;
-  return ok && op >= out.store ? CODAG_OK : CODAG_ECORRUPT;
+  return !(last & kBadChunk) && op >= out.store ? CODAG_OK : CODAG_ECORRUPT;
 }
 
 }  // namespace codag_dev

@@ -21,7 +21,7 @@ __global__ void __launch_bounds__(32 * kTeamWarps, 3)
     if (status && threadIdx.x == 0) status[chunk] = CODAG_ECORRUPT;
     return;
   }
-  if (threadIdx.x == 0) sm.stop = 0;
+  if (threadIdx.x == 0) sm.stop = sm.dead = 0;
   __syncthreads();
   InflateRing in;
   TokenRing tin;
@@ -29,15 +29,17 @@ __global__ void __launch_bounds__(32 * kTeamWarps, 3)
   if (warp < 2) {
     in.begin(comp + off, static_cast<uint32_t>(next - off));
     inflate_scan(in, sm, wrapper, warp, lane);
-  } else if (warp == 2) {
+  } else if (warp < 4) {
     tin.begin(comp + off, static_cast<uint32_t>(next - off));
-    inflate_tokens(tin, sm, lane);
+    inflate_tokens(tin, sm, warp - 2u, lane);
+  } else if (warp == 4) {
+    inflate_place(sm, chunk_bytes, lane);
   } else {
     const uint64_t base = chunk * chunk_bytes;
     InflateWin o;
     inflate_window(o, sm, lane);
     o.begin(out + base, store_bytes(base, chunk_bytes, out_bytes));
-    const int st = inflate_expander(sm, o, chunk_bytes, lane);
+    const int st = inflate_copy(sm, o, lane);
     if (status && lane == 0) status[chunk] = st;
   }
 }
