@@ -3,29 +3,41 @@
 //
 // CODAG encodes on the GPU with one thread per chunk (rlev1/encoder.h:1728-1847 setup_deflate_orig
 // / deflate_orig, rlev2/encoder_trans.h:184-357 block_encode_orig driven by compress_gpu_orig
-// :482-564), then scans the stream lengths and moves every stream to its aligned offset.  The
-// same three steps run here as three kernels on the caller's stream:
-//   k_encode_rlev1_warp  RLE v1: one warp per chunk runs the shared writer of ../rle_writers.h (the
-//                    code the host producers run, so the bytes are the same) into its own slot of
-//                    the caller's workspace, literal streams and runs 32 values at a time;
-//   k_encode_rlev2_warp  RLE v2: one warp per chunk runs the same writer, its group operations
-//                    split over the lanes (see below);
+// :482-564), then scans the stream lengths and moves every stream to its aligned offset.  Here:
+//   k_encode         one CTA per chunk, see below; the streams go to slots of the caller's workspace;
 //   k_scan_offsets   one CTA turns the stream lengths into the aligned offsets (blk_off);
-//   k_gather         one warp per chunk copies its stream to its offset with the alignment
+//   k_gather         one CTA per chunk copies its stream to its offset with the alignment
 //                    padding zeroed, and fills col_len.
 // Nothing is allocated; a stream that overruns its workspace slot, or a file larger than the
 // caller's output capacity, is reported in *d_status.
+//
+// Both writers (../rle_writers.h, which the host producers run) look like state machines over
+// the values, but where their items (a run, a group of literals) begin and end depends only on
+// where the last one ended and on comparisons of neighbouring values:
+//   RLE v1: a run starts at p if its first step is in [-128, 127] and the next step equals it; it
+//     goes on while the steps stay equal, for at most 129 values.  What lies between runs is
+//     literals, in groups of 127.
+//   RLE v2: from p, the first three equal values in a row within 128 values start a fixed run, which
+//     goes on for at most 128 values; what lies before them, else 128 values, is a variable group.
+// So a CTA first writes the comparisons of kTile values as bit masks, in parallel; then one warp
+// walks the items, a search for a set bit each; then all warps encode the items, one warp per
+// item, eight at a time, each with its size first and its bytes once the sizes of the
+// others are known.  With one warp per chunk running the state machine, an item cost about 9000 warp
+// instructions and a chunk had one warp to wait for.
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <type_traits>
 
 #include "../../../include/codag.h"
-#include "../rle_writers.h"
+#include "../rlev2_widths.h"
+#include "device_common.cuh"
+
+using namespace codag_dev;
 
 namespace {
 
 constexpr uint64_t kOverflow = ~0ull;
-
 
 // element j of one chunk of the input zero padded past in_bytes (d_in is element aligned)
 template <typename T>
@@ -55,280 +67,467 @@ struct Wide<uint32_t> { using T = unsigned int; };
 template <>
 struct Wide<uint64_t> { using T = unsigned long long; };
 
+constexpr uint32_t kEncWarps = 8;
+constexpr uint32_t kTile = 4096;             // values whose items are found at a time
+constexpr uint32_t kMaskWords = kTile / 32 + 5;  // and the 129 values an item may reach beyond them
+constexpr uint32_t kItems = kTile / 2 + 64;  // a literal between runs of three: two items per four values
 
-// ---------------------------------------------------------------------------------------
-// RLE v2, one warp per chunk.  With one thread per chunk the 32 threads of a warp take
-// different paths through the writer's decisions (a warp ran them largely one after another,
-// 6.4 GB/s on 1 GiB).  Here every lane of a warp runs the writer on the same chunk (same values,
-// same branches, the pending values and the patch list in shared memory, every lane storing the
-// same value to the same place), and WarpGroups splits each group operation over the lanes.
-// The writer's decisions are the ones the host producers run, so the bytes are the same.
-// ---------------------------------------------------------------------------------------
-constexpr uint32_t FULL_MASK = 0xffffffffu;
+struct EncodeShared {
+  uint32_t a[kMaskWords];  // RLE v1: a run starts here; RLE v2: the third of three equal values
+  uint32_t b[kMaskWords];  // RLE v1: the step to the next value equals the one after; RLE v2: equals the value before
+  uint32_t item[kItems];   // start (12 bits), values (8 bits), run (1 bit)
+  uint32_t items, next;
+  uint32_t size[2][kEncWarps];
+  uint32_t hist[kEncWarps][32];
+  uint64_t val[kEncWarps][128], list[kEncWarps][128];  // PATCHED_BASE: reduced values, patch list
+};
 
-// output of one warp: lane 0 writes the writer's single bytes, all lanes write packed bodies
-struct WarpSink {
+// bytes of one stream; what passes the slot's end is dropped (and reported by the stream's length)
+struct Slot {
   uint8_t* p;
   uint64_t cap;
-  uint64_t n;  // the same on every lane
-  uint32_t lane;
-  __device__ void put(uint8_t b) {
-    if (lane == 0 && n < cap) p[n] = b;
-    n++;
-  }
-  __device__ void put_at(uint64_t k, uint8_t b) {
-    if (n + k < cap) p[n + k] = b;
-  }
-  __device__ void advance(uint64_t k) { n += k; }
-  __device__ uint64_t size() const { return n; }
-  __device__ void set(uint64_t i, uint8_t b) {
-    if (lane == 0 && i < cap) p[i] = b;
+  __device__ __forceinline__ void put(uint64_t at, uint32_t b) const {
+    if (at < cap) p[at] = static_cast<uint8_t>(b);
   }
 };
 
-__device__ __forceinline__ uint64_t umin64(uint64_t a, uint64_t b) { return a < b ? a : b; }
-__device__ __forceinline__ uint64_t umax64(uint64_t a, uint64_t b) { return a > b ? a : b; }
-
-// codag_fmt::SerialGroups' operations, split over the 32 lanes; each starts and ends with the warp
-// converged, so what one lane writes the others read afterwards and no lane overwrites what
-// another still reads
-struct WarpGroups {
-  uint64_t* lit;   // kMaxLiterals pending values (shared memory)
-  uint64_t* list;  // kMaxLiterals patch entries (shared memory)
-  uint32_t* hs;    // 32 histogram counters (shared memory)
-  uint32_t lane;
-  using Scan = codag_fmt::SerialGroups::Scan;
-  static constexpr bool kBulk = true;
-  __device__ uint64_t* lits() { return lit; }
-
-  // Up to min(32, lim) values i, i+1, ... that extend a variable run: lane k takes value i+k and
-  // its step from the value before; the run stops before the first value whose step and the
-  // step before it are both zero (the writer's fixed-run test) and at the end of the input.
-  // Appends the values taken to l[nl..], leaves the last step taken in prev_delta, and returns
-  // the count (0: the writer's per-value steps take value i).
-  template <class Get>
-  __device__ uint32_t append_run(const Get& get, uint64_t i, uint64_t n, uint64_t* l, uint32_t nl,
-                                 uint64_t& prev_delta, uint32_t lim) const {
-    __syncwarp();
-    const uint64_t j = i + lane;
-    const bool in = j < n;
-    const uint64_t v = in ? static_cast<uint64_t>(get(j)) : 0ull;
-    uint64_t before = __shfl_up_sync(FULL_MASK, v, 1);
-    if (lane == 0) before = l[nl - 1];
-    const uint64_t d = v - before;
-    const uint32_t zero = __ballot_sync(FULL_MASK, in && d == 0);
-    const uint32_t zero_before = (zero << 1) | (prev_delta == 0 ? 1u : 0u);
-    const uint32_t stop = (zero & zero_before) | __ballot_sync(FULL_MASK, !in);
-    uint32_t take = stop ? static_cast<uint32_t>(__ffs(stop)) - 1u : 32u;
-    if (take > lim) take = lim;
-    if (lane < take) l[nl + lane] = v;
-    if (take) prev_delta = __shfl_sync(FULL_MASK, d, static_cast<int>(take - 1));
-    __syncwarp();
-    return take;
-  }
-
-  // Up to min(32, lim) values i, i+1, ... equal to the last pending value (a fixed run going on),
-  // appended to l[nl..]; returns the count
-  template <class Get>
-  __device__ uint32_t append_equal(const Get& get, uint64_t i, uint64_t n, uint64_t* l, uint32_t nl,
-                                   uint32_t lim) const {
-    __syncwarp();
-    const uint64_t last = l[nl - 1];
-    const uint64_t j = i + lane;
-    const bool eq = j < n && static_cast<uint64_t>(get(j)) == last;
-    const uint32_t stop = __ballot_sync(FULL_MASK, !eq);
-    uint32_t take = stop ? static_cast<uint32_t>(__ffs(stop)) - 1u : 32u;
-    if (take > lim) take = lim;
-    if (lane < take) l[nl + lane] = last;
-    __syncwarp();
-    return take;
-  }
-  __device__ uint64_t* lists() { return list; }
-
-  __device__ Scan scan(const uint64_t* l, uint32_t n) const {
-    __syncwarp();
-    const uint64_t initial = l[1] - l[0];
-    uint64_t lmin = l[0], lmax = l[0], md = 0;
-    bool inc = true, dec = true, fix = true;
-    for (uint32_t i = 1 + lane; i < n; i += 32) {
-      const uint64_t l1 = l[i], l0 = l[i - 1], d = l1 - l0;
-      lmin = umin64(lmin, l1);
-      lmax = umax64(lmax, l1);
-      inc &= l0 <= l1;
-      dec &= l0 >= l1;
-      fix &= d == initial;
-      md = umax64(md, d);
-    }
-    for (int o = 16; o; o >>= 1) {
-      lmin = umin64(lmin, __shfl_xor_sync(FULL_MASK, lmin, o));
-      lmax = umax64(lmax, __shfl_xor_sync(FULL_MASK, lmax, o));
-      md = umax64(md, __shfl_xor_sync(FULL_MASK, md, o));
-    }
-    Scan r{lmin, lmax, md, __all_sync(FULL_MASK, inc) != 0, __all_sync(FULL_MASK, dec) != 0,
-           __all_sync(FULL_MASK, fix) != 0};
-    return r;
-  }
-
-  template <class D>
-  __device__ void hist(const D& d, uint32_t n, uint8_t* h) const {
-    __syncwarp();
-    hs[lane] = 0;
-    __syncwarp();
-    for (uint32_t i = lane; i < n; i += 32) atomicAdd(&hs[v2_code(codag_fmt::closest_width(d(i)))], 1u);
-    __syncwarp();
-    for (int k = 0; k < 32; k++) h[k] = static_cast<uint8_t>(hs[k]);
-    __syncwarp();
-  }
-
-  // output byte k of the aligned packing, computed by lane k mod 32
-  template <class S, class D>
-  __device__ void pack_aligned(S& out, const D& d, uint32_t n, uint8_t bits) const {
-    __syncwarp();
-    uint64_t total;
-    if (bits < 8) {
-      const uint32_t per = 8u / bits;
-      const uint32_t mask = (1u << bits) - 1u;
-      total = (n + per - 1) / per;
-      for (uint64_t k = lane; k < total; k += 32) {
-        uint32_t b = 0;
-        for (uint32_t j = 0; j < per; j++) {
-          const uint64_t i = k * per + j;
-          if (i < n) b |= (static_cast<uint32_t>(d(static_cast<uint32_t>(i))) & mask) << (8u - (j + 1u) * bits);
-        }
-        out.put_at(k, static_cast<uint8_t>(b));
-      }
-    } else {
-      const uint32_t bytes = bits / 8u;
-      total = static_cast<uint64_t>(n) * bytes;
-      for (uint64_t k = lane; k < total; k += 32) {
-        const uint32_t i = static_cast<uint32_t>(k / bytes);
-        const uint32_t j = bytes - 1u - static_cast<uint32_t>(k % bytes);
-        out.put_at(k, static_cast<uint8_t>(d(i) >> (8u * j)));
-      }
-    }
-    out.advance(total);
-    __syncwarp();
-  }
-
-  // output byte k of the MSB-first packing: the bits of every value that overlaps it
-  template <class S, class D>
-  __device__ void pack_unaligned(S& out, const D& d, uint32_t n, uint8_t bits) const {
-    __syncwarp();
-    const uint64_t tb = static_cast<uint64_t>(n) * bits, total = (tb + 7) / 8;
-    for (uint64_t k = lane; k < total; k += 32) {
-      const uint64_t s = 8 * k, e = s + 8 < tb ? s + 8 : tb;
-      uint32_t byte = 0;
-      for (uint64_t i = s / bits; i * bits < e; i++) {
-        const uint64_t vs = i * bits, ve = vs + bits;
-        const uint64_t a = vs > s ? vs : s, b = ve < e ? ve : e;
-        const uint64_t field = (d(static_cast<uint32_t>(i)) >> (ve - b)) & ((1ull << (b - a)) - 1ull);
-        byte |= static_cast<uint32_t>(field << (s + 8 - b));
-      }
-      out.put_at(k, static_cast<uint8_t>(byte));
-    }
-    out.advance(total);
-    __syncwarp();
-  }
-
-  __device__ uint32_t patches(const uint64_t* l, uint32_t n, uint64_t lmin, uint64_t mask, uint32_t b95,
-                              uint32_t pwidth, uint64_t* out, uint64_t* max_gap) const {
-    static_assert(codag_fmt::kMaxLiterals == 128, "four rounds of 32 values");
-    __syncwarp();
-    uint32_t before = 0;
-    int32_t prev_pos = -1;  // last patched position of the earlier rounds
-    uint64_t mg = 0;
+__device__ __forceinline__ uint32_t scan_add(uint32_t v, uint32_t lane) {  // inclusive
 #pragma unroll
-    for (uint32_t q = 0; q < 4; q++) {
-      const uint32_t i = q * 32 + lane;
-      const uint64_t r = i < n ? l[i] - lmin : 0ull;
-      const bool hit = i < n && r > mask;
-      const uint32_t bq = __ballot_sync(FULL_MASK, hit);
-      if (hit) {
-        const uint32_t below = bq & ((1u << lane) - 1u);
-        const uint32_t prev = below ? q * 32 + 31 - __clz(below) : (prev_pos >= 0 ? static_cast<uint32_t>(prev_pos) : 0u);
-        const uint64_t gap = i - prev;
-        out[before + __popc(below)] = (gap << pwidth) | (r >> b95);
-        mg = umax64(mg, gap);
-      }
-      if (bq) prev_pos = static_cast<int32_t>(q * 32 + 31 - __clz(bq));
-      before += __popc(bq);
-    }
-    for (int o = 16; o; o >>= 1) mg = umax64(mg, __shfl_xor_sync(FULL_MASK, mg, o));
-    *max_gap = mg;
-    __syncwarp();
-    return before;
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t o = __shfl_up_sync(FULL, v, d);
+    if (lane >= static_cast<uint32_t>(d)) v += o;
   }
-};
+  return v;
+}
+__device__ __forceinline__ uint64_t max64(uint64_t v) {
+  const uint32_t h = static_cast<uint32_t>(v >> 32), hi = __reduce_max_sync(FULL, h);
+  return (static_cast<uint64_t>(hi) << 32) | __reduce_max_sync(FULL, h == hi ? static_cast<uint32_t>(v) : 0u);
+}
+__device__ __forceinline__ uint64_t min64(uint64_t v) { return ~max64(~v); }
 
-constexpr uint32_t kEncWarps = 4;
-
-// codag_fmt::RleV1Writer's bulk steps for a warp whose lanes all run the writer on one chunk
-struct WarpV1 {
-  static constexpr bool kBulk = true;
-  uint32_t lane_;
-  __device__ uint32_t lane() const { return lane_; }
-  __device__ uint32_t ballot(bool p) const { return __ballot_sync(FULL_MASK, p); }
-  __device__ uint32_t ffs(uint32_t m) const { return static_cast<uint32_t>(__ffs(m)); }
-  __device__ void sync() const { __syncwarp(); }
-  template <typename V>
-  __device__ V shfl(V v, int src) const {
-    if constexpr (sizeof(V) == 8) return static_cast<V>(__shfl_sync(FULL_MASK, static_cast<unsigned long long>(v), src));
-    else return static_cast<V>(__shfl_sync(FULL_MASK, static_cast<uint32_t>(v), src));
-  }
-  // the value of the lane below (lane 0 gets its own)
-  template <typename V>
-  __device__ V shfl_up(V v) const {
-    if constexpr (sizeof(V) == 8) return static_cast<V>(__shfl_up_sync(FULL_MASK, static_cast<unsigned long long>(v), 1));
-    else return static_cast<V>(__shfl_up_sync(FULL_MASK, static_cast<uint32_t>(v), 1));
-  }
-  // sum of v over the lanes below
-  __device__ uint32_t excl_sum(uint32_t v) const {
-    uint32_t s = v;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const uint32_t o = __shfl_up_sync(FULL_MASK, s, d);
-      if (lane_ >= static_cast<uint32_t>(d)) s += o;
-    }
-    return s - v;
-  }
-};
-
-// RLE v1, one warp per chunk: every lane runs the writer on the same values (lane 0 writes its
-// single bytes); literal streams and runs going on are taken 32 values at a time (WarpV1)
-template <typename T>
-__global__ void __launch_bounds__(32 * kEncWarps) k_encode_rlev1_warp(const uint8_t* __restrict__ in, uint64_t in_bytes,
-                                                                     uint64_t chunk_bytes, uint64_t n,
-                                                                     uint8_t* __restrict__ scratch, uint64_t slot,
-                                                                     uint64_t* __restrict__ lens) {
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint64_t i = static_cast<uint64_t>(blockIdx.x) * kEncWarps + (threadIdx.x >> 5);
-  if (i >= n) return;  // the whole warp
-  WarpSink s{scratch + i * slot, slot, 0, lane};
-  using W = typename Wide<T>::T;
-  const PaddedChunk<W> get{in, in_bytes, i * chunk_bytes};
-  codag_fmt::RleV1Writer<T, WarpSink, WarpV1> w(s, WarpV1{lane});
-  w.encode([&](uint64_t j) { return static_cast<T>(get(j)); }, chunk_bytes / sizeof(T));
-  if (lane == 0) lens[i] = s.n > slot ? kOverflow : s.n;
+// position of the first set bit of `mask` (xor `flip`) at or after `from`, if it lies within 31 words;
+// else kFar, which is past everything but leaves room for sums
+constexpr uint32_t kFar = 1u << 30;
+__device__ __forceinline__ uint32_t first_set(const uint32_t* mask, uint32_t flip, uint32_t from, uint32_t lane) {
+  const uint32_t w = from / 32u + lane;
+  uint32_t v = w < kMaskWords ? mask[w] ^ flip : FULL;
+  if (lane == 0) v &= FULL << (from & 31u);
+  const uint32_t f = __ffs(__ballot_sync(FULL, v != 0));
+  return f ? (from / 32u + f - 1u) * 32u + __ffs(__shfl_sync(FULL, v, f - 1u)) - 1u : kFar;
 }
 
+// step from one value to the next as the writer computes it: in the type's own arithmetic, so never
+// negative for 32-bit values, and as an int for narrower ones
 template <typename T>
-__global__ void __launch_bounds__(32 * kEncWarps) k_encode_rlev2_warp(const uint8_t* __restrict__ in, uint64_t in_bytes,
-                                                                     uint64_t chunk_bytes, uint64_t n,
-                                                                     uint8_t* __restrict__ scratch, uint64_t slot,
-                                                                     uint64_t* __restrict__ lens) {
-  __shared__ uint64_t s_lit[kEncWarps][codag_fmt::kMaxLiterals];
-  __shared__ uint64_t s_list[kEncWarps][codag_fmt::kMaxLiterals];
-  __shared__ uint32_t s_h[kEncWarps][32];
-  const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
-  const uint64_t i = static_cast<uint64_t>(blockIdx.x) * kEncWarps + w;
-  if (i >= n) return;  // the whole warp
-  WarpSink s{scratch + i * slot, slot, 0, lane};
-  const WarpGroups g{s_lit[w], s_list[w], s_h[w], lane};
+__device__ __forceinline__ int64_t step_of(T a, T b) {
+  return static_cast<int64_t>(b - a);
+}
+
+// number of significant bits rounded up to a representable width
+__device__ __forceinline__ uint32_t width_of(uint64_t v) {
+  return v2_closest(64u - static_cast<uint32_t>(__clzll(static_cast<long long>(v))));
+}
+__device__ __forceinline__ uint32_t varint_len(uint64_t v) {
+  return (70u - static_cast<uint32_t>(__clzll(static_cast<long long>(v | 1u)))) / 7u;
+}
+// byte k of the unsigned LEB128 form of v, whose length is len
+__device__ __forceinline__ uint32_t varint_byte(uint64_t v, uint32_t k, uint32_t len) {
+  return (static_cast<uint32_t>(v >> (7u * k)) & 0x7fu) | (k + 1u < len ? 0x80u : 0u);
+}
+
+// --- RLE v1 items ---------------------------------------------------------------------------------
+template <typename T>
+struct ItemV1 {
+  static constexpr uint32_t kRunMax = 129, kLitMax = 127;
+  T v[4];  // value 32 q + lane (a run needs the first two only)
+  uint32_t n, size;
+  bool run;
+  uint32_t at[4];  // literals: offset of each value's bytes
+
+  template <class Get>
+  __device__ __forceinline__ void measure(const Get& get, uint64_t start, uint32_t count, bool is_run, EncodeShared&, uint32_t,
+                                          uint32_t lane) {
+    n = count;
+    run = is_run;
+    if (run) {
+      v[0] = static_cast<T>(get(start));
+      v[1] = static_cast<T>(get(start + 1));
+      size = 2u + varint_len(v[0]);
+      return;
+    }
+    uint32_t sum = 1;
+#pragma unroll
+    for (uint32_t q = 0; q < 4; q++) {
+      const uint32_t i = 32u * q + lane;
+      v[q] = i < n ? static_cast<T>(get(start + i)) : T(0);
+      const uint32_t len = i < n ? varint_len(v[q]) : 0u;
+      const uint32_t s = scan_add(len, lane);
+      at[q] = sum + s - len;
+      sum += __shfl_sync(FULL, s, 31);
+    }
+    size = sum;
+  }
+  __device__ __forceinline__ void write(const Slot& out, uint64_t off, EncodeShared&, uint32_t, uint32_t lane) const {
+    if (run) {
+      if (lane < size) {
+        const uint32_t b = lane == 0 ? n - 3u
+                           : lane == 1 ? static_cast<uint32_t>(step_of<T>(v[0], v[1]))
+                                       : varint_byte(v[0], lane - 2u, size - 2u);
+        out.put(off + lane, b);
+      }
+      return;
+    }
+    if (lane == 0) out.put(off, 0u - n);
+#pragma unroll
+    for (uint32_t q = 0; q < 4; q++) {
+      if (32u * q + lane < n) {
+        const uint32_t len = varint_len(v[q]);
+        for (uint32_t k = 0; k < len; k++) out.put(off + at[q] + k, varint_byte(v[q], k, len));
+      }
+    }
+  }
+};
+
+// --- RLE v2 items (the choices are those of RleV2Writer, ../rle_writers.h) ------------------------------
+template <typename T>
+struct ItemV2 {
+  enum : uint32_t { kShortRepeat, kDirect, kDeltaFixed, kDelta, kPatched };
+  uint64_t v[4];   // value 32 q + lane
+  uint64_t first, second, lmin;
+  uint32_t n, size, kind, bits;
+  uint32_t b95, pwidth, npatch, gap_width;
+
+  // suffix sums of the histogram of width codes: lane c has the number of values of code c and above
+  template <class D>
+  __device__ __forceinline__ uint32_t code_suffix(const D& d, uint32_t* hist, uint32_t lane) const {
+    __syncwarp();
+    hist[lane] = 0;
+    __syncwarp();
+#pragma unroll
+    for (uint32_t q = 0; q < 4; q++)
+      if (32u * q + lane < n) atomicAdd(&hist[v2_code(width_of(d(q)))], 1u);
+    __syncwarp();
+    const uint32_t c = hist[lane];
+    return n - (scan_add(c, lane) - c);
+  }
+  // smallest width that covers all but the top (100 - p)% of the values
+  __device__ __forceinline__ uint32_t percentile(uint32_t suffix, uint32_t p) const {
+    p = 100u - p;
+    const uint32_t left = p == 0 ? 0u : (n * p - 1u) / 100u + 1u;
+    const uint32_t m = __ballot_sync(FULL, suffix > left);
+    return m ? v2_width(31u - __clz(m)) : 0u;
+  }
+  static __device__ __forceinline__ uint32_t aligned_bytes(uint32_t count, uint32_t w) { return (count * w + 7u) / 8u; }
+  static __device__ __forceinline__ uint64_t zigzag(uint64_t d) {
+    const int64_t s = static_cast<int64_t>(d);
+    return static_cast<uint64_t>((s << 1) ^ (s >> 63));
+  }
+
+  __device__ __forceinline__ void set_direct(uint32_t suffix) {
+    kind = kDirect;
+    bits = v2_closest_aligned(percentile(suffix, 100));
+    size = 2u + aligned_bytes(n, bits);
+  }
+
+  template <class Get>
+  __device__ __forceinline__ void measure(const Get& get, uint64_t start, uint32_t count, bool is_run, EncodeShared& sh,
+                                          uint32_t warp, uint32_t lane) {
+    n = count;
+    if (is_run && n < 128u) {  // a fixed run that ended before the limit
+      first = second = get(start);
+      const uint32_t nb = (width_of(first) - 1u) / 8u + 1u;
+      kind = n <= 10u ? kShortRepeat : kDeltaFixed;
+      size = n <= 10u ? 1u + nb : 3u + varint_len(first);
+      return;
+    }
+#pragma unroll
+    for (uint32_t q = 0; q < 4; q++) v[q] = 32u * q + lane < n ? static_cast<uint64_t>(get(start + 32u * q + lane)) : 0ull;
+    uint32_t* hist = sh.hist[warp];
+    const auto value = [&](uint32_t q) { return v[q]; };
+    if (n <= 3u) {
+      set_direct(code_suffix(value, hist, lane));
+      return;
+    }
+    first = shfl64(v[0], 0);
+    second = shfl64(v[0], 1);
+    const uint64_t initial = second - first;
+    uint64_t lo = first, hi = first, md = 0;
+    bool inc = true, dec = true, fix = true;
+    uint64_t last = 0;
+#pragma unroll
+    for (uint32_t q = 0; q < 4; q++) {
+      uint64_t prev = shfl_up64(v[q], 1);
+      if (lane == 0) prev = last;
+      last = shfl64(v[q], 31);
+      const uint32_t i = 32u * q + lane;
+      if (i > 0 && i < n) {
+        const uint64_t d = v[q] - prev;
+        lo = v[q] < lo ? v[q] : lo;
+        hi = v[q] > hi ? v[q] : hi;
+        md = d > md ? d : md;
+        inc &= prev <= v[q];
+        dec &= prev >= v[q];
+        fix &= d == initial;
+      }
+    }
+    lmin = min64(lo);
+    const uint64_t lmax = max64(hi);
+    // subtracting the minimum is taken for unsafe only for a minimum of 0 and a maximum up to 128
+    if (!(lmin > 0 || lmax > 128u)) {
+      set_direct(code_suffix(value, hist, lane));
+      return;
+    }
+    if (__all_sync(FULL, fix)) {
+      kind = kDeltaFixed;
+      size = 2u + varint_len(first) + varint_len(zigzag(initial));
+      return;
+    }
+    if (initial != 0 && (__all_sync(FULL, inc) || __all_sync(FULL, dec))) {
+      kind = kDelta;
+      bits = v2_closest_aligned(width_of(max64(md)));
+      if (bits == 1u) bits = 2u;
+      size = 2u + varint_len(first) + varint_len(zigzag(initial)) + aligned_bytes(n - 2u, bits);
+      return;
+    }
+    const uint32_t plain = code_suffix(value, hist, lane);
+    if (percentile(plain, 100) - percentile(plain, 90) <= 1u) {
+      set_direct(plain);
+      return;
+    }
+    const uint32_t reduced = code_suffix([&](uint32_t q) { return v[q] - lmin; }, hist, lane);
+    b95 = percentile(reduced, 95);
+    const uint32_t r100 = percentile(reduced, 100);
+    if (r100 == b95) {
+      set_direct(plain);
+      return;
+    }
+    // PATCHED_BASE: values above b95 bits keep their low bits and give an entry (gap, high bits) of the
+    // patch list, gaps counted from the patch before (0 before the first)
+    kind = kPatched;
+    pwidth = v2_closest(r100 - b95);
+    if (pwidth == 64u) {
+      pwidth = 56u;
+      b95 = 8u;
+    }
+    const uint64_t mask = (1ull << b95) - 1ull;
+    uint32_t before = 0, max_gap = 0;
+    int32_t prev_pos = -1;
+    __syncwarp();
+#pragma unroll
+    for (uint32_t q = 0; q < 4; q++) {
+      const uint32_t i = 32u * q + lane;
+      const uint64_t r = i < n ? v[q] - lmin : 0ull;
+      if (i < n) sh.val[warp][i] = r & mask;
+      const bool hit = r > mask;
+      const uint32_t bq = __ballot_sync(FULL, hit);
+      if (hit) {
+        const uint32_t below = bq & lanemask_lt(lane);
+        const uint32_t prev = below ? 32u * q + 31u - __clz(below) : (prev_pos >= 0 ? static_cast<uint32_t>(prev_pos) : 0u);
+        sh.list[warp][before + __popc(below)] = (static_cast<uint64_t>(i - prev) << pwidth) | (r >> b95);
+        max_gap = max_gap > i - prev ? max_gap : i - prev;
+      }
+      if (bq) prev_pos = static_cast<int32_t>(32u * q + 31u - __clz(bq));
+      before += __popc(bq);
+    }
+    __syncwarp();
+    npatch = before;
+    max_gap = __reduce_max_sync(FULL, max_gap);
+    gap_width = max_gap == 0 && npatch != 0 ? 1u : width_of(max_gap);
+    size = 4u + base_bytes() + aligned_bytes(n, b95) + aligned_bytes(npatch, v2_closest(gap_width + pwidth));
+  }
+  __device__ __forceinline__ uint32_t base_bytes() const { return width_of(lmin) / 8u + 1u; }
+
+  // x[q] is element 32 q + lane, at an aligned width, most significant bit first
+  __device__ __forceinline__ void put_aligned(const Slot& out, uint64_t off, const uint64_t* x, uint32_t count, uint32_t w,
+                                              uint32_t lane) const {
+    if (w >= 8u) {
+      const uint32_t nb = w / 8u;
+#pragma unroll
+      for (uint32_t q = 0; q < 4; q++) {
+        const uint32_t i = 32u * q + lane;
+        if (i < count)
+          for (uint32_t j = 0; j < nb; j++) out.put(off + i * nb + j, static_cast<uint32_t>(x[q] >> (8u * (nb - 1u - j))));
+      }
+      return;
+    }
+    const uint32_t per = 8u / w;  // 2, 4 or 8 lanes share a byte
+#pragma unroll
+    for (uint32_t q = 0; q < 4; q++) {
+      const uint32_t i = 32u * q + lane;
+      uint32_t b = i < count ? (static_cast<uint32_t>(x[q]) & ((1u << w) - 1u)) << (8u - (i % per + 1u) * w) : 0u;
+      for (uint32_t d = 1; d < per; d <<= 1) b |= __shfl_xor_sync(FULL, b, d);
+      if (i < count && i % per == 0) out.put(off + i / per, b);
+    }
+  }
+  // `count` values of w bits from shared memory, most significant bit first
+  static __device__ __forceinline__ void put_packed(const Slot& out, uint64_t off, const uint64_t* x, uint32_t count,
+                                                    uint32_t w, uint32_t lane) {
+    const uint32_t tb = count * w;
+    for (uint32_t s = 8u * lane; s < tb; s += 256u) {
+      const uint32_t e = s + 8u < tb ? s + 8u : tb;
+      uint32_t byte = 0;
+      for (uint32_t i = s / w; i * w < e; i++) {
+        const uint32_t vs = i * w, ve = vs + w, a = vs > s ? vs : s, b = ve < e ? ve : e;
+        byte |= (static_cast<uint32_t>(x[i] >> (ve - b)) & ((1u << (b - a)) - 1u)) << (s + 8u - b);
+      }
+      out.put(off + s / 8u, byte);
+    }
+  }
+
+  __device__ __forceinline__ void write(const Slot& out, uint64_t off, EncodeShared& sh, uint32_t warp, uint32_t lane) const {
+    const uint32_t len = n - 1u;
+    if (kind == kShortRepeat) {
+      if (lane == 0) out.put(off, ((size - 2u) << 3) | (n - 3u));
+      else if (lane < size) out.put(off + lane, static_cast<uint32_t>(first >> (8u * (size - 1u - lane))));
+      return;
+    }
+    const uint32_t top = kind == kDirect ? 0x40u : kind == kPatched ? 0x80u : 0xC0u;
+    const uint32_t code = kind == kDeltaFixed ? 0u : v2_code(kind == kPatched ? b95 : bits);
+    if (lane == 0) out.put(off, top | (code << 1) | ((len >> 8) & 1u));
+    if (lane == 1) out.put(off + 1, len);
+    off += 2;
+    if (kind == kDirect) {
+      put_aligned(out, off, v, n, bits, lane);
+      return;
+    }
+    if (kind == kPatched) {
+      const uint32_t nb = base_bytes(), w2 = v2_closest(gap_width + pwidth);
+      if (lane == 0) out.put(off, ((nb - 1u) << 5) | v2_code(pwidth));
+      if (lane == 1) out.put(off + 1, ((gap_width - 1u) << 5) | npatch);
+      off += 2;
+      if (lane < nb) out.put(off + lane, static_cast<uint32_t>(shr64(lmin, 8u * (nb - 1u - lane))));
+      off += nb;
+      put_packed(out, off, sh.val[warp], n, b95, lane);
+      put_packed(out, off + aligned_bytes(n, b95), sh.list[warp], npatch, w2, lane);
+      return;
+    }
+    // DELTA: base and first step as varints, then the further steps unless they are all the same
+    const uint64_t zz = zigzag(second - first);
+    const uint32_t l1 = varint_len(first), l2 = varint_len(zz);
+    if (lane < l1) out.put(off + lane, varint_byte(first, lane, l1));
+    else if (lane < l1 + l2) out.put(off + lane, varint_byte(zz, lane - l1, l2));
+    if (kind == kDeltaFixed) return;
+    uint64_t d[4], x[4], last = 0;
+#pragma unroll
+    for (uint32_t q = 0; q < 4; q++) {
+      uint64_t prev = shfl_up64(v[q], 1);
+      if (lane == 0) prev = last;
+      last = shfl64(v[q], 31);
+      d[q] = v[q] - prev;
+    }
+#pragma unroll
+    for (uint32_t q = 0; q < 4; q++) {  // element i is the step to value i + 2
+      const uint64_t here = shfl64(d[q], (lane + 2u) & 31u);
+      const uint64_t next = q < 3 ? shfl64(d[q + 1], (lane + 2u) & 31u) : 0ull;
+      x[q] = lane < 30u ? here : next;
+    }
+    put_aligned(out, off + l1 + l2, x, n - 2u, bits, lane);
+  }
+};
+
+// One CTA per chunk.  Bound by the latency of its serial parts (the walk, a barrier every eight
+// items); several CTAs per SM overlap theirs.
+template <int CODEC, typename T>
+__global__ void __launch_bounds__(32 * kEncWarps) k_encode(const uint8_t* __restrict__ in, uint64_t in_bytes,
+                                                          uint64_t chunk_bytes, uint8_t* __restrict__ scratch,
+                                                          uint64_t slot, uint64_t* __restrict__ lens) {
+  __shared__ EncodeShared sh;
+  constexpr bool V1 = CODEC == CODAG_CODEC_RLEV1;
+  using Item = std::conditional_t<V1, ItemV1<T>, ItemV2<T>>;
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint64_t chunk = blockIdx.x;
+  const uint64_t n = chunk_bytes / sizeof(T);
   using W = typename Wide<T>::T;
-  const PaddedChunk<W> get{in, in_bytes, i * chunk_bytes};
-  codag_fmt::RleV2Writer<WarpSink, WarpGroups> wr(s, g);
-  wr.encode([&](uint64_t j) { return static_cast<uint64_t>(get(j)); }, chunk_bytes / sizeof(T));
-  if (lane == 0) lens[i] = s.n > slot ? kOverflow : s.n;
+  const PaddedChunk<W> raw{in, in_bytes, chunk * chunk_bytes};
+  const auto get = [&](uint64_t i) { return static_cast<T>(raw(i)); };
+  const Slot out{scratch + chunk * slot, slot};
+  uint64_t base = 0;
+  uint32_t par = 0;
+  for (uint64_t t0 = 0; t0 < n;) {
+    // comparisons of values t0 + b
+    for (uint32_t w = warp; w < kMaskWords; w += kEncWarps) {
+      const uint64_t j = t0 + 32u * w + lane;
+      bool pa = false, pb = false;
+      if constexpr (V1) {
+        if (j + 2 < n) {
+          const T x0 = get(j), x1 = get(j + 1), x2 = get(j + 2);
+          const int64_t d = step_of<T>(x0, x1);
+          pb = d == step_of<T>(x1, x2);
+          pa = pb && d >= -128 && d <= 127;
+        }
+      } else {
+        const uint32_t b = 32u * w + lane;
+        if (b >= 1 && j < n) {
+          const T x0 = get(j), x1 = get(j - 1);
+          pb = x0 == x1;
+          pa = pb && b >= 2 && x1 == get(j - 2);
+        }
+      }
+      const uint32_t ma = __ballot_sync(FULL, pa), mb = __ballot_sync(FULL, pb);
+      if (lane == 0) {
+        sh.a[w] = ma;
+        sh.b[w] = mb;
+      }
+    }
+    __syncthreads();
+    if (warp == 0) {  // items that start in the tile
+      const uint32_t end = static_cast<uint32_t>(n - t0 < kTile + 256u ? n - t0 : kTile + 256u);
+      uint32_t p = 0, items = 0;
+      while (p < kTile && p < end) {
+        uint32_t count, run = 0;
+        if constexpr (V1) {
+          const uint32_t r = first_set(sh.a, 0u, p, lane);
+          if (r == p) {
+            const uint32_t z = first_set(sh.b, FULL, p, lane) - p + 2u;
+            count = z < Item::kRunMax ? z : Item::kRunMax;
+            run = 1;
+          } else {
+            const uint32_t stop = r < end ? r : end;
+            count = stop - p < Item::kLitMax ? stop - p : Item::kLitMax;
+          }
+        } else {
+          const uint32_t j = first_set(sh.a, 0u, p + 2u, lane), lim = end - p < 128u ? end : p + 128u;
+          if (j >= lim) {
+            count = lim - p;
+          } else if (j - 2u > p) {
+            count = j - 2u - p;
+          } else {
+            const uint32_t z = first_set(sh.b, FULL, p + 1u, lane);
+            const uint32_t stop = z < end ? z : end;
+            count = stop - p < 128u ? stop - p : 128u;
+            run = 1;
+          }
+        }
+        if (lane == 0) sh.item[items] = p | (count << 12) | (run << 20);
+        items++;
+        p += count;
+      }
+      if (lane == 0) {
+        sh.items = items;
+        sh.next = p;
+      }
+    }
+    __syncthreads();
+    const uint32_t items = sh.items, step = sh.next;
+    for (uint32_t r = 0; r < items; r += kEncWarps, par ^= 1u) {
+      Item it;
+      it.size = 0;
+      if (r + warp < items) {
+        const uint32_t d = sh.item[r + warp];
+        it.measure(get, t0 + (d & 0xfffu), (d >> 12) & 0xffu, (d >> 20) != 0, sh, warp, lane);
+      }
+      if (lane == 0) sh.size[par][warp] = it.size;
+      __syncthreads();
+      const uint32_t s = lane < kEncWarps ? sh.size[par][lane] : 0u;
+      const uint32_t upto = scan_add(s, lane);
+      const uint32_t before = __shfl_sync(FULL, upto - s, warp);
+      if (r + warp < items) it.write(out, base + before, sh, warp, lane);
+      base += __shfl_sync(FULL, upto, 31);
+    }
+    t0 += step;
+    __syncthreads();  // the masks and items are overwritten
+  }
+  if (threadIdx.x == 0) lens[chunk] = base > slot ? kOverflow : base;
 }
 
 // blk_off[i] = sum of round_up(lens[k], ALIGN) for k < i, blk_off[n] = the total; one CTA of
@@ -364,17 +563,15 @@ __global__ void __launch_bounds__(1024) k_scan_offsets(const uint64_t* __restric
   if (t == 0 && bad && status) *status = CODAG_ECORRUPT;
 }
 
-// One warp per chunk: stream i goes to out + head + blk_off[i] and is zero padded to ALIGN
+// One CTA per chunk: stream i goes to out + head + blk_off[i] and is zero padded to ALIGN
 // bytes.  RLE v1 (head 8): the blob starts with the original size.  RLE v2: blk_off[n] is
 // overwritten with the original size.  The file is out_bytes = head + blk_off[n] long.
 template <uint64_t ALIGN, uint32_t HEAD>
 __global__ void __launch_bounds__(256) k_gather(const uint8_t* __restrict__ scratch, uint64_t slot,
                                                 const uint64_t* __restrict__ lens, uint64_t n, uint8_t* __restrict__ out,
-                                                uint64_t capacity, uint64_t* __restrict__ blk_off,
+                                                uint64_t capacity, const uint64_t* __restrict__ blk_off,
                                                 uint64_t* __restrict__ col_len, uint64_t in_bytes,
                                                 uint64_t* __restrict__ out_bytes, int32_t* __restrict__ status) {
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint64_t warps = static_cast<uint64_t>(gridDim.x) * (blockDim.x >> 5);
   const uint64_t total = HEAD + blk_off[n];
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     if (out_bytes) *out_bytes = total;
@@ -382,23 +579,19 @@ __global__ void __launch_bounds__(256) k_gather(const uint8_t* __restrict__ scra
     if (HEAD == 8 && capacity >= 8) *reinterpret_cast<uint64_t*>(out) = in_bytes;
   }
   if (total > capacity) return;
-  for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += warps) {
-    const uint64_t len = lens[i], off = HEAD + blk_off[i];
-    if (lane == 0) col_len[i] = len;
-    if (len == kOverflow) continue;
-    const uint64_t padded = (len + ALIGN - 1) / ALIGN * ALIGN;
-    const uint32_t* src = reinterpret_cast<const uint32_t*>(scratch + i * slot);
-    uint32_t* dst = reinterpret_cast<uint32_t*>(out + off);  // 4-byte aligned: HEAD, ALIGN multiples of 4
-    for (uint64_t w = lane; w < padded / 4; w += 32) {
-      uint32_t v = 0;
-      const uint64_t b0 = 4 * w;
-      if (b0 + 4 <= len) {
-        v = src[w];
-      } else if (b0 < len) {
-        v = src[w] & ((1u << (8 * (len - b0))) - 1u);  // keep the stream's bytes, zero the padding
-      }
-      dst[w] = v;
-    }
+  const uint64_t i = blockIdx.x;
+  const uint64_t len = lens[i], off = HEAD + blk_off[i];
+  if (threadIdx.x == 0) col_len[i] = len;
+  if (len == kOverflow) return;
+  const uint64_t padded = (len + ALIGN - 1) / ALIGN * ALIGN;
+  const uint32_t* src = reinterpret_cast<const uint32_t*>(scratch + i * slot);
+  uint32_t* dst = reinterpret_cast<uint32_t*>(out + off);  // 4-byte aligned: HEAD, ALIGN multiples of 4
+  const uint64_t full = len / 4;
+#pragma unroll 4
+  for (uint64_t w = threadIdx.x; w < full; w += 256) dst[w] = src[w];
+  for (uint64_t w = full + threadIdx.x; w < padded / 4; w += 256) {
+    const uint64_t b0 = 4 * w;  // keep the stream's bytes, zero the padding
+    dst[w] = b0 < len ? src[w] & ((1u << (8 * (len - b0))) - 1u) : 0u;
   }
 }
 
@@ -422,13 +615,7 @@ uint64_t slot_of(int codec, uint64_t chunk_bytes, int e) {
 template <int CODEC, typename T>
 void launch_encode(const uint8_t* in, uint64_t in_bytes, uint64_t chunk, uint64_t n, uint8_t* scratch, uint64_t slot,
                    uint64_t* lens, cudaStream_t s) {
-  if constexpr (CODEC == CODAG_CODEC_RLEV2) {
-    k_encode_rlev2_warp<T><<<static_cast<unsigned>((n + kEncWarps - 1) / kEncWarps), 32 * kEncWarps, 0, s>>>(
-        in, in_bytes, chunk, n, scratch, slot, lens);
-  } else {
-    k_encode_rlev1_warp<T><<<static_cast<unsigned>((n + kEncWarps - 1) / kEncWarps), 32 * kEncWarps, 0, s>>>(
-        in, in_bytes, chunk, n, scratch, slot, lens);
-  }
+  k_encode<CODEC, T><<<static_cast<unsigned>(n), 32 * kEncWarps, 0, s>>>(in, in_bytes, chunk, scratch, slot, lens);
 }
 
 template <int CODEC>
@@ -456,9 +643,8 @@ codag_status compress(const uint8_t* d_in, uint64_t in_bytes, uint64_t chunk, in
   constexpr uint64_t A = CODEC == CODAG_CODEC_RLEV1 ? 4 : 128;  // encoder.h:780-783 / encoder_trans.h:352
   constexpr uint32_t H = CODEC == CODAG_CODEC_RLEV1 ? 8 : 0;    // rlev1.h:103-192: [u64 size][streams]
   k_scan_offsets<A><<<1, 1024, 0, s>>>(lens, n, d_blk_off, d_status);
-  const uint64_t blocks = (n + 7) / 8;
-  k_gather<A, H><<<static_cast<unsigned>(blocks < 4096 ? blocks : 4096), 256, 0, s>>>(
-      scratch, slot, lens, n, d_out, capacity, d_blk_off, d_col_len, in_bytes, d_out_bytes, d_status);
+  k_gather<A, H><<<static_cast<unsigned>(n), 256, 0, s>>>(scratch, slot, lens, n, d_out, capacity, d_blk_off, d_col_len,
+                                                          in_bytes, d_out_bytes, d_status);
   if (CODEC == CODAG_CODEC_RLEV2) k_set_last_offset<<<1, 1, 0, s>>>(d_blk_off, n, in_bytes);  // encoder_trans.h:545
   return cudaGetLastError() == cudaSuccess ? CODAG_OK : CODAG_ECUDA;
 }
