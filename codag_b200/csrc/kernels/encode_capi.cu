@@ -19,11 +19,11 @@
 //     literals, in groups of 127.
 //   RLE v2: from p, the first three equal values in a row within 128 values start a fixed run, which
 //     goes on for at most 128 values; what lies before them, else 128 values, is a variable group.
-// So a CTA first writes the comparisons of kTile values as bit masks, in parallel; then one warp
-// walks the items, a search for a set bit each; then all warps encode the items, one warp per
-// item, eight at a time, each with its size first and its bytes once the sizes of the
-// others are known.  With one warp per chunk running the state machine, an item cost about 9000 warp
-// instructions and a chunk had one warp to wait for.
+// So a CTA takes kTile values at a time into shared memory and writes their comparisons as bit masks,
+// in parallel; one warp walks the items, a search for a set bit each; then the warps measure the
+// items, one warp per item, the CTA sums the sizes, and the warps write the items' bytes.  With one
+// warp per chunk running the state machine, an item cost about 9000 warp instructions and a
+// chunk had one warp to wait for.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -31,7 +31,7 @@
 
 #include "../../../include/codag.h"
 #include "../rlev2_widths.h"
-#include "device_common.cuh"
+#include "capi_common.cuh"
 
 using namespace codag_dev;
 
@@ -67,19 +67,23 @@ struct Wide<uint32_t> { using T = unsigned int; };
 template <>
 struct Wide<uint64_t> { using T = unsigned long long; };
 
-constexpr uint32_t kEncWarps = 8;
-constexpr uint32_t kTile = 4096;             // values whose items are found at a time
-constexpr uint32_t kMaskWords = kTile / 32 + 5;  // and the 129 values an item may reach beyond them
-constexpr uint32_t kItems = kTile / 2 + 64;  // a literal between runs of three: two items per four values
+constexpr uint32_t kTile = 2048;                 // values whose items are found at a time
+constexpr uint32_t kAhead = 160;                 // values of an item beyond them (at most 129)
+constexpr uint32_t kMaskWords = (kTile + kAhead) / 32;
+constexpr uint32_t kItems = kTile / 2 + 64;      // a literal between runs of three: two items per four values
 
+template <typename T, uint32_t WARPS, bool V1>
 struct EncodeShared {
+  T val[kTile + kAhead];
   uint32_t a[kMaskWords];  // RLE v1: a run starts here; RLE v2: the third of three equal values
   uint32_t b[kMaskWords];  // RLE v1: the step to the next value equals the one after; RLE v2: equals the value before
   uint32_t item[kItems];   // start (12 bits), values (8 bits), run (1 bit)
+  uint32_t off[kItems];    // size, then offset in the tile's bytes
+  uint32_t how[V1 ? 1 : kItems];  // RLE v2: see ItemV2::pack
   uint32_t items, next;
-  uint32_t size[2][kEncWarps];
-  uint32_t hist[kEncWarps][32];
-  uint64_t val[kEncWarps][128], list[kEncWarps][128];  // PATCHED_BASE: reduced values, patch list
+  uint32_t part[WARPS];
+  uint32_t hist[V1 ? 1 : WARPS][32];
+  uint64_t red[V1 ? 1 : WARPS][128], list[V1 ? 1 : WARPS][32];  // PATCHED_BASE: reduced values, patch list
 };
 
 // bytes of one stream; what passes the slot's end is dropped (and reported by the stream's length)
@@ -105,16 +109,24 @@ __device__ __forceinline__ uint64_t max64(uint64_t v) {
 }
 __device__ __forceinline__ uint64_t min64(uint64_t v) { return ~max64(~v); }
 
-// position of the first set bit of `mask` (xor `flip`) at or after `from`, if it lies within 31 words;
-// else kFar, which is past everything but leaves room for sums
+// position past everything that leaves room for sums
 constexpr uint32_t kFar = 1u << 30;
-__device__ __forceinline__ uint32_t first_set(const uint32_t* mask, uint32_t flip, uint32_t from, uint32_t lane) {
-  const uint32_t w = from / 32u + lane;
-  uint32_t v = w < kMaskWords ? mask[w] ^ flip : FULL;
-  if (lane == 0) v &= FULL << (from & 31u);
-  const uint32_t f = __ffs(__ballot_sync(FULL, v != 0));
-  return f ? (from / 32u + f - 1u) * 32u + __ffs(__shfl_sync(FULL, v, f - 1u)) - 1u : kFar;
-}
+
+// 32 words of a mask, one per lane, from word `base`
+struct MaskWindow {
+  uint32_t v, base, lane;
+  __device__ __forceinline__ void load(const uint32_t* mask, uint32_t flip, uint32_t at) {
+    base = at;
+    v = base + lane < kMaskWords ? mask[base + lane] ^ flip : FULL;
+  }
+  // the first set bit at or after `from`, or kFar if the window has none
+  __device__ __forceinline__ uint32_t first(uint32_t from) const {
+    const uint32_t w = from / 32u - base;
+    const uint32_t x = lane < w ? 0u : lane == w ? v & (FULL << (from & 31u)) : v;
+    const uint32_t f = __ffs(__ballot_sync(FULL, x != 0));
+    return f ? (base + f - 1u) * 32u + __ffs(__shfl_sync(FULL, x, f - 1u)) - 1u : kFar;
+  }
+};
 
 // step from one value to the next as the writer computes it: in the type's own arithmetic, so never
 // negative for 32-bit values, and as an int for narrower ones
@@ -138,52 +150,42 @@ __device__ __forceinline__ uint32_t varint_byte(uint64_t v, uint32_t k, uint32_t
 // --- RLE v1 items ---------------------------------------------------------------------------------
 template <typename T>
 struct ItemV1 {
-  static constexpr uint32_t kRunMax = 129, kLitMax = 127;
-  T v[4];  // value 32 q + lane (a run needs the first two only)
-  uint32_t n, size;
-  bool run;
-  uint32_t at[4];  // literals: offset of each value's bytes
+  static constexpr uint32_t kWarps = 16;
+  using Shared = EncodeShared<T, kWarps, true>;
 
-  template <class Get>
-  __device__ __forceinline__ void measure(const Get& get, uint64_t start, uint32_t count, bool is_run, EncodeShared&, uint32_t,
-                                          uint32_t lane) {
-    n = count;
-    run = is_run;
-    if (run) {
-      v[0] = static_cast<T>(get(start));
-      v[1] = static_cast<T>(get(start + 1));
-      size = 2u + varint_len(v[0]);
-      return;
-    }
-    uint32_t sum = 1;
+  static __device__ __forceinline__ uint32_t measure(const T* v, uint32_t n, bool run, Shared&, uint32_t, uint32_t,
+                                                     uint32_t lane) {
+    if (run) return 2u + varint_len(v[0]);
+    uint32_t sum = 0;
 #pragma unroll
-    for (uint32_t q = 0; q < 4; q++) {
-      const uint32_t i = 32u * q + lane;
-      v[q] = i < n ? static_cast<T>(get(start + i)) : T(0);
-      const uint32_t len = i < n ? varint_len(v[q]) : 0u;
-      const uint32_t s = scan_add(len, lane);
-      at[q] = sum + s - len;
-      sum += __shfl_sync(FULL, s, 31);
-    }
-    size = sum;
+    for (uint32_t q = 0; q < 4; q++)
+      if (32u * q + lane < n) sum += varint_len(v[32u * q + lane]);
+    return 1u + __reduce_add_sync(FULL, sum);
   }
-  __device__ __forceinline__ void write(const Slot& out, uint64_t off, EncodeShared&, uint32_t, uint32_t lane) const {
+  static __device__ __forceinline__ void write(const T* v, uint32_t n, bool run, const Slot& out, uint64_t off, Shared&,
+                                               uint32_t, uint32_t, uint32_t lane) {
     if (run) {
-      if (lane < size) {
+      const uint32_t len = varint_len(v[0]);
+      if (lane < 2u + len) {
         const uint32_t b = lane == 0 ? n - 3u
                            : lane == 1 ? static_cast<uint32_t>(step_of<T>(v[0], v[1]))
-                                       : varint_byte(v[0], lane - 2u, size - 2u);
+                                       : varint_byte(v[0], lane - 2u, len);
         out.put(off + lane, b);
       }
       return;
     }
     if (lane == 0) out.put(off, 0u - n);
+    off++;
 #pragma unroll
     for (uint32_t q = 0; q < 4; q++) {
-      if (32u * q + lane < n) {
-        const uint32_t len = varint_len(v[q]);
-        for (uint32_t k = 0; k < len; k++) out.put(off + at[q] + k, varint_byte(v[q], k, len));
-      }
+      if (32u * q >= n) break;
+      const bool on = 32u * q + lane < n;
+      const T x = on ? v[32u * q + lane] : T(0);
+      const uint32_t len = on ? varint_len(x) : 0u;
+      const uint32_t upto = scan_add(len, lane);
+      const uint64_t at = off + (upto - len);
+      for (uint32_t k = 0; k < len; k++) out.put(at + k, varint_byte(x, k, len));
+      off += __shfl_sync(FULL, upto, 31);
     }
   }
 };
@@ -191,11 +193,24 @@ struct ItemV1 {
 // --- RLE v2 items (the choices are those of RleV2Writer, ../rle_writers.h) ------------------------------
 template <typename T>
 struct ItemV2 {
+  static constexpr uint32_t kWarps = 8;
+  using Shared = EncodeShared<T, kWarps, false>;
   enum : uint32_t { kShortRepeat, kDirect, kDeltaFixed, kDelta, kPatched };
   uint64_t v[4];   // value 32 q + lane
   uint64_t first, second, lmin;
   uint32_t n, size, kind, bits;
-  uint32_t b95, pwidth, npatch, gap_width;
+  uint32_t pwidth, npatch, gap_width;  // kPatched, whose `bits` is the width of the reduced values
+
+  __device__ __forceinline__ uint32_t pack() const {
+    return kind | (bits << 3) | (kind == kPatched ? (pwidth << 10) | (npatch << 17) | (gap_width << 25) : 0u);
+  }
+  __device__ __forceinline__ void unpack(uint32_t p) {
+    kind = p & 7u;
+    bits = (p >> 3) & 127u;
+    pwidth = (p >> 10) & 127u;
+    npatch = (p >> 17) & 255u;
+    gap_width = p >> 25;
+  }
 
   // suffix sums of the histogram of width codes: lane c has the number of values of code c and above
   template <class D>
@@ -229,27 +244,28 @@ struct ItemV2 {
     size = 2u + aligned_bytes(n, bits);
   }
 
-  template <class Get>
-  __device__ __forceinline__ void measure(const Get& get, uint64_t start, uint32_t count, bool is_run, EncodeShared& sh,
-                                          uint32_t warp, uint32_t lane) {
+  __device__ __forceinline__ void load(const T* val, uint32_t count, uint32_t lane) {
     n = count;
+#pragma unroll
+    for (uint32_t q = 0; q < 4; q++) v[q] = 32u * q + lane < n ? static_cast<uint64_t>(val[32u * q + lane]) : 0ull;
+    first = val[0];
+    second = val[n > 1u ? 1 : 0];
+  }
+
+  __device__ __forceinline__ void choose(bool is_run, Shared& sh, uint32_t warp, uint32_t lane) {
+    bits = 0;
     if (is_run && n < 128u) {  // a fixed run that ended before the limit
-      first = second = get(start);
       const uint32_t nb = (width_of(first) - 1u) / 8u + 1u;
       kind = n <= 10u ? kShortRepeat : kDeltaFixed;
       size = n <= 10u ? 1u + nb : 3u + varint_len(first);
       return;
     }
-#pragma unroll
-    for (uint32_t q = 0; q < 4; q++) v[q] = 32u * q + lane < n ? static_cast<uint64_t>(get(start + 32u * q + lane)) : 0ull;
     uint32_t* hist = sh.hist[warp];
     const auto value = [&](uint32_t q) { return v[q]; };
     if (n <= 3u) {
       set_direct(code_suffix(value, hist, lane));
       return;
     }
-    first = shfl64(v[0], 0);
-    second = shfl64(v[0], 1);
     const uint64_t initial = second - first;
     uint64_t lo = first, hi = first, md = 0;
     bool inc = true, dec = true, fix = true;
@@ -295,7 +311,7 @@ struct ItemV2 {
       return;
     }
     const uint32_t reduced = code_suffix([&](uint32_t q) { return v[q] - lmin; }, hist, lane);
-    b95 = percentile(reduced, 95);
+    uint32_t b95 = percentile(reduced, 95);
     const uint32_t r100 = percentile(reduced, 100);
     if (r100 == b95) {
       set_direct(plain);
@@ -309,31 +325,53 @@ struct ItemV2 {
       pwidth = 56u;
       b95 = 8u;
     }
+    bits = b95;
     const uint64_t mask = (1ull << b95) - 1ull;
-    uint32_t before = 0, max_gap = 0;
+    uint32_t max_gap = 0;
+    npatch = 0;
+    int32_t prev_pos = -1;
+#pragma unroll
+    for (uint32_t q = 0; q < 4; q++) {
+      const uint32_t bq = __ballot_sync(FULL, 32u * q + lane < n && v[q] - lmin > mask);
+      for (uint32_t m = bq; m; m &= m - 1u) {
+        const int32_t pos = static_cast<int32_t>(32u * q + __ffs(m) - 1u);
+        const uint32_t gap = static_cast<uint32_t>(pos - (prev_pos >= 0 ? prev_pos : 0));
+        max_gap = max_gap > gap ? max_gap : gap;
+        prev_pos = pos;
+      }
+      npatch += __popc(bq);
+    }
+    gap_width = max_gap == 0 && npatch != 0 ? 1u : width_of(max_gap);
+    size = 4u + base_bytes() + aligned_bytes(n, bits) + aligned_bytes(npatch, v2_closest(gap_width + pwidth));
+  }
+
+  // reduced values and patch list of a PATCHED_BASE group, into shared memory
+  __device__ __forceinline__ void stage_patched(Shared& sh, uint32_t warp, uint32_t lane) {
+    uint64_t lo = first;
+#pragma unroll
+    for (uint32_t q = 0; q < 4; q++)
+      if (32u * q + lane < n) lo = v[q] < lo ? v[q] : lo;
+    lmin = min64(lo);
+    const uint64_t mask = (1ull << bits) - 1ull;
+    uint32_t before = 0;
     int32_t prev_pos = -1;
     __syncwarp();
 #pragma unroll
     for (uint32_t q = 0; q < 4; q++) {
       const uint32_t i = 32u * q + lane;
       const uint64_t r = i < n ? v[q] - lmin : 0ull;
-      if (i < n) sh.val[warp][i] = r & mask;
+      if (i < n) sh.red[warp][i] = r & mask;
       const bool hit = r > mask;
       const uint32_t bq = __ballot_sync(FULL, hit);
       if (hit) {
         const uint32_t below = bq & lanemask_lt(lane);
         const uint32_t prev = below ? 32u * q + 31u - __clz(below) : (prev_pos >= 0 ? static_cast<uint32_t>(prev_pos) : 0u);
-        sh.list[warp][before + __popc(below)] = (static_cast<uint64_t>(i - prev) << pwidth) | (r >> b95);
-        max_gap = max_gap > i - prev ? max_gap : i - prev;
+        sh.list[warp][before + __popc(below)] = (static_cast<uint64_t>(i - prev) << pwidth) | (r >> bits);
       }
       if (bq) prev_pos = static_cast<int32_t>(32u * q + 31u - __clz(bq));
       before += __popc(bq);
     }
     __syncwarp();
-    npatch = before;
-    max_gap = __reduce_max_sync(FULL, max_gap);
-    gap_width = max_gap == 0 && npatch != 0 ? 1u : width_of(max_gap);
-    size = 4u + base_bytes() + aligned_bytes(n, b95) + aligned_bytes(npatch, v2_closest(gap_width + pwidth));
   }
   __device__ __forceinline__ uint32_t base_bytes() const { return width_of(lmin) / 8u + 1u; }
 
@@ -374,15 +412,16 @@ struct ItemV2 {
     }
   }
 
-  __device__ __forceinline__ void write(const Slot& out, uint64_t off, EncodeShared& sh, uint32_t warp, uint32_t lane) const {
+  __device__ __forceinline__ void put_item(const Slot& out, uint64_t off, Shared& sh, uint32_t warp, uint32_t lane) {
     const uint32_t len = n - 1u;
     if (kind == kShortRepeat) {
-      if (lane == 0) out.put(off, ((size - 2u) << 3) | (n - 3u));
-      else if (lane < size) out.put(off + lane, static_cast<uint32_t>(first >> (8u * (size - 1u - lane))));
+      const uint32_t nb = (width_of(first) - 1u) / 8u + 1u;
+      if (lane == 0) out.put(off, ((nb - 1u) << 3) | (n - 3u));
+      else if (lane <= nb) out.put(off + lane, static_cast<uint32_t>(first >> (8u * (nb - lane))));
       return;
     }
     const uint32_t top = kind == kDirect ? 0x40u : kind == kPatched ? 0x80u : 0xC0u;
-    const uint32_t code = kind == kDeltaFixed ? 0u : v2_code(kind == kPatched ? b95 : bits);
+    const uint32_t code = kind == kDeltaFixed ? 0u : v2_code(bits);
     if (lane == 0) out.put(off, top | (code << 1) | ((len >> 8) & 1u));
     if (lane == 1) out.put(off + 1, len);
     off += 2;
@@ -391,14 +430,15 @@ struct ItemV2 {
       return;
     }
     if (kind == kPatched) {
+      stage_patched(sh, warp, lane);
       const uint32_t nb = base_bytes(), w2 = v2_closest(gap_width + pwidth);
       if (lane == 0) out.put(off, ((nb - 1u) << 5) | v2_code(pwidth));
       if (lane == 1) out.put(off + 1, ((gap_width - 1u) << 5) | npatch);
       off += 2;
       if (lane < nb) out.put(off + lane, static_cast<uint32_t>(shr64(lmin, 8u * (nb - 1u - lane))));
       off += nb;
-      put_packed(out, off, sh.val[warp], n, b95, lane);
-      put_packed(out, off + aligned_bytes(n, b95), sh.list[warp], npatch, w2, lane);
+      put_packed(out, off, sh.red[warp], n, bits, lane);
+      put_packed(out, off + aligned_bytes(n, bits), sh.list[warp], npatch, w2, lane);
       return;
     }
     // DELTA: base and first step as varints, then the further steps unless they are all the same
@@ -423,44 +463,68 @@ struct ItemV2 {
     }
     put_aligned(out, off + l1 + l2, x, n - 2u, bits, lane);
   }
+
+  static __device__ __forceinline__ uint32_t measure(const T* val, uint32_t n, bool run, Shared& sh, uint32_t item,
+                                                     uint32_t warp, uint32_t lane) {
+    ItemV2 it;
+    it.load(val, n, lane);
+    it.choose(run, sh, warp, lane);
+    if (lane == 0) sh.how[item] = it.pack();
+    return it.size;
+  }
+  static __device__ __forceinline__ void write(const T* val, uint32_t n, bool, const Slot& out, uint64_t off, Shared& sh,
+                                               uint32_t item, uint32_t warp, uint32_t lane) {
+    ItemV2 it;
+    it.load(val, n, lane);
+    it.unpack(sh.how[item]);
+    it.put_item(out, off, sh, warp, lane);
+  }
 };
 
-// One CTA per chunk.  Bound by the latency of its serial parts (the walk, a barrier every eight
-// items); several CTAs per SM overlap theirs.
-template <int CODEC, typename T>
-__global__ void __launch_bounds__(32 * kEncWarps) k_encode(const uint8_t* __restrict__ in, uint64_t in_bytes,
-                                                          uint64_t chunk_bytes, uint8_t* __restrict__ scratch,
-                                                          uint64_t slot, uint64_t* __restrict__ lens) {
-  __shared__ EncodeShared sh;
-  constexpr bool V1 = CODEC == CODAG_CODEC_RLEV1;
-  using Item = std::conditional_t<V1, ItemV1<T>, ItemV2<T>>;
+// One CTA per chunk.  Bound by the latency of its serial part, the walk, and of the barriers around it;
+// several CTAs per SM overlap theirs.
+template <class Item, typename T, bool V1>
+__global__ void __launch_bounds__(32 * Item::kWarps) k_encode(const uint8_t* __restrict__ in, uint64_t in_bytes,
+                                                             uint64_t chunk_bytes, uint8_t* __restrict__ scratch,
+                                                             uint64_t slot, uint64_t* __restrict__ lens) {
+  constexpr uint32_t kWarps = Item::kWarps, kThreads = 32 * kWarps;
+  extern __shared__ __align__(16) uint8_t smem[];
+  auto& sh = *reinterpret_cast<typename Item::Shared*>(smem);
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint64_t chunk = blockIdx.x;
   const uint64_t n = chunk_bytes / sizeof(T);
   using W = typename Wide<T>::T;
-  const PaddedChunk<W> raw{in, in_bytes, chunk * chunk_bytes};
-  const auto get = [&](uint64_t i) { return static_cast<T>(raw(i)); };
+  const PaddedChunk<W> get{in, in_bytes, chunk * chunk_bytes};
   const Slot out{scratch + chunk * slot, slot};
   uint64_t base = 0;
-  uint32_t par = 0;
   for (uint64_t t0 = 0; t0 < n;) {
-    // comparisons of values t0 + b
-    for (uint32_t w = warp; w < kMaskWords; w += kEncWarps) {
-      const uint64_t j = t0 + 32u * w + lane;
+    const uint32_t end = static_cast<uint32_t>(n - t0 < kTile + kAhead ? n - t0 : kTile + kAhead);
+    {
+      T x[4];  // several loads in flight
+      for (uint32_t i = threadIdx.x; i < end; i += 4 * kThreads) {
+#pragma unroll
+        for (uint32_t k = 0; k < 4; k++)
+          if (i + k * kThreads < end) x[k] = static_cast<T>(get(t0 + i + k * kThreads));
+#pragma unroll
+        for (uint32_t k = 0; k < 4; k++)
+          if (i + k * kThreads < end) sh.val[i + k * kThreads] = x[k];
+      }
+    }
+    __syncthreads();
+    for (uint32_t w = warp; w < kMaskWords; w += kWarps) {  // comparisons of values t0 + j
+      const uint32_t j = 32u * w + lane;
       bool pa = false, pb = false;
       if constexpr (V1) {
-        if (j + 2 < n) {
-          const T x0 = get(j), x1 = get(j + 1), x2 = get(j + 2);
+        if (j + 2u < end) {
+          const T x0 = sh.val[j], x1 = sh.val[j + 1], x2 = sh.val[j + 2];
           const int64_t d = step_of<T>(x0, x1);
           pb = d == step_of<T>(x1, x2);
           pa = pb && d >= -128 && d <= 127;
         }
       } else {
-        const uint32_t b = 32u * w + lane;
-        if (b >= 1 && j < n) {
-          const T x0 = get(j), x1 = get(j - 1);
-          pb = x0 == x1;
-          pa = pb && b >= 2 && x1 == get(j - 2);
+        if (j >= 1u && j < end) {
+          pb = sh.val[j] == sh.val[j - 1];
+          pa = pb && j >= 2u && sh.val[j - 1] == sh.val[j - 2];
         }
       }
       const uint32_t ma = __ballot_sync(FULL, pa), mb = __ballot_sync(FULL, pb);
@@ -471,28 +535,34 @@ __global__ void __launch_bounds__(32 * kEncWarps) k_encode(const uint8_t* __rest
     }
     __syncthreads();
     if (warp == 0) {  // items that start in the tile
-      const uint32_t end = static_cast<uint32_t>(n - t0 < kTile + 256u ? n - t0 : kTile + 256u);
       uint32_t p = 0, items = 0;
+      MaskWindow a{0, 0, lane}, b{0, 0, lane};
+      a.load(sh.a, 0u, 0);
+      b.load(sh.b, FULL, 0);
       while (p < kTile && p < end) {
+        if (p / 32u > a.base + 26u) {  // an item reaches at most five words on
+          a.load(sh.a, 0u, p / 32u);
+          b.load(sh.b, FULL, p / 32u);
+        }
         uint32_t count, run = 0;
         if constexpr (V1) {
-          const uint32_t r = first_set(sh.a, 0u, p, lane);
+          const uint32_t r = a.first(p);
           if (r == p) {
-            const uint32_t z = first_set(sh.b, FULL, p, lane) - p + 2u;
-            count = z < Item::kRunMax ? z : Item::kRunMax;
+            const uint32_t z = b.first(p) - p + 2u;
+            count = z < 129u ? z : 129u;
             run = 1;
           } else {
             const uint32_t stop = r < end ? r : end;
-            count = stop - p < Item::kLitMax ? stop - p : Item::kLitMax;
+            count = stop - p < 127u ? stop - p : 127u;
           }
         } else {
-          const uint32_t j = first_set(sh.a, 0u, p + 2u, lane), lim = end - p < 128u ? end : p + 128u;
+          const uint32_t j = a.first(p + 2u), lim = end - p < 128u ? end : p + 128u;
           if (j >= lim) {
             count = lim - p;
           } else if (j - 2u > p) {
             count = j - 2u - p;
           } else {
-            const uint32_t z = first_set(sh.b, FULL, p + 1u, lane);
+            const uint32_t z = b.first(p + 1u);
             const uint32_t stop = z < end ? z : end;
             count = stop - p < 128u ? stop - p : 128u;
             run = 1;
@@ -509,23 +579,31 @@ __global__ void __launch_bounds__(32 * kEncWarps) k_encode(const uint8_t* __rest
     }
     __syncthreads();
     const uint32_t items = sh.items, step = sh.next;
-    for (uint32_t r = 0; r < items; r += kEncWarps, par ^= 1u) {
-      Item it;
-      it.size = 0;
-      if (r + warp < items) {
-        const uint32_t d = sh.item[r + warp];
-        it.measure(get, t0 + (d & 0xfffu), (d >> 12) & 0xffu, (d >> 20) != 0, sh, warp, lane);
-      }
-      if (lane == 0) sh.size[par][warp] = it.size;
-      __syncthreads();
-      const uint32_t s = lane < kEncWarps ? sh.size[par][lane] : 0u;
-      const uint32_t upto = scan_add(s, lane);
-      const uint32_t before = __shfl_sync(FULL, upto - s, warp);
-      if (r + warp < items) it.write(out, base + before, sh, warp, lane);
-      base += __shfl_sync(FULL, upto, 31);
+    for (uint32_t i = warp; i < items; i += kWarps) {
+      const uint32_t d = sh.item[i];
+      const uint32_t size = Item::measure(sh.val + (d & 0xfffu), (d >> 12) & 0xffu, (d >> 20) != 0, sh, i, warp, lane);
+      if (lane == 0) sh.off[i] = size;
     }
+    __syncthreads();
+    // offsets: every warp sums its share of the items, then starts from the sums of the warps below
+    const uint32_t per = (items + kWarps - 1u) / kWarps, i0 = warp * per < items ? warp * per : items;
+    const uint32_t i1 = i0 + per < items ? i0 + per : items;
+    uint32_t sum = 0;
+    for (uint32_t i = i0 + lane; i < i1; i += 32) sum += sh.off[i];
+    sum = __reduce_add_sync(FULL, sum);
+    if (lane == 0) sh.part[warp] = sum;
+    __syncthreads();
+    const uint32_t mine = lane < kWarps ? sh.part[lane] : 0u;
+    uint32_t at = __reduce_add_sync(FULL, lane < warp ? mine : 0u);
+    const uint32_t total = __reduce_add_sync(FULL, mine);
+    for (uint32_t i = i0; i < i1; i++) {
+      const uint32_t d = sh.item[i], size = sh.off[i];
+      Item::write(sh.val + (d & 0xfffu), (d >> 12) & 0xffu, (d >> 20) != 0, out, base + at, sh, i, warp, lane);
+      at += size;
+    }
+    base += total;
     t0 += step;
-    __syncthreads();  // the masks and items are overwritten
+    __syncthreads();  // the tile's memory is overwritten
   }
   if (threadIdx.x == 0) lens[chunk] = base > slot ? kOverflow : base;
 }
@@ -613,9 +691,15 @@ uint64_t slot_of(int codec, uint64_t chunk_bytes, int e) {
 }
 
 template <int CODEC, typename T>
-void launch_encode(const uint8_t* in, uint64_t in_bytes, uint64_t chunk, uint64_t n, uint8_t* scratch, uint64_t slot,
+bool launch_encode(const uint8_t* in, uint64_t in_bytes, uint64_t chunk, uint64_t n, uint8_t* scratch, uint64_t slot,
                    uint64_t* lens, cudaStream_t s) {
-  k_encode<CODEC, T><<<static_cast<unsigned>(n), 32 * kEncWarps, 0, s>>>(in, in_bytes, chunk, scratch, slot, lens);
+  constexpr bool V1 = CODEC == CODAG_CODEC_RLEV1;
+  using Item = std::conditional_t<V1, ItemV1<T>, ItemV2<T>>;
+  auto kern = k_encode<Item, T, V1>;
+  constexpr uint32_t bytes = sizeof(typename Item::Shared);
+  if (codag_capi::allow_smem(kern, bytes) != cudaSuccess) return false;
+  kern<<<static_cast<unsigned>(n), 32 * Item::kWarps, bytes, s>>>(in, in_bytes, chunk, scratch, slot, lens);
+  return true;
 }
 
 template <int CODEC>
@@ -634,12 +718,14 @@ codag_status compress(const uint8_t* d_in, uint64_t in_bytes, uint64_t chunk, in
   uint8_t* scratch = static_cast<uint8_t*>(ws);
   uint64_t* lens = reinterpret_cast<uint64_t*>(scratch + n * slot);
   if (d_status && cudaMemsetAsync(d_status, 0, sizeof(int32_t), s) != cudaSuccess) return CODAG_ECUDA;
+  bool ok;
   switch (e) {
-    case 8: launch_encode<CODEC, uint64_t>(d_in, in_bytes, chunk, n, scratch, slot, lens, s); break;
-    case 4: launch_encode<CODEC, uint32_t>(d_in, in_bytes, chunk, n, scratch, slot, lens, s); break;
-    case 2: launch_encode<CODEC, uint16_t>(d_in, in_bytes, chunk, n, scratch, slot, lens, s); break;
-    default: launch_encode<CODEC, uint8_t>(d_in, in_bytes, chunk, n, scratch, slot, lens, s); break;
+    case 8: ok = launch_encode<CODEC, uint64_t>(d_in, in_bytes, chunk, n, scratch, slot, lens, s); break;
+    case 4: ok = launch_encode<CODEC, uint32_t>(d_in, in_bytes, chunk, n, scratch, slot, lens, s); break;
+    case 2: ok = launch_encode<CODEC, uint16_t>(d_in, in_bytes, chunk, n, scratch, slot, lens, s); break;
+    default: ok = launch_encode<CODEC, uint8_t>(d_in, in_bytes, chunk, n, scratch, slot, lens, s); break;
   }
+  if (!ok) return CODAG_ECUDA;
   constexpr uint64_t A = CODEC == CODAG_CODEC_RLEV1 ? 4 : 128;  // encoder.h:780-783 / encoder_trans.h:352
   constexpr uint32_t H = CODEC == CODAG_CODEC_RLEV1 ? 8 : 0;    // rlev1.h:103-192: [u64 size][streams]
   k_scan_offsets<A><<<1, 1024, 0, s>>>(lens, n, d_blk_off, d_status);
