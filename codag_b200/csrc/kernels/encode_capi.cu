@@ -11,7 +11,7 @@
 // Nothing is allocated; a stream that overruns its workspace slot, or a file larger than the
 // caller's output capacity, is reported in *d_status.
 //
-// Both writers (../rle_writers.h, which the host producers run) look like state machines over
+// The host producers' writers (../rle_writers.h) look like state machines over
 // the values, but where their items (a run, a group of literals) begin and end depends only on
 // where the last one ended and on comparisons of neighbouring values:
 //   RLE v1: a run starts at p if its first step is in [-128, 127] and the next step equals it; it
@@ -19,11 +19,13 @@
 //     literals, in groups of 127.
 //   RLE v2: from p, the first three equal values in a row within 128 values start a fixed run, which
 //     goes on for at most 128 values; what lies before them, else 128 values, is a variable group.
-// So a CTA takes kTile values at a time into shared memory and writes their comparisons as bit masks,
-// in parallel; one warp walks the items, a search for a set bit each; then the warps measure the
-// items, one warp per item, the CTA sums the sizes, and the warps write the items' bytes.  With one
-// warp per chunk running the state machine, an item cost about 9000 warp instructions and a
-// chunk had one warp to wait for.
+// So a CTA's front warps take kTile values at a time into shared memory and write their comparisons as
+// bit masks, then the length that an item starting at each of the values would have, all in parallel;
+// one lane follows the lengths from item to item (searching the masks there instead took 480 cycles
+// an item).  Meanwhile
+// the back warps measure the items of the tile before, one warp per item, sum the sizes, and write
+// the items' bytes.  With one warp per chunk running the state machine, an item cost about 9000 warp
+// instructions and a chunk had one warp to wait for.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -72,27 +74,38 @@ constexpr uint32_t kAhead = 160;                 // values of an item beyond the
 constexpr uint32_t kMaskWords = (kTile + kAhead) / 32;
 constexpr uint32_t kItems = kTile / 2 + 64;      // a literal between runs of three: two items per four values
 
-template <typename T, uint32_t WARPS, bool V1>
-struct EncodeShared {
+// one tile: its values, comparisons and items
+template <typename T>
+struct EncodeTile {
   T val[kTile + kAhead];
   uint32_t a[kMaskWords];  // RLE v1: a run starts here; RLE v2: the third of three equal values
   uint32_t b[kMaskWords];  // RLE v1: the step to the next value equals the one after; RLE v2: equals the value before
+  uint16_t len[kTile];     // values of an item that starts here, and whether it is a run (bit 8)
   uint32_t item[kItems];   // start (12 bits), values (8 bits), run (1 bit)
-  uint32_t off[kItems];    // size, then offset in the tile's bytes
-  uint32_t how[V1 ? 1 : kItems];  // RLE v2: see ItemV2::pack
-  uint32_t items, next;
-  uint32_t part[WARPS];
-  uint32_t hist[V1 ? 1 : WARPS][32];
-  uint64_t red[V1 ? 1 : WARPS][128], list[V1 ? 1 : WARPS][32];  // PATCHED_BASE: reduced values, patch list
+  uint32_t items;
+  uint64_t next;           // first value of the tile after
 };
 
-// bytes of one stream; what passes the slot's end is dropped (and reported by the stream's length)
-struct Slot {
+template <typename T, uint32_t FRONT, uint32_t BACK, bool V1>
+struct EncodeShared {
+  static constexpr uint32_t kFront = FRONT, kBack = BACK;
+  EncodeTile<T> tile[2];
+  uint32_t off[kItems];           // size of each item, then offset in the tile's bytes
+  uint32_t how[V1 ? 1 : kItems];  // RLE v2: see ItemV2::pack
+  uint32_t part[BACK];
+  uint32_t hist[V1 ? 1 : BACK][32];
+  uint64_t red[V1 ? 1 : BACK][128], list[V1 ? 1 : BACK][32];  // PATCHED_BASE: reduced values, patch list
+};
+
+template <uint32_t ID, uint32_t WARPS>
+__device__ __forceinline__ void group_barrier() {
+  asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(32 * WARPS) : "memory");
+}
+
+// bytes of one item, which lies inside its slot
+struct Bytes {
   uint8_t* p;
-  uint64_t cap;
-  __device__ __forceinline__ void put(uint64_t at, uint32_t b) const {
-    if (at < cap) p[at] = static_cast<uint8_t>(b);
-  }
+  __device__ __forceinline__ void put(uint32_t at, uint32_t b) const { p[at] = static_cast<uint8_t>(b); }
 };
 
 __device__ __forceinline__ uint32_t scan_add(uint32_t v, uint32_t lane) {  // inclusive
@@ -112,21 +125,20 @@ __device__ __forceinline__ uint64_t min64(uint64_t v) { return ~max64(~v); }
 // position past everything that leaves room for sums
 constexpr uint32_t kFar = 1u << 30;
 
-// 32 words of a mask, one per lane, from word `base`
-struct MaskWindow {
-  uint32_t v, base, lane;
-  __device__ __forceinline__ void load(const uint32_t* mask, uint32_t flip, uint32_t at) {
-    base = at;
-    v = base + lane < kMaskWords ? mask[base + lane] ^ flip : FULL;
+// Distance from bit 32 w + lane + skip (skip at most 2) of `mask` (xor `flip`) to the first set bit at or
+// after it, if that lies within five words; else kFar.
+__device__ __forceinline__ uint32_t distance_to_set(const uint32_t* mask, uint32_t flip, uint32_t w, uint32_t skip,
+                                                    uint32_t lane) {
+  const uint64_t two = (static_cast<uint64_t>(mask[w + 1] ^ flip) << 32) | (mask[w] ^ flip);
+  const uint64_t x = two >> (lane + skip);
+  uint32_t far = kFar;
+#pragma unroll
+  for (uint32_t k = 5; k >= 2; k--) {
+    const uint32_t v = mask[w + k] ^ flip;
+    if (v) far = 32u * k + __ffs(v) - 1u;
   }
-  // the first set bit at or after `from`, or kFar if the window has none
-  __device__ __forceinline__ uint32_t first(uint32_t from) const {
-    const uint32_t w = from / 32u - base;
-    const uint32_t x = lane < w ? 0u : lane == w ? v & (FULL << (from & 31u)) : v;
-    const uint32_t f = __ffs(__ballot_sync(FULL, x != 0));
-    return f ? (base + f - 1u) * 32u + __ffs(__shfl_sync(FULL, x, f - 1u)) - 1u : kFar;
-  }
-};
+  return x ? static_cast<uint32_t>(__ffsll(static_cast<long long>(x))) - 1u : far - (lane + skip);
+}
 
 // step from one value to the next as the writer computes it: in the type's own arithmetic, so never
 // negative for 32-bit values, and as an int for narrower ones
@@ -150,8 +162,7 @@ __device__ __forceinline__ uint32_t varint_byte(uint64_t v, uint32_t k, uint32_t
 // --- RLE v1 items ---------------------------------------------------------------------------------
 template <typename T>
 struct ItemV1 {
-  static constexpr uint32_t kWarps = 16;
-  using Shared = EncodeShared<T, kWarps, true>;
+  using Shared = EncodeShared<T, 8, 8, true>;
 
   static __device__ __forceinline__ uint32_t measure(const T* v, uint32_t n, bool run, Shared&, uint32_t, uint32_t,
                                                      uint32_t lane) {
@@ -162,8 +173,9 @@ struct ItemV1 {
       if (32u * q + lane < n) sum += varint_len(v[32u * q + lane]);
     return 1u + __reduce_add_sync(FULL, sum);
   }
-  static __device__ __forceinline__ void write(const T* v, uint32_t n, bool run, const Slot& out, uint64_t off, Shared&,
-                                               uint32_t, uint32_t, uint32_t lane) {
+  static __device__ __forceinline__ void write(const T* v, uint32_t n, bool run, const Bytes& out, Shared&, uint32_t,
+                                               uint32_t, uint32_t lane) {
+    uint32_t off = 0;
     if (run) {
       const uint32_t len = varint_len(v[0]);
       if (lane < 2u + len) {
@@ -183,7 +195,7 @@ struct ItemV1 {
       const T x = on ? v[32u * q + lane] : T(0);
       const uint32_t len = on ? varint_len(x) : 0u;
       const uint32_t upto = scan_add(len, lane);
-      const uint64_t at = off + (upto - len);
+      const uint32_t at = off + (upto - len);
       for (uint32_t k = 0; k < len; k++) out.put(at + k, varint_byte(x, k, len));
       off += __shfl_sync(FULL, upto, 31);
     }
@@ -193,8 +205,7 @@ struct ItemV1 {
 // --- RLE v2 items (the choices are those of RleV2Writer, ../rle_writers.h) ------------------------------
 template <typename T>
 struct ItemV2 {
-  static constexpr uint32_t kWarps = 8;
-  using Shared = EncodeShared<T, kWarps, false>;
+  using Shared = EncodeShared<T, 4, 12, false>;
   enum : uint32_t { kShortRepeat, kDirect, kDeltaFixed, kDelta, kPatched };
   uint64_t v[4];   // value 32 q + lane
   uint64_t first, second, lmin;
@@ -212,15 +223,19 @@ struct ItemV2 {
     gap_width = p >> 25;
   }
 
-  // suffix sums of the histogram of width codes: lane c has the number of values of code c and above
-  template <class D>
-  __device__ __forceinline__ uint32_t code_suffix(const D& d, uint32_t* hist, uint32_t lane) const {
+  // suffix sums of the histogram of the width codes of the values less `sub`: lane c has the number of
+  // values of code c and above.  Out of line, as are the packers: the kernel waits for instructions
+  // more than for anything else.
+  static __device__ __noinline__ uint32_t code_suffix(uint64_t v0, uint64_t v1, uint64_t v2, uint64_t v3, uint64_t sub,
+                                                      uint32_t n, uint32_t* hist) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t v[4] = {v0, v1, v2, v3};
     __syncwarp();
     hist[lane] = 0;
     __syncwarp();
 #pragma unroll
     for (uint32_t q = 0; q < 4; q++)
-      if (32u * q + lane < n) atomicAdd(&hist[v2_code(width_of(d(q)))], 1u);
+      if (32u * q + lane < n) atomicAdd(&hist[v2_code(width_of(v[q] - sub))], 1u);
     __syncwarp();
     const uint32_t c = hist[lane];
     return n - (scan_add(c, lane) - c);
@@ -261,9 +276,9 @@ struct ItemV2 {
       return;
     }
     uint32_t* hist = sh.hist[warp];
-    const auto value = [&](uint32_t q) { return v[q]; };
+    const auto suffix = [&](uint64_t sub) { return code_suffix(v[0], v[1], v[2], v[3], sub, n, hist); };
     if (n <= 3u) {
-      set_direct(code_suffix(value, hist, lane));
+      set_direct(suffix(0));
       return;
     }
     const uint64_t initial = second - first;
@@ -290,7 +305,7 @@ struct ItemV2 {
     const uint64_t lmax = max64(hi);
     // subtracting the minimum is taken for unsafe only for a minimum of 0 and a maximum up to 128
     if (!(lmin > 0 || lmax > 128u)) {
-      set_direct(code_suffix(value, hist, lane));
+      set_direct(suffix(0));
       return;
     }
     if (__all_sync(FULL, fix)) {
@@ -305,12 +320,12 @@ struct ItemV2 {
       size = 2u + varint_len(first) + varint_len(zigzag(initial)) + aligned_bytes(n - 2u, bits);
       return;
     }
-    const uint32_t plain = code_suffix(value, hist, lane);
+    const uint32_t plain = suffix(0);
     if (percentile(plain, 100) - percentile(plain, 90) <= 1u) {
       set_direct(plain);
       return;
     }
-    const uint32_t reduced = code_suffix([&](uint32_t q) { return v[q] - lmin; }, hist, lane);
+    const uint32_t reduced = suffix(lmin);
     uint32_t b95 = percentile(reduced, 95);
     const uint32_t r100 = percentile(reduced, 100);
     if (r100 == b95) {
@@ -375,16 +390,21 @@ struct ItemV2 {
   }
   __device__ __forceinline__ uint32_t base_bytes() const { return width_of(lmin) / 8u + 1u; }
 
-  // x[q] is element 32 q + lane, at an aligned width, most significant bit first
-  __device__ __forceinline__ void put_aligned(const Slot& out, uint64_t off, const uint64_t* x, uint32_t count, uint32_t w,
-                                              uint32_t lane) const {
+  // x0..x3 are elements lane, 32 + lane, ...; at an aligned width, most significant bit first
+  static __device__ __noinline__ void put_aligned(uint8_t* out, uint64_t x0, uint64_t x1, uint64_t x2, uint64_t x3,
+                                                  uint32_t count, uint32_t w) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t x[4] = {x0, x1, x2, x3};
     if (w >= 8u) {
       const uint32_t nb = w / 8u;
 #pragma unroll
       for (uint32_t q = 0; q < 4; q++) {
         const uint32_t i = 32u * q + lane;
-        if (i < count)
-          for (uint32_t j = 0; j < nb; j++) out.put(off + i * nb + j, static_cast<uint32_t>(x[q] >> (8u * (nb - 1u - j))));
+        if (i < count) {
+          uint8_t* p = out + i * nb + nb;
+          uint64_t y = x[q];
+          for (uint32_t j = 0; j < nb; j++, y >>= 8) *--p = static_cast<uint8_t>(y);
+        }
       }
       return;
     }
@@ -394,25 +414,24 @@ struct ItemV2 {
       const uint32_t i = 32u * q + lane;
       uint32_t b = i < count ? (static_cast<uint32_t>(x[q]) & ((1u << w) - 1u)) << (8u - (i % per + 1u) * w) : 0u;
       for (uint32_t d = 1; d < per; d <<= 1) b |= __shfl_xor_sync(FULL, b, d);
-      if (i < count && i % per == 0) out.put(off + i / per, b);
+      if (i < count && i % per == 0) out[i / per] = static_cast<uint8_t>(b);
     }
   }
   // `count` values of w bits from shared memory, most significant bit first
-  static __device__ __forceinline__ void put_packed(const Slot& out, uint64_t off, const uint64_t* x, uint32_t count,
-                                                    uint32_t w, uint32_t lane) {
+  static __device__ __noinline__ void put_packed(uint8_t* out, const uint64_t* x, uint32_t count, uint32_t w) {
     const uint32_t tb = count * w;
-    for (uint32_t s = 8u * lane; s < tb; s += 256u) {
+    for (uint32_t s = 8u * (threadIdx.x & 31u); s < tb; s += 256u) {
       const uint32_t e = s + 8u < tb ? s + 8u : tb;
       uint32_t byte = 0;
       for (uint32_t i = s / w; i * w < e; i++) {
         const uint32_t vs = i * w, ve = vs + w, a = vs > s ? vs : s, b = ve < e ? ve : e;
         byte |= (static_cast<uint32_t>(x[i] >> (ve - b)) & ((1u << (b - a)) - 1u)) << (s + 8u - b);
       }
-      out.put(off + s / 8u, byte);
+      out[s / 8u] = static_cast<uint8_t>(byte);
     }
   }
 
-  __device__ __forceinline__ void put_item(const Slot& out, uint64_t off, Shared& sh, uint32_t warp, uint32_t lane) {
+  __device__ __forceinline__ void put_item(const Bytes& out, uint32_t off, Shared& sh, uint32_t warp, uint32_t lane) {
     const uint32_t len = n - 1u;
     if (kind == kShortRepeat) {
       const uint32_t nb = (width_of(first) - 1u) / 8u + 1u;
@@ -426,7 +445,7 @@ struct ItemV2 {
     if (lane == 1) out.put(off + 1, len);
     off += 2;
     if (kind == kDirect) {
-      put_aligned(out, off, v, n, bits, lane);
+      put_aligned(out.p + off, v[0], v[1], v[2], v[3], n, bits);
       return;
     }
     if (kind == kPatched) {
@@ -437,8 +456,8 @@ struct ItemV2 {
       off += 2;
       if (lane < nb) out.put(off + lane, static_cast<uint32_t>(shr64(lmin, 8u * (nb - 1u - lane))));
       off += nb;
-      put_packed(out, off, sh.red[warp], n, bits, lane);
-      put_packed(out, off + aligned_bytes(n, bits), sh.list[warp], npatch, w2, lane);
+      put_packed(out.p + off, sh.red[warp], n, bits);
+      put_packed(out.p + off + aligned_bytes(n, bits), sh.list[warp], npatch, w2);
       return;
     }
     // DELTA: base and first step as varints, then the further steps unless they are all the same
@@ -461,7 +480,7 @@ struct ItemV2 {
       const uint64_t next = q < 3 ? shfl64(d[q + 1], (lane + 2u) & 31u) : 0ull;
       x[q] = lane < 30u ? here : next;
     }
-    put_aligned(out, off + l1 + l2, x, n - 2u, bits, lane);
+    put_aligned(out.p + off + l1 + l2, x[0], x[1], x[2], x[3], n - 2u, bits);
   }
 
   static __device__ __forceinline__ uint32_t measure(const T* val, uint32_t n, bool run, Shared& sh, uint32_t item,
@@ -472,208 +491,204 @@ struct ItemV2 {
     if (lane == 0) sh.how[item] = it.pack();
     return it.size;
   }
-  static __device__ __forceinline__ void write(const T* val, uint32_t n, bool, const Slot& out, uint64_t off, Shared& sh,
-                                               uint32_t item, uint32_t warp, uint32_t lane) {
+  static __device__ __forceinline__ void write(const T* val, uint32_t n, bool, const Bytes& out, Shared& sh, uint32_t item,
+                                               uint32_t warp, uint32_t lane) {
     ItemV2 it;
     it.load(val, n, lane);
     it.unpack(sh.how[item]);
-    it.put_item(out, off, sh, warp, lane);
+    it.put_item(out, 0, sh, warp, lane);
   }
 };
 
-// One CTA per chunk.  Bound by the latency of its serial part, the walk, and of the barriers around it;
-// several CTAs per SM overlap theirs.
+// Front warps: the tile whose first value is t0.
+template <bool V1, typename T, uint32_t FRONT, class Get>
+__device__ __forceinline__ void prepare_tile(EncodeTile<T>& t, const Get& get, uint64_t t0, uint64_t n, uint32_t warp,
+                                             uint32_t lane) {
+  const uint32_t end = static_cast<uint32_t>(n - t0 < kTile + kAhead ? n - t0 : kTile + kAhead);
+  constexpr uint32_t kStep = 32 * FRONT;
+  for (uint32_t i = 32u * warp + lane; i < end; i += 8 * kStep) {
+    T x[8];  // several loads in flight
+#pragma unroll
+    for (uint32_t k = 0; k < 8; k++)
+      if (i + k * kStep < end) x[k] = static_cast<T>(get(t0 + i + k * kStep));
+#pragma unroll
+    for (uint32_t k = 0; k < 8; k++)
+      if (i + k * kStep < end) t.val[i + k * kStep] = x[k];
+  }
+  group_barrier<1, FRONT>();
+#pragma unroll 2
+  for (uint32_t w = warp; w < kMaskWords; w += FRONT) {  // comparisons of values t0 + j
+    const uint32_t j = 32u * w + lane;
+    bool pa = false, pb = false;
+    if constexpr (V1) {
+      if (j + 2u < end) {
+        const T x0 = t.val[j], x1 = t.val[j + 1], x2 = t.val[j + 2];
+        const int64_t d = step_of<T>(x0, x1);
+        pb = d == step_of<T>(x1, x2);
+        pa = pb && d >= -128 && d <= 127;
+      }
+    } else {
+      if (j >= 1u && j < end) {
+        pb = t.val[j] == t.val[j - 1];
+        pa = pb && j >= 2u && t.val[j - 1] == t.val[j - 2];
+      }
+    }
+    const uint32_t ma = __ballot_sync(FULL, pa), mb = __ballot_sync(FULL, pb);
+    if (lane == 0) {
+      t.a[w] = ma;
+      t.b[w] = mb;
+    }
+  }
+  group_barrier<1, FRONT>();
+  for (uint32_t w = warp; w < kTile / 32u; w += FRONT) {  // the item that would start at p
+    const uint32_t p = 32u * w + lane, left = p < end ? end - p : 0u;
+    uint32_t len, run;
+    if constexpr (V1) {
+      const uint32_t r = distance_to_set(t.a, 0u, w, 0, lane), z = distance_to_set(t.b, FULL, w, 0, lane) + 2u;
+      run = r == 0u;
+      len = run ? (z < 129u ? z : 129u) : (r < 127u ? r : 127u);
+    } else {
+      const uint32_t r = distance_to_set(t.a, 0u, w, 2, lane), z = distance_to_set(t.b, FULL, w, 1, lane) + 1u;
+      run = r == 0u;
+      len = run ? (z < 128u ? z : 128u) : (r < 126u ? r : 128u);
+    }
+    t.len[p] = static_cast<uint16_t>((len < left ? len : left) | (run << 8));
+  }
+  group_barrier<1, FRONT>();
+  if (warp != 0 || lane != 0) return;
+  uint32_t p = 0, items = 0;  // items that start in the tile
+  while (p < kTile && p < end) {
+    const uint32_t v = t.len[p];
+    t.item[items++] = p | (v << 12);
+    p += v & 0xffu;
+  }
+  t.items = items;
+  t.next = t0 + p;
+}
+
+// One CTA per chunk.  Bound by the latency of the front's walk and of the back's longest items.
 template <class Item, typename T, bool V1>
-__global__ void __launch_bounds__(32 * Item::kWarps) k_encode(const uint8_t* __restrict__ in, uint64_t in_bytes,
-                                                             uint64_t chunk_bytes, uint8_t* __restrict__ scratch,
-                                                             uint64_t slot, uint64_t* __restrict__ lens) {
-  constexpr uint32_t kWarps = Item::kWarps, kThreads = 32 * kWarps;
+__global__ void __launch_bounds__(32 * (Item::Shared::kFront + Item::Shared::kBack), 2)
+    k_encode(const uint8_t* __restrict__ in, uint64_t in_bytes, uint64_t chunk_bytes, uint8_t* __restrict__ scratch,
+             uint64_t slot, uint64_t* __restrict__ lens) {
+  constexpr uint32_t kFront = Item::Shared::kFront, kBack = Item::Shared::kBack;
   extern __shared__ __align__(16) uint8_t smem[];
   auto& sh = *reinterpret_cast<typename Item::Shared*>(smem);
-  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t lane = threadIdx.x & 31u;
+  const bool front = threadIdx.x < 32u * kFront;
+  const uint32_t warp = (threadIdx.x >> 5) - (front ? 0u : kFront);
   const uint64_t chunk = blockIdx.x;
   const uint64_t n = chunk_bytes / sizeof(T);
   using W = typename Wide<T>::T;
   const PaddedChunk<W> get{in, in_bytes, chunk * chunk_bytes};
-  const Slot out{scratch + chunk * slot, slot};
-  uint64_t base = 0;
-  for (uint64_t t0 = 0; t0 < n;) {
-    const uint32_t end = static_cast<uint32_t>(n - t0 < kTile + kAhead ? n - t0 : kTile + kAhead);
-    {
-      T x[4];  // several loads in flight
-      for (uint32_t i = threadIdx.x; i < end; i += 4 * kThreads) {
-#pragma unroll
-        for (uint32_t k = 0; k < 4; k++)
-          if (i + k * kThreads < end) x[k] = static_cast<T>(get(t0 + i + k * kThreads));
-#pragma unroll
-        for (uint32_t k = 0; k < 4; k++)
-          if (i + k * kThreads < end) sh.val[i + k * kThreads] = x[k];
+  uint8_t* out = scratch + chunk * slot;
+  uint64_t base = 0, ready = 0;  // bytes written; first value of the tile to prepare
+  bool have = false;             // the back has a tile
+  for (uint32_t c = 0; ready < n || have; c ^= 1u) {
+    if (front) {
+      if (ready < n) prepare_tile<V1, T, kFront>(sh.tile[c], get, ready, n, warp, lane);
+    } else if (have) {
+      const EncodeTile<T>& t = sh.tile[c ^ 1u];
+      const uint32_t items = t.items;
+      for (uint32_t i = warp; i < items; i += kBack) {
+        const uint32_t d = t.item[i];
+        const uint32_t size = Item::measure(t.val + (d & 0xfffu), (d >> 12) & 0xffu, (d >> 20) != 0, sh, i, warp, lane);
+        if (lane == 0) sh.off[i] = size;
       }
+      group_barrier<2, kBack>();
+      // every warp sums its share of the items, then starts from the sums of the warps below
+      const uint32_t per = (items + kBack - 1u) / kBack, i0 = warp * per < items ? warp * per : items;
+      const uint32_t i1 = i0 + per < items ? i0 + per : items;
+      uint32_t sum = 0;
+      for (uint32_t i = i0 + lane; i < i1; i += 32) sum += sh.off[i];
+      sum = __reduce_add_sync(FULL, sum);
+      if (lane == 0) sh.part[warp] = sum;
+      group_barrier<2, kBack>();
+      const uint32_t mine = lane < kBack ? sh.part[lane] : 0u;
+      uint32_t at = __reduce_add_sync(FULL, lane < warp ? mine : 0u);
+      const uint32_t total = __reduce_add_sync(FULL, mine);
+      for (uint32_t i = i0; i < i1; i++) {
+        const uint32_t d = t.item[i], size = sh.off[i];
+        if (base + at + size <= slot)  // else the stream's length will say that it did not fit
+          Item::write(t.val + (d & 0xfffu), (d >> 12) & 0xffu, (d >> 20) != 0, Bytes{out + base + at}, sh, i, warp, lane);
+        at += size;
+      }
+      base += total;
     }
     __syncthreads();
-    for (uint32_t w = warp; w < kMaskWords; w += kWarps) {  // comparisons of values t0 + j
-      const uint32_t j = 32u * w + lane;
-      bool pa = false, pb = false;
-      if constexpr (V1) {
-        if (j + 2u < end) {
-          const T x0 = sh.val[j], x1 = sh.val[j + 1], x2 = sh.val[j + 2];
-          const int64_t d = step_of<T>(x0, x1);
-          pb = d == step_of<T>(x1, x2);
-          pa = pb && d >= -128 && d <= 127;
-        }
-      } else {
-        if (j >= 1u && j < end) {
-          pb = sh.val[j] == sh.val[j - 1];
-          pa = pb && j >= 2u && sh.val[j - 1] == sh.val[j - 2];
-        }
-      }
-      const uint32_t ma = __ballot_sync(FULL, pa), mb = __ballot_sync(FULL, pb);
-      if (lane == 0) {
-        sh.a[w] = ma;
-        sh.b[w] = mb;
-      }
-    }
-    __syncthreads();
-    if (warp == 0) {  // items that start in the tile
-      uint32_t p = 0, items = 0;
-      MaskWindow a{0, 0, lane}, b{0, 0, lane};
-      a.load(sh.a, 0u, 0);
-      b.load(sh.b, FULL, 0);
-      while (p < kTile && p < end) {
-        if (p / 32u > a.base + 26u) {  // an item reaches at most five words on
-          a.load(sh.a, 0u, p / 32u);
-          b.load(sh.b, FULL, p / 32u);
-        }
-        uint32_t count, run = 0;
-        if constexpr (V1) {
-          const uint32_t r = a.first(p);
-          if (r == p) {
-            const uint32_t z = b.first(p) - p + 2u;
-            count = z < 129u ? z : 129u;
-            run = 1;
-          } else {
-            const uint32_t stop = r < end ? r : end;
-            count = stop - p < 127u ? stop - p : 127u;
-          }
-        } else {
-          const uint32_t j = a.first(p + 2u), lim = end - p < 128u ? end : p + 128u;
-          if (j >= lim) {
-            count = lim - p;
-          } else if (j - 2u > p) {
-            count = j - 2u - p;
-          } else {
-            const uint32_t z = b.first(p + 1u);
-            const uint32_t stop = z < end ? z : end;
-            count = stop - p < 128u ? stop - p : 128u;
-            run = 1;
-          }
-        }
-        if (lane == 0) sh.item[items] = p | (count << 12) | (run << 20);
-        items++;
-        p += count;
-      }
-      if (lane == 0) {
-        sh.items = items;
-        sh.next = p;
-      }
-    }
-    __syncthreads();
-    const uint32_t items = sh.items, step = sh.next;
-    for (uint32_t i = warp; i < items; i += kWarps) {
-      const uint32_t d = sh.item[i];
-      const uint32_t size = Item::measure(sh.val + (d & 0xfffu), (d >> 12) & 0xffu, (d >> 20) != 0, sh, i, warp, lane);
-      if (lane == 0) sh.off[i] = size;
-    }
-    __syncthreads();
-    // offsets: every warp sums its share of the items, then starts from the sums of the warps below
-    const uint32_t per = (items + kWarps - 1u) / kWarps, i0 = warp * per < items ? warp * per : items;
-    const uint32_t i1 = i0 + per < items ? i0 + per : items;
-    uint32_t sum = 0;
-    for (uint32_t i = i0 + lane; i < i1; i += 32) sum += sh.off[i];
-    sum = __reduce_add_sync(FULL, sum);
-    if (lane == 0) sh.part[warp] = sum;
-    __syncthreads();
-    const uint32_t mine = lane < kWarps ? sh.part[lane] : 0u;
-    uint32_t at = __reduce_add_sync(FULL, lane < warp ? mine : 0u);
-    const uint32_t total = __reduce_add_sync(FULL, mine);
-    for (uint32_t i = i0; i < i1; i++) {
-      const uint32_t d = sh.item[i], size = sh.off[i];
-      Item::write(sh.val + (d & 0xfffu), (d >> 12) & 0xffu, (d >> 20) != 0, out, base + at, sh, i, warp, lane);
-      at += size;
-    }
-    base += total;
-    t0 += step;
-    __syncthreads();  // the tile's memory is overwritten
+    have = ready < n;
+    if (have) ready = sh.tile[c].next;
   }
-  if (threadIdx.x == 0) lens[chunk] = base > slot ? kOverflow : base;
+  if (threadIdx.x == 32u * kFront) lens[chunk] = base > slot ? kOverflow : base;
 }
 
-// blk_off[i] = sum of round_up(lens[k], ALIGN) for k < i, blk_off[n] = the total; one CTA of
-// 1024 threads, each summing a contiguous range.
 template <uint64_t ALIGN>
-__global__ void __launch_bounds__(1024) k_scan_offsets(const uint64_t* __restrict__ lens, uint64_t n,
+__device__ __forceinline__ uint64_t round_up(uint64_t len) {
+  return (len + ALIGN - 1) / ALIGN * ALIGN;
+}
+
+// blk_off[i] = sum of round_up(lens[k], ALIGN) for k < i, and blk_off[n] = the total or, for RLE v2,
+// the original size (encoder_trans.h:545); one CTA of 1024 threads, each summing a contiguous range.
+template <uint64_t ALIGN, bool LAST_IS_SIZE>
+__global__ void __launch_bounds__(1024) k_scan_offsets(const uint64_t* __restrict__ lens, uint64_t n, uint64_t in_bytes,
                                                        uint64_t* __restrict__ blk_off, int32_t* __restrict__ status) {
-  __shared__ uint64_t part[1024];
-  __shared__ int bad;
-  const uint32_t t = threadIdx.x;
-  if (t == 0) bad = 0;
-  const uint64_t per = (n + 1023) / 1024, a = t * per, b = a + per < n ? a + per : n;
+  __shared__ uint64_t part[32];
+  const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+  const uint64_t per = (n + 1023) / 1024, a = t * per < n ? t * per : n, b = a + per < n ? a + per : n;
   uint64_t s = 0;
+  bool over = false;
   for (uint64_t i = a; i < b; i++) {
-    const uint64_t l = lens[i];
-    if (l == kOverflow) bad = 1;
-    s += (l + ALIGN - 1) / ALIGN * ALIGN;
+    over |= lens[i] == kOverflow;
+    s += round_up<ALIGN>(lens[i]);
   }
-  part[t] = s;
-  __syncthreads();
-  for (uint32_t d = 1; d < 1024; d <<= 1) {  // inclusive scan of the partial sums
-    const uint64_t o = t >= d ? part[t - d] : 0;
-    __syncthreads();
-    part[t] += o;
-    __syncthreads();
-  }
-  uint64_t run = part[t] - s;
+  const uint64_t upto = warp_scan_add64(s, lane);
+  if (lane == 31) part[warp] = upto;
+  const int bad = __syncthreads_or(over);
+  const uint64_t below = warp_scan_add64(part[lane], lane);  // of the warps up to `lane`
+  uint64_t run = upto - s + (warp ? shfl64(below, static_cast<int>(warp) - 1) : 0);
   for (uint64_t i = a; i < b; i++) {
     blk_off[i] = run;
-    run += (lens[i] + ALIGN - 1) / ALIGN * ALIGN;
+    run += round_up<ALIGN>(lens[i]);
   }
-  if (t == 1023) blk_off[n] = part[1023];
-  if (t == 0 && bad && status) *status = CODAG_ECORRUPT;
+  const uint64_t total = shfl64(below, 31);
+  if (t == 0) {
+    blk_off[n] = LAST_IS_SIZE ? in_bytes : total;
+    if (status) *status = bad ? CODAG_ECORRUPT : CODAG_OK;
+  }
 }
 
-// One CTA per chunk: stream i goes to out + head + blk_off[i] and is zero padded to ALIGN
-// bytes.  RLE v1 (head 8): the blob starts with the original size.  RLE v2: blk_off[n] is
-// overwritten with the original size.  The file is out_bytes = head + blk_off[n] long.
+// Stream i = blockIdx.x, or one of gridDim.y shares of it, goes to out + head + blk_off[i] and is zero
+// padded to ALIGN bytes.  RLE v1 (head 8): the blob starts with the original size.
 template <uint64_t ALIGN, uint32_t HEAD>
 __global__ void __launch_bounds__(256) k_gather(const uint8_t* __restrict__ scratch, uint64_t slot,
                                                 const uint64_t* __restrict__ lens, uint64_t n, uint8_t* __restrict__ out,
                                                 uint64_t capacity, const uint64_t* __restrict__ blk_off,
                                                 uint64_t* __restrict__ col_len, uint64_t in_bytes,
                                                 uint64_t* __restrict__ out_bytes, int32_t* __restrict__ status) {
-  const uint64_t total = HEAD + blk_off[n];
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
+  const uint64_t total = HEAD + blk_off[n - 1] + round_up<ALIGN>(lens[n - 1]);
+  const uint64_t i = blockIdx.x;
+  const bool first = threadIdx.x == 0 && blockIdx.y == 0;
+  if (first && i == 0) {
     if (out_bytes) *out_bytes = total;
     if (total > capacity && status) *status = CODAG_ELIMIT;
     if (HEAD == 8 && capacity >= 8) *reinterpret_cast<uint64_t*>(out) = in_bytes;
   }
   if (total > capacity) return;
-  const uint64_t i = blockIdx.x;
   const uint64_t len = lens[i], off = HEAD + blk_off[i];
-  if (threadIdx.x == 0) col_len[i] = len;
+  if (first) col_len[i] = len;
   if (len == kOverflow) return;
-  const uint64_t padded = (len + ALIGN - 1) / ALIGN * ALIGN;
+  const uint64_t words = round_up<ALIGN>(len) / 4, full = len / 4;
   const uint32_t* src = reinterpret_cast<const uint32_t*>(scratch + i * slot);
   uint32_t* dst = reinterpret_cast<uint32_t*>(out + off);  // 4-byte aligned: HEAD, ALIGN multiples of 4
-  const uint64_t full = len / 4;
+  const uint64_t share = (words + gridDim.y - 1) / gridDim.y, w0 = blockIdx.y * share;
+  const uint64_t w1 = w0 + share < words ? w0 + share : words, wf = w1 < full ? w1 : full;
 #pragma unroll 4
-  for (uint64_t w = threadIdx.x; w < full; w += 256) dst[w] = src[w];
-  for (uint64_t w = full + threadIdx.x; w < padded / 4; w += 256) {
+  for (uint64_t w = w0 + threadIdx.x; w < wf; w += 256) dst[w] = src[w];
+  for (uint64_t w = (w0 > full ? w0 : full) + threadIdx.x; w < w1; w += 256) {
     const uint64_t b0 = 4 * w;  // keep the stream's bytes, zero the padding
     dst[w] = b0 < len ? src[w] & ((1u << (8 * (len - b0))) - 1u) : 0u;
   }
 }
-
-__global__ void k_set_last_offset(uint64_t* blk_off, uint64_t n, uint64_t in_bytes) { blk_off[n] = in_bytes; }
 
 bool valid_elem(int e) { return e == 1 || e == 2 || e == 4 || e == 8; }
 
@@ -698,7 +713,7 @@ bool launch_encode(const uint8_t* in, uint64_t in_bytes, uint64_t chunk, uint64_
   auto kern = k_encode<Item, T, V1>;
   constexpr uint32_t bytes = sizeof(typename Item::Shared);
   if (codag_capi::allow_smem(kern, bytes) != cudaSuccess) return false;
-  kern<<<static_cast<unsigned>(n), 32 * Item::kWarps, bytes, s>>>(in, in_bytes, chunk, scratch, slot, lens);
+  kern<<<static_cast<unsigned>(n), 32 * (Item::Shared::kFront + Item::Shared::kBack), bytes, s>>>(in, in_bytes, chunk, scratch, slot, lens);
   return true;
 }
 
@@ -717,7 +732,6 @@ codag_status compress(const uint8_t* d_in, uint64_t in_bytes, uint64_t chunk, in
   (void)cudaGetLastError();  // an error earlier work left pending is not this call's
   uint8_t* scratch = static_cast<uint8_t*>(ws);
   uint64_t* lens = reinterpret_cast<uint64_t*>(scratch + n * slot);
-  if (d_status && cudaMemsetAsync(d_status, 0, sizeof(int32_t), s) != cudaSuccess) return CODAG_ECUDA;
   bool ok;
   switch (e) {
     case 8: ok = launch_encode<CODEC, uint64_t>(d_in, in_bytes, chunk, n, scratch, slot, lens, s); break;
@@ -728,10 +742,11 @@ codag_status compress(const uint8_t* d_in, uint64_t in_bytes, uint64_t chunk, in
   if (!ok) return CODAG_ECUDA;
   constexpr uint64_t A = CODEC == CODAG_CODEC_RLEV1 ? 4 : 128;  // encoder.h:780-783 / encoder_trans.h:352
   constexpr uint32_t H = CODEC == CODAG_CODEC_RLEV1 ? 8 : 0;    // rlev1.h:103-192: [u64 size][streams]
-  k_scan_offsets<A><<<1, 1024, 0, s>>>(lens, n, d_blk_off, d_status);
-  k_gather<A, H><<<static_cast<unsigned>(n), 256, 0, s>>>(scratch, slot, lens, n, d_out, capacity, d_blk_off, d_col_len,
-                                                          in_bytes, d_out_bytes, d_status);
-  if (CODEC == CODAG_CODEC_RLEV2) k_set_last_offset<<<1, 1, 0, s>>>(d_blk_off, n, in_bytes);  // encoder_trans.h:545
+  constexpr bool V2 = CODEC == CODAG_CODEC_RLEV2;
+  k_scan_offsets<A, V2><<<1, 1024, 0, s>>>(lens, n, in_bytes, d_blk_off, d_status);
+  // eight CTAs a chunk where one each would leave SMs idle
+  k_gather<A, H><<<dim3(static_cast<unsigned>(n), n < 1024 ? 8 : 1), 256, 0, s>>>(
+      scratch, slot, lens, n, d_out, capacity, d_blk_off, d_col_len, in_bytes, d_out_bytes, d_status);
   return cudaGetLastError() == cudaSuccess ? CODAG_OK : CODAG_ECUDA;
 }
 

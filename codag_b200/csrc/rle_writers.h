@@ -1,5 +1,5 @@
-// ORC RLE v1 and RLE v2 chunk writers, shared by the host producers (host/encode_rle*.cpp) and
-// the GPU encoders (kernels/encode_capi.cu), so both emit the same bytes.
+// ORC RLE v1 and RLE v2 chunk writers of the host producers (host/encode_rle*.cpp).  The GPU encoders
+// (kernels/encode_capi.cu) make the same choices item by item, so both emit the same bytes.
 //
 // RleV1Writer produces the byte stream of CODAG's encoder include/rlev1/encoder.h:1352-1695
 // (compression_warp_orig, driven by deflate_orig :1800-1840).  Format, one stream per chunk:
@@ -35,23 +35,14 @@
 
 namespace codag_fmt {
 
-// The RLE v1 writer's bulk steps: none when one thread runs the writer (host producers).  A warp
-// whose lanes all run the writer on the same values (the GPU encoder) supplies lane(), ballot(),
-// shuffles and an exclusive sum, and takes the values of a literal stream or of a run going on
-// many at a time (RleV1Writer::bulk).
-struct SerialV1 {
-  static constexpr bool kBulk = false;
-};
-
-template <typename T, class Sink, class G = SerialV1>
+template <typename T, class Sink>
 class RleV1Writer {
  public:
-  CODAG_HD explicit RleV1Writer(Sink& out) : out_(out) {}
-  CODAG_HD RleV1Writer(Sink& out, const G& g) : out_(out), g_(g) {}
+  explicit RleV1Writer(Sink& out) : out_(out) {}
 
   // n >= 2 values, value i read as get(i)
   template <class Get>
-  CODAG_HD void encode(const Get& get, uint64_t n) {
+  void encode(const Get& get, uint64_t n) {
     // first value
     uint64_t i = 0;
     T x = get(i++);
@@ -80,13 +71,6 @@ class RleV1Writer {
     held_++;
 
     for (; i < n; i++) {
-      if constexpr (G::kBulk) {
-        const uint32_t took = bulk(get, i, n);
-        if (took) {
-          i += took - 1;  // the loop's increment moves to the first value not taken
-          continue;
-        }
-      }
       if (lit_n_ == 127) close_literals();
       x = get(i);
 
@@ -196,90 +180,10 @@ class RleV1Writer {
   }
 
  private:
-  // Values i, i+1, ... (at most one per lane) that take the same steps as the value before them:
-  // in a run going on (three or more values, step in range), values that continue it, while the
-  // run stays below 130 values; in a literal stream (one value held), values whose step from the
-  // one before is out of range, each writing the value before it as a literal.  The steps are
-  // the per-value ones of encode() below, done for all taken values at once; returns the count
-  // (0: encode() takes value i).
-  template <class Get>
-  CODAG_HD uint32_t bulk(const Get& get, uint64_t i, uint64_t n) {
-    const uint32_t lane = g_.lane();
-    const uint64_t j = i + lane;
-    const bool in = j < n;
-    const T x = in ? static_cast<T>(get(j)) : T(0);
-    T before = g_.template shfl_up<T>(x);
-    if (lane == 0) before = prev_;
-    uint32_t take;
-    if (run_len_ >= 3 && in_run_) {
-      const uint32_t stop = g_.ballot(!(in && before + step_ == x));
-      take = stop ? g_.ffs(stop) - 1u : 32u;
-      const uint32_t room = 129u - run_len_;  // the value making 130 writes the run (encode())
-      if (take > room) take = room;
-      if (!take) return 0;
-      run_len_ = static_cast<uint16_t>(run_len_ + take);
-      held_ = static_cast<uint8_t>(held_ + take < 2 ? held_ + take : 2);
-    } else if (run_len_ == 1) {
-      const int64_t d = static_cast<int64_t>(x - before);
-      const uint32_t stop = g_.ballot(!(in && (d > 127 || d < -128)));
-      take = stop ? g_.ffs(stop) - 1u : 32u;
-      if (!take) return 0;
-      // literal k writes `before`; a group header goes before literal k when L0 + k is a multiple
-      // of 127 (at most once in 32 literals): a close of the full group and an open, or only an
-      // open when nothing was pending
-      const uint32_t l0 = lit_n_;
-      const uint32_t ev = l0 == 0 ? 0u : (127u - l0) % 127u;  // literal index of the header
-      const bool has_ev = ev < take;
-      const bool mine = lane < take;
-      const uint32_t hdr = (mine && has_ev && lane == ev) ? 1u : 0u;
-      uint32_t vlen = 0;
-      if (mine) {
-        T w = before;
-        do {
-          vlen++;
-          w = static_cast<T>(w >> 7);
-        } while (w != 0);
-      }
-      const uint32_t at = g_.excl_sum(hdr + vlen);
-      const uint32_t total = g_.template shfl<uint32_t>(at + hdr + vlen, 31);
-      if (has_ev && l0 != 0) out_.set(lit_hdr_, static_cast<uint8_t>(static_cast<int8_t>(-127)));
-      if (mine) {
-        uint32_t p = at;
-        if (hdr) out_.put_at(p++, 1);  // the placeholder open_literals(1) writes
-        T w = before;
-        do {
-          int8_t b = static_cast<int8_t>(w & 0x7F);
-          if ((w & (~0x7f)) != 0) b = static_cast<int8_t>(b | 0x80);
-          out_.put_at(p++, static_cast<uint8_t>(b));
-          w = static_cast<T>(w >> 7);
-        } while (w != 0);
-      }
-      if (has_ev) {
-        lit_hdr_ = out_.size() + g_.template shfl<uint32_t>(at, static_cast<int>(ev));
-        lit_n_ = static_cast<uint16_t>(take - ev);
-      } else {
-        lit_n_ = static_cast<uint16_t>(l0 + take);
-      }
-      out_.advance(total);
-      in_run_ = false;
-    } else {
-      return 0;
-    }
-    // the last two values taken become the history (push_hist per value)
-    const T last = g_.template shfl<T>(x, static_cast<int>(take - 1));
-    const T second = take >= 2 ? g_.template shfl<T>(x, static_cast<int>(take - 2)) : prev_;
-    head_ = static_cast<uint8_t>(head_ ^ (take & 1u));
-    hist_[head_ ^ 1] = last;
-    hist_[head_] = second;
-    prev_ = last;
-    g_.sync();
-    return take;
-  }
-
-  CODAG_HD void put(uint8_t b) { out_.put(b); }
+  void put(uint8_t b) { out_.put(b); }
 
   // unsigned LEB128 in the element type's arithmetic (encoder.h:839-853)
-  CODAG_HD void put_varint(T val) {
+  void put_varint(T val) {
     T w = val;
     do {
       int8_t b = static_cast<int8_t>(w & 0x7F);
@@ -289,23 +193,22 @@ class RleV1Writer {
     } while (w != 0);
   }
 
-  CODAG_HD void open_literals(uint8_t placeholder) {
+  void open_literals(uint8_t placeholder) {
     lit_hdr_ = out_.size();
     put(placeholder);
   }
 
-  CODAG_HD void close_literals() {
+  void close_literals() {
     out_.set(lit_hdr_, static_cast<uint8_t>(static_cast<int8_t>(-static_cast<int>(lit_n_))));
     lit_n_ = 0;
   }
 
-  CODAG_HD void push_hist(T x) {
+  void push_hist(T x) {
     hist_[head_] = x;
     head_ ^= 1;
   }
 
   Sink& out_;
-  G g_;
   T hist_[2] = {0, 0};
   uint8_t head_ = 0;
   uint8_t held_ = 0;
@@ -324,43 +227,23 @@ constexpr int kMinRepeat = 3;      // utils.h:65
 constexpr int kMaxShortRepeat = 10;
 
 // number of significant bits rounded up to a representable width (find_closes_num_bits)
-CODAG_HD uint8_t closest_width(uint64_t v) {
+inline uint8_t closest_width(uint64_t v) {
   // bits needed for v (0 for 0): a leading-zero count rather than a 64-step shift loop
-#if defined(__CUDA_ARCH__)
-  const uint32_t c = 64u - static_cast<uint32_t>(__clzll(static_cast<long long>(v)));
-#else
   const uint32_t c = v ? 64u - static_cast<uint32_t>(__builtin_clzll(v)) : 0u;
-#endif
   return static_cast<uint8_t>(v2_closest(c));
 }
 
-// The RLE v2 writer's work on a closed group of up to 128 pending values, run by one thread: the
-// host producers.  A warp can stand in for it (the GPU encoder, one warp per chunk): it keeps
-// the pending values and the patch list where all its lanes see them and splits each operation
-// over its lanes, while every lane runs the writer's decisions on the same data.
-struct SerialGroups {
-  // no bulk path: every value takes the writer's per-value steps (see RleV2Writer::encode)
-  static constexpr bool kBulk = false;
-  template <class Get>
-  CODAG_HD uint32_t append_run(const Get&, uint64_t, uint64_t, uint64_t*, uint32_t, uint64_t&, uint32_t) const {
-    return 0;
-  }
-  template <class Get>
-  CODAG_HD uint32_t append_equal(const Get&, uint64_t, uint64_t, uint64_t*, uint32_t, uint32_t) const {
-    return 0;
-  }
+// The RLE v2 writer's work on a closed group of up to 128 pending values.
+struct Groups {
   uint64_t lit[kMaxLiterals] = {};
   uint64_t list[kMaxLiterals];
-  CODAG_HD uint64_t* lits() { return lit; }
-  CODAG_HD uint64_t* lists() { return list; }
-
   struct Scan {
     uint64_t lmin, lmax, max_delta;
     bool increasing, decreasing, fixed;
   };
   // over l[0..n), n >= 2: extremes, monotonicity, whether every step equals the first, the largest
   // step (steps as unsigned differences)
-  CODAG_HD Scan scan(const uint64_t* l, uint32_t n) const {
+  Scan scan(const uint64_t* l, uint32_t n) const {
     Scan r{l[0], l[0], 0, true, true, true};
     const uint64_t initial = l[1] - l[0];
     for (uint32_t i = 1; i < n; i++) {
@@ -378,14 +261,14 @@ struct SerialGroups {
 
   // histogram of representable widths (compute_bit_width)
   template <class D>
-  CODAG_HD void hist(const D& d, uint32_t n, uint8_t* h) const {
+  void hist(const D& d, uint32_t n, uint8_t* h) const {
     for (int i = 0; i < 32; i++) h[i] = 0;
     for (uint32_t i = 0; i < n; ++i) h[v2_code(closest_width(d(i)))]++;
   }
 
   // fixed width big-endian packing used by DIRECT and DELTA (write_aligned_ints)
   template <class S, class D>
-  CODAG_HD void pack_aligned(S& out, const D& d, uint32_t n, uint8_t bits) const {
+  void pack_aligned(S& out, const D& d, uint32_t n, uint8_t bits) const {
     if (bits < 8) {
       const uint8_t mask = static_cast<uint8_t>((1 << bits) - 1);
       const uint32_t per_byte = 8 / bits;
@@ -415,7 +298,7 @@ struct SerialGroups {
 
   // MSB-first packing at any width (write_unaligned_ints)
   template <class S, class D>
-  CODAG_HD void pack_unaligned(S& out, const D& d, uint32_t n, uint8_t bits) const {
+  void pack_unaligned(S& out, const D& d, uint32_t n, uint8_t bits) const {
     uint32_t room = 8;
     uint8_t cur = 0;
     for (uint32_t i = 0; i < n; ++i) {
@@ -444,7 +327,7 @@ struct SerialGroups {
   // (gap << pwidth) | (value >> b95) per base-reduced value above mask, gaps from the previous
   // patched position (0 before the first); a group holds at most 128 values, so every gap is
   // below 256 and takes one entry.  Returns the entry count and the largest gap.
-  CODAG_HD uint32_t patches(const uint64_t* l, uint32_t n, uint64_t lmin, uint64_t mask, uint32_t b95,
+  uint32_t patches(const uint64_t* l, uint32_t n, uint64_t lmin, uint64_t mask, uint32_t b95,
                             uint32_t pwidth, uint64_t* out, uint64_t* max_gap) const {
     uint32_t np = 0;
     uint64_t prev = 0, mg = 0;
@@ -462,51 +345,18 @@ struct SerialGroups {
   }
 };
 
-template <class Sink, class G = SerialGroups>
+template <class Sink>
 class RleV2Writer {
  public:
-  CODAG_HD explicit RleV2Writer(Sink& out) : out_(out), lit_(g_.lits()) {}
-  // a group executor with its own storage (one warp per chunk)
-  CODAG_HD RleV2Writer(Sink& out, const G& g) : out_(out), g_(g), lit_(g_.lits()) {}
+  explicit RleV2Writer(Sink& out) : out_(out), lit_(g_.lit) {}
   RleV2Writer(const RleV2Writer&) = delete;  // lit_ points into g_
   RleV2Writer& operator=(const RleV2Writer&) = delete;
 
   // n values, value i read as get(i) (zero-extended to 64 bits)
   template <class Get>
-  CODAG_HD void encode(const Get& get, uint64_t n) {
+  void encode(const Get& get, uint64_t n) {
     uint64_t prev_delta = 0;
     for (uint64_t i = 0; i < n; i++) {
-      if constexpr (G::kBulk) {
-        // Inside a variable run (no fixed run pending, two or more values held) a value only
-        // appends to the pending values, until two zero steps in a row start a fixed run or the
-        // group reaches 128 values: the executor may take such values many at a time.
-        if (fix_ == 0 && nlit_ >= 2) {
-          const uint32_t lim_v = static_cast<uint32_t>(kMaxLiterals) - var_;
-          const uint32_t lim_n = static_cast<uint32_t>(kMaxLiterals) - nlit_;
-          const uint32_t took = g_.append_run(get, i, n, lit_, nlit_, prev_delta, lim_v < lim_n ? lim_v : lim_n);
-          if (took) {
-            nlit_ += took;
-            var_ += took;
-            if (var_ == static_cast<uint32_t>(kMaxLiterals)) choose_encoding();
-            i += took - 1;  // the loop's increment moves to the first value not taken
-            continue;
-          }
-        }
-        // Inside a fixed run (no variable values pending) a value equal to the last only appends,
-        // until the run reaches 128 values.
-        if (var_ == 0 && fix_ >= static_cast<uint32_t>(kMinRepeat) && prev_delta == 0 && nlit_ >= 1) {
-          const uint32_t lim_f = static_cast<uint32_t>(kMaxLiterals) - fix_;
-          const uint32_t lim_n = static_cast<uint32_t>(kMaxLiterals) - nlit_;
-          const uint32_t took = g_.append_equal(get, i, n, lit_, nlit_, lim_f < lim_n ? lim_f : lim_n);
-          if (took) {
-            nlit_ += took;
-            fix_ += took;
-            if (fix_ == static_cast<uint32_t>(kMaxLiterals)) choose_encoding();
-            i += took - 1;
-            continue;
-          }
-        }
-      }
       const uint64_t val = get(i);
       if (nlit_ == 0) {
         lit_[nlit_++] = val;
@@ -584,13 +434,13 @@ class RleV2Writer {
   }
 
  private:
-  CODAG_HD void put(uint8_t b) { out_.put(b); }
+  void put(uint8_t b) { out_.put(b); }
 
   // The writer keeps only the pending values (lit_) and the patch list: deltas and base-reduced
-  // values are derived from lit_ where they are read, which keeps a GPU thread's state small.
+  // values are derived from lit_ where they are read.
 
   // smallest width covering all but the top (100-p)% of values (compute_percentile_bit_width)
-  CODAG_HD static uint8_t percentile_width(const uint8_t* hist, uint32_t n, uint8_t p) {
+  static uint8_t percentile_width(const uint8_t* hist, uint32_t n, uint8_t p) {
     p = static_cast<uint8_t>(100 - p);
     int32_t left = (p == 0 ? 0 : static_cast<int32_t>((n * p - 1) / 100 + 1));
     for (int8_t i = 31; i >= 0; --i) {
@@ -600,7 +450,7 @@ class RleV2Writer {
     return 0;
   }
 
-  CODAG_HD void put_uvarint(int64_t val) {
+  void put_uvarint(int64_t val) {
     for (;;) {
       if ((val & ~0x7f) == 0) {
         put(static_cast<uint8_t>(val));
@@ -610,9 +460,9 @@ class RleV2Writer {
       val = static_cast<int64_t>(static_cast<uint64_t>(val) >> 7);
     }
   }
-  CODAG_HD void put_svarint(int64_t val) { put_uvarint((val << 1) ^ (val >> 63)); }
+  void put_svarint(int64_t val) { put_uvarint((val << 1) ^ (val >> 63)); }
 
-  CODAG_HD_CALL void write_short_repeat() {
+  void write_short_repeat() {
     const uint64_t val = lit_[0];
     const uint8_t nbytes = static_cast<uint8_t>((closest_width(val) - 1) / 8 + 1);
     put(static_cast<uint8_t>(((nbytes - 1) << 3) | (fix_ - kMinRepeat)));
@@ -622,7 +472,7 @@ class RleV2Writer {
     var_ = 0;
   }
 
-  CODAG_HD_CALL void write_direct() {
+  void write_direct() {
     uint8_t hist[32];
     const uint64_t* l = lit_;
     const auto lit = [l](uint32_t i) { return l[i]; };
@@ -642,7 +492,7 @@ class RleV2Writer {
     nlit_ = 0;
   }
 
-  CODAG_HD_CALL void write_delta() {
+  void write_delta() {
     uint16_t len;
     uint8_t enc = 0;
     uint8_t bits = v2_closest_aligned(delta_bits_);
@@ -673,7 +523,7 @@ class RleV2Writer {
     var_ = 0;
   }
 
-  CODAG_HD_CALL void write_patched(uint64_t lit_min, uint8_t b95, uint8_t b100) {
+  void write_patched(uint64_t lit_min, uint8_t b95, uint8_t b100) {
     // patch list (preparePatchedBlob1, encoder.h:182-268); a group holds at most 128 values, so
     // every gap is below 256 and each patch takes one list entry
     int64_t mask = static_cast<int64_t>((static_cast<uint64_t>(1) << b95) - 1);
@@ -683,7 +533,7 @@ class RleV2Writer {
       b95 = 8;
       mask = static_cast<int64_t>((static_cast<uint64_t>(1) << b95) - 1);
     }
-    uint64_t* list = g_.lists();
+    uint64_t* list = g_.list;
     uint64_t max_gap = 0;
     const uint32_t npatch = g_.patches(lit_, nlit_, lit_min, static_cast<uint64_t>(mask), b95, pwidth, list, &max_gap);
     const uint32_t gap_width = (max_gap == 0 && npatch != 0) ? 1u : closest_width(max_gap);
@@ -712,12 +562,12 @@ class RleV2Writer {
   }
 
   // determineEncoding (encoder.h:270-387)
-  CODAG_HD_CALL void choose_encoding() {
+  void choose_encoding() {
     if (nlit_ <= static_cast<uint32_t>(kMinRepeat)) {
       write_direct();
       return;
     }
-    const typename G::Scan sc = g_.scan(lit_, nlit_);
+    const Groups::Scan sc = g_.scan(lit_, nlit_);
     const uint64_t lmin = sc.lmin, lmax = sc.lmax, max_delta = sc.max_delta;
     const uint64_t initial = lit_[1] - lit_[0];
     const bool increasing = sc.increasing, decreasing = sc.decreasing;
@@ -759,7 +609,7 @@ class RleV2Writer {
   }
 
   Sink& out_;
-  G g_;
+  Groups g_;
   uint64_t* lit_;
   uint32_t nlit_ = 0, fix_ = 0, var_ = 0;
   uint8_t delta_bits_ = 0;
