@@ -1,0 +1,226 @@
+// One CTA per RLE chunk: a walk warp finds the headers, the other warps expand them.
+//
+// A warp that walks the headers of its chunk and expands them one after another leaves 31 lanes idle
+// while it reads a header, and a chunk of 128 KiB takes it 0.2 to 0.6 ms whatever the GPU has to
+// spare.  Here the two jobs run side by side: in every step the walk warp lists the next headers
+// (where each starts, and which value its first is) while the expand warps take the headers of the
+// step before, one warp per header, straight from a shared ring of the stream to the output.
+//
+// RLE v1 headers do not say how long they are: a literal group ends with the last of its varints.  So
+// two more warps run ahead of the walk and write down, for every byte that ends a varint, where it is
+// (`term`, by ordinal) and how many come before each 32 bytes of the stream.  The end of a header is
+// then one look-up, and so is each literal's place: no value needs its neighbours to be found.
+//
+// Whatever these stages do not expect (a header that does not fit, a varint of more than 16 bytes, a
+// stream that ends early) is left to the one-warp decoder, which starts the chunk over and reports
+// the exact error.
+#pragma once
+#include "decode_rle.cuh"
+
+namespace codag_dev {
+
+using TeamRing = InRing<16>;
+
+// A view of a ring for the warps that do not fill it: everything listed for them is resident.
+__device__ __forceinline__ TeamRing resident_view(const TeamRing& r) {
+  TeamRing v = r;
+  v.ready = 0xffffffffu;
+  v.release_at = 0xffffffffu;
+  return v;
+}
+
+struct TeamItem {
+  uint32_t pos;   // header, in ring coordinates
+  uint32_t n;     // its first value
+  uint32_t ord;   // RLE v1 literals: ordinal of the first one's last byte; runs: kRunItem
+  uint32_t cnt;
+};
+constexpr uint32_t kRunItem = 0xffffffffu;
+
+enum : uint32_t { kTeamGo = 0, kTeamDone = 1, kTeamFallback = 2, kTeamTimeout = 3 };
+
+template <uint32_t ITEMS>
+struct TeamBatch {
+  TeamItem item[ITEMS];
+  uint32_t items;
+  uint32_t first;  // position of its first header: what the ring has to keep
+};
+
+// --- RLE v1 -----------------------------------------------------------------------------------------
+constexpr uint32_t kBlockBytes = 2048;  // the look-ahead warps' step: two slots of the ring
+constexpr uint32_t kBlocks = 4;         // blocks whose terminators are kept
+constexpr uint32_t kV1Items = 128;
+struct TeamV1 {
+  alignas(128) uint8_t ring[TeamRing::kBytes];
+  uint16_t term[kBlocks * kBlockBytes];                  // low half of the position, by ordinal
+  uint32_t bits[kBlocks * kBlockBytes / 32];             // varint ends of 32 bytes
+  uint32_t pre[kBlocks * kBlockBytes / 32];              // ordinal of the first at or after them
+  TeamBatch<kV1Items> batch[2];
+  uint32_t count[2];      // look-ahead warps: varint ends of their slots
+  uint32_t prepared, ords;  // blocks done, and varint ends in them
+  uint32_t state;
+  uint64_t bar[16], bar4[4];
+};
+constexpr uint32_t kTermMask = kBlocks * kBlockBytes - 1u, kWordMask = kBlocks * kBlockBytes / 32u - 1u;
+
+// Look-ahead warps (me 0 and 1): slot 2 * block + me, the ordinals going on from `base`.
+__device__ __forceinline__ void find_ends(const TeamRing& in, TeamV1& sm, uint32_t block, uint32_t base, uint32_t me,
+                                          uint32_t lane) {
+  const uint32_t p0 = block * kBlockBytes + me * kSlotBytes;
+  uint32_t ends = 0;  // bits 4r .. 4r+3: the lane's four bytes of the slot's 128 bytes r
+#pragma unroll
+  for (uint32_t r = 0; r < 8; r++) {
+    const uint32_t p = p0 + 128u * r + 4u * lane;
+    const uint32_t t = ~in.rd32(p) & 0x80808080u;
+    uint32_t nib = ((t >> 7) & 1u) | ((t >> 14) & 2u) | ((t >> 21) & 4u) | (t >> 28);
+    if (p + 4u > in.hi) nib &= p >= in.hi ? 0u : (1u << (in.hi - p)) - 1u;
+    if (p < in.lo) nib &= p + 4u <= in.lo ? 0u : 15u << (in.lo - p);
+    ends |= nib << (4u * r);
+  }
+  const uint32_t total = __reduce_add_sync(FULL, __popc(ends));
+  if (lane == 0) sm.count[me] = total;
+  asm volatile("bar.sync 1, 64;" ::: "memory");
+  if (me) base += sm.count[0];
+#pragma unroll
+  for (uint32_t r = 0; r < 8; r++) {
+    const uint32_t nib = (ends >> (4u * r)) & 15u, p = p0 + 128u * r + 4u * lane;
+    uint32_t upto = __popc(nib), word = nib << (4u * (lane & 7u));
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t o = __shfl_up_sync(FULL, upto, d);
+      if (lane >= static_cast<uint32_t>(d)) upto += o;
+    }
+#pragma unroll
+    for (int d = 1; d < 8; d <<= 1) word |= __shfl_xor_sync(FULL, word, d);
+    uint32_t o = base + upto - __popc(nib);
+    if ((lane & 7u) == 0) {
+      sm.bits[(p >> 5) & kWordMask] = word;
+      sm.pre[(p >> 5) & kWordMask] = o;
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < 4; k++)
+      if ((nib >> k) & 1u) sm.term[o++ & kTermMask] = static_cast<uint16_t>(p + k);
+    base += __shfl_sync(FULL, upto, 31);
+  }
+}
+
+// ordinal of the first varint end at or after position q
+__device__ __forceinline__ uint32_t end_rank(const TeamV1& sm, uint32_t q) {
+  const uint32_t w = (q >> 5) & kWordMask;
+  return sm.pre[w] + __popc(sm.bits[w] & ((1u << (q & 31u)) - 1u));
+}
+
+// Walk warp, one lane: headers from `pos` (value n) into `b` while their ends are known.
+__device__ __forceinline__ void walk_v1(const TeamRing& in, TeamV1& sm, TeamBatch<kV1Items>& b, uint32_t& pos, uint32_t& n,
+                                        uint32_t cap, uint32_t blocks, bool stuck) {
+  const uint32_t ords = sm.ords, known = sm.prepared * kBlockBytes;
+  const bool all = sm.prepared >= blocks;
+  uint32_t items = 0, state = kTeamGo;
+  b.first = pos;
+  while (items < kV1Items) {
+    if (n >= cap) {
+      state = kTeamDone;
+      break;
+    }
+    if (!all && pos + 2u >= known) break;
+    // a literal group of one one-byte value may end the stream, a run may not
+    if (pos + 2u > in.hi || (pos + 2u == in.hi && in.rd8(pos) < 0x80u)) {
+      state = kTeamFallback;
+      break;
+    }
+    const uint32_t h = in.rd8(pos);
+    const bool run = h < 0x80u;
+    const uint32_t q = pos + (run ? 2u : 1u), cnt = run ? h + 3u : 256u - h;
+    const uint32_t r = end_rank(sm, q), last = run ? r : r + cnt - 1u;
+    if (last >= ords) {
+      if (all) state = kTeamFallback;
+      break;
+    }
+    const uint32_t next = q + ((sm.term[last & kTermMask] - q) & 0xffffu) + 1u;
+    if (n + cnt > cap || (run && next - q > 16u)) {
+      state = kTeamFallback;
+      break;
+    }
+    b.item[items++] = TeamItem{pos, n, run ? kRunItem : r, cnt};
+    pos = next;
+    n += cnt;
+  }
+  if (stuck && items == 0 && state == kTeamGo) state = kTeamFallback;  // longer than the look-ahead
+  b.items = items;
+  if (state != kTeamGo) sm.state = state;
+}
+
+template <int E>
+__device__ __forceinline__ void expand_v1(TeamRing& in, const TeamV1& sm, DirectOut& out, const TeamItem& it, uint32_t lane) {
+  constexpr uint64_t M = emask<E>();
+  if (it.ord == kRunItem) {
+    const int64_t delta = static_cast<int8_t>(in.rd8(it.pos + 1u));
+    const uint64_t lo8 = in.peek_le64(it.pos + 2u), hi8 = in.peek_le64(it.pos + 10u);
+    body_fill<E>(out, it.n, it.cnt, leb_value(lo8, hi8, leb_len(lo8, hi8)), static_cast<uint64_t>(delta), lane);
+    return;
+  }
+  for (uint32_t i = lane; i < it.cnt; i += 32) {
+    const uint32_t t1 = sm.term[(it.ord + i) & kTermMask];
+    const uint32_t t0 = i ? sm.term[(it.ord + i - 1u) & kTermMask] + 1u : it.pos + 1u;
+    const uint32_t start = it.pos + ((t0 - it.pos) & 0xffffu), len = ((t1 - t0) & 0xffffu) + 1u;
+    uint64_t v;
+    if (len <= 4u) {
+      v = leb_compact32(in.peek_le32(start), len);
+    } else {
+      const uint64_t lo8 = in.peek_le64(start);
+      v = leb_value(lo8, len > 8u ? in.peek_le64(start + 8u) : 0ull, len);
+    }
+    put_elem<E>(out, it.n + i, v & M);
+  }
+}
+
+// --- RLE v2 -----------------------------------------------------------------------------------------
+constexpr uint32_t kV2Items = 32;
+struct TeamV2 {
+  alignas(128) uint8_t ring[TeamRing::kBytes];
+  TeamBatch<kV2Items> batch[2];
+  uint32_t state;
+  uint64_t bar[16], bar4[4];
+};
+
+// Walk warp, all lanes on the same data: headers from `pos` (value n) into `b`.
+__device__ __forceinline__ void walk_v2(TeamRing& in, TeamV2& sm, TeamBatch<kV2Items>& b, uint32_t& pos, uint32_t& n,
+                                        uint32_t cap, uint32_t keep, uint32_t lane) {
+  uint32_t items = 0, state = kTeamGo;
+  if (lane == 0) b.first = pos;
+  if (!in.release(keep)) state = kTeamTimeout;
+  while (state == kTeamGo && items < kV2Items) {
+    if (pos >= in.hi) {
+      state = kTeamDone;
+      break;
+    }
+    // the largest header spans 4 + 8 + 2040 + 248 bytes; past what the ring can hold it waits for the
+    // headers listed before to be expanded
+    const uint32_t want = pos + 2304u < in.hi ? pos + 2304u : in.hi;
+    if (want > in.ready) {
+      if ((want - 1u) >> kSlotLog2 >= in.issued) break;
+      if (in.ensure(want)) {
+        state = kTeamTimeout;
+        break;
+      }
+    }
+    const uint32_t size = rlev2_size(in, pos);
+    const uint32_t w = in.peek_be32(pos), kind = w >> 30;
+    const uint32_t len8 = (((w >> 16) & 0x1ffu) + 1u) & 0xffu;
+    const uint32_t cnt = kind == 0 ? ((w >> 24) & 7u) + 3u : kind == 3 ? ((len8 - 2u) & 0xffu) + 2u : len8;
+    if (!size || pos + size > in.hi || n + cnt > cap) {
+      state = kTeamFallback;
+      break;
+    }
+    if (lane == 0) b.item[items] = TeamItem{pos, n, 0, cnt};
+    items++;
+    pos += size;
+    n += cnt;
+  }
+  if (lane == 0) {
+    b.items = items;
+    if (state != kTeamGo) sm.state = state;
+  }
+}
+
+}  // namespace codag_dev
