@@ -117,18 +117,19 @@ __global__ void __launch_bounds__(256) k_rle_plain(const uint8_t* __restrict__ c
 // ---------------------------------------------------------------------------------------
 // one CTA per chunk (decode_rle_team.cuh), values straight to global memory
 // ---------------------------------------------------------------------------------------
-constexpr uint32_t kTeamWarps = 8;
+template <int CODEC>
+using TeamOf = std::conditional_t<CODEC == CODAG_CODEC_RLEV1, TeamV1, TeamV2>;
 
 template <int CODEC, int E>
-__global__ void __launch_bounds__(32 * kTeamWarps)
+__global__ void __launch_bounds__(32 * TeamOf<CODEC>::kWarps)
     k_rle_team(const uint8_t* __restrict__ comp, uint64_t comp_bytes, const uint64_t* __restrict__ blk_off,
                const uint64_t* __restrict__ col_len, uint64_t chunk_bytes, uint8_t* __restrict__ out, uint64_t out_bytes,
                int32_t* __restrict__ status, uint64_t wait_cycles) {
   extern __shared__ __align__(128) uint8_t smem[];
   constexpr bool V1 = CODEC == CODAG_CODEC_RLEV1;
-  using Team = std::conditional_t<V1, TeamV1, TeamV2>;
-  // warp 0 walks; RLE v1: warps 1 and 2 look ahead and fill the ring; RLE v2: the walk warp fills it
-  constexpr uint32_t kFirst = V1 ? 3 : 1, kExpand = kTeamWarps - kFirst;
+  using Team = TeamOf<CODEC>;
+  // warp 0 walks, the next kAhead look ahead (the first of them fills the ring), the others expand
+  constexpr uint32_t kFirst = 1u + Team::kAhead, kExpand = Team::kWarps - kFirst;
   Team& sm = *reinterpret_cast<Team*>(smem);
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint64_t chunk = blockIdx.x;
@@ -147,44 +148,41 @@ __global__ void __launch_bounds__(32 * kTeamWarps)
   in.wait_cycles = wait_cycles;
   in.lane = lane;
   in.begin(comp + off, static_cast<uint32_t>(len));
-  constexpr uint32_t kFiller = V1 ? 1 : 0;
-  if (warp == kFiller) init_ring_barriers<16>(sm.bar, lane);
+  if (warp == 1) init_ring_barriers<16>(sm.bar, lane);
   if (threadIdx.x == 0) {
     sm.state = kTeamGo;
     sm.batch[0].items = sm.batch[1].items = 0;
     sm.batch[0].first = sm.batch[1].first = in.lo;
-    if constexpr (V1) sm.prepared = sm.ords = 0;
+    sm.prepared = sm.ords = 0;
   }
   __syncthreads();
   DirectOut o;
   o.lane = lane;
   o.begin(out + cbase, store_bytes(cbase, chunk_bytes, out_bytes));
-  uint32_t pos = in.lo, n = 0;  // walk warp
-  uint32_t prepared = 0;        // RLE v1: blocks looked over so far
+  uint32_t pos = in.lo, n = 0;  // the walk
+  uint32_t prepared = 0;        // blocks looked over so far
   uint32_t state;
   const uint32_t blocks = (in.hi + kBlockBytes - 1u) / kBlockBytes;
   for (uint32_t k = 0;; k ^= 1u) {  // the walk fills batch k while batch k ^ 1 is expanded
     auto& mine = sm.batch[k];
     const auto& prev = sm.batch[k ^ 1u];
-    const uint32_t keep = prev.first;
+    const uint32_t keep = prev.first;  // what comes before it is done with
+    const bool room = prepared < keep / kBlockBytes + kBlocks, ahead = prepared < blocks && room;
     if (warp == 0) {
-      if constexpr (V1) {
-        if (lane == 0) walk_v1(in, sm, mine, pos, n, cap, blocks, prev.items == 0 && prepared >= keep / kBlockBytes + kBlocks);
-        __syncwarp();
-      } else {
-        walk_v2(in, sm, mine, pos, n, cap, keep, lane);
+      if (lane == 0) {
+        if constexpr (V1) walk_v1(in, sm, mine, pos, n, cap, blocks, prev.items == 0 && !room);
+        else walk_v2(in, sm, mine, pos, n, cap, blocks);
       }
-    } else if (V1 && warp < kFirst) {
-      if constexpr (V1) {
-        // the next block, if its terminators' room is free again
-        if (prepared < blocks && prepared < keep / kBlockBytes + kBlocks) {
-          if (warp == 1) {
-            const uint32_t end = (prepared + 1u) * kBlockBytes;
-            if ((!in.release(keep) || in.ensure(end < in.hi ? end : in.hi)) && lane == 0) sm.state = kTeamTimeout;
-          }
-          asm volatile("bar.sync 1, 64;" ::: "memory");
-          find_ends(in, sm, prepared, sm.ords, warp - 1u, lane);
+      __syncwarp();
+    } else if (warp < kFirst) {
+      if (ahead) {
+        if (warp == 1) {  // RLE v2 headers are read from some bytes past the block, too
+          const uint32_t end = (prepared + 1u) * kBlockBytes + (V1 ? 0u : 64u);
+          if ((!in.release(keep) || in.ensure(end < in.hi ? end : in.hi)) && lane == 0) sm.state = kTeamTimeout;
         }
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * Team::kAhead) : "memory");
+        if constexpr (V1) find_ends(in, sm, prepared, sm.ords, warp - 1u, lane);
+        else read_headers(in, sm, prepared, warp - 1u, lane);
       }
     } else {
       TeamRing view = resident_view(in);
@@ -201,25 +199,22 @@ __global__ void __launch_bounds__(32 * kTeamWarps)
     __syncthreads();
     state = sm.state;
     const bool last = mine.items == 0;
-    if constexpr (V1) {
-      const bool more = prepared < blocks && prepared < keep / kBlockBytes + kBlocks;
-      __syncthreads();  // everyone has seen this step's state before the next one changes it
-      if (more) {
-        prepared++;
-        if (threadIdx.x == 0) {
-          sm.prepared = prepared;
-          sm.ords += sm.count[0] + sm.count[1];
-        }
-        __syncthreads();
+    __syncthreads();  // everyone has seen this step's state before the next one changes it
+    if (ahead) {
+      prepared++;
+      if (threadIdx.x == 0) {
+        sm.prepared = prepared;
+        if constexpr (V1) sm.ords += sm.count[0] + sm.count[1];
       }
-    } else {
-      __syncthreads();
     }
+    __syncthreads();
     if (state >= kTeamFallback || (state == kTeamDone && last)) break;
   }
   int st = CODAG_OK;
-  if (warp == kFiller && !in.drain()) state = kTeamTimeout;
-  if (warp == kFiller && lane == 0) sm.batch[0].items = state;
+  if (warp == 1) {
+    if (!in.drain()) state = kTeamTimeout;
+    if (lane == 0) sm.batch[0].items = state;
+  }
   if (warp == 0 && lane == 0) sm.batch[0].first = n;
   __syncthreads();
   state = sm.batch[0].items;
@@ -334,11 +329,11 @@ template <int CODEC, int E>
 codag_status launch_rle_team(const uint8_t* comp, uint64_t comp_bytes, const uint64_t* blk_off, const uint64_t* col_len,
                              uint64_t n, uint64_t chunk_bytes, uint8_t* out, uint64_t out_bytes, int32_t* status,
                              cudaStream_t s) {
-  constexpr uint32_t smem = CODEC == CODAG_CODEC_RLEV1 ? sizeof(TeamV1) : sizeof(TeamV2);
+  constexpr uint32_t smem = sizeof(TeamOf<CODEC>);
   auto kern = k_rle_team<CODEC, E>;
   if (allow_smem(kern, smem) != cudaSuccess) return CODAG_ECUDA;
   if (n > 0x7fffffffull) return CODAG_EINVAL;
-  kern<<<static_cast<unsigned>(n), 32 * kTeamWarps, smem, s>>>(comp, comp_bytes, blk_off, col_len, chunk_bytes, out,
+  kern<<<static_cast<unsigned>(n), 32 * TeamOf<CODEC>::kWarps, smem, s>>>(comp, comp_bytes, blk_off, col_len, chunk_bytes, out,
                                                               out_bytes, status, wait_of());
   return finish_launch();
 }

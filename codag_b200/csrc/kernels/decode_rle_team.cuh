@@ -6,10 +6,12 @@
 // (where each starts, and which value its first is) while the expand warps take the headers of the
 // step before, one warp per header, straight from a shared ring of the stream to the output.
 //
-// RLE v1 headers do not say how long they are: a literal group ends with the last of its varints.  So
-// two more warps run ahead of the walk and write down, for every byte that ends a varint, where it is
-// (`term`, by ordinal) and how many come before each 32 bytes of the stream.  The end of a header is
-// then one look-up, and so is each literal's place: no value needs its neighbours to be found.
+// More warps run ahead of the walk so that its step from header to header is a look-up or two.  RLE v1
+// headers do not say how long they are: a literal group ends with the last of its varints.  So the
+// look-ahead writes down, for every byte that ends a varint, where it is (`term`, by ordinal) and how
+// many come before each 32 bytes of the stream; each literal's place is a look-up, too.  RLE v2
+// headers do say, in a way that takes some 60 instructions to read: the look-ahead reads every byte of
+// the stream as if it were a header, 32 at a time, and writes down bytes and values.
 //
 // Whatever these stages do not expect (a header that does not fit, a varint of more than 16 bytes, a
 // stream that ends early) is left to the one-warp decoder, which starts the chunk over and reports
@@ -33,9 +35,12 @@ struct TeamItem {
   uint32_t pos;   // header, in ring coordinates
   uint32_t n;     // its first value
   uint32_t ord;   // RLE v1 literals: ordinal of the first one's last byte; runs: kRunItem
-  uint32_t cnt;
+  uint32_t cnt;   // values
 };
 constexpr uint32_t kRunItem = 0xffffffffu;
+
+constexpr uint32_t kBlockBytes = 2048;  // the look-ahead's step: two slots of the ring
+constexpr uint32_t kBlocks = 4;         // blocks whose look-ahead is kept
 
 enum : uint32_t { kTeamGo = 0, kTeamDone = 1, kTeamFallback = 2, kTeamTimeout = 3 };
 
@@ -47,16 +52,15 @@ struct TeamBatch {
 };
 
 // --- RLE v1 -----------------------------------------------------------------------------------------
-constexpr uint32_t kBlockBytes = 2048;  // the look-ahead warps' step: two slots of the ring
-constexpr uint32_t kBlocks = 4;         // blocks whose terminators are kept
 constexpr uint32_t kV1Items = 128;
 struct TeamV1 {
+  static constexpr uint32_t kWarps = 8, kAhead = 2;
   alignas(128) uint8_t ring[TeamRing::kBytes];
   uint16_t term[kBlocks * kBlockBytes];                  // low half of the position, by ordinal
   uint32_t bits[kBlocks * kBlockBytes / 32];             // varint ends of 32 bytes
   uint32_t pre[kBlocks * kBlockBytes / 32];              // ordinal of the first at or after them
   TeamBatch<kV1Items> batch[2];
-  uint32_t count[2];      // look-ahead warps: varint ends of their slots
+  uint32_t count[kAhead];   // varint ends of the look-ahead warps' slots
   uint32_t prepared, ords;  // blocks done, and varint ends in them
   uint32_t state;
   uint64_t bar[16], bar4[4];
@@ -175,52 +179,75 @@ __device__ __forceinline__ void expand_v1(TeamRing& in, const TeamV1& sm, Direct
 }
 
 // --- RLE v2 -----------------------------------------------------------------------------------------
-constexpr uint32_t kV2Items = 32;
+constexpr uint32_t kV2Items = 64;
 struct TeamV2 {
+  static constexpr uint32_t kWarps = 16, kAhead = 6;
   alignas(128) uint8_t ring[TeamRing::kBytes];
+  uint32_t info[kBlocks * kBlockBytes];  // of a header that starts here: bytes (12 bits), values; 0: not a usual one
   TeamBatch<kV2Items> batch[2];
+  uint32_t prepared, ords;  // blocks done
   uint32_t state;
   uint64_t bar[16], bar4[4];
 };
 
-// Walk warp, all lanes on the same data: headers from `pos` (value n) into `b`.
-__device__ __forceinline__ void walk_v2(TeamRing& in, TeamV2& sm, TeamBatch<kV2Items>& b, uint32_t& pos, uint32_t& n,
-                                        uint32_t cap, uint32_t keep, uint32_t lane) {
+// Look-ahead warps: every byte of `block` read as a header (as rlev2_size does for one).
+__device__ __forceinline__ void read_headers(const TeamRing& in, TeamV2& sm, uint32_t block, uint32_t me, uint32_t lane) {
+#pragma unroll 2
+  for (uint32_t g = me; g < kBlockBytes / 32u; g += TeamV2::kAhead) {
+    const uint32_t p = block * kBlockBytes + 32u * g + lane;
+    const uint32_t w = in.peek_be32(p);
+    // varint ends of the bytes from p + 2 on
+    const uint32_t e0 = __ballot_sync(FULL, !(w >> 31) && p < in.hi);
+    const uint32_t e1 = __ballot_sync(FULL, in.rd8(p + 32u) < 0x80u && p + 32u < in.hi);
+    const uint32_t ends = static_cast<uint32_t>(((static_cast<uint64_t>(e1) << 32) | e0) >> (lane + 2u)) & 0xffu;
+    const uint32_t two = ends & (ends - 1u);  // from the second on
+    const uint32_t first = w >> 24, kind = w >> 30, enc = (first >> 1) & 0x1fu;
+    const uint32_t len8 = (((w >> 16) & 0x1ffu) + 1u) & 0xffu, nd = (len8 - 2u) & 0xffu;
+    const uint32_t fbw = v2_width(enc), body = (len8 * fbw + 7u) / 8u;
+    uint32_t size, cnt = len8;
+    if (kind == 0) {
+      size = 2u + ((first >> 3) & 7u);
+      cnt = (first & 7u) + 3u;
+    } else if (kind == 1) {
+      size = 2u + body;
+    } else if (kind == 3) {
+      size = two ? 2u + __ffs(two) + (enc ? (nd * fbw + 7u) / 8u : 0u) : 0u;
+      cnt = nd + 2u;
+    } else {
+      const uint32_t third = (w >> 8) & 0xffu, fourth = w & 0xffu;
+      const uint32_t both = v2_width(third & 0x1fu) + ((fourth >> 5) & 7u) + 1u;
+      size = both > 64u ? 0u : 5u + ((third >> 5) & 7u) + body + ((fourth & 0x1fu) * v2_closest(both) + 7u) / 8u;
+    }
+    sm.info[p & (kBlocks * kBlockBytes - 1u)] = size ? size | (cnt << 12) : 0u;
+  }
+}
+
+// Walk warp, one lane: headers from `pos` (value n) into `b` while they are known.
+__device__ __forceinline__ void walk_v2(const TeamRing& in, TeamV2& sm, TeamBatch<kV2Items>& b, uint32_t& pos, uint32_t& n,
+                                        uint32_t cap, uint32_t blocks) {
+  const bool all = sm.prepared >= blocks;
+  const uint32_t known = all ? in.hi : sm.prepared * kBlockBytes;
   uint32_t items = 0, state = kTeamGo;
-  if (lane == 0) b.first = pos;
-  if (!in.release(keep)) state = kTeamTimeout;
-  while (state == kTeamGo && items < kV2Items) {
+  b.first = pos;
+  while (items < kV2Items) {
     if (pos >= in.hi) {
       state = kTeamDone;
       break;
     }
-    // the largest header spans 4 + 8 + 2040 + 248 bytes; past what the ring can hold it waits for the
-    // headers listed before to be expanded
-    const uint32_t want = pos + 2304u < in.hi ? pos + 2304u : in.hi;
-    if (want > in.ready) {
-      if ((want - 1u) >> kSlotLog2 >= in.issued) break;
-      if (in.ensure(want)) {
-        state = kTeamTimeout;
-        break;
-      }
-    }
-    const uint32_t size = rlev2_size(in, pos);
-    const uint32_t w = in.peek_be32(pos), kind = w >> 30;
-    const uint32_t len8 = (((w >> 16) & 0x1ffu) + 1u) & 0xffu;
-    const uint32_t cnt = kind == 0 ? ((w >> 24) & 7u) + 3u : kind == 3 ? ((len8 - 2u) & 0xffu) + 2u : len8;
-    if (!size || pos + size > in.hi || n + cnt > cap) {
+    if (pos >= known) break;
+    const uint32_t v = sm.info[pos & (kBlocks * kBlockBytes - 1u)];
+    const uint32_t next = pos + (v & 0xfffu), cnt = v >> 12;
+    if (!v || next > in.hi || n + cnt > cap) {
       state = kTeamFallback;
       break;
     }
-    if (lane == 0) b.item[items] = TeamItem{pos, n, 0, cnt};
-    items++;
-    pos += size;
+    if (next > known) break;  // its bytes are not all there yet
+    b.item[items++] = TeamItem{pos, n, 0, cnt};
+    pos = next;
     n += cnt;
   }
-  if (lane == 0) {
-    b.items = items;
-    if (state != kTeamGo) sm.state = state;
-  }
+  b.items = items;
+  if (state != kTeamGo) sm.state = state;
 }
 
 }  // namespace codag_dev
