@@ -31,7 +31,7 @@ __device__ __forceinline__ TeamRing resident_view(const TeamRing& r) {
   return v;
 }
 
-struct TeamItem {
+struct __align__(16) TeamItem {
   uint32_t pos;   // header, in ring coordinates
   uint32_t n;     // its first value
   uint32_t ord;   // RLE v1 literals: ordinal of the first one's last byte; runs: kRunItem
@@ -57,8 +57,7 @@ struct TeamV1 {
   static constexpr uint32_t kWarps = 8, kAhead = 2;
   alignas(128) uint8_t ring[TeamRing::kBytes];
   uint16_t term[kBlocks * kBlockBytes];                  // low half of the position, by ordinal
-  uint32_t bits[kBlocks * kBlockBytes / 32];             // varint ends of 32 bytes
-  uint32_t pre[kBlocks * kBlockBytes / 32];              // ordinal of the first at or after them
+  uint2 ends[kBlocks * kBlockBytes / 32];                // of 32 bytes: the varint ends, and the ordinal of the first
   TeamBatch<kV1Items> batch[2];
   uint32_t count[kAhead];   // varint ends of the look-ahead warps' slots
   uint32_t prepared, ords;  // blocks done, and varint ends in them
@@ -98,8 +97,7 @@ __device__ __forceinline__ void find_ends(const TeamRing& in, TeamV1& sm, uint32
     for (int d = 1; d < 8; d <<= 1) word |= __shfl_xor_sync(FULL, word, d);
     uint32_t o = base + upto - __popc(nib);
     if ((lane & 7u) == 0) {
-      sm.bits[(p >> 5) & kWordMask] = word;
-      sm.pre[(p >> 5) & kWordMask] = o;
+      sm.ends[(p >> 5) & kWordMask] = make_uint2(word, o);
     }
 #pragma unroll
     for (uint32_t k = 0; k < 4; k++)
@@ -108,17 +106,12 @@ __device__ __forceinline__ void find_ends(const TeamRing& in, TeamV1& sm, uint32
   }
 }
 
-// ordinal of the first varint end at or after position q
-__device__ __forceinline__ uint32_t end_rank(const TeamV1& sm, uint32_t q) {
-  const uint32_t w = (q >> 5) & kWordMask;
-  return sm.pre[w] + __popc(sm.bits[w] & ((1u << (q & 31u)) - 1u));
-}
-
 // Walk warp, one lane: headers from `pos` (value n) into `b` while their ends are known.
 __device__ __forceinline__ void walk_v1(const TeamRing& in, TeamV1& sm, TeamBatch<kV1Items>& b, uint32_t& pos, uint32_t& n,
                                         uint32_t cap, uint32_t blocks, bool stuck) {
   const uint32_t ords = sm.ords, known = sm.prepared * kBlockBytes;
   const bool all = sm.prepared >= blocks;
+  const uint32_t limit = all ? in.hi : known;
   uint32_t items = 0, state = kTeamGo;
   b.first = pos;
   while (items < kV1Items) {
@@ -126,27 +119,28 @@ __device__ __forceinline__ void walk_v1(const TeamRing& in, TeamV1& sm, TeamBatc
       state = kTeamDone;
       break;
     }
-    if (!all && pos + 2u >= known) break;
-    // a literal group of one one-byte value may end the stream, a run may not
-    if (pos + 2u > in.hi || (pos + 2u == in.hi && in.rd8(pos) < 0x80u)) {
-      state = kTeamFallback;
+    if (pos + 2u >= limit) {
+      if (!all) break;
+      // a literal group of one one-byte value may end the stream, a run may not
+      if (pos + 2u > limit || in.rd8(pos) < 0x80u) {
+        state = kTeamFallback;
+        break;
+      }
+    }
+    const uint32_t h = in.rd8(pos), a = pos + 1u;
+    const uint2 e = sm.ends[(a >> 5) & kWordMask];
+    const uint32_t rank = e.y + __popc(e.x & ((1u << (a & 31u)) - 1u));  // ordinal of the first varint end from a on
+    const bool run = h < 0x80u;  // run: the base's varint starts a byte later, and that byte may be an end, too
+    const uint32_t cnt = run ? h + 3u : 256u - h;
+    const uint32_t last = rank + (run ? (e.x >> (a & 31u)) & 1u : cnt - 1u);
+    const uint32_t q = run ? a + 1u : a;
+    const uint32_t bytes = ((sm.term[last & kTermMask] - q) & 0xffffu) + 1u;
+    if (last >= ords || n + cnt > cap || (run && bytes > 16u)) {
+      if (last < ords || all) state = kTeamFallback;
       break;
     }
-    const uint32_t h = in.rd8(pos);
-    const bool run = h < 0x80u;
-    const uint32_t q = pos + (run ? 2u : 1u), cnt = run ? h + 3u : 256u - h;
-    const uint32_t r = end_rank(sm, q), last = run ? r : r + cnt - 1u;
-    if (last >= ords) {
-      if (all) state = kTeamFallback;
-      break;
-    }
-    const uint32_t next = q + ((sm.term[last & kTermMask] - q) & 0xffffu) + 1u;
-    if (n + cnt > cap || (run && next - q > 16u)) {
-      state = kTeamFallback;
-      break;
-    }
-    b.item[items++] = TeamItem{pos, n, run ? kRunItem : r, cnt};
-    pos = next;
+    b.item[items++] = TeamItem{pos, n, run ? kRunItem : rank, cnt};
+    pos = q + bytes;
     n += cnt;
   }
   if (stuck && items == 0 && state == kTeamGo) state = kTeamFallback;  // longer than the look-ahead
@@ -222,6 +216,17 @@ __device__ __forceinline__ void read_headers(const TeamRing& in, TeamV2& sm, uin
   }
 }
 
+// The same for a DELTA header whose varints take more than 8 bytes, up to 16 each; 0: neither is it that.
+__device__ __noinline__ uint32_t long_delta(const TeamRing& in, uint32_t p) {
+  const uint32_t w = in.peek_be32(p);
+  if (w >> 30 != 3u) return 0;
+  const uint32_t l1 = leb_len(in.peek_le64(p + 2u), in.peek_le64(p + 10u));
+  const uint32_t l2 = l1 ? leb_len(in.peek_le64(p + 2u + l1), in.peek_le64(p + 10u + l1)) : 0u;
+  if (!l2) return 0;
+  const uint32_t enc = (w >> 25) & 0x1fu, nd = (((w >> 16) & 0x1ffu) - 1u) & 0xffu;
+  return (2u + l1 + l2 + (enc ? (nd * v2_width(enc) + 7u) / 8u : 0u)) | ((nd + 2u) << 12);
+}
+
 // Walk warp, one lane: headers from `pos` (value n) into `b` while they are known.
 __device__ __forceinline__ void walk_v2(const TeamRing& in, TeamV2& sm, TeamBatch<kV2Items>& b, uint32_t& pos, uint32_t& n,
                                         uint32_t cap, uint32_t blocks) {
@@ -235,7 +240,11 @@ __device__ __forceinline__ void walk_v2(const TeamRing& in, TeamV2& sm, TeamBatc
       break;
     }
     if (pos >= known) break;
-    const uint32_t v = sm.info[pos & (kBlocks * kBlockBytes - 1u)];
+    uint32_t v = sm.info[pos & (kBlocks * kBlockBytes - 1u)];
+    if (!v) {
+      if (!all && pos + 64u > known) break;
+      v = long_delta(in, pos);
+    }
     const uint32_t next = pos + (v & 0xfffu), cnt = v >> 12;
     if (!v || next > in.hi || n + cnt > cap) {
       state = kTeamFallback;
