@@ -34,10 +34,10 @@ __device__ __forceinline__ TeamRing resident_view(const TeamRing& r) {
 struct __align__(16) TeamItem {
   uint32_t pos;   // header, in ring coordinates
   uint32_t n;     // its first value
-  uint32_t ord;   // RLE v1 literals: ordinal of the first one's last byte; runs: kRunItem
+  uint32_t ord;   // RLE v1 literals: ordinal of the first one's last byte; runs: kRunItem plus the base's bytes
   uint32_t cnt;   // values
 };
-constexpr uint32_t kRunItem = 0xffffffffu;
+constexpr uint32_t kRunItem = 0xffffff00u;
 
 constexpr uint32_t kBlockBytes = 2048;  // the look-ahead's step: two slots of the ring
 constexpr uint32_t kBlocks = 4;         // blocks whose look-ahead is kept
@@ -66,44 +66,33 @@ struct TeamV1 {
 };
 constexpr uint32_t kTermMask = kBlocks * kBlockBytes - 1u, kWordMask = kBlocks * kBlockBytes / 32u - 1u;
 
-// Look-ahead warps (me 0 and 1): slot 2 * block + me, the ordinals going on from `base`.
+// Look-ahead warps (me 0 and 1): slot 2 * block + me, 32 bytes a lane, the ordinals going on from `base`.
 __device__ __forceinline__ void find_ends(const TeamRing& in, TeamV1& sm, uint32_t block, uint32_t base, uint32_t me,
                                           uint32_t lane) {
-  const uint32_t p0 = block * kBlockBytes + me * kSlotBytes;
-  uint32_t ends = 0;  // bits 4r .. 4r+3: the lane's four bytes of the slot's 128 bytes r
+  const uint32_t p = block * kBlockBytes + me * kSlotBytes + 32u * lane;
+  uint32_t ends = 0;  // bit i: byte p + i ends a varint
 #pragma unroll
-  for (uint32_t r = 0; r < 8; r++) {
-    const uint32_t p = p0 + 128u * r + 4u * lane;
-    const uint32_t t = ~in.rd32(p) & 0x80808080u;
-    uint32_t nib = ((t >> 7) & 1u) | ((t >> 14) & 2u) | ((t >> 21) & 4u) | (t >> 28);
-    if (p + 4u > in.hi) nib &= p >= in.hi ? 0u : (1u << (in.hi - p)) - 1u;
-    if (p < in.lo) nib &= p + 4u <= in.lo ? 0u : 15u << (in.lo - p);
-    ends |= nib << (4u * r);
+  for (uint32_t h = 0; h < 2; h++) {
+    const uint4 v = ld_s128(in.sbuf + ((p + 16u * h) & TeamRing::kMask));
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (uint32_t k = 0; k < 4; k++)  // the four top bits gathered by a product
+      ends |= (((((~w[k] & 0x80808080u) >> 7) * 0x01020408u) >> 24) & 15u) << (16u * h + 4u * k);
   }
-  const uint32_t total = __reduce_add_sync(FULL, __popc(ends));
-  if (lane == 0) sm.count[me] = total;
+  if (p + 32u > in.hi) ends &= p >= in.hi ? 0u : (1u << (in.hi - p)) - 1u;
+  if (p < in.lo) ends &= FULL << (in.lo - p);  // lo is below 16
+  uint32_t upto = __popc(ends);
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t o = __shfl_up_sync(FULL, upto, d);
+    if (lane >= static_cast<uint32_t>(d)) upto += o;
+  }
+  if (lane == 31) sm.count[me] = upto;
   asm volatile("bar.sync 1, 64;" ::: "memory");
   if (me) base += sm.count[0];
-#pragma unroll
-  for (uint32_t r = 0; r < 8; r++) {
-    const uint32_t nib = (ends >> (4u * r)) & 15u, p = p0 + 128u * r + 4u * lane;
-    uint32_t upto = __popc(nib), word = nib << (4u * (lane & 7u));
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const uint32_t o = __shfl_up_sync(FULL, upto, d);
-      if (lane >= static_cast<uint32_t>(d)) upto += o;
-    }
-#pragma unroll
-    for (int d = 1; d < 8; d <<= 1) word |= __shfl_xor_sync(FULL, word, d);
-    uint32_t o = base + upto - __popc(nib);
-    if ((lane & 7u) == 0) {
-      sm.ends[(p >> 5) & kWordMask] = make_uint2(word, o);
-    }
-#pragma unroll
-    for (uint32_t k = 0; k < 4; k++)
-      if ((nib >> k) & 1u) sm.term[o++ & kTermMask] = static_cast<uint16_t>(p + k);
-    base += __shfl_sync(FULL, upto, 31);
-  }
+  base += upto - __popc(ends);
+  sm.ends[(p >> 5) & kWordMask] = make_uint2(ends, base);
+  for (uint32_t m = ends; m; m &= m - 1u) sm.term[base++ & kTermMask] = static_cast<uint16_t>(p + __ffs(m) - 1u);
 }
 
 // Walk warp, one lane: headers from `pos` (value n) into `b` while their ends are known.
@@ -139,7 +128,7 @@ __device__ __forceinline__ void walk_v1(const TeamRing& in, TeamV1& sm, TeamBatc
       if (last < ords || all) state = kTeamFallback;
       break;
     }
-    b.item[items++] = TeamItem{pos, n, run ? kRunItem : rank, cnt};
+    b.item[items++] = TeamItem{pos, n, run ? kRunItem + bytes : rank, cnt};
     pos = q + bytes;
     n += cnt;
   }
@@ -151,10 +140,12 @@ __device__ __forceinline__ void walk_v1(const TeamRing& in, TeamV1& sm, TeamBatc
 template <int E>
 __device__ __forceinline__ void expand_v1(TeamRing& in, const TeamV1& sm, DirectOut& out, const TeamItem& it, uint32_t lane) {
   constexpr uint64_t M = emask<E>();
-  if (it.ord == kRunItem) {
+  if (it.ord > kRunItem) {
     const int64_t delta = static_cast<int8_t>(in.rd8(it.pos + 1u));
-    const uint64_t lo8 = in.peek_le64(it.pos + 2u), hi8 = in.peek_le64(it.pos + 10u);
-    body_fill<E>(out, it.n, it.cnt, leb_value(lo8, hi8, leb_len(lo8, hi8)), static_cast<uint64_t>(delta), lane);
+    const uint32_t len = it.ord - kRunItem;
+    const uint64_t base = len <= 4u ? leb_compact32(in.peek_le32(it.pos + 2u), len)
+                                    : leb_value(in.peek_le64(it.pos + 2u), in.peek_le64(it.pos + 10u), len);
+    body_fill<E>(out, it.n, it.cnt, base, static_cast<uint64_t>(delta), lane);
     return;
   }
   for (uint32_t i = lane; i < it.cnt; i += 32) {
