@@ -339,14 +339,14 @@ codag_status launch_rle_team(const uint8_t* comp, uint64_t comp_bytes, const uin
 }
 
 // Up to how many chunks a team each is faster than a warp each (measured, us, team | warp):
-//   RLE v1, 64-bit values: 64 chunks 51 | 215, 2560 276 | 344, 5120 510 | 553, 8192 791 | 723; narrower
-//   values at every count (32 bits: 64 91 | 466, 8192 1583 | 1603; 8 bits: 2560 2026 | 2823)
+//   RLE v1, 64-bit values: 33 chunks 49 | 214, 2048 187 | 273, 8192 656 | 722; 32 bits: 33 83 | 468,
+//   8192 1249 | 1601; 8 bits: 33 356 | 1830, 2048 1376 | 2211: at every count
 //   RLE v2 (the look-ahead reads every byte as a header, which pays while SMs have room for it): 64-bit
 //   values: 32 chunks 80 | 138, 400 146 | 157, 640 204 | 175; 16 bits: 32 168 | 424, 400 370 | 479,
 //   640 527 | 484; 8 bits: 640 808 | 825, 1280 1389 | 884
 constexpr uint64_t kSms = 148;
-template <int CODEC, int E>
-constexpr uint64_t kTeamChunks = CODEC == CODAG_CODEC_RLEV2 ? 3 * kSms : E == 8 ? 40 * kSms : ~0ull;
+template <int CODEC>
+constexpr uint64_t kTeamChunks = CODEC == CODAG_CODEC_RLEV2 ? 3 * kSms : ~0ull;
 
 // Values go straight to global memory when the output is element aligned (DirectOut),
 // through the shared-memory ring otherwise; with cta_per_chunk (and no workspace) a whole
@@ -357,7 +357,7 @@ codag_status launch_rle(const codag_tune& t, const uint8_t* comp, uint64_t comp_
                         int32_t* status, void* ws, uint64_t ws_bytes, cudaStream_t s) {
   // direct stores write whole elements: the output and out_bytes must be element aligned
   const bool direct = (reinterpret_cast<uintptr_t>(out) % E) == 0 && out_bytes % E == 0;
-  if (direct && !ws && (t.cta_per_chunk || n <= kTeamChunks<CODEC, E>))
+  if (direct && !ws && (t.cta_per_chunk || n <= kTeamChunks<CODEC>))
     return launch_rle_team<CODEC, E>(comp, comp_bytes, blk_off, col_len, n, chunk_bytes, out, out_bytes, status, s);
   if (direct)
     return launch_rle_out<NSLOT, CODEC, E, true>(t, comp, comp_bytes, blk_off, col_len, n, chunk_bytes, out,

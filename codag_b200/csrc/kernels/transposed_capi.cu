@@ -47,7 +47,7 @@ struct LaneReader {
   uint32_t p;              // next byte
   uint32_t cw, cv;         // cached word index and value
   uint32_t s;              // segment of cw (rows only grow, so it only moves forward)
-  bool bad;
+  bool bad = false;
 
   // where word w of this substream sits in the region; w < its word count <= the last
   // segment's hi keeps the walk inside the table, and the region has `total` words
@@ -75,6 +75,48 @@ struct LaneReader {
     return (cv >> (8u * (p++ & 3u))) & 0xffu;
   }
 
+  // MSB-first bit fields of the `total` bytes from p on (decoder_new.h:1024-1040), read through a 64-bit
+  // buffer a word at a time; p moves past them at once
+  uint64_t bb;   // bits not yet read, the next on top
+  uint32_t bc;   // how many
+  uint32_t bw;   // next word
+  __device__ __forceinline__ void fields(uint32_t total) {
+    if (total > len - p) {
+      bad = true;
+      return;
+    }
+    bb = 0;
+    bc = 0;
+    bw = p >> 2;
+    if (total) {
+      refill();
+      bb <<= 8u * (p & 3u);
+      bc -= 8u * (p & 3u);
+    }
+    p += total;
+  }
+  __device__ __forceinline__ void refill() {
+    if (bw != cw) {
+      cw = bw;
+      cv = __ldg(region + start(bw));
+    }
+    bb |= static_cast<uint64_t>(__byte_perm(cv, 0u, 0x0123u)) << (32u - bc);
+    bc += 32;
+    bw++;
+  }
+  __device__ __forceinline__ uint32_t field32(uint32_t n) {  // 1..32 bits
+    if (bc < n) refill();
+    const uint32_t v = static_cast<uint32_t>(bb >> (64u - n));
+    bb <<= n;
+    bc -= n;
+    return v;
+  }
+  __device__ __forceinline__ uint64_t field(uint32_t n) {  // 1..64 bits
+    if (n <= 32u) return field32(n);
+    const uint64_t hi = field32(n - 32u);
+    return (hi << 32) | field32(32);
+  }
+
   // the next k (1..8) bytes as one big-endian number, a word's worth of bytes per step
   __device__ __forceinline__ uint64_t take(uint32_t k) {
     if (k > len - p) {
@@ -95,24 +137,6 @@ struct LaneReader {
       k -= m;
     }
     return v;
-  }
-};
-
-// MSB-first bits local to one header (decoder_new.h:1024-1040): `cur` holds the last byte
-// taken, its low `left` bits not yet read
-struct HeaderBits {
-  uint32_t cur, left;
-  __device__ __forceinline__ uint64_t read(LaneReader& r, uint32_t n) {  // n <= 64
-    if (n <= left) {
-      left -= n;
-      return (cur >> left) & ((1u << n) - 1u);
-    }
-    const uint32_t need = n - left, k = (need + 7u) >> 3;
-    const uint64_t hi = cur & ((1u << left) - 1u);
-    const uint64_t lo = r.take(k);
-    left = 8u * k - need;
-    cur = static_cast<uint32_t>(lo) & 0xffu;
-    return shl64(hi, need) | (lo >> left);
   }
 };
 
@@ -162,11 +186,12 @@ __device__ __forceinline__ uint64_t uvarint(LaneReader& r) {
 }
 
 // One lane's substream as a state machine that yields one value per pass: a lane whose run
-// ends reads its next header while the other lanes go on with theirs, so the warp's lanes
-// meet again after every value instead of waiting for the longest run among them.  Every run
-// kind yields its next value by one step, x = v + d or v - d (v kept as x for the kinds that
+// has ended reads its next header first, so the warp's lanes meet again after every value instead of
+// waiting for the longest run among them (two and more values a pass: slower for 64-bit values).
+// Every run kind yields its next value by one step, x = v + d or v - d (v kept as x for the kinds that
 // accumulate), d being the run's next bit field or a constant, so the only fork inside the
 // step is whether the lane reads bits.
+constexpr int kEnd = -1;
 
 template <typename T>
 __device__ int decode_substream(LaneReader& r, LaneOut<T>& o) {
@@ -175,30 +200,30 @@ __device__ int decode_substream(LaneReader& r, LaneOut<T>& o) {
   uint64_t v = 0, bd = 0;  // repeat: the value; delta: running value and base delta; patched: base
   bool bits = false, acc = false, sub = false, patched = false;
   uint32_t pw = 0, pgw = 0, pll = 0, base_out = 0;  // patched: patch width, gap width, list length
-  HeaderBits b{0, 0};
-  for (;;) {
-    if (rem == 0) {
+  int st = CODAG_OK;
+  bool go = true;
+  const auto header = [&]() -> int {  // the next header with values; kEnd at the end of the substream
+    for (;;) {
       if (patched) {  // the run's values are out: patch them (decoder_new.h:1166-1183)
         if (pw + pgw > 64) return CODAG_ECORRUPT;
         const uint64_t pmask = pw >= 32 ? 0xFFFFFFFFull : ((1ull << pw) - 1ull);  // 32-bit mask (:1103)
         const uint32_t cfb = v2_closest(pw + pgw);
-        b = HeaderBits{0, 0};
+        r.fields((pll * cfb + 7u) / 8u);
+        if (r.bad) return CODAG_ECORRUPT;
         uint64_t gap = 0;
         while (pll-- > 0) {
-          const uint64_t ent = b.read(r, cfb);
+          const uint64_t ent = r.field(cfb);
           gap += shr64(ent, pw);
           const uint64_t idx = base_out + gap;
-          if (r.bad || idx >= o.n || o.over) return CODAG_ECORRUPT;
+          if (idx >= o.n) return CODAG_ECORRUPT;
           const uint64_t patch = shl64((ent & pmask) & M, fbw) & M;
           const uint64_t x = o.get(static_cast<uint32_t>(idx));
           o.set(static_cast<uint32_t>(idx), ((((x - v) & M) | patch) + v) & M);
         }
-        if (r.bad || o.over) return CODAG_ECORRUPT;
       }
       patched = false;
-      if (r.p >= r.len) break;
+      if (r.p >= r.len) return kEnd;
       const uint32_t first = r.byte();
-      b = HeaderBits{0, 0};
       switch (first & 0xC0u) {
         case 0x00: {  // SHORT_REPEAT (decoder_new.h:1004-1014)
           rem = (first & 7u) + 3u;
@@ -242,17 +267,30 @@ __device__ int decode_substream(LaneReader& r, LaneOut<T>& o) {
           acc = sub = false;
         } break;
       }
+      if (bits && !r.bad) r.fields((rem * fbw + 7u) / 8u);
       if (r.bad || o.over) return CODAG_ECORRUPT;
-      if (rem == 0) continue;
+      if (rem) return CODAG_OK;
     }
-    const uint64_t d = bits ? b.read(r, fbw) & M : bd;
-    const uint64_t x = (sub ? v - d : v + d) & M;
-    if (acc) v = x;
-    o.put(x);
-    rem--;
-    if (r.bad || o.over) return CODAG_ECORRUPT;
+  };
+  while (__any_sync(FULL, go)) {
+    if (go && rem == 0) {
+      st = header();
+      go = st == CODAG_OK;
+    }
+    __syncwarp();
+    if (go) {
+      const uint64_t d = bits ? r.field(fbw) & M : bd;
+      const uint64_t x = (sub ? v - d : v + d) & M;
+      if (acc) v = x;
+      o.put(x);
+      rem--;
+      if (o.over) {
+        st = CODAG_ECORRUPT;
+        go = false;
+      }
+    }
   }
-  return CODAG_OK;
+  return st == kEnd ? CODAG_OK : st;
 }
 
 // values of substream t whose elements fall below `store`
@@ -301,7 +339,7 @@ __global__ void __launch_bounds__(32 * kWarps)
     }
     __syncwarp();
     LaneReader r{reinterpret_cast<const uint32_t*>(comp + off), seg, run, (1u << lane) - 1u,
-                 static_cast<uint32_t>(len64), 0, 0xffffffffu, 0, 0, false};
+                 static_cast<uint32_t>(len64), 0, 0xffffffffu, 0, 0};
     LaneOut<T> o{reinterpret_cast<T*>(out) + base_e, lane, ru,
                  static_cast<uint32_t>(chunk_bytes / sizeof(T) / 32), store, 0, lane * ru, 0, false};
     int s = decode_substream<T>(r, o);
