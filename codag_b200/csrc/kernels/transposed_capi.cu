@@ -20,14 +20,11 @@
 #include <cstdint>
 
 #include "../../../include/codag.h"
-#include "../rlev2_widths.h"
+#include "decode_rle.cuh"
+
+using namespace codag_dev;
 
 namespace {
-
-constexpr uint32_t FULL = 0xffffffffu;
-
-__device__ __forceinline__ uint64_t shl64(uint64_t v, uint32_t s) { return s >= 64 ? 0ull : v << s; }
-__device__ __forceinline__ uint64_t shr64(uint64_t v, uint32_t s) { return s >= 64 ? 0ull : v >> s; }
 
 // bytes of one lane's substream, read word by word from the interleaved region
 // row segments of one chunk (shared memory): rows lo[s] <= w < hi[s] hold a word of exactly the
@@ -43,9 +40,10 @@ struct LaneReader {
   const Segments* seg;
   uint32_t total;          // words in the region
   uint32_t lt;             // lanes below this one
-  uint32_t len;            // substream bytes
+  uint32_t len, words;     // substream bytes, and words
   uint32_t p;              // next byte
   uint32_t cw, cv;         // cached word index and value
+  uint32_t far = 0;        // where in the region the last word loaded lies
   uint32_t s;              // segment of cw (rows only grow, so it only moves forward)
   bool bad = false;
 
@@ -59,6 +57,7 @@ struct LaneReader {
       bad = true;
       return 0;
     }
+    far = at;
     return at;
   }
 
@@ -73,6 +72,29 @@ struct LaneReader {
       cv = __ldg(region + start(w));
     }
     return (cv >> (8u * (p++ & 3u))) & 0xffu;
+  }
+
+  // the 16 bytes from p on, least significant first; bytes past the substream's last word are 0
+  __device__ __forceinline__ void window(uint32_t* l) {
+    const uint32_t w = p >> 2, at = start(w), n = words - w;
+    const uint32_t same = seg->hi[s] - w, step = __popc(seg->mask[s]);  // words of this row segment
+    uint32_t x[5];
+    x[0] = __ldg(region + at);
+#pragma unroll
+    for (uint32_t i = 1; i < 5; i++) x[i] = i < n && i < same ? __ldg(region + at + i * step) : 0u;
+    if (same < 5u && same < n) {  // the others lie in later segments
+      const uint32_t s0 = s;
+      for (uint32_t i = same; i < 5u && i < n; i++) {
+        const uint32_t v = __ldg(region + start(w + i));
+        if (i == 1) x[1] = v;
+        else if (i == 2) x[2] = v;
+        else if (i == 3) x[3] = v;
+        else x[4] = v;
+      }
+      s = s0;
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < 4; i++) l[i] = __funnelshift_r(x[i], x[i + 1], 8u * (p & 3u));
   }
 
   // MSB-first bit fields of the `total` bytes from p on (decoder_new.h:1024-1040), read through a 64-bit
@@ -116,28 +138,6 @@ struct LaneReader {
     const uint64_t hi = field32(n - 32u);
     return (hi << 32) | field32(32);
   }
-
-  // the next k (1..8) bytes as one big-endian number, a word's worth of bytes per step
-  __device__ __forceinline__ uint64_t take(uint32_t k) {
-    if (k > len - p) {
-      bad = true;
-      return 0;
-    }
-    uint64_t v = 0;
-    while (k) {
-      const uint32_t w = p >> 2;
-      if (w != cw) {
-        cw = w;
-        cv = __ldg(region + start(w));
-      }
-      const uint32_t o = p & 3u, m = k < 4u - o ? k : 4u - o;
-      const uint32_t be = __byte_perm(cv, 0u, 0x0123u) << (8u * o);  // stream bytes o.. at the top
-      v = (v << (8u * m)) | (be >> (32u - 8u * m));
-      p += m;
-      k -= m;
-    }
-    return v;
-  }
 };
 
 // value k of substream t lands on element t*ru + (k/ru)*32*ru + k%ru of the chunk
@@ -173,7 +173,7 @@ struct LaneOut {
   }
 };
 
-__device__ __forceinline__ uint64_t uvarint(LaneReader& r) {
+__device__ __noinline__ uint64_t uvarint(LaneReader& r) {
   uint64_t v = 0;
   uint32_t off = 0, b;
   do {
@@ -192,6 +192,7 @@ __device__ __forceinline__ uint64_t uvarint(LaneReader& r) {
 // accumulate), d being the run's next bit field or a constant, so the only fork inside the
 // step is whether the lane reads bits.
 constexpr int kEnd = -1;
+constexpr uint32_t kAhead = 512;  // words
 
 template <typename T>
 __device__ int decode_substream(LaneReader& r, LaneOut<T>& o) {
@@ -202,6 +203,11 @@ __device__ int decode_substream(LaneReader& r, LaneOut<T>& o) {
   uint32_t pw = 0, pgw = 0, pll = 0, base_out = 0;  // patched: patch width, gap width, list length
   int st = CODAG_OK;
   bool go = true;
+  // The lanes go through the region together, so what they read next is brought into L1 4 KiB at a time, a
+  // line by each lane.  (A word loaded ahead into a register costs the warp its latency all the same:
+  // whichever lane needs one waits for the last lane's load.)
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t ahead = 0, pass = 0;
   const auto header = [&]() -> int {  // the next header with values; kEnd at the end of the substream
     for (;;) {
       if (patched) {  // the run's values are out: patch them (decoder_new.h:1166-1183)
@@ -223,49 +229,65 @@ __device__ int decode_substream(LaneReader& r, LaneOut<T>& o) {
       }
       patched = false;
       if (r.p >= r.len) return kEnd;
-      const uint32_t first = r.byte();
-      switch (first & 0xC0u) {
-        case 0x00: {  // SHORT_REPEAT (decoder_new.h:1004-1014)
-          rem = (first & 7u) + 3u;
-          v = r.take(((first >> 3) & 7u) + 1u) & M;  // a big-endian value of 1..8 bytes
-          bd = 0;
-          bits = sub = false;
-          acc = true;
-        } break;
-        case 0x40:  // DIRECT (decoder_new.h:1015-1043)
-          fbw = v2_width((first >> 1) & 0x1fu);
-          rem = static_cast<uint8_t>((((first & 1u) << 8) | r.byte()) + 1u);  // a uint8_t length (:1018)
-          v = 0;
-          bits = true;
-          acc = sub = false;
-          break;
-        case 0xC0: {  // DELTA (decoder_new.h:1044-1091)
-          const uint32_t enc = (first >> 1) & 0x1fu;
-          fbw = v2_width(enc);
-          const uint8_t len = static_cast<uint8_t>((((first & 1u) << 8) | r.byte()) + 1u);
-          v = uvarint(r) & M;
-          const int64_t u = static_cast<int64_t>(uvarint(r));
-          bd = static_cast<uint64_t>((u >> 1) ^ -(u & 1)) & M;  // arithmetic shift (:990)
-          o.put(v);
-          v = (v + bd) & M;
-          o.put(v);
-          rem = static_cast<uint8_t>(len - 2);
-          bits = enc != 0;  // else every step adds the base delta
-          sub = bits && bd == 0;  // multiplier = base_delta > 0 ? 1 : -1 on the unsigned type (:1057)
-          acc = true;
-        } break;
-        default: {  // PATCHED_BASE (decoder_new.h:1092-1165)
-          fbw = v2_width((first >> 1) & 0x1fu);
-          rem = static_cast<uint8_t>((((first & 1u) << 8) | r.byte()) + 1u);
-          const uint32_t h = static_cast<uint32_t>(r.take(2));  // third and fourth header bytes
-          pw = v2_width((h >> 8) & 0x1fu);
-          pgw = ((h >> 5) & 7u) + 1u;
-          pll = h & 0x1fu;
-          base_out = o.n;
-          v = r.take(((h >> 13) & 7u) + 1u);  // the big-endian base, 1..8 bytes
-          bits = patched = true;
-          acc = sub = false;
-        } break;
+      // every kind from the same 16 bytes, so that lanes at different kinds go together
+      uint32_t l[4];
+      r.window(l);
+      const uint64_t x0 = (static_cast<uint64_t>(l[1]) << 32) | l[0], x8 = (static_cast<uint64_t>(l[3]) << 32) | l[2];
+      const uint32_t first = l[0] & 0xffu, kind = first >> 6, enc = (first >> 1) & 0x1fu;
+      const uint32_t third = (l[0] >> 16) & 0xffu, fourth = l[0] >> 24;
+      const uint32_t len8 = ((((first & 1u) << 8) | ((l[0] >> 8) & 0xffu)) + 1u) & 0xffu;  // a uint8_t length (:1018)
+      // SHORT_REPEAT's value (decoder_new.h:1004-1014) after 1 byte, PATCHED_BASE's base (:1092-1165) after 4: 1 to 8
+      // bytes, big-endian
+      const uint32_t lead = kind == 0 ? 1u : 4u, nb = (kind == 0 ? (first >> 3) & 7u : (third >> 5) & 7u) + 1u;
+      const uint64_t big = bswap64((x0 >> (8u * lead)) | (x8 << (64u - 8u * lead))) >> (64u - 8u * nb);
+      uint32_t bytes = kind & 1u ? 2u : lead + nb;
+      fbw = v2_width(enc);
+      rem = len8;
+      v = kind & 1u ? 0 : big;
+      bd = 0;
+      bits = kind != 0;
+      acc = kind == 0 || kind == 3;
+      sub = false;
+      if (kind == 0) {
+        rem = (first & 7u) + 3u;
+        v &= M;
+      }
+      patched = kind == 2;
+      if (patched) {
+        pw = v2_width(third & 0x1fu);
+        pgw = ((fourth >> 5) & 7u) + 1u;
+        pll = fourth & 0x1fu;
+        base_out = o.n;
+      }
+      if (kind == 3) {  // DELTA (decoder_new.h:1044-1091): base and base delta as varints
+        const uint64_t lo = (x0 >> 16) | (x8 << 48), ends = ~lo & 0x8080808080808080ull, second = ends & (ends - 1ull);
+        uint64_t u;
+        if (second) {  // both within 8 bytes
+          const uint32_t l1 = (ctz64(ends) >> 3) + 1u, l12 = (ctz64(second) >> 3) + 1u;
+          v = leb_compact(lo, l1);
+          u = leb_compact(lo >> (8u * l1), l12 - l1);
+          bytes += l12;
+        } else {
+          LaneReader t = r;  // a copy, so that the reader itself stays in registers
+          t.p += 2;
+          v = uvarint(t);
+          u = uvarint(t);
+          if (t.bad) return CODAG_ECORRUPT;
+          bytes = t.p - r.p;
+        }
+        v &= M;
+        const int64_t t = static_cast<int64_t>(u);
+        bd = static_cast<uint64_t>((t >> 1) ^ -(t & 1)) & M;  // arithmetic shift (:990)
+        rem = (len8 - 2u) & 0xffu;
+        bits = enc != 0;        // else every step adds the base delta
+        sub = bits && bd == 0;  // multiplier = base_delta > 0 ? 1 : -1 on the unsigned type (:1057)
+      }
+      if (bytes > r.len - r.p) return CODAG_ECORRUPT;
+      r.p += bytes;
+      if (kind == 3) {
+        o.put(v);
+        v = (v + bd) & M;
+        o.put(v);
       }
       if (bits && !r.bad) r.fields((rem * fbw + 7u) / 8u);
       if (r.bad || o.over) return CODAG_ECORRUPT;
@@ -273,6 +295,14 @@ __device__ int decode_substream(LaneReader& r, LaneOut<T>& o) {
     }
   };
   while (__any_sync(FULL, go)) {
+    if ((pass++ & 7u) == 0) {
+      const uint32_t at = __reduce_max_sync(FULL, r.far);
+      while (ahead < r.total && ahead < at + kAhead) {
+        const uint32_t line = ahead + 32u * lane;
+        if (line < r.total) asm volatile("prefetch.global.L1 [%0];" ::"l"(r.region + line));
+        ahead += 1024u;
+      }
+    }
     if (go && rem == 0) {
       st = header();
       go = st == CODAG_OK;
@@ -339,7 +369,7 @@ __global__ void __launch_bounds__(32 * kWarps)
     }
     __syncwarp();
     LaneReader r{reinterpret_cast<const uint32_t*>(comp + off), seg, run, (1u << lane) - 1u,
-                 static_cast<uint32_t>(len64), 0, 0xffffffffu, 0, 0};
+                 static_cast<uint32_t>(len64), words, 0, 0xffffffffu, 0};
     LaneOut<T> o{reinterpret_cast<T*>(out) + base_e, lane, ru,
                  static_cast<uint32_t>(chunk_bytes / sizeof(T) / 32), store, 0, lane * ru, 0, false};
     int s = decode_substream<T>(r, o);
