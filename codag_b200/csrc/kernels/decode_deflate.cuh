@@ -30,15 +30,14 @@
 
 namespace codag_dev {
 
-__constant__ uint16_t kLenBase[29] = {3,  4,  5,  6,  7,  8,  9,  10, 11,  13,  15,  17,  19,  23, 27,
-                                      31, 35, 43, 51, 59, 67, 83, 99, 115, 131, 163, 195, 227, 258};
-__constant__ uint8_t kLenExtra[29] = {0, 0, 0, 0, 0, 0, 0, 0, 1, 1, 1, 1, 2, 2, 2,
-                                      2, 3, 3, 3, 3, 4, 4, 4, 4, 5, 5, 5, 5, 0};
-__constant__ uint16_t kDistBase[30] = {1,    2,    3,    4,    5,    7,     9,     13,    17,  25,
-                                       33,   49,   65,   97,   129,  193,   257,   385,   513, 769,
-                                       1025, 1537, 2049, 3073, 4097, 6145, 8193, 12289, 16385, 24577};
-__constant__ uint8_t kDistExtra[30] = {0, 0, 0, 0, 1, 1, 2, 2,  3,  3,  4,  4,  5,  5,  6,
-                                       6, 7, 7, 8, 8, 9, 9, 10, 10, 11, 11, 12, 12, 13, 13};
+// Length code k = symbol - 257 and distance code k (RFC 1951 3.2.5), computed: 32 lanes at different
+// codes would read a table in constant memory one after another.
+__device__ __forceinline__ uint32_t len_extra(uint32_t k) { return k < 8 || k == 28 ? 0u : (k >> 2) - 1u; }
+__device__ __forceinline__ uint32_t len_base(uint32_t k) {
+  return k < 8 ? k + 3u : k == 28 ? 258u : ((4u + (k & 3u)) << ((k >> 2) - 1u)) + 3u;
+}
+__device__ __forceinline__ uint32_t dist_extra(uint32_t k) { return k < 4 ? 0u : (k >> 1) - 1u; }
+__device__ __forceinline__ uint32_t dist_base(uint32_t k) { return k < 4 ? k + 1u : ((2u + (k & 1u)) << ((k >> 1) - 1u)) + 1u; }
 __constant__ uint8_t kCodeLenOrder[19] = {16, 17, 18, 0, 8, 7, 9, 6, 10, 5, 11, 4, 12, 3, 13, 2, 14, 1, 15};
 
 constexpr uint32_t kLitLB = 10;  // codes of 11 and more bits: 0.02-0.3% of the symbols measured
@@ -73,12 +72,12 @@ __device__ __forceinline__ uint32_t make_entry(uint32_t sym, uint32_t len, int a
     if (sym == 256) return entry_bits(len, len) | kKindEndBits;
     if (sym <= 285) {
       const uint32_t k = sym - 257;
-      return entry_bits(len + kLenExtra[k], len) | kKindLenBits | (static_cast<uint32_t>(kLenBase[k]) << 16);
+      return entry_bits(len + len_extra(k), len) | kKindLenBits | (len_base(k) << 16);
     }
     return entry_bits(len, len) | kKindBadBits;
   }
   if (alpha == kAlphaDist) {
-    if (sym < 30) return entry_bits(len + kDistExtra[sym], len) | (static_cast<uint32_t>(kDistBase[sym] - 1u) << 16);
+    if (sym < 30) return entry_bits(len + dist_extra(sym), len) | ((dist_base(sym) - 1u) << 16);
     return entry_bits(len, len) | kKindBadBits;
   }
   return entry_bits(len, len) | (sym << 16);
@@ -177,15 +176,21 @@ __device__ __noinline__ bool build_table(const uint8_t* lens, uint32_t nsym, Huf
   return true;
 }
 
-// Codes longer than the table width: walk lengths LB+1..15 (zlib.h:459-527 does 6..15).
+// Codes longer than the table width: the range of lengths LB+1..15 that holds the bits (zlib.h:459-527
+// walks 6..15), all looked at side by side.
 template <uint32_t LB>
-__device__ __noinline__ uint32_t slow_entry(uint32_t bits, HuffTable t, int alpha) {
+__device__ __forceinline__ uint32_t slow_entry(uint32_t bits, HuffTable t, int alpha) {
   const uint32_t rev = __brev(bits);
+  uint32_t len = 0, at = 0;
+#pragma unroll
   for (uint32_t l = LB + 1; l < 16; l++) {
     const uint32_t k = (rev >> (32 - l)) - t.first[l];
-    if (k < t.cnt[l]) return make_entry(t.sorted[t.index[l] + k], l, alpha);
+    if (k < t.cnt[l]) {
+      len = l;
+      at = t.index[l] + k;
+    }
   }
-  return kKindBadBits;
+  return len ? make_entry(t.sorted[at], len, alpha) : static_cast<uint32_t>(kKindBadBits);
 }
 
 // Tables of one block.
@@ -346,6 +351,16 @@ __device__ __forceinline__ Symbol symbol(uint32_t lo, uint32_t hi, uint32_t s_li
   }
   y.used = (y.e & 31u) + (y.d & 31u);
   return y;
+}
+
+// inclusive prefix sum over the lanes
+__device__ __forceinline__ uint32_t warp_scan_add(uint32_t v, uint32_t lane) {
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t o = __shfl_up_sync(FULL, v, d);
+    if (lane >= static_cast<uint32_t>(d)) v += o;
+  }
+  return v;
 }
 
 // ---------------------------------------------------------------------------------------
@@ -570,40 +585,45 @@ struct InflateScan {
     pos += 3u * hclen;
     scan_barrier();
     if (!sm.header_ok) return CODAG_ECORRUPT;
-    // literal/length and distance code lengths, run-length coded with symbols 16..18.  Lane l decodes
-    // at bit l of a 32-bit stretch; the warp then steps from symbol to symbol by shuffles.
+    // Literal/length and distance code lengths, run-length coded with symbols 16..18.  Lane l decodes at
+    // bit l of a 32-bit stretch; following the lanes' steps from lane 0 by doubling finds the lanes that
+    // hold symbols, and a prefix sum of their runs where each run goes.
     uint32_t idx = 0, prev = 0;
     const uint32_t total = hlit + hdist;
-    uint32_t at = 0;
     while (idx < total) {
-      pos += at;
-      at = 0;
       if (pos > hi8) return CODAG_ECORRUPT;
       const uint32_t bits = peek(pos + lane);
       const uint32_t e = ld_s32(s_cl + 4u * (bits & ((1u << kCodeLenLB) - 1u)));
       const uint32_t n = e & 31u, sym = e >> 16, x = bits >> n;
-      // the run this symbol stands for: value (or 255: the previous one), repeats, bits
       const uint32_t rep = sym < 16 ? 1u : sym == 16 ? 3u + (x & 3u) : sym == 17 ? 3u + (x & 7u) : 11u + (x & 127u);
       const uint32_t took = n + (sym < 16 ? 0u : sym == 16 ? 2u : sym == 17 ? 3u : 7u);
-      const uint32_t val = sym < 16 ? sym : sym == 16 ? 255u : 0u;
-      const uint32_t run = (e & kSlowFlag) ? 0u : rep | (took << 8) | (val << 16);  // code lengths are at most 7 bits
-      while (at < 32 && idx < total) {
-        const uint32_t r = __shfl_sync(FULL, run, at);
-        if (!r) return CODAG_ECORRUPT;
-        const uint32_t rr = r & 0xffu;
-        uint32_t vv = r >> 16;
-        if (vv == 255u) {
-          if (idx == 0) return CODAG_ECORRUPT;
-          vv = prev;
-        }
-        if (idx + rr > total) return CODAG_ECORRUPT;
-        if (warp == 0 && vv && lane < rr) sm.lens[idx + lane] = static_cast<uint8_t>(vv);  // a repeat of 7 or more is zeros
-        prev = vv;
-        idx += rr;
-        at += (r >> 8) & 0xffu;
+      const bool bad = (e & kSlowFlag) != 0;  // code lengths are at most 7 bits
+      // lanes reached from lane 0: those of `mask` step to `mask` shifted by their steps, once, twice, four times ...
+      uint32_t next = bad ? 63u : lane + took, mask = 1u;
+#pragma unroll
+      for (int d = 0; d < 5; d++) {
+        const uint32_t to = ((mask >> lane) & 1u) && next < 32u ? 1u << next : 0u;
+        mask |= __reduce_or_sync(FULL, to);
+        const uint32_t further = __shfl_sync(FULL, next, next & 31u);
+        next = next < 32u ? further : next;
       }
+      const bool here = (mask >> lane) & 1u;
+      const uint32_t mine = here && !bad ? rep : 0u, first = idx + warp_scan_add(mine, lane) - mine;
+      const bool on = here && first < total;  // symbols past the last length belong to the data
+      if (__any_sync(FULL, on && (bad || first + rep > total || (sym == 16 && first == 0)))) return CODAG_ECORRUPT;
+      // a repeat takes the value of the last symbol below that is none, else the last stretch's
+      const uint32_t own = sym < 16 ? sym : 0u;
+      const uint32_t below = __ballot_sync(FULL, here && sym != 16) & lanemask_lt(lane);
+      const uint32_t from = __shfl_sync(FULL, own, below ? 31 - __clz(below) : 0);
+      const uint32_t val = sym == 16 ? (below ? from : prev) : own;
+      if (warp == 0 && on && val)  // a run of more than 6 is zeros
+        for (uint32_t t = 0; t < rep; t++) sm.lens[first + t] = static_cast<uint8_t>(val);
+      const uint32_t used = __ballot_sync(FULL, on);
+      const int last = 31 - __clz(used);
+      idx = __shfl_sync(FULL, first + rep, last);
+      prev = __shfl_sync(FULL, val, last);
+      pos += __shfl_sync(FULL, lane + took, last);
     }
-    pos += at;
     scan_barrier();
     if (sm.lens[256] == 0) return CODAG_ECORRUPT;
     bool ok;
@@ -696,16 +716,6 @@ __device__ __forceinline__ void inflate_scan(InflateRing& in, InflateTeam& sm, u
 // ---------------------------------------------------------------------------------------
 // token warps
 // ---------------------------------------------------------------------------------------
-// inclusive prefix sum over the lanes
-__device__ __forceinline__ uint32_t warp_scan_add(uint32_t v, uint32_t lane) {
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const uint32_t o = __shfl_up_sync(FULL, v, d);
-    if (lane >= static_cast<uint32_t>(d)) v += o;
-  }
-  return v;
-}
-
 // Token warps (2 and 3 of the team: `me` 0 and 1), taking turns at 32 cells or kTokens stored bytes; `in`
 // is bound to the stream.  Every turn ends in a batch, an empty one when no more are wanted, so the
 // place warp knows whose turn it is.
@@ -927,6 +937,28 @@ __device__ __forceinline__ void inflate_place(InflateTeam& sm, uint64_t chunk_by
           const uint32_t f = some ? __ffs(some) - 1u : 32u;  // the first 32 bytes with a start
           lead = f - q / 32u < kSteps ? 32u * (f - q / 32u) + __ffs(__shfl_sync(FULL, word, f & 31u)) - 1u : 32u * kSteps;
           lead++;
+          bool inside = false;
+#pragma unroll
+          for (uint32_t i = 0; i < kSteps; i++) inside |= w[i] < lane;
+          if (lead <= n && __any_sync(FULL, inside)) {
+            // Sources among a step's own 32 bytes are followed to a lane that starts outside or is a literal,
+            // chains of up to 31 links halved five times, and its word taken over; all steps side by side.
+            uint32_t root[kSteps];
+#pragma unroll
+            for (uint32_t i = 0; i < kSteps; i++) root[i] = w[i] < lane ? lane - 1u - w[i] : lane;
+#pragma unroll
+            for (int d = 0; d < 5; d++) {
+#pragma unroll
+              for (uint32_t i = 0; i < kSteps; i++) root[i] = __shfl_sync(FULL, root[i], root[i]);
+            }
+#pragma unroll
+            for (uint32_t i = 0; i < kSteps; i++) {
+              const uint32_t v = __shfl_sync(FULL, w[i], root[i]);
+              const uint32_t to = v >> 15 ? v : v + (lane - root[i]);
+              // a distance past 32768 has no word: the copy warp follows that step's chains itself
+              if (!__any_sync(FULL, !(v >> 15) && to >= kLiteral)) w[i] = to;
+            }
+          }
         }
         if (handed >= 2u) team_wait<64>(kBytesFree + k);
 #pragma unroll
