@@ -98,11 +98,9 @@ struct HuffTable {
   uint32_t* index;   // [16] position of the first code of each length in `sorted`
 };
 
-// Builds `t` from code lengths lens[0..nsym).  False when the lengths over-subscribe the
-// code space.  Incomplete codes are accepted; their unused codes decode as invalid.
-template <uint32_t LB, int ALPHA>
-__device__ __noinline__ bool build_table(const uint8_t* lens, uint32_t nsym, HuffTable t, uint32_t* fill,
-                                         uint32_t lane) {
+// Orders the codes of lens[0..nsym) into `t`, without its look-up table.  False when the lengths
+// over-subscribe the code space.  Incomplete codes are accepted; their unused codes decode as invalid.
+static __device__ __noinline__ bool order_codes(const uint8_t* lens, uint32_t nsym, HuffTable t, uint32_t* fill, uint32_t lane) {
   if (lane < 16) t.cnt[lane] = 0;
   __syncwarp();
   for (uint32_t s = lane; s < nsym; s += 32) {
@@ -137,43 +135,40 @@ __device__ __noinline__ bool build_table(const uint8_t* lens, uint32_t nsym, Huf
     if (l && rank == 0) fill[l] += __popc(grp);
     __syncwarp();
   }
-  // canonical codes tiled in MSB-first order: slot x finds its code by comparing its prefix of
-  // every length with that length's range of codes (ranges of two lengths never both match)
-  uint32_t first[LB], cnt[LB];
-#pragma unroll
-  for (uint32_t l = 1; l <= LB; l++) {
-    first[l - 1] = t.first[l];
-    cnt[l - 1] = t.cnt[l];
-  }
-  for (uint32_t x = lane; x < (1u << LB); x += 32) {
-    const uint32_t v = __brev(x) >> (32 - LB);  // MSB-first code prefix of table slot x
-    uint32_t len = 0, k = 0;
-#pragma unroll
-    for (uint32_t l = 1; l <= LB; l++) {
-      const uint32_t d = (v >> (LB - l)) - first[l - 1];
-      if (d < cnt[l - 1]) {
-        len = l;
-        k = d;
-      }
-    }
-    t.lut[x] = len ? make_entry(t.sorted[t.index[len] + k], len, ALPHA) : static_cast<uint32_t>(kSlowEntry);
-  }
-  __syncwarp();
-  if (ALPHA == kAlphaLitLen) {
-    // literal pairs: when the bits of slot x after its literal code hold a whole literal
-    // code too, the entry carries both.  Only the first-literal fields of the other slot
-    // are read, and a pair rewrite leaves those fields unchanged, so lanes need no order.
-    for (uint32_t x = lane; x < (1u << LB); x += 32) {
-      const uint32_t e1 = t.lut[x];
-      const uint32_t l1 = (e1 >> 5) & 15u;
-      const uint32_t e2 = t.lut[x >> l1];
-      const uint32_t l2 = (e2 >> 5) & 15u;
-      if (((e1 | e2) & (kKindMask | kSlowFlag)) == kKindLitBits && l1 + l2 <= LB)
-        t.lut[x] = (e1 & ~31u & 0x00ffffffu) | (l1 + l2) | kPairFlag | ((e2 & 0x00ff0000u) << 8);
-    }
-    __syncwarp();
-  }
   return true;
+}
+
+// The look-up table of ordered codes, by `threads` threads of which this is number `id`.  Canonical codes
+// tile the code space in MSB-first order, shorter ones first: slot x's code length is one more than the
+// number of lengths whose codes all lie below its prefix.
+template <uint32_t LB, int ALPHA>
+__device__ __noinline__ void fill_table(HuffTable t, uint32_t id, uint32_t threads) {
+  uint32_t end[LB];  // where the codes of each length end, as LB-bit prefixes
+#pragma unroll
+  for (uint32_t l = 1; l <= LB; l++) end[l - 1] = (t.first[l] + t.cnt[l]) << (LB - l);
+  for (uint32_t x = id; x < (1u << LB); x += threads) {
+    const uint32_t v = __brev(x) >> (32 - LB);  // MSB-first code prefix of table slot x
+    uint32_t len = 1;
+#pragma unroll
+    for (uint32_t l = 1; l <= LB; l++) len += v >= end[l - 1] ? 1u : 0u;
+    t.lut[x] = len <= LB ? make_entry(t.sorted[t.index[len] + (v >> (LB - len)) - t.first[len]], len, ALPHA)
+                         : static_cast<uint32_t>(kSlowEntry);
+  }
+}
+
+// Literal pairs: when the bits of slot x after its literal code hold a whole literal code too, the entry
+// carries both.  Only the first-literal fields of the other slot are read, and a pair rewrite leaves
+// those fields unchanged, so threads need no order.
+template <uint32_t LB>
+__device__ __forceinline__ void pair_literals(uint32_t* lut, uint32_t id, uint32_t threads) {
+  for (uint32_t x = id; x < (1u << LB); x += threads) {
+    const uint32_t e1 = lut[x];
+    const uint32_t l1 = (e1 >> 5) & 15u;
+    const uint32_t e2 = lut[x >> l1];
+    const uint32_t l2 = (e2 >> 5) & 15u;
+    if (((e1 | e2) & (kKindMask | kSlowFlag)) == kKindLitBits && l1 + l2 <= LB)
+      lut[x] = (e1 & ~31u & 0x00ffffffu) | (l1 + l2) | kPairFlag | ((e2 & 0x00ff0000u) << 8);
+  }
 }
 
 // Codes longer than the table width: the range of lengths LB+1..15 that holds the bits (zlib.h:459-527
@@ -210,11 +205,13 @@ constexpr uint32_t kCell = 15;         // symbols from one noted start to the ne
 constexpr uint32_t kCellMax = 16;      // where two literals were read at once
 constexpr uint32_t kCells = 13;        // noted starts of one piece: an odd row spreads over the banks
 // A piece aims at kPieceTokens symbols (by the last stretch's bits per symbol), so far below the
-// kCell * kCells it may hold that few stretches end early at a full row, and is at most kMaxSpan words long, so that 64 pieces fit the 15 KiB of
-// the input ring that are resident behind any read position.  Spans are odd numbers of words: the
+// kCell * kCells it may hold that few stretches end early at a full row, and is at most kMaxSpan words
+// long, so that 64 pieces fit the 7 KiB of the input ring that are resident behind any read position.
+// (Longer pieces, in a ring of twice the size, warm up less often but lose more where a block ends in
+// the stretch: as many turns on text, a fifth more on columns.)  Spans are odd numbers of words: the
 // lanes' first words lie in different banks.
-constexpr uint32_t kPieceTokens = 110;
-constexpr uint32_t kMinSpan = 13, kMaxSpan = 47;
+constexpr uint32_t kPieceTokens = 90;
+constexpr uint32_t kMinSpan = 13, kMaxSpan = 27;
 constexpr uint32_t kWarmBits = 640;
 
 enum : uint32_t { kBatchTokens = 0, kBatchStored = 1, kBatchDone = 2 };
@@ -237,7 +234,8 @@ constexpr uint32_t kTokens = 32 * kCellMax;
 constexpr uint32_t kRange = 3072;  // output bytes of one token batch
 struct TokenBatch {
   uint32_t starts[kRange / 32];  // bit b: a token starts at byte b of the range
-  uint32_t before;  // tokens of the list that start before the range
+  uint32_t list;    // which of the token warp's lists
+  uint32_t before;  // its tokens that start before the range
   uint32_t bytes;   // bytes of the range
   uint32_t what;    // kMore: another range of the same list follows; kLast: the chunk's last batch
 };
@@ -254,7 +252,7 @@ struct ByteBatch {
 };
 constexpr uint32_t kBadChunk = 2;
 
-using InflateRing = InRing<16, true>;  // the scan's input
+using InflateRing = InRing<8, true>;   // the scan's input
 using TokenRing = InRing<2, true>;     // a token warp's, which lags by up to two stretches
 constexpr uint32_t align16(uint32_t v) { return (v + 15u) & ~15u; }
 using InflateWin = OutRing<15, 11, true>;  // 32 KiB window, 2 KiB drains by TMA bulk stores
@@ -267,8 +265,8 @@ struct InflateTeam {
   alignas(16) uint8_t token_ring[2][align16(TokenRing::kAlloc)];
   InflateTables tab[2];  // the scan warps build the next block's while the token warps read the last's
   ScanBatch batch[2];
-  alignas(16) uint32_t tok[2][kTokens];  // one list and one batch per token warp
-  TokenBatch out[2];
+  alignas(16) uint32_t tok[2][2][kTokens];  // two lists and two batches per token warp
+  TokenBatch out[2][2];
   ByteBatch place[2];
   uint16_t cell_end[2][kPieces];
   uint8_t lens[320];
@@ -282,7 +280,7 @@ struct InflateTeam {
   uint32_t dead;       // a token warp's wait for its input ran out
   uint32_t stopped[2]; // `stop` as the first token warp saw it, one word per batch buffer
   uint32_t job;     // batched kernel: the team's current job
-  uint64_t bar[16], token_bar[2][2];
+  uint64_t bar[8], token_bar[2][2];
 };
 static_assert(sizeof(InflateTeam) <= 76800, "three teams per SM: 228 KiB / 3 less 1 KiB each");
 
@@ -302,8 +300,9 @@ __device__ __forceinline__ void team_signal(uint32_t id) {  // arrives without w
 __device__ __forceinline__ void scan_barrier() { team_barrier<1, 64>(); }                    // the scan warps
 __device__ __forceinline__ void batch_barrier() { team_barrier<2, 128>(); }                  // scan -> tokens
 __device__ __forceinline__ void job_barrier() { team_barrier<3, 32 * kTeamWarps>(); }
-// buffer k of a producer and a consumer warp is full (the producer signals) or free (the consumer does)
-enum : uint32_t { kTokensFull = 4, kTokensFree = 6, kBytesFull = 8, kBytesFree = 10 };
+// buffer k of a producer and a consumer warp is full (the producer signals) or free (the consumer does);
+// batch k of token warp w is 2 w + k
+enum : uint32_t { kTokensFull = 4, kTokensFree = 8, kBytesFull = 12, kBytesFree = 14 };
 
 // One symbol, with its distance if it is a length, or two literals.
 struct Symbol {
@@ -553,7 +552,7 @@ struct InflateScan {
     if (len && !handoff(kBatchStored, pos >> 3, len, CODAG_OK)) return CODAG_ECORRUPT;
     // the ring goes on in steps it can hold
     for (uint32_t left = len * 8u; left;) {
-      const uint32_t step = left < 8192u * 8u ? left : 8192u * 8u;
+      const uint32_t step = left < 4096u * 8u ? left : 4096u * 8u;
       st = need(step);
       if (st) return st;
       pos += step;
@@ -577,7 +576,9 @@ struct InflateScan {
       if (lane < 19)  // code length code lengths, 3 bits each in kCodeLenOrder order
         sm.lens[kCodeLenOrder[lane]] = lane < hclen ? static_cast<uint8_t>(peek(pos + 3u * lane) & 7u) : 0;
       __syncwarp();
-      const bool ok = build_table<kCodeLenLB, kAlphaCodeLen>(sm.lens, 19, cl, sm.fill[0], lane);
+      const bool ok = order_codes(sm.lens, 19, cl, sm.fill[0], lane);
+      __syncwarp();
+      if (ok) fill_table<kCodeLenLB, kAlphaCodeLen>(cl, lane, 32);
       __syncwarp();
       for (uint32_t s = lane; s < 80; s += 32) reinterpret_cast<uint32_t*>(sm.lens)[s] = 0;
       if (lane == 0) sm.header_ok = ok;
@@ -626,21 +627,30 @@ struct InflateScan {
     }
     scan_barrier();
     if (sm.lens[256] == 0) return CODAG_ECORRUPT;
-    bool ok;
-    if (warp == 0) ok = build_table<kLitLB, kAlphaLitLen>(sm.lens, hlit, sm.tab[tab].lit(), sm.fill[0], lane);
-    else ok = build_table<kDistLB, kAlphaDist>(sm.lens + hlit, hdist, sm.tab[tab].dist(), sm.fill[1], lane);
+    return build_tables(hlit, sm.lens + hlit, hdist) ? CODAG_OK : CODAG_ECORRUPT;
+  }
+
+  // Tables of literal/length codes lens[0..hlit) and distance codes dlens[0..hdist): each warp orders one
+  // alphabet, then both fill.
+  __device__ __forceinline__ bool build_tables(uint32_t hlit, const uint8_t* dlens, uint32_t hdist) {
+    InflateTables& t = sm.tab[tab];
+    const bool ok = order_codes(warp ? dlens : sm.lens, warp ? hdist : hlit, warp ? t.dist() : t.lit(), sm.fill[warp], lane);
     if (lane == 0) sm.sum[warp] = ok;
     scan_barrier();
-    return sm.sum[0] & sm.sum[1] ? CODAG_OK : CODAG_ECORRUPT;
+    if (!(sm.sum[0] & sm.sum[1])) return false;
+    fill_table<kLitLB, kAlphaLitLen>(t.lit(), id, 64);
+    fill_table<kDistLB, kAlphaDist>(t.dist(), id, 64);
+    scan_barrier();
+    pair_literals<kLitLB>(t.lit_lut, id, 64);
+    scan_barrier();
+    return true;
   }
 
   // fixed Huffman codes (RFC 1951 3.2.6)
   __device__ __forceinline__ void fixed_tables() {
     for (uint32_t s = id; s < 320; s += 64) sm.lens[s] = s < 144 ? 8 : s < 256 ? 9 : s < 280 ? 7 : s < 288 ? 8 : 5;
     scan_barrier();
-    if (warp == 0) build_table<kLitLB, kAlphaLitLen>(sm.lens, 288, sm.tab[tab].lit(), sm.fill[0], lane);
-    else build_table<kDistLB, kAlphaDist>(sm.lens + 288, 30, sm.tab[tab].dist(), sm.fill[1], lane);
-    scan_barrier();
+    build_tables(288, sm.lens + 288, 30);
   }
 
   // The stream bound to `in`, `wrapper` header bytes first.
@@ -648,7 +658,7 @@ struct InflateScan {
     if (in.lo + wrapper > in.hi) return CODAG_ECORRUPT;
     pos = (in.lo + wrapper) * 8u;
     hi8 = in.hi * 8u;
-    span = 41;
+    span = kMaxSpan;
     bool last = false;
     while (!last) {
       if (pos >= hi8) return CODAG_ECORRUPT;
@@ -720,21 +730,23 @@ __device__ __forceinline__ void inflate_scan(InflateRing& in, InflateTeam& sm, u
 // is bound to the stream.  Every turn ends in a batch, an empty one when no more are wanted, so the
 // place warp knows whose turn it is.
 __device__ __forceinline__ void inflate_tokens(TokenRing& in, InflateTeam& sm, uint32_t me, uint32_t lane) {
-  uint32_t kb = 0, turn = 0;
-  bool used = false;  // the list and the batch have been handed over before
-  TokenBatch& o = sm.out[me];
-  const auto reuse = [&]() {  // waits until the place warp is done with them
-    if (used) team_wait<64>(kTokensFree + me);
-    used = true;
+  uint32_t kb = 0, turn = 0, list = 0, k = 0, used = 0;
+  const auto reuse = [&]() {  // waits until the place warp is done with the batch before last, and its list
+    if (used >= 2u) team_wait<64>(kTokensFree + 2u * me + k);
+    used++;
   };
   const auto handoff = [&](uint32_t before, uint32_t bytes, uint32_t what) {
     if (lane == 0) {
+      TokenBatch& o = sm.out[me][k];
+      o.list = list;
       o.before = before;
       o.bytes = bytes;
       o.what = what;
     }
     __syncwarp();
-    team_signal<64>(kTokensFull + me);
+    team_signal<64>(kTokensFull + 2u * me + k);
+    k ^= 1u;
+    if (!(what & kMore)) list ^= 1u;
   };
   // the place warp's word, the same for every lane
   const auto stopped = [&]() {
@@ -764,7 +776,8 @@ __device__ __forceinline__ void inflate_tokens(TokenRing& in, InflateTeam& sm, u
         reuse();
         handoff(0, 0, kLast);
       }
-      if (used) team_wait<64>(kTokensFree + me);
+      if (used >= 2u) team_wait<64>(kTokensFree + 2u * me + k);
+      if (used) team_wait<64>(kTokensFree + 2u * me + (k ^ 1u));
       return;
     }
     if (kind == kBatchStored) {
@@ -777,8 +790,8 @@ __device__ __forceinline__ void inflate_tokens(TokenRing& in, InflateTeam& sm, u
           handoff(0, 0, 0);
           continue;
         }
-        for (uint32_t q = lane; q < n; q += 32) sm.tok[me][q] = kLiteralToken | in.rd8(at + i + q);
-        if (32u * lane < n) o.starts[lane] = n - 32u * lane >= 32u ? FULL : (1u << (n - 32u * lane)) - 1u;
+        for (uint32_t q = lane; q < n; q += 32) sm.tok[me][list][q] = kLiteralToken | in.rd8(at + i + q);
+        if (32u * lane < n) sm.out[me][k].starts[lane] = n - 32u * lane >= 32u ? FULL : (1u << (n - 32u * lane)) - 1u;
         handoff(0, n, 0);
       }
       continue;
@@ -807,7 +820,7 @@ __device__ __forceinline__ void inflate_tokens(TokenRing& in, InflateTeam& sm, u
       uint32_t p = base + q * bits + (row[0] & 0x7fffu);
       const uint32_t next = j + 1u < b.cnt[q] >> 8 ? kCell * (j + 1u) + (row[1] >> 15) : b.cnt[q] & 0xffu;
       const uint32_t n = lane < count ? next - (kCell * j + (row[0] >> 15)) : 0u;
-      uint32_t* dst = sm.tok[me] + (warp_scan_add(n, lane) - n);
+      uint32_t* dst = sm.tok[me][list] + (warp_scan_add(n, lane) - n);
       uint32_t len = 0;  // bytes of this lane's tokens
       reuse();
       bool ok = !stopped();
@@ -851,21 +864,22 @@ __device__ __forceinline__ void inflate_tokens(TokenRing& in, InflateTeam& sm, u
       // the tokens' bytes in ranges the bit map covers: one, unless there are long matches
       for (uint32_t r = 0; r < total; r += kRange) {
         if (r) reuse();
-        for (uint32_t i = lane; i < kRange / 32u; i += 32) o.starts[i] = 0;
+        uint32_t* starts = sm.out[me][k].starts;
+        for (uint32_t i = lane; i < kRange / 32u; i += 32) starts[i] = 0;
         __syncwarp();
         uint32_t s = s0, before = 0;
         if (total <= kRange) {
 #pragma unroll 4
           for (uint32_t i = 0; i < n; i++) {
             const uint32_t tok = dst[i];
-            atomicOr(&o.starts[s >> 5], 1u << (s & 31u));
+            atomicOr(&starts[s >> 5], 1u << (s & 31u));
             s += tok >> 16;
           }
         } else {
           for (uint32_t i = 0; i < n; i++) {
             const uint32_t tok = dst[i];
             if (s < r) before++;
-            else if (s - r < kRange) atomicOr(&o.starts[(s - r) >> 5], 1u << (s & 31u));
+            else if (s - r < kRange) atomicOr(&starts[(s - r) >> 5], 1u << (s & 31u));
             s += tok >> 16;
           }
           before = __reduce_add_sync(FULL, before);
@@ -885,7 +899,7 @@ __device__ __forceinline__ void inflate_tokens(TokenRing& in, InflateTeam& sm, u
 __device__ __forceinline__ void inflate_place(InflateTeam& sm, uint64_t chunk_bytes, uint32_t lane) {
   const uint32_t cap = static_cast<uint32_t>(chunk_bytes);
   const uint32_t le = 0xffffffffu >> (31u - lane);
-  uint32_t op = 0, me = 0, k = 0, handed = 0;
+  uint32_t op = 0, me = 0, from = 0, k = 0, handed = 0;  // from: bit w, the batch token warp w fills next
   bool ok = true;
   const auto handoff = [&](uint32_t bytes, uint32_t near, uint32_t last) {
     if (lane == 0) {
@@ -899,9 +913,10 @@ __device__ __forceinline__ void inflate_place(InflateTeam& sm, uint64_t chunk_by
     handed++;
   };
   for (;;) {
-    team_wait<64>(kTokensFull + me);
-    const TokenBatch& b = sm.out[me];
-    const uint32_t bytes = b.bytes, what = b.what, s_tok = smem_u32(sm.tok[me]);
+    const uint32_t buf = (from >> me) & 1u;
+    team_wait<64>(kTokensFull + 2u * me + buf);
+    const TokenBatch& b = sm.out[me][buf];
+    const uint32_t bytes = b.bytes, what = b.what, s_tok = smem_u32(sm.tok[me][b.list]);
     if (bytes > cap - op) ok = false;
     uint32_t count = b.before;  // tokens that start before the 1 KiB at c
     for (uint32_t c = 0; ok && c < bytes; c += 1024) {
@@ -966,7 +981,8 @@ __device__ __forceinline__ void inflate_place(InflateTeam& sm, uint64_t chunk_by
         handoff(n < 32u * kSteps ? n : 32u * kSteps, lead, 0);
       }
     }
-    team_signal<64>(kTokensFree + me);
+    team_signal<64>(kTokensFree + 2u * me + buf);
+    from ^= 1u << me;
     if (ok) op += bytes;
     else if (lane == 0) sm.stop = 1;
     __syncwarp();
