@@ -9,24 +9,31 @@
 
 #include "capi_common.cuh"
 #include "decode_deflate.cuh"
-#include "decode_rle.cuh"
+#include "decode_rle_team.cuh"
 
 using namespace codag_dev;
 using namespace codag_capi;
 
 namespace {
 
-constexpr uint32_t kWarps = 8;       // warps per CTA: a Deflate team uses six, the RLE files all
-constexpr uint32_t kRleFirst = 3;    // with both kinds of work, every 3rd CTA takes RLE files first
+constexpr uint32_t kWarps = kTeamWarps;  // warps per CTA (eight, for RLE files, cost Deflate 7% in registers)
 using RleRing = InRing<4>;
+using BatchV2 = TeamV2<3>;
 struct BatchShared {
   union {
-    InflateTeam team;
-    alignas(128) uint8_t ring[kWarps][RleRing::kBytes];  // overlays the team's window only
+    InflateTeam inflate;
+    TeamV1 v1;
+    BatchV2 v2;
+    alignas(128) uint8_t ring[kWarps][RleRing::kBytes];
   };
-  uint64_t bar[kWarps][4];  // the RLE rings' barriers (the team has its own)
+  TeamBars tb;
+  uint64_t bar[kWarps][4];  // of the warps' own rings
+  uint32_t job;
+  int32_t st;
 };
-static_assert(kWarps * RleRing::kBytes <= sizeof(InflateTeam::win), "the team's barriers keep their place");
+static_assert(sizeof(TeamV1) <= offsetof(InflateTeam, bar) && sizeof(BatchV2) <= offsetof(InflateTeam, bar) &&
+                  kWarps * RleRing::kBytes <= offsetof(InflateTeam, bar),
+              "the Deflate team's barriers keep their place");
 static_assert(sizeof(BatchShared) <= 76800, "three CTAs per SM");
 
 struct BatchArgs {
@@ -74,57 +81,93 @@ __device__ __forceinline__ void rle_ring(RleRing& in, BatchShared& sh, uint64_t 
   init_ring_barriers<4>(in.bar, lane);
 }
 
-// Entries [0, n) of the order, taken by the CTA's first six warps together: a Deflate stream by the
-// team, anything else by its first warp alone (in the window's memory, which is idle then).
-__device__ __forceinline__ void team_jobs(const BatchArgs& a, uint64_t n, uint32_t* queue, BatchShared& sh,
+// An RLE stream on the whole CTA
+template <int CODEC, int E, class Team>
+__device__ __noinline__ uint32_t rle_team_job(Team& sm, TeamBars& tb, const uint8_t* src, uint32_t len, uint8_t* dst,
+                                              uint32_t out_len, uint64_t wait_cycles) {
+  return rle_team<CODEC, E, kWarps>(sm, tb, src, len, dst, out_len, out_len / E, wait_cycles);
+}
+template <int CODEC, class Team>
+__device__ __forceinline__ uint32_t rle_team_any(Team& sm, TeamBars& tb, const BatchArgs& a, const codag_chunk_desc& d,
+                                                 uint64_t wait_cycles) {
+  const uint8_t* src = a.comp + d.comp_off;
+  uint8_t* dst = a.out + d.out_off;
+  switch (d.elem_bytes) {
+    case 8: return rle_team_job<CODEC, 8>(sm, tb, src, d.comp_len, dst, d.out_len, wait_cycles);
+    case 4: return rle_team_job<CODEC, 4>(sm, tb, src, d.comp_len, dst, d.out_len, wait_cycles);
+    case 2: return rle_team_job<CODEC, 2>(sm, tb, src, d.comp_len, dst, d.out_len, wait_cycles);
+    default: return rle_team_job<CODEC, 1>(sm, tb, src, d.comp_len, dst, d.out_len, wait_cycles);
+  }
+}
+__device__ __forceinline__ bool rle_team_takes(const BatchArgs& a, const codag_chunk_desc& d) {
+  const uint32_t e = d.elem_bytes;
+  return job_in_bounds(a, d) && (d.codec == CODAG_CODEC_RLEV1 || d.codec == CODAG_CODEC_RLEV2) && valid_elem_dev(e) &&
+         (reinterpret_cast<uintptr_t>(a.out + d.out_off) % e) == 0 && d.out_len % e == 0 &&
+         (d.comp_len | d.out_len) < 0x80000000u;
+}
+
+// Entries [0, n) of the order, each taken by the CTA's warps together, an RLE stream that a team cannot take by
+// the first alone.  False after a timeout.
+__device__ __forceinline__ bool team_jobs(const BatchArgs& a, uint64_t n, uint32_t* queue, BatchShared& sh,
                                           uint64_t wait_cycles, uint32_t warp, uint32_t lane, RleRing& rle) {
-  InflateTeam& sm = sh.team;
+  InflateTeam& sm = sh.inflate;
   InflateRing in;
   TokenRing tin;
   InflateWin o;
   inflate_rings(in, tin, sm, wait_cycles, warp, lane);
   inflate_window(o, sm, lane);
+  if (warp == 5) init_ring_barriers<16>(sh.tb.bar, lane);
+  if (threadIdx.x == 0) sh.tb.phase = 0;
   for (;;) {
-    if (warp == 0 && lane == 0) {
-      sm.job = atomicAdd(queue, 1u);
+    if (threadIdx.x == 0) {
+      sh.job = atomicAdd(queue, 1u);
+      sh.st = CODAG_OK;
       sm.stop = sm.dead = 0;
-      sm.status = CODAG_OK;
     }
-    job_barrier();
-    const uint32_t k = sm.job;
-    if (k >= n) break;
+    __syncthreads();
+    const uint32_t k = sh.job;
+    if (k >= n) return true;
     const uint32_t i = a.order ? a.order[k] : k;
     const codag_chunk_desc d = a.descs[i];
     if (d.codec != CODAG_CODEC_DEFLATE) {
+      uint32_t state = kTeamFallback;
+      if (rle_team_takes(a, d))
+        state = d.codec == CODAG_CODEC_RLEV1 ? rle_team_any<CODAG_CODEC_RLEV1>(sh.v1, sh.tb, a, d, wait_cycles)
+                                             : rle_team_any<CODAG_CODEC_RLEV2>(sh.v2, sh.tb, a, d, wait_cycles);
       if (warp == 0) {
-        const int st = rle_job(a, d, rle, lane);
+        int st = state == kTeamTimeout ? CODAG_ETIMEOUT : state == kTeamShort ? CODAG_ECORRUPT : CODAG_OK;
+        if (state == kTeamFallback) {
+          fence_proxy_async_smem();
+          st = rle_job(a, d, rle, lane);
+        }
         if (lane == 0) {
           if (a.status) a.status[i] = st;
-          sm.status = st;
+          sh.st = st;
         }
-        fence_proxy_async_smem();
       }
     } else if (!job_in_bounds(a, d)) {
-      if (a.status && warp == 0 && lane == 0) a.status[i] = CODAG_ECORRUPT;
+      if (a.status && threadIdx.x == 0) a.status[i] = CODAG_ECORRUPT;
+    } else if (warp < 2) {
+      in.begin(a.comp + d.comp_off, d.comp_len);
+      inflate_scan(in, sm, d.wrapper_bytes, warp, lane);
+    } else if (warp < 4) {
+      tin.begin(a.comp + d.comp_off, d.comp_len);
+      inflate_tokens(tin, sm, warp - 2u, lane);
+    } else if (warp == 4) {
+      inflate_place(sm, d.out_len, lane);
     } else {
-      if (warp < 2) {
-        in.begin(a.comp + d.comp_off, d.comp_len);
-        inflate_scan(in, sm, d.wrapper_bytes, warp, lane);
-      } else if (warp < 4) {
-        tin.begin(a.comp + d.comp_off, d.comp_len);
-        inflate_tokens(tin, sm, warp - 2u, lane);
-      } else if (warp == 4) {
-        inflate_place(sm, d.out_len, lane);
-      } else {
-        o.begin(a.out + d.out_off, d.out_len);
-        const int st = inflate_copy(sm, o, lane);
-        if (a.status && lane == 0) a.status[i] = st;
+      o.begin(a.out + d.out_off, d.out_len);
+      const int st = inflate_copy(sm, o, lane);
+      if (lane == 0) {
+        if (a.status) a.status[i] = st;
+        sh.st = sm.dead || sm.status == CODAG_ETIMEOUT ? static_cast<int>(CODAG_ETIMEOUT) : st;
       }
     }
-    job_barrier();
-    const bool timed_out = sm.status == CODAG_ETIMEOUT || sm.dead;
-    job_barrier();  // every warp has looked before the next job resets it
-    if (timed_out) break;  // ring state unknown: the team stops
+    fence_proxy_async_smem();  // the next stream's bytes may come in where this one's tables are
+    __syncthreads();
+    const bool timed_out = sh.st == CODAG_ETIMEOUT;
+    __syncthreads();  // every warp has looked before the next job resets it
+    if (timed_out) return false;  // ring state unknown: the CTA stops
   }
 }
 
@@ -143,10 +186,9 @@ __device__ __forceinline__ void rle_jobs(const BatchArgs& a, uint64_t n0, uint64
   }
 }
 
-// Persistent grid, three CTAs per SM.  The first n_team entries of the order are taken by teams
-// (queue[0]), the others, RLE files of a plan, by single warps (queue[1]).  A CTA does both: most start
-// with the team's entries and turn all eight warps to RLE files when those run out; every
-// kRleFirst-th begins with the RLE files, so that the longest of both kinds start at once.
+// Persistent grid, three CTAs per SM.  The first n_team entries of the order are taken by CTAs
+// (queue[0]), longest first; the others, a plan's short RLE files, by single warps (queue[1]), which
+// fills the SMs while the last of the CTAs' streams are decoded.
 __global__ void __launch_bounds__(32 * kWarps, 3)
     k_batch(BatchArgs a, uint64_t n, uint64_t n_team, uint32_t* __restrict__ queue, uint64_t wait_cycles) {
   extern __shared__ __align__(128) uint8_t smem[];
@@ -154,23 +196,15 @@ __global__ void __launch_bounds__(32 * kWarps, 3)
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   RleRing rle;
   rle_ring(rle, sh, wait_cycles, warp, lane);
-  const bool rle_first = blockIdx.x % kRleFirst == kRleFirst - 1u;
-  for (uint32_t phase = 0; phase < 2; phase++) {
-    if ((phase == 0) == rle_first) {
-      if (n_team < n) rle_jobs(a, n_team, n, queue + 1, lane, rle);
-    } else if (n_team && warp < kTeamWarps) {
-      team_jobs(a, n_team, queue, sh, wait_cycles, warp, lane, rle);
-    }
-    __syncthreads();  // the phases share the memory
-    fence_proxy_async_smem();
-  }
+  if (n_team && !team_jobs(a, n_team, queue, sh, wait_cycles, warp, lane, rle)) return;
+  if (n_team < n) rle_jobs(a, n_team, n, queue + 1, lane, rle);
 }
 
 }  // namespace
 
 struct codag_plan {
   uint64_t n = 0;
-  uint64_t n_team = 0;  // leading entries of the order taken by teams: the Deflate files
+  uint64_t n_team = 0;  // leading entries of the order, taken by CTAs
   codag_chunk_desc* d_descs = nullptr;
   uint32_t* d_order = nullptr;
   uint32_t* d_queue = nullptr;
@@ -202,10 +236,22 @@ void batch_enqueue(const BatchArgs& a, uint64_t n, uint64_t n_team, uint32_t* qu
   k_batch<<<grid, 32 * kWarps, sizeof(BatchShared), s>>>(a, n, n_team, queue, wait_of());
 }
 
-// Work estimate that orders the queue within a kind of work: compressed bytes, and for RLE files,
-// whose runs expand at store speed, a share of the output.
+// Work estimate that orders the queue: a Deflate stream takes some 3 us per KiB of output, an RLE
+// stream on a CTA a third to a sixth of that.
 uint64_t chunk_cost(const codag_chunk_desc& d) {
   return d.codec == CODAG_CODEC_DEFLATE ? 8ull * d.comp_len + d.out_len : static_cast<uint64_t>(d.comp_len) + d.out_len / 4;
+}
+
+// RLE files of up to this size are taken by a warp each; so are all RLE v2 files when there are more
+// longer ones than CTAs are resident, as in codag_decompress_rlev2 (2048 of 128 KiB: 389 us | 1091).
+constexpr uint32_t kWarpBytes = 32768;
+
+// CTAs of the grid.  One stream alone on an SM is decoded 2.5 times as fast as three side by side, so
+// when the longest takes more than an even share of the work on two CTAs per SM, no more are started
+// (2000 files of 4 KiB to 1 MiB: 3.2 ms | 3.7; 2048 Deflate files of 128 KiB: 2.9 | 2.3).
+uint64_t grid_cap(uint64_t resident, uint64_t longest, uint64_t total) {
+  const uint64_t two = std::max<uint64_t>(resident * 2 / 3, 1);
+  return longest > total / two ? two : resident;
 }
 
 bool valid_shape(const codag_tune& t) {
@@ -233,7 +279,24 @@ extern "C" codag_status codag_batch_plan(const codag_chunk_desc* h_descs, uint64
   p->n = n;
   std::vector<uint32_t> order(n);
   for (uint64_t i = 0; i < n; i++) order[i] = static_cast<uint32_t>(i);
-  auto team = [&](uint32_t i) { return h_descs[i].codec == CODAG_CODEC_DEFLATE; };
+  int cap = 0;
+  const codag_status st = batch_grid_cap(&cap);
+  if (st != CODAG_OK) {
+    codag_batch_destroy(p);
+    return st;
+  }
+  uint64_t long_v2 = 0, longest = 0, total = 0;
+  for (uint64_t i = 0; i < n; i++) {
+    const uint64_t cost = chunk_cost(h_descs[i]);
+    long_v2 += h_descs[i].codec == CODAG_CODEC_RLEV2 && h_descs[i].out_len > kWarpBytes;
+    longest = std::max(longest, cost);
+    total += cost;
+  }
+  const auto team = [&](uint32_t i) {
+    const codag_chunk_desc& d = h_descs[i];
+    if (d.codec == CODAG_CODEC_DEFLATE) return true;
+    return d.out_len > kWarpBytes && (d.codec == CODAG_CODEC_RLEV1 || long_v2 <= static_cast<uint64_t>(cap));
+  };
   std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) {
     if (team(a) != team(b)) return team(a);
     return chunk_cost(h_descs[a]) > chunk_cost(h_descs[b]);
@@ -247,14 +310,8 @@ extern "C" codag_status codag_batch_plan(const codag_chunk_desc* h_descs, uint64
     codag_batch_destroy(p);
     return CODAG_ECUDA;
   }
-  int cap = 0;
-  const codag_status st = batch_grid_cap(&cap);
-  if (st != CODAG_OK) {
-    codag_batch_destroy(p);
-    return st;
-  }
   const uint64_t need = p->n_team + (n - p->n_team + kWarps - 1) / kWarps;
-  p->grid = static_cast<int>(std::min<uint64_t>(need, static_cast<uint64_t>(cap)));
+  p->grid = static_cast<int>(std::min<uint64_t>(need, grid_cap(static_cast<uint64_t>(cap), longest, total)));
   *plan = p;
   return CODAG_OK;
 }

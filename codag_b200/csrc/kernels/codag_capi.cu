@@ -118,123 +118,52 @@ __global__ void __launch_bounds__(256) k_rle_plain(const uint8_t* __restrict__ c
 // one CTA per chunk (decode_rle_team.cuh), values straight to global memory
 // ---------------------------------------------------------------------------------------
 template <int CODEC>
-using TeamOf = std::conditional_t<CODEC == CODAG_CODEC_RLEV1, TeamV1, TeamV2>;
+constexpr uint32_t kTeamWarpsOf = CODEC == CODAG_CODEC_RLEV1 ? 8 : 16;
+template <int CODEC>
+struct TeamShared {
+  std::conditional_t<CODEC == CODAG_CODEC_RLEV1, TeamV1, TeamV2<6>> team;
+  TeamBars tb;
+  uint64_t bar4[4];
+};
 
 template <int CODEC, int E>
-__global__ void __launch_bounds__(32 * TeamOf<CODEC>::kWarps)
+__global__ void __launch_bounds__(32 * kTeamWarpsOf<CODEC>)
     k_rle_team(const uint8_t* __restrict__ comp, uint64_t comp_bytes, const uint64_t* __restrict__ blk_off,
                const uint64_t* __restrict__ col_len, uint64_t chunk_bytes, uint8_t* __restrict__ out, uint64_t out_bytes,
                int32_t* __restrict__ status, uint64_t wait_cycles) {
   extern __shared__ __align__(128) uint8_t smem[];
-  constexpr bool V1 = CODEC == CODAG_CODEC_RLEV1;
-  using Team = TeamOf<CODEC>;
-  // warp 0 walks, the next kAhead look ahead (the first of them fills the ring), the others expand
-  constexpr uint32_t kFirst = 1u + Team::kAhead, kExpand = Team::kWarps - kFirst;
-  Team& sm = *reinterpret_cast<Team*>(smem);
+  TeamShared<CODEC>& sh = *reinterpret_cast<TeamShared<CODEC>*>(smem);
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint64_t chunk = blockIdx.x;
   const uint64_t off = blk_off[chunk], len = col_len[chunk];
   const uint64_t cbase = chunk * chunk_bytes;
-  const uint32_t cap = static_cast<uint32_t>(chunk_bytes / E);
+  const uint32_t cap = static_cast<uint32_t>(chunk_bytes / E), store = store_bytes(cbase, chunk_bytes, out_bytes);
   if (!stream_in_bounds(off, len, comp_bytes)) {
     if (status && threadIdx.x == 0) status[chunk] = CODAG_ECORRUPT;
     return;
   }
-  TeamRing in;
-  in.buf = sm.ring;
-  in.sbuf = smem_u32(sm.ring);
-  in.bar = sm.bar;
-  in.phase = 0;
-  in.wait_cycles = wait_cycles;
-  in.lane = lane;
-  in.begin(comp + off, static_cast<uint32_t>(len));
-  if (warp == 1) init_ring_barriers<16>(sm.bar, lane);
-  if (threadIdx.x == 0) {
-    sm.state = kTeamGo;
-    sm.batch[0].items = sm.batch[1].items = 0;
-    sm.batch[0].first = sm.batch[1].first = in.lo;
-    sm.prepared = sm.ords = 0;
-  }
+  if (warp == 1) init_ring_barriers<16>(sh.tb.bar, lane);
+  if (threadIdx.x == 0) sh.tb.phase = 0;
   __syncthreads();
-  DirectOut o;
-  o.lane = lane;
-  o.begin(out + cbase, store_bytes(cbase, chunk_bytes, out_bytes));
-  uint32_t pos = in.lo, n = 0;  // the walk
-  uint32_t prepared = 0;        // blocks looked over so far
-  uint32_t state;
-  const uint32_t blocks = (in.hi + kBlockBytes - 1u) / kBlockBytes;
-  for (uint32_t k = 0;; k ^= 1u) {  // the walk fills batch k while batch k ^ 1 is expanded
-    auto& mine = sm.batch[k];
-    const auto& prev = sm.batch[k ^ 1u];
-    const uint32_t keep = prev.first;  // what comes before it is done with
-    const bool room = prepared < keep / kBlockBytes + kBlocks, ahead = prepared < blocks && room;
-    if (warp == 0) {
-      if (lane == 0) {
-        if constexpr (V1) walk_v1(in, sm, mine, pos, n, cap, blocks, prev.items == 0 && !room);
-        else walk_v2(in, sm, mine, pos, n, cap, blocks);
-      }
-      __syncwarp();
-    } else if (warp < kFirst) {
-      if (ahead) {
-        if (warp == 1) {  // RLE v2 headers are read from some bytes past the block, too
-          const uint32_t end = (prepared + 1u) * kBlockBytes + (V1 ? 0u : 64u);
-          if ((!in.release(keep) || in.ensure(end < in.hi ? end : in.hi)) && lane == 0) sm.state = kTeamTimeout;
-        }
-        asm volatile("bar.sync 1, %0;" ::"n"(32 * Team::kAhead) : "memory");
-        if constexpr (V1) find_ends(in, sm, prepared, sm.ords, warp - 1u, lane);
-        else read_headers(in, sm, prepared, warp - 1u, lane);
-      }
-    } else {
-      TeamRing view = resident_view(in);
-      for (uint32_t i = warp - kFirst; i < prev.items; i += kExpand) {
-        const TeamItem it = prev.item[i];
-        if constexpr (V1) {
-          expand_v1<E>(view, sm, o, it, lane);
-        } else {
-          uint32_t p = it.pos, v = it.n;
-          if (rlev2_header<16, E>(view, o, p, v, cap, in.hi, lane) && lane == 0) sm.state = kTeamFallback;
-        }
-      }
-    }
-    __syncthreads();
-    state = sm.state;
-    const bool last = mine.items == 0;
-    __syncthreads();  // everyone has seen this step's state before the next one changes it
-    if (ahead) {
-      prepared++;
-      if (threadIdx.x == 0) {
-        sm.prepared = prepared;
-        if constexpr (V1) sm.ords += sm.count[0] + sm.count[1];
-      }
-    }
-    __syncthreads();
-    if (state >= kTeamFallback || (state == kTeamDone && last)) break;
-  }
-  int st = CODAG_OK;
-  if (warp == 1) {
-    if (!in.drain()) state = kTeamTimeout;
-    if (lane == 0) sm.batch[0].items = state;
-  }
-  if (warp == 0 && lane == 0) sm.batch[0].first = n;
-  __syncthreads();
-  state = sm.batch[0].items;
+  const uint32_t state = rle_team<CODEC, E, kTeamWarpsOf<CODEC>>(sh.team, sh.tb, comp + off, static_cast<uint32_t>(len),
+                                                                 out + cbase, store, cap, wait_cycles);
   if (warp != 0) return;
-  if (state == kTeamTimeout) {
-    st = CODAG_ETIMEOUT;
-  } else if (state == kTeamFallback) {  // in one pass, from the start
+  int st = state == kTeamTimeout ? CODAG_ETIMEOUT : state == kTeamShort ? CODAG_ECORRUPT : CODAG_OK;
+  if (state == kTeamFallback) {  // in one pass, from the start
+    DirectOut o;
+    o.lane = lane;
+    o.begin(out + cbase, store);
     InRing<4> one;
-    one.buf = sm.ring;
-    one.sbuf = smem_u32(sm.ring);
-    one.bar = sm.bar4;
+    one.buf = sh.team.ring;
+    one.sbuf = smem_u32(sh.team.ring);
+    one.bar = sh.bar4;
     one.phase = 0;
     one.wait_cycles = wait_cycles;
     one.lane = lane;
     init_ring_barriers<4>(one.bar, lane);
     fence_proxy_async_smem();
     one.begin(comp + off, static_cast<uint32_t>(len));
-    st = V1 ? decode_rlev1_chunk<4, E>(one, o, cap) : decode_rlev2_chunk<4, E>(one, o, cap);
-  } else if (static_cast<uint64_t>(sm.batch[0].first) * E < o.store) {
-    st = CODAG_ECORRUPT;
+    st = CODEC == CODAG_CODEC_RLEV1 ? decode_rlev1_chunk<4, E>(one, o, cap) : decode_rlev2_chunk<4, E>(one, o, cap);
   }
   if (status && lane == 0) status[chunk] = st;
 }
@@ -329,12 +258,12 @@ template <int CODEC, int E>
 codag_status launch_rle_team(const uint8_t* comp, uint64_t comp_bytes, const uint64_t* blk_off, const uint64_t* col_len,
                              uint64_t n, uint64_t chunk_bytes, uint8_t* out, uint64_t out_bytes, int32_t* status,
                              cudaStream_t s) {
-  constexpr uint32_t smem = sizeof(TeamOf<CODEC>);
+  constexpr uint32_t smem = sizeof(TeamShared<CODEC>);
   auto kern = k_rle_team<CODEC, E>;
   if (allow_smem(kern, smem) != cudaSuccess) return CODAG_ECUDA;
   if (n > 0x7fffffffull) return CODAG_EINVAL;
-  kern<<<static_cast<unsigned>(n), 32 * TeamOf<CODEC>::kWarps, smem, s>>>(comp, comp_bytes, blk_off, col_len, chunk_bytes, out,
-                                                              out_bytes, status, wait_of());
+  kern<<<static_cast<unsigned>(n), 32 * kTeamWarpsOf<CODEC>, smem, s>>>(comp, comp_bytes, blk_off, col_len, chunk_bytes, out,
+                                                                      out_bytes, status, wait_of());
   return finish_launch();
 }
 

@@ -279,7 +279,6 @@ struct InflateTeam {
   uint32_t stop;       // set by the place warp: the output is full or a distance is bad
   uint32_t dead;       // a token warp's wait for its input ran out
   uint32_t stopped[2]; // `stop` as the first token warp saw it, one word per batch buffer
-  uint32_t job;     // batched kernel: the team's current job
   uint64_t bar[8], token_bar[2][2];
 };
 static_assert(sizeof(InflateTeam) <= 76800, "three teams per SM: 228 KiB / 3 less 1 KiB each");
@@ -299,7 +298,6 @@ __device__ __forceinline__ void team_signal(uint32_t id) {  // arrives without w
 }
 __device__ __forceinline__ void scan_barrier() { team_barrier<1, 64>(); }                    // the scan warps
 __device__ __forceinline__ void batch_barrier() { team_barrier<2, 128>(); }                  // scan -> tokens
-__device__ __forceinline__ void job_barrier() { team_barrier<3, 32 * kTeamWarps>(); }
 // buffer k of a producer and a consumer warp is full (the producer signals) or free (the consumer does);
 // batch k of token warp w is 2 w + k
 enum : uint32_t { kTokensFull = 4, kTokensFree = 8, kBytesFull = 12, kBytesFree = 14 };

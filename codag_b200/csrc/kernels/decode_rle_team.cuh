@@ -42,7 +42,13 @@ constexpr uint32_t kRunItem = 0xffffff00u;
 constexpr uint32_t kBlockBytes = 2048;  // the look-ahead's step: two slots of the ring
 constexpr uint32_t kBlocks = 4;         // blocks whose look-ahead is kept
 
-enum : uint32_t { kTeamGo = 0, kTeamDone = 1, kTeamFallback = 2, kTeamTimeout = 3 };
+enum : uint32_t { kTeamGo = 0, kTeamDone = 1, kTeamFallback = 2, kTeamTimeout = 3, kTeamShort = 4 };
+
+// The ring's barriers, which outlive a stream where a CTA takes several
+struct TeamBars {
+  uint64_t bar[16];
+  uint32_t phase;
+};
 
 template <uint32_t ITEMS>
 struct TeamBatch {
@@ -54,7 +60,7 @@ struct TeamBatch {
 // --- RLE v1 -----------------------------------------------------------------------------------------
 constexpr uint32_t kV1Items = 128;
 struct TeamV1 {
-  static constexpr uint32_t kWarps = 8, kAhead = 2;
+  static constexpr uint32_t kAhead = 2;
   alignas(128) uint8_t ring[TeamRing::kBytes];
   uint16_t term[kBlocks * kBlockBytes];                  // low half of the position, by ordinal
   uint2 ends[kBlocks * kBlockBytes / 32];                // of 32 bytes: the varint ends, and the ordinal of the first
@@ -62,7 +68,6 @@ struct TeamV1 {
   uint32_t count[kAhead];   // varint ends of the look-ahead warps' slots
   uint32_t prepared, ords;  // blocks done, and varint ends in them
   uint32_t state;
-  uint64_t bar[16], bar4[4];
 };
 constexpr uint32_t kTermMask = kBlocks * kBlockBytes - 1u, kWordMask = kBlocks * kBlockBytes / 32u - 1u;
 
@@ -165,20 +170,21 @@ __device__ __forceinline__ void expand_v1(TeamRing& in, const TeamV1& sm, Direct
 
 // --- RLE v2 -----------------------------------------------------------------------------------------
 constexpr uint32_t kV2Items = 64;
+template <uint32_t AHEAD>
 struct TeamV2 {
-  static constexpr uint32_t kWarps = 16, kAhead = 6;
+  static constexpr uint32_t kAhead = AHEAD;
   alignas(128) uint8_t ring[TeamRing::kBytes];
   uint32_t info[kBlocks * kBlockBytes];  // of a header that starts here: bytes (12 bits), values; 0: not a usual one
   TeamBatch<kV2Items> batch[2];
   uint32_t prepared, ords;  // blocks done
   uint32_t state;
-  uint64_t bar[16], bar4[4];
 };
 
 // Look-ahead warps: every byte of `block` read as a header (as rlev2_size does for one).
-__device__ __forceinline__ void read_headers(const TeamRing& in, TeamV2& sm, uint32_t block, uint32_t me, uint32_t lane) {
+template <uint32_t AHEAD>
+__device__ __forceinline__ void read_headers(const TeamRing& in, TeamV2<AHEAD>& sm, uint32_t block, uint32_t me, uint32_t lane) {
 #pragma unroll 2
-  for (uint32_t g = me; g < kBlockBytes / 32u; g += TeamV2::kAhead) {
+  for (uint32_t g = me; g < kBlockBytes / 32u; g += AHEAD) {
     const uint32_t p = block * kBlockBytes + 32u * g + lane;
     const uint32_t w = in.peek_be32(p);
     // varint ends of the bytes from p + 2 on
@@ -208,7 +214,7 @@ __device__ __forceinline__ void read_headers(const TeamRing& in, TeamV2& sm, uin
 }
 
 // The same for a DELTA header whose varints take more than 8 bytes, up to 16 each; 0: neither is it that.
-__device__ __noinline__ uint32_t long_delta(const TeamRing& in, uint32_t p) {
+static __device__ __noinline__ uint32_t long_delta(const TeamRing& in, uint32_t p) {
   const uint32_t w = in.peek_be32(p);
   if (w >> 30 != 3u) return 0;
   const uint32_t l1 = leb_len(in.peek_le64(p + 2u), in.peek_le64(p + 10u));
@@ -219,7 +225,8 @@ __device__ __noinline__ uint32_t long_delta(const TeamRing& in, uint32_t p) {
 }
 
 // Walk warp, one lane: headers from `pos` (value n) into `b` while they are known.
-__device__ __forceinline__ void walk_v2(const TeamRing& in, TeamV2& sm, TeamBatch<kV2Items>& b, uint32_t& pos, uint32_t& n,
+template <uint32_t AHEAD>
+__device__ __forceinline__ void walk_v2(const TeamRing& in, TeamV2<AHEAD>& sm, TeamBatch<kV2Items>& b, uint32_t& pos, uint32_t& n,
                                         uint32_t cap, uint32_t blocks) {
   const bool all = sm.prepared >= blocks;
   const uint32_t known = all ? in.hi : sm.prepared * kBlockBytes;
@@ -248,6 +255,97 @@ __device__ __forceinline__ void walk_v2(const TeamRing& in, TeamV2& sm, TeamBatc
   }
   b.items = items;
   if (state != kTeamGo) sm.state = state;
+}
+
+// The stream src[0, len) by all WARPS warps of the CTA: warp 0 walks, the next kAhead look ahead (the
+// first of them fills the ring), the others expand.  kTeamDone, kTeamShort when the stream ends before
+// `store` bytes, kTeamTimeout, or kTeamFallback: the one-warp decoder has to start it over.
+template <int CODEC, int E, uint32_t WARPS, class Team>
+__device__ __forceinline__ uint32_t rle_team(Team& sm, TeamBars& tb, const uint8_t* src, uint32_t len, uint8_t* dst,
+                                             uint32_t store, uint32_t cap, uint64_t wait_cycles) {
+  constexpr bool V1 = CODEC == CODAG_CODEC_RLEV1;
+  constexpr uint32_t kFirst = 1u + Team::kAhead, kExpand = WARPS - kFirst;
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  TeamRing in;
+  in.buf = sm.ring;
+  in.sbuf = smem_u32(sm.ring);
+  in.bar = tb.bar;
+  in.phase = tb.phase;
+  in.wait_cycles = wait_cycles;
+  in.lane = lane;
+  in.begin(src, len);
+  if (threadIdx.x == 0) {
+    sm.state = kTeamGo;
+    sm.batch[0].items = sm.batch[1].items = 0;
+    sm.batch[0].first = sm.batch[1].first = in.lo;
+    sm.prepared = sm.ords = 0;
+  }
+  __syncthreads();
+  DirectOut o;
+  o.lane = lane;
+  o.begin(dst, store);
+  uint32_t pos = in.lo, n = 0;  // the walk
+  uint32_t prepared = 0;        // blocks looked over so far
+  uint32_t state;
+  const uint32_t blocks = (in.hi + kBlockBytes - 1u) / kBlockBytes;
+  for (uint32_t k = 0;; k ^= 1u) {  // the walk fills batch k while batch k ^ 1 is expanded
+    auto& mine = sm.batch[k];
+    const auto& prev = sm.batch[k ^ 1u];
+    const uint32_t keep = prev.first;  // what comes before it is done with
+    const bool room = prepared < keep / kBlockBytes + kBlocks, ahead = prepared < blocks && room;
+    if (warp == 0) {
+      if (lane == 0) {
+        if constexpr (V1) walk_v1(in, sm, mine, pos, n, cap, blocks, prev.items == 0 && !room);
+        else walk_v2(in, sm, mine, pos, n, cap, blocks);
+      }
+      __syncwarp();
+    } else if (warp < kFirst) {
+      if (ahead) {
+        if (warp == 1) {  // RLE v2 headers are read from some bytes past the block, too
+          const uint32_t end = (prepared + 1u) * kBlockBytes + (V1 ? 0u : 64u);
+          if ((!in.release(keep) || in.ensure(end < in.hi ? end : in.hi)) && lane == 0) sm.state = kTeamTimeout;
+        }
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * Team::kAhead) : "memory");
+        if constexpr (V1) find_ends(in, sm, prepared, sm.ords, warp - 1u, lane);
+        else read_headers(in, sm, prepared, warp - 1u, lane);
+      }
+    } else {
+      TeamRing view = resident_view(in);
+      for (uint32_t i = warp - kFirst; i < prev.items; i += kExpand) {
+        const TeamItem it = prev.item[i];
+        if constexpr (V1) {
+          expand_v1<E>(view, sm, o, it, lane);
+        } else {
+          uint32_t p = it.pos, v = it.n;
+          if (rlev2_header<16, E>(view, o, p, v, cap, in.hi, lane) && lane == 0) sm.state = kTeamFallback;
+        }
+      }
+    }
+    __syncthreads();
+    state = sm.state;
+    const bool last = mine.items == 0;
+    __syncthreads();  // everyone has seen this step's state before the next one changes it
+    if (ahead) {
+      prepared++;
+      if (threadIdx.x == 0) {
+        sm.prepared = prepared;
+        if constexpr (V1) sm.ords += sm.count[0] + sm.count[1];
+      }
+    }
+    __syncthreads();
+    if (state >= kTeamFallback || (state == kTeamDone && last)) break;
+  }
+  if (warp == 1) {
+    if (!in.drain()) state = kTeamTimeout;
+    if (lane == 0) {
+      sm.batch[0].items = state;
+      tb.phase = in.phase;  // the next stream through this ring goes on from here
+    }
+  }
+  if (warp == 0 && lane == 0) sm.batch[0].first = n;
+  __syncthreads();
+  state = sm.batch[0].items;
+  return state == kTeamDone && static_cast<uint64_t>(sm.batch[0].first) * E < o.store ? kTeamShort : state;
 }
 
 }  // namespace codag_dev
