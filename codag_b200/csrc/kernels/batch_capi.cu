@@ -24,7 +24,7 @@ struct BatchShared {
     InflateTeam inflate;
     TeamV1 v1;
     BatchV2 v2;
-    alignas(128) uint8_t ring[kWarps][RleRing::kBytes];
+    alignas(128) uint8_t ring[kWarps][align_up(RleRing::kAlloc, 128)];
   };
   TeamBars tb;
   uint64_t bar[kWarps][4];  // of the warps' own rings
@@ -32,7 +32,7 @@ struct BatchShared {
   int32_t st;
 };
 static_assert(sizeof(TeamV1) <= offsetof(InflateTeam, bar) && sizeof(BatchV2) <= offsetof(InflateTeam, bar) &&
-                  kWarps * RleRing::kBytes <= offsetof(InflateTeam, bar),
+                  kWarps * align_up(RleRing::kAlloc, 128) <= offsetof(InflateTeam, bar),
               "the Deflate team's barriers keep their place");
 static_assert(sizeof(BatchShared) <= 76800, "three CTAs per SM");
 

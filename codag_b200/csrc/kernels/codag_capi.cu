@@ -23,13 +23,12 @@ namespace {
 // ---------------------------------------------------------------------------------------
 // per-warp shared memory layouts
 // ---------------------------------------------------------------------------------------
-constexpr uint32_t align_up(uint32_t v, uint32_t a) { return (v + a - 1) / a * a; }
 
 using RleOut = OutRing<12, 10, true>;  // 4 KiB ring, 1 KiB drains by TMA bulk stores
 template <int NSLOT>
 struct RleLayout {
   static constexpr uint32_t kIn = 0;
-  static constexpr uint32_t kOut = kIn + NSLOT * kSlotBytes;
+  static constexpr uint32_t kOut = kIn + align_up(InRing<NSLOT>::kAlloc, 128);
   static constexpr uint32_t kBar = kOut + RleOut::kBytes;
   static constexpr uint32_t kPerWarp = align_up(kBar + NSLOT * 8, 128);
 };
@@ -38,7 +37,7 @@ struct RleLayout {
 template <int NSLOT>
 struct RleDirectLayout {
   static constexpr uint32_t kIn = 0;
-  static constexpr uint32_t kBar = kIn + NSLOT * kSlotBytes;
+  static constexpr uint32_t kBar = kIn + InRing<NSLOT>::kAlloc;
   static constexpr uint32_t kPerWarp = align_up(kBar + NSLOT * 8, 128);
 };
 
@@ -170,7 +169,7 @@ __global__ void __launch_bounds__(32 * kTeamWarpsOf<CODEC>)
 
 // A wait that no copy ever completes: exercises the bounded-wait path of InRing.
 __global__ void k_selftest_timeout(int32_t* status, uint64_t wait_cycles) {
-  __shared__ __align__(128) uint8_t buf[kSlotBytes];
+  __shared__ __align__(128) uint8_t buf[InRing<1>::kAlloc];
   __shared__ uint64_t bar[1];
   const uint32_t lane = threadIdx.x & 31u;
   InRing<1> in;

@@ -252,8 +252,8 @@ struct ByteBatch {
 };
 constexpr uint32_t kBadChunk = 2;
 
-using InflateRing = InRing<8, true>;   // the scan's input
-using TokenRing = InRing<2, true>;     // a token warp's, which lags by up to two stretches
+using InflateRing = InRing<8>;   // the scan's input
+using TokenRing = InRing<2>;     // a token warp's, which lags by up to two stretches
 constexpr uint32_t align16(uint32_t v) { return (v + 15u) & ~15u; }
 using InflateWin = OutRing<15, 11, true>;  // 32 KiB window, 2 KiB drains by TMA bulk stores
 constexpr uint32_t kTeamWarps = 6;
@@ -687,7 +687,7 @@ struct InflateScan {
 
 // Binds a warp's input ring (it initialises the barriers) and the window of a team.
 template <int NSLOT>
-__device__ __forceinline__ void bind_ring(InRing<NSLOT, true>& in, uint8_t* buf, uint64_t* bar, uint64_t wait_cycles,
+__device__ __forceinline__ void bind_ring(InRing<NSLOT>& in, uint8_t* buf, uint64_t* bar, uint64_t wait_cycles,
                                           uint32_t lane, bool init) {
   in.buf = buf;
   in.sbuf = smem_u32(buf);

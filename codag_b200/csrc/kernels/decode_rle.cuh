@@ -144,8 +144,6 @@ __device__ __forceinline__ void body_fill(OUT& out, uint32_t n, uint32_t cnt, ui
 template <int NSLOT, int E, class OUT>
 __device__ __forceinline__ void body_unpack(const InRing<NSLOT>& in, OUT& out, uint32_t n, uint32_t cnt, uint32_t bit0,
                                             uint32_t fbw, uint64_t add, uint32_t lane) {
-  constexpr uint32_t IM = InRing<NSLOT>::kMask;
-  const uint32_t ib = in.sbuf;
   if (lane >= cnt) return;
   uint32_t bp = bit0 + lane * fbw;
   const uint32_t bstep = fbw << 5;
@@ -158,18 +156,18 @@ __device__ __forceinline__ void body_unpack(const InRing<NSLOT>& in, OUT& out, u
       T* dst = reinterpret_cast<T*>(out.gdst) + n + lane;
 #pragma unroll 4
       for (uint32_t j = lane; j < lim; j += 32, bp += bstep, dst += 32) {
-        const uint32_t wa = (bp >> 3) & ~3u;
-        const uint32_t w0 = __byte_perm(ld_s32(ib + (wa & IM)), 0, 0x0123);
-        const uint32_t w1 = __byte_perm(ld_s32(ib + ((wa + 4) & IM)), 0, 0x0123);
+        const uint32_t a = in.word_at(bp >> 3);
+        const uint32_t w0 = be_s32(a);
+        const uint32_t w1 = be_s32(a + 4);
         const uint32_t v = __funnelshift_l(w1, w0, bp & 31u) >> rs;
         *dst = static_cast<T>(static_cast<uint64_t>(v) + add);
       }
       return;
     }
     for (uint32_t j = lane; j < cnt; j += 32, bp += bstep, oa += 32 * E) {
-      const uint32_t wa = (bp >> 3) & ~3u;
-      const uint32_t w0 = __byte_perm(ld_s32(ib + (wa & IM)), 0, 0x0123);
-      const uint32_t w1 = __byte_perm(ld_s32(ib + ((wa + 4) & IM)), 0, 0x0123);
+      const uint32_t a = in.word_at(bp >> 3);
+      const uint32_t w0 = be_s32(a);
+      const uint32_t w1 = be_s32(a + 4);
       const uint32_t v = __funnelshift_l(w1, w0, bp & 31u) >> rs;
       out.template put<E>(oa, static_cast<uint64_t>(v) + add);
     }
@@ -181,20 +179,20 @@ __device__ __forceinline__ void body_unpack(const InRing<NSLOT>& in, OUT& out, u
       T* dst = reinterpret_cast<T*>(out.gdst) + n + lane;
 #pragma unroll 4
       for (uint32_t j = lane; j < lim; j += 32, bp += bstep, dst += 32) {
-        const uint32_t wa = (bp >> 3) & ~3u, s = bp & 31u;
-        const uint32_t w0 = __byte_perm(ld_s32(ib + (wa & IM)), 0, 0x0123);
-        const uint32_t w1 = __byte_perm(ld_s32(ib + ((wa + 4) & IM)), 0, 0x0123);
-        const uint32_t w2 = __byte_perm(ld_s32(ib + ((wa + 8) & IM)), 0, 0x0123);
+        const uint32_t a = in.word_at(bp >> 3), s = bp & 31u;
+        const uint32_t w0 = be_s32(a);
+        const uint32_t w1 = be_s32(a + 4);
+        const uint32_t w2 = be_s32(a + 8);
         const uint64_t v = ((static_cast<uint64_t>(__funnelshift_l(w1, w0, s)) << 32) | __funnelshift_l(w2, w1, s)) >> rs;
         *dst = static_cast<T>(v + add);
       }
       return;
     }
     for (uint32_t j = lane; j < cnt; j += 32, bp += bstep, oa += 32 * E) {
-      const uint32_t wa = (bp >> 3) & ~3u, s = bp & 31u;
-      const uint32_t w0 = __byte_perm(ld_s32(ib + (wa & IM)), 0, 0x0123);
-      const uint32_t w1 = __byte_perm(ld_s32(ib + ((wa + 4) & IM)), 0, 0x0123);
-      const uint32_t w2 = __byte_perm(ld_s32(ib + ((wa + 8) & IM)), 0, 0x0123);
+      const uint32_t a = in.word_at(bp >> 3), s = bp & 31u;
+      const uint32_t w0 = be_s32(a);
+      const uint32_t w1 = be_s32(a + 4);
+      const uint32_t w2 = be_s32(a + 8);
       const uint64_t v = ((static_cast<uint64_t>(__funnelshift_l(w1, w0, s)) << 32) | __funnelshift_l(w2, w1, s)) >> rs;
       out.template put<E>(oa, v + add);
     }
@@ -222,11 +220,13 @@ __device__ __forceinline__ void body_delta_packed(const InRing<NSLOT>& in, OUT& 
   }
 }
 
-// PATCHED_BASE patch list (decoder_new.h:1142-1182), applied to the len8 values at n
+// PATCHED_BASE patch list (decoder_new.h:1142-1182), applied to the len8 values at n, which were unpacked from
+// bit `val0` on.  A patched value's field is read again from the ring: reading the value back from global memory
+// made the warp wait for its own store (1 GiB of 64-bit values 449 us, @NEW@ now).
 template <int NSLOT, int E, class OUT>
 __device__ __forceinline__ int body_patches(const InRing<NSLOT>& in, OUT& out, uint32_t n, uint32_t len8, uint32_t fbw,
-                                            uint32_t pw, uint32_t cfb, uint32_t pll, uint64_t base, uint32_t bit0,
-                                            uint32_t lane) {
+                                            uint32_t pw, uint32_t cfb, uint32_t pll, uint64_t base, uint32_t val0,
+                                            uint32_t bit0, uint32_t lane) {
   constexpr uint64_t M = emask<E>();
   // the reference masks patches with a 32-bit mask (decoder_new.h:1103)
   const uint64_t pmask = pw >= 32 ? 0xffffffffull : ((1ull << pw) - 1ull);
@@ -256,8 +256,8 @@ __device__ __forceinline__ int body_patches(const InRing<NSLOT>& in, OUT& out, u
   }
   __syncwarp();
   if (lane < pll && (lane == 0 || prev != off)) {
-    const uint64_t v = get_elem<E>(out, n + off);
-    put_elem<E>(out, n + off, ((((v - base) & M) | patch) + base) & M);
+    const uint64_t v = in.msb_bits64(val0 + off * fbw, fbw);
+    put_elem<E>(out, n + off, (((v & M) | patch) + base) & M);
   }
   return CODAG_OK;
 }
@@ -434,7 +434,7 @@ __device__ __forceinline__ int rlev2_header(InRing<NSLOT>& in, OUT& out, uint32_
     body_unpack<NSLOT, E>(in, out, n, cnt, vals * 8u, fbw, base, lane);
     if (pll) {
       __syncwarp();
-      st = body_patches<NSLOT, E>(in, out, n, len8, fbw, pw, cfb, pll, base, patches * 8u, lane);
+      st = body_patches<NSLOT, E>(in, out, n, len8, fbw, pw, cfb, pll, base, vals * 8u, patches * 8u, lane);
       if (st) return st;
     }
   }
@@ -567,9 +567,9 @@ __device__ int decode_rlev2_chunk(InRing<NSLOT>& in, OUT& out, uint32_t cap) {
         const uint32_t pi = __shfl_sync(FULL, pinfo, j);
         body_unpack<NSLOT, E>(in, out, n, cnt, __shfl_sync(FULL, bit, j), fbw, base, lane);
         if (pi >> 16) {
-          const uint32_t pb = __shfl_sync(FULL, pbit, j);
+          const uint32_t pb = __shfl_sync(FULL, pbit, j), vbit = __shfl_sync(FULL, bit, j);
           __syncwarp();
-          st = body_patches<NSLOT, E>(in, out, n, cnt, fbw, pi & 0xffu, (pi >> 8) & 0xffu, pi >> 16, base, pb, lane);
+          st = body_patches<NSLOT, E>(in, out, n, cnt, fbw, pi & 0xffu, (pi >> 8) & 0xffu, pi >> 16, base, vbit, pb, lane);
           if (st) break;
         }
       }

@@ -61,7 +61,7 @@ struct TeamBatch {
 constexpr uint32_t kV1Items = 128;
 struct TeamV1 {
   static constexpr uint32_t kAhead = 2;
-  alignas(128) uint8_t ring[TeamRing::kBytes];
+  alignas(128) uint8_t ring[TeamRing::kAlloc];
   uint16_t term[kBlocks * kBlockBytes];                  // low half of the position, by ordinal
   uint2 ends[kBlocks * kBlockBytes / 32];                // of 32 bytes: the varint ends, and the ordinal of the first
   TeamBatch<kV1Items> batch[2];
@@ -173,7 +173,7 @@ constexpr uint32_t kV2Items = 64;
 template <uint32_t AHEAD>
 struct TeamV2 {
   static constexpr uint32_t kAhead = AHEAD;
-  alignas(128) uint8_t ring[TeamRing::kBytes];
+  alignas(128) uint8_t ring[TeamRing::kAlloc];
   uint32_t info[kBlocks * kBlockBytes];  // of a header that starts here: bytes (12 bits), values; 0: not a usual one
   TeamBatch<kV2Items> batch[2];
   uint32_t prepared, ords;  // blocks done

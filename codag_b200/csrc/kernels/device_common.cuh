@@ -167,23 +167,28 @@ __device__ __forceinline__ uint64_t warp_scan_add64(uint64_t v, uint32_t lane) {
 
 __device__ __forceinline__ uint32_t lanemask_lt(uint32_t lane) { return (1u << lane) - 1u; }
 
+// big-endian word at a shared address
+__device__ __forceinline__ uint32_t be_s32(uint32_t a) { return __byte_perm(ld_s32(a), 0, 0x0123); }
+
+__host__ __device__ constexpr uint32_t align_up(uint32_t v, uint32_t a) { return (v + a - 1) / a * a; }
+
 // ---------------------------------------------------------------------------------------
 // TMA input ring
 // ---------------------------------------------------------------------------------------
 constexpr uint32_t kSlotLog2 = 10;
 constexpr uint32_t kSlotBytes = 1u << kSlotLog2;
 
-// MIRROR: the buffer is kMirror bytes longer and repeats its first bytes behind its end, so that a
-// few words that follow one another in the stream can be read from one masked address.
-template <int NSLOT, bool MIRROR = false>
+// The buffer is kMirror bytes longer and repeats its first bytes behind its end, so that a few words
+// that follow one another in the stream are read from one masked address.
+template <int NSLOT>
 struct InRing {
   static constexpr uint32_t kBytes = NSLOT * kSlotBytes;
   static constexpr uint32_t kMask = kBytes - 1;
   static constexpr uint32_t kMirror = 16;
-  static constexpr uint32_t kAlloc = kBytes + (MIRROR ? kMirror : 0u);
+  static constexpr uint32_t kAlloc = kBytes + kMirror;
   static_assert((NSLOT & (NSLOT - 1)) == 0, "ring depth must be a power of two");
 
-  uint8_t* buf;            // kBytes of shared memory, 16-byte aligned
+  uint8_t* buf;            // kAlloc bytes of shared memory, 16-byte aligned
   uint32_t sbuf;           // shared-space address of buf
   uint64_t* bar;           // NSLOT mbarriers
   const uint8_t* gbase;    // stream start rounded down to 16 bytes
@@ -234,13 +239,13 @@ struct InRing {
       const uint32_t p = tail_lo + lane;
       if (p < hi) {
         st_s8(sbuf + (p & kMask), gbase[p]);
-        if (MIRROR && (p & kMask) < kMirror) st_s8(sbuf + kBytes + (p & kMask), gbase[p]);
+        if ((p & kMask) < kMirror) st_s8(sbuf + kBytes + (p & kMask), gbase[p]);
       }
     }
     if (lane == 0) {
       fence_proxy_async_smem();
       // a slot that wraps to the buffer's start (never the stream's first, so its body starts with it)
-      const bool again = MIRROR && r == 0 && s != 0 && bytes >= kMirror;
+      const bool again = r == 0 && s != 0 && bytes >= kMirror;
       mbar_arrive_expect_tx(&bar[r], again ? bytes + kMirror : bytes);
       if (bytes) bulk_g2s(buf + (a & kMask), gbase + a, bytes, &bar[r]);
       if (again) bulk_g2s(buf + kBytes, gbase + a, kMirror, &bar[r]);
@@ -311,51 +316,37 @@ struct InRing {
 
   __device__ __forceinline__ uint32_t rd8(uint32_t p) const { return ld_s8(sbuf + (p & kMask)); }
   __device__ __forceinline__ uint32_t rd32(uint32_t p4) const { return ld_s32(sbuf + (p4 & kMask)); }
+  // shared address of the aligned word at or before p; the next three words follow it
+  __device__ __forceinline__ uint32_t word_at(uint32_t p) const { return sbuf + (p & (kMask & ~3u)); }
   // bytes p..p+7, little-endian
   __device__ __forceinline__ uint64_t peek_le64(uint32_t p) const {
-    const uint32_t a = p & ~3u;
-    const uint32_t w0 = rd32(a), w1 = rd32(a + 4), w2 = rd32(a + 8);
-    const uint64_t v = (static_cast<uint64_t>(w1) << 32) | w0;
-    const uint32_t sh = (p & 3u) * 8u;
-    return sh ? (v >> sh) | (static_cast<uint64_t>(w2) << (64 - sh)) : v;
+    const uint32_t a = word_at(p), sh = (p & 3u) * 8u;
+    const uint32_t w0 = ld_s32(a), w1 = ld_s32(a + 4), w2 = ld_s32(a + 8);
+    return (static_cast<uint64_t>(__funnelshift_r(w1, w2, sh)) << 32) | __funnelshift_r(w0, w1, sh);
   }
   // bytes p..p+7 as a big-endian value (byte p on top): two byte permutes of three aligned words
   __device__ __forceinline__ uint64_t peek_be64(uint32_t p) const {
-    const uint32_t a = p & ~3u, sel = 0x0123u + 0x1111u * (p & 3u);
-    const uint32_t w0 = rd32(a), w1 = rd32(a + 4), w2 = rd32(a + 8);
+    const uint32_t a = word_at(p), sel = 0x0123u + 0x1111u * (p & 3u);
+    const uint32_t w0 = ld_s32(a), w1 = ld_s32(a + 4), w2 = ld_s32(a + 8);
     return (static_cast<uint64_t>(__byte_perm(w0, w1, sel)) << 32) | __byte_perm(w1, w2, sel);
   }
   // bytes p..p+3 as a big-endian word (byte p on top): one byte permute of two aligned words
   __device__ __forceinline__ uint32_t peek_be32(uint32_t p) const {
-    const uint32_t a = p & ~3u;
-    return __byte_perm(rd32(a), rd32(a + 4), 0x0123u + 0x1111u * (p & 3u));
+    const uint32_t a = word_at(p);
+    return __byte_perm(ld_s32(a), ld_s32(a + 4), 0x0123u + 0x1111u * (p & 3u));
   }
   // bytes p..p+3, little-endian (two aligned loads)
   __device__ __forceinline__ uint32_t peek_le32(uint32_t p) const {
-    const uint32_t a = p & ~3u;
-    return __funnelshift_r(rd32(a), rd32(a + 4), (p & 3u) * 8u);
-  }
-  // big-endian 32-bit word at a 4-byte aligned position
-  __device__ __forceinline__ uint32_t be32(uint32_t p4) const { return __byte_perm(rd32(p4), 0, 0x0123); }
-  // w (1..32) bits at stream bit bitpos, most significant bit first (two aligned loads)
-  __device__ __forceinline__ uint32_t msb_bits32(uint32_t bitpos, uint32_t w) const {
-    const uint32_t a = (bitpos >> 5) << 2;
-    const uint32_t top = __funnelshift_l(be32(a + 4), be32(a), bitpos & 31u);
-    return top >> (32u - w);
+    const uint32_t a = word_at(p);
+    return __funnelshift_r(ld_s32(a), ld_s32(a + 4), (p & 3u) * 8u);
   }
   // w (1..64) bits at stream bit bitpos, most significant bit first (three aligned loads
   // cover the 64 bits that start anywhere within the first word)
   __device__ __forceinline__ uint64_t msb_bits64(uint32_t bitpos, uint32_t w) const {
-    const uint32_t a = (bitpos >> 5) << 2, s = bitpos & 31u;
-    const uint32_t w0 = be32(a), w1 = be32(a + 4), w2 = be32(a + 8);
+    const uint32_t a = word_at(bitpos >> 3), s = bitpos & 31u;
+    const uint32_t w0 = be_s32(a), w1 = be_s32(a + 4), w2 = be_s32(a + 8);
     const uint64_t v = (static_cast<uint64_t>(__funnelshift_l(w1, w0, s)) << 32) | __funnelshift_l(w2, w1, s);
     return v >> (64u - w);
-  }
-  // `w` (1..64) bits starting at stream bit `bitpos`, most significant bit first; the field
-  // must fit in the 8 bytes at bitpos/8, which holds for every ORC RLE v2 width.
-  __device__ __forceinline__ uint64_t bits_be(uint32_t bitpos, uint32_t w) const {
-    const uint64_t be = peek_be64(bitpos >> 3);
-    return (be << (bitpos & 7u)) >> (64u - w);
   }
 };
 

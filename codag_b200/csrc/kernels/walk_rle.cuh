@@ -369,7 +369,7 @@ __device__ int expand_rlev2_range(InRing<NSLOT>& in, OUT& out, const RleDesc* __
         if (pll) {
           __syncwarp();
           const uint32_t cfb = v2_closest(pw + ((fourth >> 5) & 7u) + 1u);
-          st = body_patches<NSLOT, E>(in, out, n, cnt, fbw, pw, cfb, pll, a, (data + (cnt * fbw + 7u) / 8u) * 8u, lane);
+          st = body_patches<NSLOT, E>(in, out, n, cnt, fbw, pw, cfb, pll, a, data * 8u, (data + (cnt * fbw + 7u) / 8u) * 8u, lane);
           if (st) break;
         }
       }
