@@ -12,7 +12,9 @@
 // start + (w - first row) * popc(mask) + popc(mask & lanes below t) by itself.  Then every
 // lane decodes its own substream and writes its values straight to their interleaved places
 // in global memory.  The small table leaves occupancy to the registers, so many chunks' lanes
-// wait on their word loads at once.  Header semantics are CODAG's (the oracle's restatement of
+// wait on their word loads at once.  Where there are few chunks, two or four warps share one's substreams.
+// 256 MiB of 64-bit values: 650 us with byte-wise headers and fields, 433 now; a value takes a warp some
+// 160 instructions, about half of them for the headers that one lane or another is at.  Header semantics are CODAG's (the oracle's restatement of
 // decoder_new.h:1000-1184, quirks included: the uint8_t run length, the 32-bit patch mask, the
 // arithmetic-shift zigzag and the DELTA direction taken from the base delta).
 #include <cuda_runtime.h>
@@ -33,7 +35,7 @@ struct Segments {
   uint32_t hi[32], lo[32], mask[32], words[32];
 };
 
-constexpr uint32_t kWarps = 4;  // chunks (warps) per block
+constexpr uint32_t kWarps = 4;  // warps per block
 
 struct LaneReader {
   const uint32_t* region;  // the chunk's region (128-byte aligned)
@@ -195,14 +197,13 @@ constexpr int kEnd = -1;
 constexpr uint32_t kAhead = 512;  // words
 
 template <typename T>
-__device__ int decode_substream(LaneReader& r, LaneOut<T>& o) {
+__device__ int decode_substream(LaneReader& r, LaneOut<T>& o, bool go) {
   constexpr uint64_t M = sizeof(T) == 8 ? ~0ull : ((1ull << (8 * sizeof(T))) - 1ull);
   uint32_t rem = 0, fbw = 0;
   uint64_t v = 0, bd = 0;  // repeat: the value; delta: running value and base delta; patched: base
   bool bits = false, acc = false, sub = false, patched = false;
   uint32_t pw = 0, pgw = 0, pll = 0, base_out = 0;  // patched: patch width, gap width, list length
   int st = CODAG_OK;
-  bool go = true;
   // The lanes go through the region together, so what they read next is brought into L1 4 KiB at a time, a
   // line by each lane.  (A word loaded ahead into a register costs the warp its latency all the same:
   // whichever lane needs one waits for the last lane's load.)
@@ -330,29 +331,31 @@ __device__ __forceinline__ uint32_t needed(uint32_t t, uint32_t ru, uint32_t sto
   return g * ru + (rem > lo ? (rem - lo < ru ? rem - lo : ru) : 0u);
 }
 
-template <typename T>
+// SPLIT warps share a chunk
+template <typename T, uint32_t SPLIT>
 __global__ void __launch_bounds__(32 * kWarps)
     k_rlev2_transposed(const uint8_t* __restrict__ comp, uint64_t comp_bytes, const uint64_t* __restrict__ blk_off,
                        const uint64_t* __restrict__ col_len, uint64_t n_chunks, uint64_t chunk_bytes, uint32_t ru,
                        uint8_t* __restrict__ out, uint64_t out_bytes, int32_t* __restrict__ status,
                        uint32_t max_words) {
   __shared__ Segments segs[kWarps];
+  __shared__ uint32_t part[kWarps];  // the warps' statuses
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  const uint64_t c = static_cast<uint64_t>(blockIdx.x) * (blockDim.x >> 5) + warp;
-  if (c >= n_chunks) return;
+  const uint64_t c = (static_cast<uint64_t>(blockIdx.x) * kWarps + warp) / SPLIT;
+  const bool real = c < n_chunks;
   Segments* seg = segs + warp;
-  const uint64_t len64 = col_len[32 * c + lane];
+  const uint64_t len64 = real ? col_len[32 * c + lane] : 0;
   const uint32_t words = static_cast<uint32_t>(len64 < (1ull << 34) ? (len64 + 3) / 4 : 0xffffffffu);
   const uint32_t maxw = __reduce_max_sync(FULL, words);
   const uint64_t total = 4ull * __reduce_add_sync(FULL, words);
-  const uint64_t off = blk_off[c];
+  const uint64_t off = real ? blk_off[c] : 0;
   int st = CODAG_OK;
   if (maxw > max_words || (off & 3u) || off > comp_bytes || total > comp_bytes - off) st = CODAG_ECORRUPT;
   const uint64_t base_e = c * (chunk_bytes / sizeof(T));
   const uint64_t store_b = c * chunk_bytes < out_bytes ? (out_bytes - c * chunk_bytes < chunk_bytes
                                                              ? out_bytes - c * chunk_bytes : chunk_bytes) : 0;
   const uint32_t store = static_cast<uint32_t>(store_b / sizeof(T));
-  if (st == CODAG_OK) {
+  if (st == CODAG_OK && real) {
     // one segment per distinct word count: each pass drops at least one substream, so at most 32
     uint32_t run = 0, row = 0, ns = 0;
     for (uint32_t m = __ballot_sync(FULL, words > 0); m; m = __ballot_sync(FULL, words > row)) {
@@ -368,16 +371,33 @@ __global__ void __launch_bounds__(32 * kWarps)
       ns++;
     }
     __syncwarp();
-    LaneReader r{reinterpret_cast<const uint32_t*>(comp + off), seg, run, (1u << lane) - 1u,
-                 static_cast<uint32_t>(len64), words, 0, 0xffffffffu, 0};
-    LaneOut<T> o{reinterpret_cast<T*>(out) + base_e, lane, ru,
-                 static_cast<uint32_t>(chunk_bytes / sizeof(T) / 32), store, 0, lane * ru, 0, false};
-    int s = decode_substream<T>(r, o);
-    if (s == CODAG_OK && o.n < needed(lane, ru, store)) s = CODAG_ECORRUPT;
+    // this warp's substreams, one for each of the first lanes
+    constexpr uint32_t kLanes = 32u / SPLIT;
+    const bool mine = lane < kLanes;
+    const uint32_t t = SPLIT == 1 ? lane : (warp % SPLIT) * kLanes + lane % kLanes;
+    LaneReader r{reinterpret_cast<const uint32_t*>(comp + off), seg, run, (1u << t) - 1u,
+                 __shfl_sync(FULL, static_cast<uint32_t>(len64), t), __shfl_sync(FULL, words, t), 0, 0xffffffffu, 0};
+    LaneOut<T> o{reinterpret_cast<T*>(out) + base_e, t, ru,
+                 static_cast<uint32_t>(chunk_bytes / sizeof(T) / 32), store, 0, t * ru, 0, false};
+    int s = decode_substream<T>(r, o, mine);
+    if (s == CODAG_OK && mine && o.n < needed(t, ru, store)) s = CODAG_ECORRUPT;
     st = __reduce_max_sync(FULL, static_cast<uint32_t>(s));
   }
-  if (status && lane == 0) status[c] = st;
+  if (SPLIT > 1) {
+    if (lane == 0) part[warp] = static_cast<uint32_t>(st);
+    __syncthreads();
+    if (lane < SPLIT) st = max(st, static_cast<int>(part[warp / SPLIT * SPLIT + lane]));
+    st = __reduce_max_sync(FULL, static_cast<uint32_t>(st));
+  }
+  if (status && real && lane == 0 && warp % SPLIT == 0) status[c] = st;
 }
+
+// Up to how many chunks four warps with eight substreams each, or two with sixteen, are faster than one with
+// all 32.  With fewer lanes a pass meets fewer headers, at the price of issue slots.  Measured, us, one | two |
+// four warps, 64-bit values: 300 chunks 351 | 305 | 269, 600 395 | 342 | 323, 900 395 | 352 | 382,
+// 1200 406 | 385 | 556, 2048 451 | 463 | 717; 8-bit: 600 2718 | 2495 | 2485, 900 2907 | 2708 | 3052,
+// 1200 2914 | 2949 | 3933.
+constexpr uint64_t kQuarter = 4 * 148, kHalf = 7 * 148;
 
 bool valid_elem(int e) { return e == 1 || e == 2 || e == 4 || e == 8; }
 
@@ -387,11 +407,11 @@ codag_status launch(const uint8_t* comp, uint64_t comp_bytes, const uint64_t* bl
                     cudaStream_t s) {
   // a substream is at most about twice its share of the chunk (the encoders' bound), in words
   const uint32_t max_words = static_cast<uint32_t>((chunk / 32 * 2 + 1024) / 4);
-  const uint64_t grid = (n + kWarps - 1) / kWarps;
+  const uint64_t split = n <= kQuarter ? 4 : n <= kHalf ? 2 : 1, grid = (n * split + kWarps - 1) / kWarps;
   if (grid > 0x7fffffffull) return CODAG_EINVAL;
-  k_rlev2_transposed<T><<<static_cast<unsigned>(grid), 32 * kWarps, 0, s>>>(comp, comp_bytes, blk_off, col_len, n,
-                                                                            chunk, ru, out, out_bytes, status,
-                                                                            max_words);
+  auto kern = split == 4 ? k_rlev2_transposed<T, 4> : split == 2 ? k_rlev2_transposed<T, 2> : k_rlev2_transposed<T, 1>;
+  kern<<<static_cast<unsigned>(grid), 32 * kWarps, 0, s>>>(comp, comp_bytes, blk_off, col_len, n, chunk, ru, out, out_bytes,
+                                                           status, max_words);
   return cudaGetLastError() == cudaSuccess ? CODAG_OK : CODAG_ECUDA;
 }
 
