@@ -229,15 +229,21 @@ namespace {
 constexpr uint64_t rle_ws_counts_bytes(uint64_t n) { return (n * 4 + 255) / 256 * 256; }
 constexpr uint64_t rle_ws_bytes(uint64_t n) { return rle_ws_counts_bytes(n) + n * kDescPerChunk * sizeof(RleDesc); }
 
+constexpr uint64_t kSms = 148;
+
 template <int NSLOT, int CODEC, int E, bool DIRECT>
 codag_status launch_rle_out(const codag_tune& t, const uint8_t* comp, uint64_t comp_bytes, const uint64_t* blk_off,
                             const uint64_t* col_len, uint64_t n, uint64_t chunk_bytes, uint8_t* out,
                             uint64_t out_bytes, int32_t* status, void* ws, uint64_t ws_bytes, cudaStream_t s) {
   using L = std::conditional_t<DIRECT, RleDirectLayout<NSLOT>, RleLayout<NSLOT>>;
-  const uint32_t smem = L::kPerWarp * t.warps_per_cta;
+  // With more chunks than warps are resident (32 per SM), CTAs of at most four warps: a slot is taken again
+  // as soon as its four are done (RLE v2, 1 GiB of 64-bit values 438 us with eight, 428 with four, 700 MB of 32-bit
+  // values 615 | 595; 256 MiB, all resident at once, 190 | 191).
+  const int warps = n > 32 * kSms && t.warps_per_cta > 4 ? 4 : t.warps_per_cta;
+  const uint32_t smem = L::kPerWarp * warps;
   auto kern = k_rle_plain<NSLOT, CODEC, E, DIRECT>;
   if (allow_smem(kern, smem) != cudaSuccess) return CODAG_ECUDA;
-  const uint64_t grid = (n + t.warps_per_cta - 1) / t.warps_per_cta;
+  const uint64_t grid = (n + warps - 1) / warps;
   if (grid > 0x7fffffffull) return CODAG_EINVAL;
   uint32_t* counts = nullptr;
   RleDesc* descs = nullptr;
@@ -247,9 +253,8 @@ codag_status launch_rle_out(const codag_tune& t, const uint8_t* comp, uint64_t c
     k_rle_walk<CODEC><<<static_cast<unsigned>((n + 127) / 128), 128, 0, s>>>(
         comp, comp_bytes, blk_off, col_len, n, static_cast<uint32_t>(chunk_bytes / E), counts, descs);
   }
-  kern<<<static_cast<unsigned>(grid), 32 * t.warps_per_cta, smem, s>>>(comp, comp_bytes, blk_off, col_len, n,
-                                                                         chunk_bytes, out, out_bytes, status,
-                                                                         wait_of(), counts, descs);
+  kern<<<static_cast<unsigned>(grid), 32 * warps, smem, s>>>(comp, comp_bytes, blk_off, col_len, n, chunk_bytes, out, out_bytes,
+                                                             status, wait_of(), counts, descs);
   return finish_launch();
 }
 
@@ -272,7 +277,6 @@ codag_status launch_rle_team(const uint8_t* comp, uint64_t comp_bytes, const uin
 //   RLE v2 (the look-ahead reads every byte as a header, which pays while SMs have room for it): 64-bit
 //   values: 32 chunks 80 | 138, 400 146 | 157, 640 204 | 175; 16 bits: 32 168 | 424, 400 370 | 479,
 //   640 527 | 484; 8 bits: 640 808 | 825, 1280 1389 | 884
-constexpr uint64_t kSms = 148;
 template <int CODEC>
 constexpr uint64_t kTeamChunks = CODEC == CODAG_CODEC_RLEV2 ? 3 * kSms : ~0ull;
 
