@@ -53,13 +53,15 @@ WORKLOADS = {
     "rlev1x128": dict(codec=0, n=134_217_728, elem=8, desc="ORC RLE v1, 134,217,728 uint64 (1 GiB), 8192 x 128 KiB chunks"),
     "deflate": dict(codec=2, n=1 << 30, elem=1, desc="Deflate (zlib level 6), 1 GiB Zipf text, 8192 x 128 KiB chunks"),
 }
-KERNEL_NAMES = {0: "k_rle_plain<.., RLEV1>", 1: "k_rle_plain<.., RLEV2>", 2: "k_inflate_plain"}
+TEAM_CHUNKS = 444  # up to this many RLE v2 chunks have a CTA each, RLE v1 chunks at any count
 
 
-def _kernel_name(codec: int, t) -> str:
-    if codec != 2:
-        return "k_rle_cta<RLEV1/RLEV2, E>" if t.cta_per_chunk else KERNEL_NAMES[codec]
-    return "k_inflate_cta" if t.cta_per_chunk else KERNEL_NAMES[codec]
+def _kernel_name(codec: int, t, n: int, two_pass: bool) -> str:
+    if codec == 2:
+        return "k_inflate"
+    name = "RLEV2" if codec else "RLEV1"
+    team = not two_pass and (t.cta_per_chunk or codec == 0 or n <= TEAM_CHUNKS)
+    return f"k_rle_team<{name}>" if team else f"k_rle_plain<.., {name}>"
 
 
 EXTRA_CONFIGS = ("rlev2", "rlev1", "rlev1x128", "deflate")
@@ -334,7 +336,7 @@ def measure_codec(workload: str, args, rank: int, world: int, local: int, steps:
         "gpu_launches": steps * (2 if codec != 2 and args.rle_passes == 2 else 1),
         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                      "frac": round(achieved / peak, 4), "traffic": ncu_traffic(workload), "peak_kind": peak_kind,
-                     "kernel": _kernel_name(codec, t),
+                     "kernel": _kernel_name(codec, t, n, d_ws is not None),
                      "alg_bytes_per_launch": alg_bytes,
                      "note": ("launch = header walk + expansion kernels of one call" if codec != 2 and args.rle_passes == 2
                               else "one kernel"),

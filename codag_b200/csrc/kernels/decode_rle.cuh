@@ -2,14 +2,16 @@
 //
 // CODAG decodes these with one lane walking the stream byte by byte while the other lanes
 // idle or store the same addresses (include/rlev1/decoder.h:588-798,
-// include/rlev2/decoder_new.h:909-1187).  Here each chunk is decoded in two passes when a
-// workspace is available (walk_rle.cuh):
+// include/rlev2/decoder_new.h:909-1187).  Here a chunk has a CTA where that pays (decode_rle_team.cuh),
+// else it is decoded in two passes when a workspace is available (walk_rle.cuh):
 //   1. a header walk, one THREAD per chunk (so one warp instruction advances 32 chunks),
 //      writes a 32-byte descriptor per header;
 //   2. one WARP per chunk expands the headers: descriptors arrive 32 at a time with one
 //      coalesced load, and each header's values are produced lane-parallel.
-// Without a workspace the same warp parses the headers itself (decode_rlev*_chunk).
-// Lane-parallel value expansion, shared by both paths:
+// Without a workspace the same warp parses the headers itself (decode_rlev*_chunk): RLE v2, 1 GiB of
+// 64-bit values in 440 us, 206 warp instructions a header (91 values on average): 38 of them branches and 30
+// compares; the issue slots are 76% busy.  Without expanding any value it still takes 300 us.
+// Lane-parallel value expansion, shared by all paths:
 //   - RLE v1 runs, RLE v2 SHORT_REPEAT and fixed-step DELTA: one arithmetic value per lane;
 //   - RLE v1 literal groups: 128 stream bytes per step, 4 bytes per lane; one ballot per byte
 //     lane finds the varint ends and the lane holding an end decodes that varint in registers
@@ -48,11 +50,6 @@ __device__ __forceinline__ constexpr uint64_t emask() {
 template <int E, class OUT>
 __device__ __forceinline__ void put_elem(OUT& o, uint32_t idx, uint64_t v) {
   o.template put<E>(idx * static_cast<uint32_t>(E), v);
-}
-
-template <int E, class OUT>
-__device__ __forceinline__ uint64_t get_elem(const OUT& o, uint32_t idx) {
-  return o.template get<E>(idx * static_cast<uint32_t>(E));
 }
 
 // LEB128 payload of the first `len` bytes of a little-endian window (len 1..8)
@@ -222,7 +219,7 @@ __device__ __forceinline__ void body_delta_packed(const InRing<NSLOT>& in, OUT& 
 
 // PATCHED_BASE patch list (decoder_new.h:1142-1182), applied to the len8 values at n, which were unpacked from
 // bit `val0` on.  A patched value's field is read again from the ring: reading the value back from global memory
-// made the warp wait for its own store (1 GiB of 64-bit values 449 us, @NEW@ now).
+// made the warp wait for its own store (1 GiB of 64-bit values 449 us, 440 now).
 template <int NSLOT, int E, class OUT>
 __device__ __forceinline__ int body_patches(const InRing<NSLOT>& in, OUT& out, uint32_t n, uint32_t len8, uint32_t fbw,
                                             uint32_t pw, uint32_t cfb, uint32_t pll, uint64_t base, uint32_t val0,

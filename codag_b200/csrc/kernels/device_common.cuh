@@ -461,14 +461,6 @@ struct OutRing {
     else if constexpr (E == 2) st_s16(a, static_cast<uint32_t>(v));
     else st_s8(a, static_cast<uint32_t>(v));
   }
-  template <int E>
-  __device__ __forceinline__ uint64_t get(uint32_t off) const {
-    const uint32_t a = sbuf + (off & kMask);
-    if constexpr (E == 8) return ld_s64(a);
-    else if constexpr (E == 4) return ld_s32(a);
-    else if constexpr (E == 2) return ld_s16(a);
-    else return ld_s8(a);
-  }
 };
 
 // Output straight to global memory: lane i of a warp store writes element n + i, so one warp
@@ -506,15 +498,6 @@ struct DirectOut {
     else if constexpr (E == 2) *reinterpret_cast<uint16_t*>(a) = static_cast<uint16_t>(v);
     else *a = static_cast<uint8_t>(v);
   }
-  template <int E>
-  __device__ __forceinline__ uint64_t get(uint32_t off) const {
-    if (off >= store) return 0;  // never stored: the patch result is dropped as well
-    const uint8_t* a = gdst + off;
-    if constexpr (E == 8) return *reinterpret_cast<const uint64_t*>(a);
-    else if constexpr (E == 4) return *reinterpret_cast<const uint32_t*>(a);
-    else if constexpr (E == 2) return *reinterpret_cast<const uint16_t*>(a);
-    else return *a;
-  }
 };
 
 // Output that is not element aligned, stored straight to global memory byte by byte (a
@@ -539,14 +522,6 @@ struct ByteOut {
 #pragma unroll
     for (int i = 0; i < E; i++)
       if (off + i < store) gdst[off + i] = static_cast<uint8_t>(v >> (8 * i));
-  }
-  template <int E>
-  __device__ __forceinline__ uint64_t get(uint32_t off) const {
-    uint64_t v = 0;
-#pragma unroll
-    for (int i = 0; i < E; i++)
-      if (off + i < store) v |= static_cast<uint64_t>(gdst[off + i]) << (8 * i);
-    return v;
   }
 };
 

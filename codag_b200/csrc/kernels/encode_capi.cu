@@ -26,6 +26,10 @@
 // the back warps measure the items of the tile before, one warp per item, sum the sizes, and write
 // the items' bytes.  With one warp per chunk running the state machine, an item cost about 9000 warp
 // instructions and a chunk had one warp to wait for.
+//
+// RLE v2, 256 MiB of 64-bit values: 3.75 ms with a warp per chunk, 1.07 now (2 CTAs of 16 warps per SM,
+// which registers allow; 3 or 4 with fewer registers each: 1.26, 1.40; one front warp: 1.26).  RLE v1,
+// 20 MB of 32-bit values: 1.60 ms, 0.13 now.
 #include <cuda_runtime.h>
 
 #include <cstdint>

@@ -167,11 +167,9 @@ def poisson_arrivals(rate: float, duration: float, n_files: int, seed: int):
     return list(zip(t.tolist(), rng.integers(0, n_files, t.size).tolist()))
 
 
-# Launch shapes (warps_per_cta, ring_slots, lut_bits, cta_per_chunk) tried by tune_server.  The
-# per-file Deflate default (2 warps per CTA) holds too few warps per SM for a loop whose launches
-# carry thousands of 128 KiB chunks: 36.6 GB/s against 60.0 GB/s with 8 warps per CTA at
-# 2000 requests per second on one B200.
-SERVE_SHAPES = [(w, 4, lb, 0) for w in (2, 4, 8) for lb in (9, 10)]
+# Launch shapes (warps_per_cta, ring_slots, lut_bits, cta_per_chunk) tried by tune_server: the
+# launch has one shape, whatever these say.
+SERVE_SHAPES = [(8, 4, 10, 0)]
 
 
 def tune_server(srv: "Server", n_requests: int = 96, seed: int = 7, use_cache: bool = True):

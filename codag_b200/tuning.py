@@ -2,13 +2,11 @@
 
 Per codec it times every supported combination of
   warps_per_cta  chunks decoded by one CTA (one warp per chunk): 1, 2, 4, 8
-  ring_slots     depth of the TMA input ring in 1 KiB slots: 4, 8 (2 also for Deflate)
-  lut_bits       primary Huffman table width (Deflate only): 9, 10, 11
-  cta_per_chunk  RLE only: a whole CTA of 4 or 8 warps per chunk instead of one warp
-on a resident sample of the caller's chunks, keeps the fastest, installs it with
+  ring_slots     depth of the TMA input ring in 1 KiB slots: 4, 8
+  cta_per_chunk  RLE v2: a whole CTA per chunk instead of one warp, whatever their number
+(Deflate chunks and batched plans have one shape, which the tune fields do not change) on a resident sample of the caller's chunks, keeps the fastest, installs it with
 codag_set_tune and caches it in a JSON file keyed by GPU name and codec, so later runs
-on the same kind of GPU skip the search.  Batched plans take their shape the same way
-(codag_batch_plan's tune argument), searched over a sample of the batch.
+on the same kind of GPU skip the search.
 """
 from __future__ import annotations
 
@@ -25,22 +23,16 @@ CACHE = Path(os.environ.get("CODAG_TUNE_CACHE", Path(__file__).resolve().parent 
 
 
 def candidates(codec: int):
-    warps = (1, 2, 4, 8)
     if codec == native.DEFLATE:
-        # one warp per chunk, or a decoder and an expander warp per chunk (1, 2 or 4 pairs per CTA)
-        return (list(itertools.product(warps, (2, 4, 8), (9, 10, 11), (0,))) +
-                list(itertools.product((2, 4, 8), (4,), (9, 10), (1,))))
-    # one warp per chunk, or one CTA of 4 or 8 warps per chunk
-    return list(itertools.product(warps, (4, 8), (10,), (0,))) + [(4, 4, 10, 1), (8, 4, 10, 1)]
+        return [(2, 2, 9, 0)]
+    # one warp per chunk, or one CTA per chunk
+    return list(itertools.product((1, 2, 4, 8), (4, 8), (10,), (0,))) + [(8, 4, 10, 1)]
 
 
 def batch_candidates():
-    """Launch shapes of the batched kernel: (warps_per_cta, ring_slots, lut_bits, cta_per_chunk,
-    table_global).  RLE files need rings of at least 4 slots; with cta_per_chunk = k the Deflate
-    files of at least k x 256 KiB go to warp pairs (so the warp count is even); table_global
-    places the Huffman lookup tables in global memory (through L1) rather than shared memory."""
-    return (list(itertools.product((2, 4, 8), (4, 8), (9, 10, 11), (0,), (0, 1))) +
-            list(itertools.product((4, 8), (4,), (9, 10, 11), (1, 2, 3), (0,))))
+    """Launch shapes of the batched kernel (warps_per_cta, ring_slots, lut_bits, cta_per_chunk,
+    table_global): there is one, which a plan picks by the sizes of its files."""
+    return [(8, 4, 10, 0, 0)]
 
 
 def _key(codec: int, tag: str) -> str:

@@ -169,30 +169,24 @@ codag_status codag_compress_rlev2(const uint8_t *d_in, uint64_t in_bytes, uint64
                                   void *d_workspace, uint64_t workspace_bytes, codag_stream_t stream);
 
 /* --- launch tuning --------------------------------------------------------------------
- * Process-wide launch shape for the per-file calls above, per codec.  warps_per_cta is
- * the number of chunks one CTA decodes (one warp per chunk, 1..8); ring_slots the depth of
- * the TMA input ring (2, 4 or 8 slots of 1 KiB; the RLE codecs need at least 4 because an
- * RLE v2 header with its data spans up to 2060 bytes); lut_bits the primary Huffman table width
- * (Deflate only: 9, 10 or 11), which also sizes the shared-memory history window of the
- * Deflate call (9: 1 KiB, so more warps fit per SM, for many chunks; 10 and 11: 2 KiB, fewer
- * instructions per chunk, for few chunks).  cta_per_chunk (0 or 1) shortens the decode of a single
- * chunk (few chunks, e.g. an 8 MiB column, or large files) at the cost of throughput on many:
- * for the RLE calls without a workspace it runs one CTA of warps_per_cta warps per chunk (the
- * CTA stages the chunk's stream in shared memory, one warp walks its headers and all warps
- * expand them; applies when the output and out_bytes are element aligned); for Deflate a
- * chunk takes two warps, one decoding its symbols into tokens and one expanding them into
- * bytes, warps_per_cta/2 chunks per CTA (warps_per_cta even).  Values outside the supported
- * sets return CODAG_EINVAL. */
+ * Process-wide launch shape for the per-file calls above, per codec.  It applies to the RLE
+ * kernels that give each chunk one warp: RLE v2 with more than 444 chunks, calls with a
+ * workspace, and outputs that are not element aligned.  warps_per_cta is the number of chunks
+ * one CTA decodes (1..8); ring_slots the depth of the TMA input ring (2, 4 or 8 slots of 1 KiB;
+ * the RLE codecs need at least 4 because an RLE v2 header with its data spans up to 2060 bytes).
+ * cta_per_chunk = 1 gives each RLE v2 chunk a whole CTA whatever their number (fewer chunks, and
+ * RLE v1 chunks, have one without being asked; it applies without a workspace, when the output
+ * and out_bytes are element aligned).  Deflate chunks are always decoded by a team of six warps
+ * each: their shape, and lut_bits (9, 10 or 11), are checked and kept, and change nothing.
+ * Values outside the supported sets return CODAG_EINVAL. */
 typedef struct {
     int32_t warps_per_cta;
     int32_t ring_slots;
     int32_t lut_bits;
     int32_t cta_per_chunk;
-    int32_t table_global; /* batched plans only (0 or 1): the Huffman lookup tables of every warp in
-                             global memory, read through L1, instead of shared memory; frees
-                             3-9 KiB of shared memory per warp for more resident warps.  The
-                             per-file calls and codag_batch_launch keep them in shared memory
-                             (0; other values give CODAG_EINVAL). */
+    int32_t table_global; /* accepted by batched plans (0 or 1), where it changes nothing; the
+                             per-file calls and codag_batch_launch take 0 (other values give
+                             CODAG_EINVAL) */
 } codag_tune;
 
 codag_status codag_set_tune(int codec, const codag_tune *tune);
@@ -226,9 +220,10 @@ typedef struct {
 typedef struct codag_plan codag_plan;
 
 /* Copies the descriptors to the device (the only allocating call), orders the queue and
- * picks the launch shape (tune may be NULL: 8 warps per CTA, 4 ring slots, 10-bit tables).  In a plan,
- * tune->cta_per_chunk = k (1..4, warps_per_cta even) sends the Deflate chunks of at least
- * k x 256 KiB to warp pairs (a symbol decoder and a byte expander each), decoded first. */
+ * picks the launch shape by their sizes: Deflate streams, and RLE streams of more than 32 KiB,
+ * are decoded by six warps together, longest first, short RLE streams by a warp each.  tune (may
+ * be NULL) is checked as before (cta_per_chunk 0..4, with an even warps_per_cta unless 0) and
+ * changes nothing. */
 codag_status codag_batch_plan(const codag_chunk_desc *h_descs, uint64_t n, const codag_tune *tune,
                               codag_plan **plan);
 /* One persistent launch over all planned chunks; d_status has n entries (may be NULL).
