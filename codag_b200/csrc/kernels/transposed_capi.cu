@@ -12,9 +12,10 @@
 // start + (w - first row) * popc(mask) + popc(mask & lanes below t) by itself.  Then every
 // lane decodes its own substream and writes its values straight to their interleaved places
 // in global memory.  The small table leaves occupancy to the registers, so many chunks' lanes
-// wait on their word loads at once.  Where there are few chunks, two or four warps share one's substreams.
-// 256 MiB of 64-bit values: 650 us with byte-wise headers and fields, 433 now; a value takes a warp some
-// 160 instructions, about half of them for the headers that one lane or another is at.  Header semantics are CODAG's (the oracle's restatement of
+// wait on their word loads at once.  Where there are few chunks, four warps share one's substreams.
+// 256 MiB of 64-bit values: 650 us with byte-wise headers and fields, 433 with a word at a time loaded when it
+// was needed (a step from one value to the next took 600 cycles, most of it that load, which some lane or
+// other does every time), 371 with the words copied to shared memory ahead of their use.  Header semantics are CODAG's (the oracle's restatement of
 // decoder_new.h:1000-1184, quirks included: the uint8_t run length, the 32-bit patch mask, the
 // arithmetic-shift zigzag and the DELTA direction taken from the base delta).
 #include <cuda_runtime.h>
@@ -37,6 +38,7 @@ struct Segments {
 
 constexpr uint32_t kWarps = 4;  // warps per block
 
+constexpr uint32_t kFifo = 16;
 struct LaneReader {
   const uint32_t* region;  // the chunk's region (128-byte aligned)
   const Segments* seg;
@@ -45,9 +47,45 @@ struct LaneReader {
   uint32_t len, words;     // substream bytes, and words
   uint32_t p;              // next byte
   uint32_t cw, cv;         // cached word index and value
-  uint32_t far = 0;        // where in the region the last word loaded lies
-  uint32_t s;              // segment of cw (rows only grow, so it only moves forward)
+  uint32_t s;              // segment of the last word loaded by start() (rows only grow, so it only moves forward)
+  // The words to come, kFifo at most, are copied to the lane's column of shared memory ahead of their use.
+  uint32_t fifo;           // word w at fifo + 128 * (w % kFifo)
+  uint32_t issued = 0, avail = 0;  // words asked for, and known to be there
+  uint32_t next_at = 0, next_step = 0, next_hi = 0, next_s = 0;  // place of word `issued`, as start() finds it
   bool bad = false;
+
+  // Called by all lanes every few values: what was asked for last time is there by now, and the
+  // next N words, kFifo at most behind `low`, the first one still needed, are asked for.
+  template <uint32_t N>
+  __device__ __forceinline__ void top_up(uint32_t low) {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    avail = issued;
+    if (issued < low) {
+      issued = low;
+      next_hi = 0;
+    }
+    const uint32_t lim = low + kFifo < words ? low + kFifo : words;
+#pragma unroll 2
+    for (uint32_t i = 0; i < N; i++) {
+      if (issued < lim) {
+        if (issued >= next_hi) {
+          while (issued >= seg->hi[next_s]) next_s++;
+          const uint32_t m = seg->mask[next_s];
+          next_hi = seg->hi[next_s];
+          next_step = __popc(m);
+          next_at = seg->words[next_s] + (issued - seg->lo[next_s]) * next_step + __popc(m & lt);
+        }
+        if (next_at < total) {
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(fifo + 128u * (issued % kFifo)), "l"(region + next_at)
+                       : "memory");
+          issued++;
+          next_at += next_step;
+        }
+      }
+    }
+  }
+  __device__ __forceinline__ uint32_t ahead(uint32_t w) const { return ld_s32(fifo + 128u * (w % kFifo)); }
+  __device__ __forceinline__ uint32_t word(uint32_t w) { return w < avail ? ahead(w) : __ldg(region + start(w)); }
 
   // where word w of this substream sits in the region; w < its word count <= the last
   // segment's hi keeps the walk inside the table, and the region has `total` words
@@ -59,7 +97,6 @@ struct LaneReader {
       bad = true;
       return 0;
     }
-    far = at;
     return at;
   }
 
@@ -71,29 +108,33 @@ struct LaneReader {
     const uint32_t w = p >> 2;
     if (w != cw) {
       cw = w;
-      cv = __ldg(region + start(w));
+      cv = word(w);
     }
     return (cv >> (8u * (p++ & 3u))) & 0xffu;
   }
 
   // the 16 bytes from p on, least significant first; bytes past the substream's last word are 0
   __device__ __forceinline__ void window(uint32_t* l) {
-    const uint32_t w = p >> 2, at = start(w), n = words - w;
-    const uint32_t same = seg->hi[s] - w, step = __popc(seg->mask[s]);  // words of this row segment
+    const uint32_t w = p >> 2, n = words - w;
     uint32_t x[5];
-    x[0] = __ldg(region + at);
 #pragma unroll
-    for (uint32_t i = 1; i < 5; i++) x[i] = i < n && i < same ? __ldg(region + at + i * step) : 0u;
-    if (same < 5u && same < n) {  // the others lie in later segments
-      const uint32_t s0 = s;
-      for (uint32_t i = same; i < 5u && i < n; i++) {
-        const uint32_t v = __ldg(region + start(w + i));
-        if (i == 1) x[1] = v;
-        else if (i == 2) x[2] = v;
-        else if (i == 3) x[3] = v;
-        else x[4] = v;
+    for (uint32_t i = 0; i < 5; i++) x[i] = i < n ? ahead(w + i) : 0u;
+    if (avail < (n < 5u ? words : w + 5u)) {  // not all there yet
+      const uint32_t at = start(w), same = seg->hi[s] - w, step = __popc(seg->mask[s]);  // words of this row segment
+      x[0] = __ldg(region + at);
+#pragma unroll
+      for (uint32_t i = 1; i < 5; i++) x[i] = i < n && i < same ? __ldg(region + at + i * step) : 0u;
+      if (same < 5u && same < n) {  // the others lie in later segments
+        const uint32_t s0 = s;
+        for (uint32_t i = same; i < 5u && i < n; i++) {
+          const uint32_t v = __ldg(region + start(w + i));
+          if (i == 1) x[1] = v;
+          else if (i == 2) x[2] = v;
+          else if (i == 3) x[3] = v;
+          else x[4] = v;
+        }
+        s = s0;
       }
-      s = s0;
     }
 #pragma unroll
     for (uint32_t i = 0; i < 4; i++) l[i] = __funnelshift_r(x[i], x[i + 1], 8u * (p & 3u));
@@ -122,7 +163,7 @@ struct LaneReader {
   __device__ __forceinline__ void refill() {
     if (bw != cw) {
       cw = bw;
-      cv = __ldg(region + start(bw));
+      cv = word(bw);
     }
     bb |= static_cast<uint64_t>(__byte_perm(cv, 0u, 0x0123u)) << (32u - bc);
     bc += 32;
@@ -187,28 +228,29 @@ __device__ __noinline__ uint64_t uvarint(LaneReader& r) {
   return v;
 }
 
-// One lane's substream as a state machine that yields one value per pass: a lane whose run
-// has ended reads its next header first, so the warp's lanes meet again after every value instead of
-// waiting for the longest run among them (two and more values a pass: slower for 64-bit values).
+// One lane's substream as a state machine that yields one value per pass (four where values are narrow): a lane
+// whose run has ended reads its next header first, so the warp's lanes meet again after a value or four
+// instead of waiting for the longest run among them.  2048 chunks, one | two | four values a pass: 64 bits
+// 452 us | 468 | 479, 32 bits 864 | 864 | 880, 16 bits 1615 | 1603 | 1521, 8 bits 2997 | 3097 | 2826 (before the words
+// came ahead of their use; 371, 723, 1202 and 2379 now).
 // Every run kind yields its next value by one step, x = v + d or v - d (v kept as x for the kinds that
 // accumulate), d being the run's next bit field or a constant, so the only fork inside the
 // step is whether the lane reads bits.
 constexpr int kEnd = -1;
-constexpr uint32_t kAhead = 512;  // words
 
 template <typename T>
 __device__ int decode_substream(LaneReader& r, LaneOut<T>& o, bool go) {
   constexpr uint64_t M = sizeof(T) == 8 ? ~0ull : ((1ull << (8 * sizeof(T))) - 1ull);
+  constexpr int kValues = sizeof(T) <= 2 ? 4 : 1;
   uint32_t rem = 0, fbw = 0;
   uint64_t v = 0, bd = 0;  // repeat: the value; delta: running value and base delta; patched: base
   bool bits = false, acc = false, sub = false, patched = false;
   uint32_t pw = 0, pgw = 0, pll = 0, base_out = 0;  // patched: patch width, gap width, list length
   int st = CODAG_OK;
-  // The lanes go through the region together, so what they read next is brought into L1 4 KiB at a time, a
-  // line by each lane.  (A word loaded ahead into a register costs the warp its latency all the same:
-  // whichever lane needs one waits for the last lane's load.)
-  const uint32_t lane = threadIdx.x & 31u;
-  uint32_t ahead = 0, pass = 0;
+  // 64-bit values take at most two words each, so a top-up every kPasses passes keeps ahead of them.
+  constexpr uint32_t kPasses = kValues == 1 ? 4 : 1, kTopUp = kValues == 1 ? 8 : 4;
+  uint32_t pass = 0;
+  r.template top_up<kFifo>(0);
   const auto header = [&]() -> int {  // the next header with values; kEnd at the end of the substream
     for (;;) {
       if (patched) {  // the run's values are out: patch them (decoder_new.h:1166-1183)
@@ -296,31 +338,31 @@ __device__ int decode_substream(LaneReader& r, LaneOut<T>& o, bool go) {
     }
   };
   while (__any_sync(FULL, go)) {
-    if ((pass++ & 7u) == 0) {
-      const uint32_t at = __reduce_max_sync(FULL, r.far);
-      while (ahead < r.total && ahead < at + kAhead) {
-        const uint32_t line = ahead + 32u * lane;
-        if (line < r.total) asm volatile("prefetch.global.L1 [%0];" ::"l"(r.region + line));
-        ahead += 1024u;
-      }
+    if (pass++ % kPasses == 0) {
+      // a run's last word can be the next header's first
+      r.template top_up<kTopUp>(!go ? r.words : bits && rem ? r.bw - 1u : r.p >> 2);
     }
     if (go && rem == 0) {
       st = header();
       go = st == CODAG_OK;
     }
     __syncwarp();
-    if (go) {
-      const uint64_t d = bits ? r.field(fbw) & M : bd;
-      const uint64_t x = (sub ? v - d : v + d) & M;
-      if (acc) v = x;
-      o.put(x);
-      rem--;
-      if (o.over) {
-        st = CODAG_ECORRUPT;
-        go = false;
+#pragma unroll 1
+    for (int b = 0; b < kValues; b++) {
+      if (go && rem) {
+        const uint64_t d = bits ? r.field(fbw) & M : bd;
+        const uint64_t x = (sub ? v - d : v + d) & M;
+        if (acc) v = x;
+        o.put(x);
+        rem--;
+        if (o.over) {
+          st = CODAG_ECORRUPT;
+          go = false;
+        }
       }
     }
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");
   return st == kEnd ? CODAG_OK : st;
 }
 
@@ -339,6 +381,7 @@ __global__ void __launch_bounds__(32 * kWarps)
                        uint8_t* __restrict__ out, uint64_t out_bytes, int32_t* __restrict__ status,
                        uint32_t max_words) {
   __shared__ Segments segs[kWarps];
+  __shared__ uint32_t fifos[kWarps][kFifo][32];
   __shared__ uint32_t part[kWarps];  // the warps' statuses
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint64_t c = (static_cast<uint64_t>(blockIdx.x) * kWarps + warp) / SPLIT;
@@ -376,7 +419,8 @@ __global__ void __launch_bounds__(32 * kWarps)
     const bool mine = lane < kLanes;
     const uint32_t t = SPLIT == 1 ? lane : (warp % SPLIT) * kLanes + lane % kLanes;
     LaneReader r{reinterpret_cast<const uint32_t*>(comp + off), seg, run, (1u << t) - 1u,
-                 __shfl_sync(FULL, static_cast<uint32_t>(len64), t), __shfl_sync(FULL, words, t), 0, 0xffffffffu, 0};
+                 __shfl_sync(FULL, static_cast<uint32_t>(len64), t), __shfl_sync(FULL, words, t), 0, 0xffffffffu, 0, 0,
+                 smem_u32(&fifos[warp][0][lane])};
     LaneOut<T> o{reinterpret_cast<T*>(out) + base_e, t, ru,
                  static_cast<uint32_t>(chunk_bytes / sizeof(T) / 32), store, 0, t * ru, 0, false};
     int s = decode_substream<T>(r, o, mine);
@@ -392,12 +436,11 @@ __global__ void __launch_bounds__(32 * kWarps)
   if (status && real && lane == 0 && warp % SPLIT == 0) status[c] = st;
 }
 
-// Up to how many chunks four warps with eight substreams each, or two with sixteen, are faster than one with
-// all 32.  With fewer lanes a pass meets fewer headers, at the price of issue slots.  Measured, us, one | two |
-// four warps, 64-bit values: 300 chunks 351 | 305 | 269, 600 395 | 342 | 323, 900 395 | 352 | 382,
-// 1200 406 | 385 | 556, 2048 451 | 463 | 717; 8-bit: 600 2718 | 2495 | 2485, 900 2907 | 2708 | 3052,
-// 1200 2914 | 2949 | 3933.
-constexpr uint64_t kQuarter = 4 * 148, kHalf = 7 * 148;
+// Up to how many chunks four warps with eight substreams each are faster than one with all 32: with fewer
+// lanes a pass meets fewer headers, at the price of issue slots.  Measured, us, one | four warps, 64-bit
+// values: 300 chunks 300 | 249, 592 306 | 298, 900 317 | 387; 32 bits 604 | 502, 609 | 572, 635 | 741.  Narrow values
+// gain nothing (16 bits, 300 chunks: 957 | 951), nor do two warps of sixteen over the better of the others.
+constexpr uint64_t kFewChunks = 4 * 148;
 
 bool valid_elem(int e) { return e == 1 || e == 2 || e == 4 || e == 8; }
 
@@ -407,9 +450,11 @@ codag_status launch(const uint8_t* comp, uint64_t comp_bytes, const uint64_t* bl
                     cudaStream_t s) {
   // a substream is at most about twice its share of the chunk (the encoders' bound), in words
   const uint32_t max_words = static_cast<uint32_t>((chunk / 32 * 2 + 1024) / 4);
-  const uint64_t split = n <= kQuarter ? 4 : n <= kHalf ? 2 : 1, grid = (n * split + kWarps - 1) / kWarps;
+  constexpr uint32_t kSplit = sizeof(T) >= 4 ? 4 : 1;
+  const bool few = n <= kFewChunks;
+  const uint64_t grid = (n * (few ? kSplit : 1u) + kWarps - 1) / kWarps;
   if (grid > 0x7fffffffull) return CODAG_EINVAL;
-  auto kern = split == 4 ? k_rlev2_transposed<T, 4> : split == 2 ? k_rlev2_transposed<T, 2> : k_rlev2_transposed<T, 1>;
+  auto kern = few ? k_rlev2_transposed<T, kSplit> : k_rlev2_transposed<T, 1>;
   kern<<<static_cast<unsigned>(grid), 32 * kWarps, 0, s>>>(comp, comp_bytes, blk_off, col_len, n, chunk, ru, out, out_bytes,
                                                            status, max_words);
   return cudaGetLastError() == cudaSuccess ? CODAG_OK : CODAG_ECUDA;
