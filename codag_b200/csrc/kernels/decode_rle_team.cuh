@@ -47,6 +47,7 @@ constexpr uint32_t kRunItem = 0xffffff00u;
 constexpr uint32_t kBlockBytes = 2048;  // the look-ahead's step: two slots of the ring
 constexpr uint32_t kBlocks = 4;         // blocks whose look-ahead is kept
 
+// how far the chunk has come: of what the warps say in one step, the highest counts
 enum : uint32_t { kTeamGo = 0, kTeamDone = 1, kTeamFallback = 2, kTeamTimeout = 3, kTeamShort = 4 };
 
 // The ring's barriers, which outlive a stream where a CTA takes several
@@ -144,7 +145,7 @@ __device__ __forceinline__ void walk_v1(const TeamRing& in, TeamV1& sm, TeamBatc
   }
   if (stuck && items == 0 && state == kTeamGo) state = kTeamFallback;  // longer than the look-ahead
   b.items = items;
-  if (state != kTeamGo) sm.state = state;
+  if (state != kTeamGo) atomicMax(&sm.state, state);
 }
 
 template <int E>
@@ -259,7 +260,7 @@ __device__ __forceinline__ void walk_v2(const TeamRing& in, TeamV2<AHEAD>& sm, T
     n += cnt;
   }
   b.items = items;
-  if (state != kTeamGo) sm.state = state;
+  if (state != kTeamGo) atomicMax(&sm.state, state);
 }
 
 // The stream src[0, len) by all WARPS warps of the CTA: warp 0 walks, the next kAhead look ahead (the
@@ -308,7 +309,8 @@ __device__ __forceinline__ uint32_t rle_team(Team& sm, TeamBars& tb, const uint8
       if (ahead) {
         if (warp == 1) {  // RLE v2 headers are read from some bytes past the block, too
           const uint32_t end = (prepared + 1u) * kBlockBytes + (V1 ? 0u : 64u);
-          if ((!in.release(keep) || in.ensure(end < in.hi ? end : in.hi)) && lane == 0) sm.state = kTeamTimeout;
+          if ((!in.release(keep) || in.ensure(end < in.hi ? end : in.hi)) && lane == 0)
+            atomicMax(&sm.state, static_cast<uint32_t>(kTeamTimeout));
         }
         asm volatile("bar.sync 1, %0;" ::"n"(32 * Team::kAhead) : "memory");
         if constexpr (V1) find_ends(in, sm, prepared, sm.ords, warp - 1u, lane);
@@ -322,7 +324,8 @@ __device__ __forceinline__ uint32_t rle_team(Team& sm, TeamBars& tb, const uint8
           expand_v1<E>(view, sm, o, it, lane);
         } else {
           uint32_t p = it.pos, v = it.n;
-          if (rlev2_header<16, E>(view, o, p, v, cap, in.hi, lane) && lane == 0) sm.state = kTeamFallback;
+          if (rlev2_header<16, E>(view, o, p, v, cap, in.hi, lane) && lane == 0)
+            atomicMax(&sm.state, static_cast<uint32_t>(kTeamFallback));
         }
       }
     }
