@@ -27,7 +27,7 @@
 // the items' bytes.  With one warp per chunk running the state machine, an item cost about 9000 warp
 // instructions and a chunk had one warp to wait for.
 //
-// RLE v2, 256 MiB of 64-bit values: 3.75 ms with a warp per chunk, 1.07 now (2 CTAs of 16 warps per SM,
+// RLE v2, 256 MiB of 64-bit values: 3.75 ms with a warp per chunk, 0.93 now (2 CTAs of 16 warps per SM,
 // which registers allow; 3 or 4 with fewer registers each: 1.26, 1.40; one front warp: 1.26).  RLE v1,
 // 20 MB of 32-bit values: 1.60 ms, 0.13 now.
 #include <cuda_runtime.h>
@@ -94,9 +94,11 @@ template <typename T, uint32_t FRONT, uint32_t BACK, bool V1>
 struct EncodeShared {
   static constexpr uint32_t kFront = FRONT, kBack = BACK;
   EncodeTile<T> tile[2];
-  uint32_t off[kItems];           // size of each item, then offset in the tile's bytes
+  uint32_t off[kItems];           // size of each item
+  uint32_t end[V1 ? 1 : kItems];  // RLE v2: where it ends in the tile's bytes
   uint32_t how[V1 ? 1 : kItems];  // RLE v2: see ItemV2::pack
   uint32_t part[BACK];
+  uint32_t taken[2][2];           // RLE v2: items measured and written so far, of either tile
   uint32_t hist[V1 ? 1 : BACK][32];
   uint64_t red[V1 ? 1 : BACK][128], list[V1 ? 1 : BACK][32];  // PATCHED_BASE: reduced values, patch list
 };
@@ -588,13 +590,24 @@ __global__ void __launch_bounds__(32 * (Item::Shared::kFront + Item::Shared::kBa
   uint8_t* out = scratch + chunk * slot;
   uint64_t base = 0, ready = 0;  // bytes written; first value of the tile to prepare
   bool have = false;             // the back has a tile
+  if (threadIdx.x < 4) sh.taken[threadIdx.x >> 1][threadIdx.x & 1u] = 0;
+  __syncthreads();
   for (uint32_t c = 0; ready < n || have; c ^= 1u) {
     if (front) {
       if (ready < n) prepare_tile<V1, T, kFront>(sh.tile[c], get, ready, n, warp, lane);
     } else if (have) {
       const EncodeTile<T>& t = sh.tile[c ^ 1u];
       const uint32_t items = t.items;
-      for (uint32_t i = warp; i < items; i += kBack) {
+      // RLE v2 items take from 50 to some 600 instructions, so the warps take them as they come (1064 us with
+      // every kBack-th for each warp, 1032 with the measuring as they come, 932 with the writing, too); RLE v1
+      // items are too short for that (127 | 133)
+      const auto next = [&](uint32_t i, uint32_t* taken) {
+        if (V1) return i + kBack;
+        uint32_t k = 0;
+        if (lane == 0) k = atomicAdd(taken, 1u);
+        return __shfl_sync(FULL, k, 0);
+      };
+      for (uint32_t i = V1 ? warp : next(0, &sh.taken[c][0]); i < items; i = next(i, &sh.taken[c][0])) {
         const uint32_t d = t.item[i];
         const uint32_t size = Item::measure(t.val + (d & 0xfffu), (d >> 12) & 0xffu, (d >> 20) != 0, sh, i, warp, lane);
         if (lane == 0) sh.off[i] = size;
@@ -611,11 +624,27 @@ __global__ void __launch_bounds__(32 * (Item::Shared::kFront + Item::Shared::kBa
       const uint32_t mine = lane < kBack ? sh.part[lane] : 0u;
       uint32_t at = __reduce_add_sync(FULL, lane < warp ? mine : 0u);
       const uint32_t total = __reduce_add_sync(FULL, mine);
-      for (uint32_t i = i0; i < i1; i++) {
-        const uint32_t d = t.item[i], size = sh.off[i];
+      const auto write = [&](uint32_t i, uint32_t at, uint32_t size) {
+        const uint32_t d = t.item[i];
         if (base + at + size <= slot)  // else the stream's length will say that it did not fit
           Item::write(t.val + (d & 0xfffu), (d >> 12) & 0xffu, (d >> 20) != 0, Bytes{out + base + at}, sh, i, warp, lane);
-        at += size;
+      };
+      if (V1) {
+        for (uint32_t i = i0; i < i1; i++) {
+          const uint32_t size = sh.off[i];
+          write(i, at, size);
+          at += size;
+        }
+      } else {
+        for (uint32_t i = i0; i < i1; i += 32) {
+          const uint32_t size = i + lane < i1 ? sh.off[i + lane] : 0u, upto = scan_add(size, lane);
+          if (i + lane < i1) sh.end[i + lane] = at + upto;
+          at += __shfl_sync(FULL, upto, 31);
+        }
+        if (threadIdx.x == 32u * kFront) sh.taken[c ^ 1u][0] = sh.taken[c ^ 1u][1] = 0;
+        group_barrier<2, kBack>();
+        for (uint32_t i = next(0, &sh.taken[c][1]); i < items; i = next(i, &sh.taken[c][1]))
+          write(i, sh.end[i] - sh.off[i], sh.off[i]);
       }
       base += total;
     }
