@@ -27,8 +27,9 @@
 // the items' bytes.  With one warp per chunk running the state machine, an item cost about 9000 warp
 // instructions and a chunk had one warp to wait for.
 //
-// RLE v2, 256 MiB of 64-bit values: 3.75 ms with a warp per chunk, 0.93 now (2 CTAs of 16 warps per SM,
-// which registers allow; 3 or 4 with fewer registers each: 1.26, 1.40; one front warp: 1.26).  RLE v1,
+// RLE v2, 256 MiB of 64-bit values: 3.75 ms with a warp per chunk, 0.91 now (2 CTAs of 16 warps per SM,
+// which registers allow; 3 or 4 with fewer registers each: 1.26, 1.40; three, four, six, eight
+// front warps instead of five: 0.99, 0.93, 0.93, 0.99).  RLE v1,
 // 20 MB of 32-bit values: 1.60 ms, 0.13 now.
 #include <cuda_runtime.h>
 
@@ -211,7 +212,7 @@ struct ItemV1 {
 // --- RLE v2 items (the choices are those of RleV2Writer, ../rle_writers.h) ------------------------------
 template <typename T>
 struct ItemV2 {
-  using Shared = EncodeShared<T, 4, 12, false>;
+  using Shared = EncodeShared<T, 5, 11, false>;
   enum : uint32_t { kShortRepeat, kDirect, kDeltaFixed, kDelta, kPatched };
   uint64_t v[4];   // value 32 q + lane
   uint64_t first, second, lmin;
