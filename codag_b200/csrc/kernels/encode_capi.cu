@@ -74,7 +74,7 @@ struct Wide<uint32_t> { using T = unsigned int; };
 template <>
 struct Wide<uint64_t> { using T = unsigned long long; };
 
-constexpr uint32_t kTile = 2048;                 // values whose items are found at a time
+constexpr uint32_t kTile = 3072;  // values whose items are found at a time (2048: 1 to 8% slower; 4000: one CTA per SM)
 constexpr uint32_t kAhead = 160;                 // values of an item beyond them (at most 129)
 constexpr uint32_t kMaskWords = (kTile + kAhead) / 32;
 constexpr uint32_t kItems = kTile / 2 + 64;      // a literal between runs of three: two items per four values

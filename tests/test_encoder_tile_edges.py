@@ -1,4 +1,4 @@
-"""GPU encoders at the edges of their tiles (2048 values): runs, literal groups and packed headers that
+"""GPU encoders at the edges of their tiles (3072 values): runs, literal groups and packed headers that
 start, end and are cut there, chunks of a few values and chunks one value longer or shorter than a
 tile.  The files equal the host producers' byte for byte."""
 import numpy as np
@@ -22,7 +22,7 @@ def _values(rng, n, mode):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("mode", ["runs", "literals", "patches"])
-@pytest.mark.parametrize("chunk", [1, 2, 3, 129, 2047, 2048, 2049, 4097, 16384])
+@pytest.mark.parametrize("chunk", [1, 2, 3, 129, 2047, 2048, 2049, 3071, 3072, 3073, 6145, 16384])
 @pytest.mark.parametrize("codec", [0, 1], ids=["rlev1", "rlev2"])
 def test_tile_edges(cuda, native, codec, chunk, mode):
     from codag_b200 import api
