@@ -336,7 +336,7 @@ def measure_codec(workload: str, args, rank: int, world: int, local: int, steps:
         "gpu_launches": steps * (2 if codec != 2 and args.rle_passes == 2 else 1),
         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                      "frac": round(achieved / peak, 4), "traffic": ncu_traffic(workload), "peak_kind": peak_kind,
-                     "kernel": _kernel_name(codec, t, n, d_ws is not None),
+                     "kernel": _kernel_name(codec, t, n, codec != 2 and args.rle_passes == 2),
                      "alg_bytes_per_launch": alg_bytes,
                      "note": ("launch = header walk + expansion kernels of one call" if codec != 2 and args.rle_passes == 2
                               else "one kernel"),

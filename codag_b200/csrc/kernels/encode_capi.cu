@@ -30,7 +30,7 @@
 // RLE v2, 256 MiB of 64-bit values: 3.75 ms with a warp per chunk, 0.91 now (2 CTAs of 16 warps per SM,
 // which registers allow; 3 or 4 with fewer registers each: 1.26, 1.40; three, four, six, eight
 // front warps instead of five: 0.99, 0.93, 0.93, 0.99).  RLE v1,
-// 20 MB of 32-bit values: 1.60 ms, 0.13 now.
+// 20 MB of 32-bit values: 1.60 ms, 0.12 now.
 #include <cuda_runtime.h>
 
 #include <cstdint>
