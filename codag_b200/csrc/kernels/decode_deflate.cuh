@@ -1021,6 +1021,7 @@ __device__ __forceinline__ int inflate_copy(InflateTeam& sm, OUT& out, uint32_t 
 #pragma unroll
       for (uint32_t i = 0; i < kSteps; i++)
         if (!(v[i] >> 15) && 32u * i < n) v[i] = out.get8(op + 32u * i + lane - 1u - v[i]);
+      __syncwarp();  // from distance 32513 on a source's place in the window is that of a later byte of the batch
 #pragma unroll
       for (uint32_t i = 0; i < kSteps; i++)
         if (32u * i + lane < n) out.put8(op + 32u * i + lane, v[i]);
@@ -1050,6 +1051,7 @@ __device__ __forceinline__ int inflate_copy(InflateTeam& sm, OUT& out, uint32_t 
 #pragma unroll
           for (uint32_t i = 0; i < 4; i++)
             if (!(v[i] >> 15) && h + 32u * i < n) v[i] = out.get8(op + h + 32u * i + lane - 1u - v[i]);
+          __syncwarp();
 #pragma unroll
           for (uint32_t i = 0; i < 4; i++)
             if (h + 32u * i + lane < n) out.put8(op + h + 32u * i + lane, v[i]);
@@ -1069,6 +1071,7 @@ __device__ __forceinline__ int inflate_copy(InflateTeam& sm, OUT& out, uint32_t 
             for (int j = 0; j < 5; j++) root = __shfl_sync(FULL, root, root);
             x = __shfl_sync(FULL, x, root);
           }
+          __syncwarp();
           if (i + lane < n) out.put8(op + i + lane, x);
           __syncwarp();
         }
