@@ -259,7 +259,9 @@ __device__ __forceinline__ int body_patches(const InRing<NSLOT>& in, OUT& out, u
   return CODAG_OK;
 }
 
-// RLE v1 literal group: `remaining` varints from pos (decoder.h:686-727); advances pos
+// RLE v1 literal group: `remaining` varints from pos (decoder.h:686-727); advances pos.  A step looks at 128 bytes,
+// so a longer varint, whose bytes past the 10th carry nothing, is refused.
+constexpr uint32_t kLongestLiteral = 128;
 template <int NSLOT, int E, class OUT>
 __device__ __forceinline__ int body_literals(InRing<NSLOT>& in, OUT& out, uint32_t n, uint32_t remaining, uint32_t& pos,
                                              uint32_t end, uint32_t lane) {
@@ -276,7 +278,7 @@ __device__ __forceinline__ int body_literals(InRing<NSLOT>& in, OUT& out, uint32
     const uint32_t lt = lanemask_lt(lane);
     const uint32_t before = __popc(b0 & lt) + __popc(b1 & lt) + __popc(b2 & lt) + __popc(b3 & lt);
     const uint32_t total = __popc(b0) + __popc(b1) + __popc(b2) + __popc(b3);
-    if (!total) return CODAG_ECORRUPT;  // a varint longer than 128 bytes
+    if (!total) return CODAG_ECORRUPT;  // a varint longer than kLongestLiteral
     const uint32_t take = total < remaining ? total : remaining;
     // end of the previous varint: the last end in a lower lane, or the window start
     const uint32_t nz = __ballot_sync(FULL, nib != 0) & lt;

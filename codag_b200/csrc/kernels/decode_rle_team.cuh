@@ -13,9 +13,9 @@
 // headers do say, in a way that takes some 60 instructions to read: the look-ahead reads every byte of
 // the stream as if it were a header, 32 at a time, and writes down bytes and values.
 //
-// Whatever these stages do not expect (a header that does not fit, a varint of more than 16 bytes, a
-// stream that ends early) is left to the one-warp decoder, which starts the chunk over and reports
-// the exact error.
+// Whatever these stages do not expect (a header that does not fit, a base of more than 16 bytes or a
+// literal of more than kLongestLiteral, a stream that ends early) is left to the one-warp decoder, which
+// starts the chunk over and reports the exact error.
 //
 // One warp per chunk | a team: RLE v1, 8 MiB of 64-bit values 214 us | 46, 256 MiB of 32-bit values
 // 577 | 335 (8 warps; 6, 10 or 12 gain nothing); RLE v2, 3 MB of 16-bit values 434 | 165 (16 warps; 24 or
@@ -149,7 +149,7 @@ __device__ __forceinline__ void walk_v1(const TeamRing& in, TeamV1& sm, TeamBatc
 }
 
 template <int E>
-__device__ __forceinline__ void expand_v1(TeamRing& in, const TeamV1& sm, DirectOut& out, const TeamItem& it, uint32_t lane) {
+__device__ __forceinline__ void expand_v1(TeamRing& in, TeamV1& sm, DirectOut& out, const TeamItem& it, uint32_t lane) {
   constexpr uint64_t M = emask<E>();
   if (it.ord > kRunItem) {
     const int64_t delta = static_cast<int8_t>(in.rd8(it.pos + 1u));
@@ -169,6 +169,7 @@ __device__ __forceinline__ void expand_v1(TeamRing& in, const TeamV1& sm, Direct
     } else {
       const uint64_t lo8 = in.peek_le64(start);
       v = leb_value(lo8, len > 8u ? in.peek_le64(start + 8u) : 0ull, len);
+      if (len > kLongestLiteral) atomicMax(&sm.state, static_cast<uint32_t>(kTeamFallback));
     }
     put_elem<E>(out, it.n + i, v & M);
   }
