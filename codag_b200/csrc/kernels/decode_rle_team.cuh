@@ -13,8 +13,8 @@
 // headers do say, in a way that takes some 60 instructions to read: the look-ahead reads every byte of
 // the stream as if it were a header, 32 at a time, and writes down bytes and values.
 //
-// Whatever these stages do not expect (a header that does not fit, a base of more than 16 bytes or a
-// literal of more than kLongestLiteral, a stream that ends early) is left to the one-warp decoder, which
+// Whatever these stages do not expect (a header that does not fit, a base of more than 16 bytes, a literal
+// that may be longer than kLongestLiteral, a stream that ends early) is left to the one-warp decoder, which
 // starts the chunk over and reports the exact error.
 //
 // One warp per chunk | a team: RLE v1, 8 MiB of 64-bit values 214 us | 46, 256 MiB of 32-bit values
@@ -92,6 +92,11 @@ __device__ __forceinline__ void find_ends(const TeamRing& in, TeamV1& sm, uint32
   }
   if (p + 32u > in.hi) ends &= p >= in.hi ? 0u : (1u << (in.hi - p)) - 1u;
   if (p < in.lo) ends &= FULL << (in.lo - p);  // lo is below 16
+  // A varint of more than kLongestLiteral bytes leaves three of these words in a row without an end, two of them in
+  // one slot.  (A look at every literal's length as it is expanded took 6%.)
+  static_assert(kLongestLiteral >= 127);
+  const uint32_t none = __ballot_sync(FULL, !ends && p + 32u <= in.hi);
+  if ((none & (none >> 1)) && lane == 0) atomicMax(&sm.state, static_cast<uint32_t>(kTeamFallback));
   uint32_t upto = __popc(ends);
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
@@ -149,7 +154,7 @@ __device__ __forceinline__ void walk_v1(const TeamRing& in, TeamV1& sm, TeamBatc
 }
 
 template <int E>
-__device__ __forceinline__ void expand_v1(TeamRing& in, TeamV1& sm, DirectOut& out, const TeamItem& it, uint32_t lane) {
+__device__ __forceinline__ void expand_v1(TeamRing& in, const TeamV1& sm, DirectOut& out, const TeamItem& it, uint32_t lane) {
   constexpr uint64_t M = emask<E>();
   if (it.ord > kRunItem) {
     const int64_t delta = static_cast<int8_t>(in.rd8(it.pos + 1u));
@@ -169,7 +174,6 @@ __device__ __forceinline__ void expand_v1(TeamRing& in, TeamV1& sm, DirectOut& o
     } else {
       const uint64_t lo8 = in.peek_le64(start);
       v = leb_value(lo8, len > 8u ? in.peek_le64(start + 8u) : 0ull, len);
-      if (len > kLongestLiteral) atomicMax(&sm.state, static_cast<uint32_t>(kTeamFallback));
     }
     put_elem<E>(out, it.n + i, v & M);
   }
