@@ -242,9 +242,27 @@ uint64_t chunk_cost(const codag_chunk_desc& d) {
   return d.codec == CODAG_CODEC_DEFLATE ? 8ull * d.comp_len + d.out_len : static_cast<uint64_t>(d.comp_len) + d.out_len / 4;
 }
 
-// RLE files of up to this size are taken by a warp each; so are all RLE v2 files when there are more
-// longer ones than CTAs are resident, as in codag_decompress_rlev2 (2048 of 128 KiB: 389 us | 1091).
+// RLE files of up to this size are taken by a warp each.  So are longer RLE v2 files where there are more of them
+// than CTAs are resident (as in codag_decompress_rlev2; 2048 of 128 KiB: 257 us | 581 by CTAs), but for the
+// longest: those above the smallest power of two that no more than the resident CTAs exceed, so that a few
+// long files among many are not left to single warps (450 of 40 KB and one of 8 MiB: 7.1 ms by warps | 5.3).
 constexpr uint32_t kWarpBytes = 32768;
+constexpr uint32_t kShifts = 18;  // file sizes are below kWarpBytes << 17
+__host__ __device__ __forceinline__ uint32_t shifts_below(uint32_t out_len) {  // how many j have out_len > kWarpBytes << j
+  uint32_t j = 0;
+  while (out_len > static_cast<uint64_t>(kWarpBytes) << j) j++;
+  return j;
+}
+// long_v2[j]: RLE v2 files with shifts_below of j; the result: those with more than it gives get a CTA
+__host__ __device__ __forceinline__ uint32_t v2_shift(const uint32_t* long_v2, uint64_t resident) {
+  uint64_t longer = 0;
+  uint32_t s = kShifts - 1;
+  while (s > 0 && (longer += long_v2[s]) <= resident) s--;
+  return s;
+}
+__host__ __device__ __forceinline__ bool rle_team_size(const codag_chunk_desc& d, uint32_t shift) {
+  return d.out_len > kWarpBytes && (d.codec == CODAG_CODEC_RLEV1 || shifts_below(d.out_len) > shift);
+}
 
 // CTAs of the grid.  One stream alone on an SM is decoded 2.5 times as fast as three side by side, so
 // when the longest takes more than an even share of the work on two CTAs per SM, no more are started
@@ -285,18 +303,20 @@ extern "C" codag_status codag_batch_plan(const codag_chunk_desc* h_descs, uint64
     codag_batch_destroy(p);
     return st;
   }
-  uint64_t long_v2 = 0, longest = 0, total = 0;
+  uint32_t long_v2[kShifts] = {};
+  for (uint64_t i = 0; i < n; i++)
+    if (h_descs[i].codec == CODAG_CODEC_RLEV2) long_v2[shifts_below(h_descs[i].out_len)]++;
+  const uint32_t shift = v2_shift(long_v2, static_cast<uint64_t>(cap));
+  const auto team = [&](uint32_t i) {
+    const codag_chunk_desc& d = h_descs[i];
+    return d.codec == CODAG_CODEC_DEFLATE || (rle_team_size(d, shift) && d.out_off % d.elem_bytes == 0);
+  };
+  uint64_t longest = 0, total = 0;
   for (uint64_t i = 0; i < n; i++) {
     const uint64_t cost = chunk_cost(h_descs[i]);
-    long_v2 += h_descs[i].codec == CODAG_CODEC_RLEV2 && h_descs[i].out_len > kWarpBytes;
     longest = std::max(longest, cost);
     total += cost;
   }
-  const auto team = [&](uint32_t i) {
-    const codag_chunk_desc& d = h_descs[i];
-    if (d.codec == CODAG_CODEC_DEFLATE) return true;
-    return d.out_len > kWarpBytes && (d.codec == CODAG_CODEC_RLEV1 || long_v2 <= static_cast<uint64_t>(cap));
-  };
   std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) {
     if (team(a) != team(b)) return team(a);
     return chunk_cost(h_descs[a]) > chunk_cost(h_descs[b]);
