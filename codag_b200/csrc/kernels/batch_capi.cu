@@ -29,6 +29,7 @@ struct BatchShared {
   TeamBars tb;
   uint64_t bar[kWarps][4];  // of the warps' own rings
   uint32_t job;
+  uint32_t ahead;  // the next entry for a team, as far as the threads have looked
   int32_t st;
 };
 static_assert(sizeof(TeamV1) <= offsetof(InflateTeam, bar) && sizeof(BatchV2) <= offsetof(InflateTeam, bar) &&
@@ -106,9 +107,58 @@ __device__ __forceinline__ bool rle_team_takes(const BatchArgs& a, const codag_c
          (d.comp_len | d.out_len) < 0x80000000u;
 }
 
+// RLE files of up to this size are taken by a warp each.  So are longer RLE v2 files where there are more of them
+// than CTAs are resident (as in codag_decompress_rlev2; 2048 of 128 KiB: 257 us | 581 by CTAs), but for the
+// longest: those above the smallest power of two that no more than the resident CTAs exceed, so that a few
+// long files among many are not left to single warps (450 of 40 KB and one of 8 MiB: 7.1 ms by warps | 5.3).
+constexpr uint32_t kWarpBytes = 32768;
+constexpr uint32_t kShifts = 18;  // file sizes are below kWarpBytes << 17
+__host__ __device__ __forceinline__ uint32_t shifts_below(uint32_t out_len) {  // how many j have out_len > kWarpBytes << j
+  uint32_t j = 0;
+  while (out_len > static_cast<uint64_t>(kWarpBytes) << j) j++;
+  return j;
+}
+// long_v2[j]: RLE v2 files with shifts_below of j; the result: those with more than it gives get a CTA
+__host__ __device__ __forceinline__ uint32_t v2_shift(const uint32_t* long_v2, uint64_t resident) {
+  uint64_t longer = 0;
+  uint32_t s = kShifts - 1;
+  while (s > 0 && (longer += long_v2[s]) <= resident) s--;
+  return s;
+}
+__host__ __device__ __forceinline__ bool rle_team_size(const codag_chunk_desc& d, uint32_t shift) {
+  return d.out_len > kWarpBytes && (d.codec == CODAG_CODEC_RLEV1 || shifts_below(d.out_len) > shift);
+}
+
+// Without a plan the host does not know the files.  k_classify writes to *queue what k_batch has to know of
+// them; k_batch counts its entries in the low bits.  It goes over the list twice: CTAs take the files for
+// teams, then single warps the others, which is how a plan sorts them.
+constexpr uint32_t kCountBits = 26, kAnyTeam = 1u << 31;
+constexpr uint64_t kMaxMixed = (1u << (kCountBits - 1)) - 65536u;  // counts to twice that, and once more per warp
+__device__ __forceinline__ bool wants_team(const BatchArgs& a, const codag_chunk_desc& d, uint32_t shift) {
+  return d.codec == CODAG_CODEC_DEFLATE || (rle_team_size(d, shift) && rle_team_takes(a, d));
+}
+__global__ void __launch_bounds__(1024) k_classify(BatchArgs a, uint32_t n, uint32_t resident, uint32_t* __restrict__ queue) {
+  __shared__ uint32_t long_v2[kShifts];
+  if (threadIdx.x < kShifts) long_v2[threadIdx.x] = 0;
+  __syncthreads();
+  bool any = false;
+#pragma unroll 4
+  for (uint32_t i = threadIdx.x; i < n; i += 1024) {
+    const codag_chunk_desc& d = a.descs[i];
+    if (d.codec == CODAG_CODEC_RLEV2 && d.out_len > kWarpBytes) atomicAdd(&long_v2[shifts_below(d.out_len)], 1u);
+    else any |= wants_team(a, d, 0);
+  }
+  any = __syncthreads_or(any);
+  if (threadIdx.x != 0) return;
+  const uint32_t shift = v2_shift(long_v2, resident);
+  for (uint32_t j = shift + 1; j < kShifts; j++) any |= long_v2[j] != 0;
+  *queue = (any ? kAnyTeam : 0u) | (shift << kCountBits);
+}
+
 // Entries [0, n) of the order, each taken by the CTA's warps together, an RLE stream that a team cannot take by
-// the first alone.  False after a timeout.
-__device__ __forceinline__ bool team_jobs(const BatchArgs& a, uint64_t n, uint32_t* queue, BatchShared& sh,
+// the first alone; `mixed`: those for a team, the others are passed over.  False after a timeout; else sh.job is
+// what the queue gave after the last entry.
+__device__ __forceinline__ bool team_jobs(const BatchArgs& a, uint64_t n, bool mixed, uint32_t* queue, BatchShared& sh,
                                           uint64_t wait_cycles, uint32_t warp, uint32_t lane, RleRing& rle) {
   InflateTeam& sm = sh.inflate;
   InflateRing in;
@@ -121,14 +171,33 @@ __device__ __forceinline__ bool team_jobs(const BatchArgs& a, uint64_t n, uint32
   for (;;) {
     if (threadIdx.x == 0) {
       sh.job = atomicAdd(queue, 1u);
+      sh.ahead = 0xffffffffu;
       sh.st = CODAG_OK;
       sm.stop = sm.dead = 0;
     }
     __syncthreads();
-    const uint32_t k = sh.job;
-    if (k >= n) return true;
+    const uint32_t job = sh.job, k = mixed ? job & ((1u << kCountBits) - 1u) : job;
+    if (k >= n || (mixed && !(job & kAnyTeam))) return true;
     const uint32_t i = a.order ? a.order[k] : k;
     const codag_chunk_desc d = a.descs[i];
+    if (mixed) {
+      const uint32_t shift = (job & ~kAnyTeam) >> kCountBits;
+      if (!wants_team(a, d, shift)) {  // on to the next entry for a team, if it is among those the threads look at
+        constexpr uint32_t kLook = 8;
+        uint32_t far = k + 1u + kLook * 32u * kWarps;
+        if (far > n) far = static_cast<uint32_t>(n);
+#pragma unroll
+        for (uint32_t q = 0; q < kLook; q++) {
+          const uint32_t e = k + 1u + q * 32u * kWarps + threadIdx.x;
+          if (e < far && wants_team(a, a.descs[a.order ? a.order[e] : e], shift)) far = e;
+        }
+        far = __reduce_min_sync(FULL, far);
+        if (lane == 0) atomicMin(&sh.ahead, far);
+        __syncthreads();
+        if (threadIdx.x == 0) atomicMax(queue, (job & ~((1u << kCountBits) - 1u)) | sh.ahead);
+        continue;
+      }
+    }
     if (d.codec != CODAG_CODEC_DEFLATE) {
       uint32_t state = kTeamFallback;
       if (rle_team_takes(a, d))
@@ -171,16 +240,27 @@ __device__ __forceinline__ bool team_jobs(const BatchArgs& a, uint64_t n, uint32
   }
 }
 
-// RLE entries [n0, n) of the order, one per warp.
-__device__ __forceinline__ void rle_jobs(const BatchArgs& a, uint64_t n0, uint64_t n, uint32_t* queue, uint32_t lane,
-                                         RleRing& in) {
+// RLE entries [n0, n) of the order, one per warp; `mixed`: those not for a team, the first warp beginning with
+// `job`, which its CTA has taken already.
+__device__ __forceinline__ void rle_jobs(const BatchArgs& a, uint64_t n0, uint64_t n, bool mixed, uint32_t job, uint32_t* queue,
+                                         uint32_t warp, uint32_t lane, RleRing& in) {
+  // a list of fewer than the grid's warps, and none for teams: the CTAs share it evenly (600 of 128 KiB: 217 us | 185)
+  if (mixed && !(job & kAnyTeam) && warp * gridDim.x >= n) return;
+  bool have = mixed && warp == 0;
   for (;;) {
-    uint32_t k = 0;
-    if (lane == 0) k = atomicAdd(queue, 1u);
-    k = __shfl_sync(FULL, k, 0);
+    if (!have && lane == 0) job = atomicAdd(queue, 1u);
+    have = false;
+    job = __shfl_sync(FULL, job, 0);
+    uint32_t k = job;
+    if (mixed) {
+      k &= (1u << kCountBits) - 1u;
+      if (job & kAnyTeam) k -= static_cast<uint32_t>(n);  // the list's second time
+    }
     if (k >= n - n0) break;
-    const uint32_t i = a.order[n0 + k];
-    const int st = rle_job(a, a.descs[i], in, lane);
+    const uint32_t i = a.order ? a.order[n0 + k] : static_cast<uint32_t>(n0) + k;
+    const codag_chunk_desc& d = a.descs[i];
+    if (mixed && (job & kAnyTeam) && wants_team(a, d, (job & ~kAnyTeam) >> kCountBits)) continue;
+    const int st = rle_job(a, d, in, lane);
     if (a.status && lane == 0) a.status[i] = st;
     if (st == CODAG_ETIMEOUT) break;  // ring state unknown: this warp stops pulling work
   }
@@ -188,16 +268,18 @@ __device__ __forceinline__ void rle_jobs(const BatchArgs& a, uint64_t n0, uint64
 
 // Persistent grid, three CTAs per SM.  The first n_team entries of the order are taken by CTAs
 // (queue[0]), longest first; the others, a plan's short RLE files, by single warps (queue[1]), which
-// fills the SMs while the last of the CTAs' streams are decoded.
+// fills the SMs while the last of the CTAs' streams are decoded.  `mixed`: the list is in no such order, and
+// n_team is n.
 __global__ void __launch_bounds__(32 * kWarps, 3)
-    k_batch(BatchArgs a, uint64_t n, uint64_t n_team, uint32_t* __restrict__ queue, uint64_t wait_cycles) {
+    k_batch(BatchArgs a, uint64_t n, uint64_t n_team, bool mixed, uint32_t* __restrict__ queue, uint64_t wait_cycles) {
   extern __shared__ __align__(128) uint8_t smem[];
   BatchShared& sh = *reinterpret_cast<BatchShared*>(smem);
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   RleRing rle;
   rle_ring(rle, sh, wait_cycles, warp, lane);
-  if (n_team && !team_jobs(a, n_team, queue, sh, wait_cycles, warp, lane, rle)) return;
-  if (n_team < n) rle_jobs(a, n_team, n, queue + 1, lane, rle);
+  if (n_team && !team_jobs(a, n_team, mixed, queue, sh, wait_cycles, warp, lane, rle)) return;
+  if (mixed) rle_jobs(a, 0, n, true, sh.job, queue, warp, lane, rle);
+  else if (n_team < n) rle_jobs(a, n_team, n, false, 0, queue + 1, warp, lane, rle);
 }
 
 }  // namespace
@@ -208,7 +290,7 @@ struct codag_plan {
   codag_chunk_desc* d_descs = nullptr;
   uint32_t* d_order = nullptr;
   uint32_t* d_queue = nullptr;
-  int grid = 0;
+  int grid = 0, mixed_grid = 0;
   // captured graph and the arguments it was captured with
   cudaGraphExec_t exec = nullptr;
   const void* g_comp = nullptr;
@@ -233,35 +315,24 @@ codag_status batch_grid_cap(int* cap) {
 
 void batch_enqueue(const BatchArgs& a, uint64_t n, uint64_t n_team, uint32_t* queue, int grid, cudaStream_t s) {
   cudaMemsetAsync(queue, 0, (n_team < n ? 2 : 1) * sizeof(uint32_t), s);
-  k_batch<<<grid, 32 * kWarps, sizeof(BatchShared), s>>>(a, n, n_team, queue, wait_of());
+  k_batch<<<grid, 32 * kWarps, sizeof(BatchShared), s>>>(a, n, n_team, false, queue, wait_of());
+}
+void mixed_enqueue(const BatchArgs& a, uint64_t n, uint32_t* queue, uint64_t resident, cudaStream_t s) {
+  const int grid = static_cast<int>(std::min(n, resident));
+  if (n > kMaxMixed) return batch_enqueue(a, n, n, queue, grid, s);
+  k_classify<<<1, 1024, 0, s>>>(a, static_cast<uint32_t>(n), static_cast<uint32_t>(resident), queue);
+  k_batch<<<grid, 32 * kWarps, sizeof(BatchShared), s>>>(a, n, n, true, queue, wait_of());
+}
+// CTAs decode RLE files whose output is element aligned; a plan checks the offsets, so the base has to be, too
+void plan_enqueue(const codag_plan& p, const BatchArgs& a, cudaStream_t s) {
+  if (reinterpret_cast<uintptr_t>(a.out) % 8) mixed_enqueue(a, p.n, p.d_queue, static_cast<uint64_t>(p.mixed_grid), s);
+  else batch_enqueue(a, p.n, p.n_team, p.d_queue, p.grid, s);
 }
 
 // Work estimate that orders the queue: a Deflate stream takes some 3 us per KiB of output, an RLE
 // stream on a CTA a third to a sixth of that.
 uint64_t chunk_cost(const codag_chunk_desc& d) {
   return d.codec == CODAG_CODEC_DEFLATE ? 8ull * d.comp_len + d.out_len : static_cast<uint64_t>(d.comp_len) + d.out_len / 4;
-}
-
-// RLE files of up to this size are taken by a warp each.  So are longer RLE v2 files where there are more of them
-// than CTAs are resident (as in codag_decompress_rlev2; 2048 of 128 KiB: 257 us | 581 by CTAs), but for the
-// longest: those above the smallest power of two that no more than the resident CTAs exceed, so that a few
-// long files among many are not left to single warps (450 of 40 KB and one of 8 MiB: 7.1 ms by warps | 5.3).
-constexpr uint32_t kWarpBytes = 32768;
-constexpr uint32_t kShifts = 18;  // file sizes are below kWarpBytes << 17
-__host__ __device__ __forceinline__ uint32_t shifts_below(uint32_t out_len) {  // how many j have out_len > kWarpBytes << j
-  uint32_t j = 0;
-  while (out_len > static_cast<uint64_t>(kWarpBytes) << j) j++;
-  return j;
-}
-// long_v2[j]: RLE v2 files with shifts_below of j; the result: those with more than it gives get a CTA
-__host__ __device__ __forceinline__ uint32_t v2_shift(const uint32_t* long_v2, uint64_t resident) {
-  uint64_t longer = 0;
-  uint32_t s = kShifts - 1;
-  while (s > 0 && (longer += long_v2[s]) <= resident) s--;
-  return s;
-}
-__host__ __device__ __forceinline__ bool rle_team_size(const codag_chunk_desc& d, uint32_t shift) {
-  return d.out_len > kWarpBytes && (d.codec == CODAG_CODEC_RLEV1 || shifts_below(d.out_len) > shift);
 }
 
 // CTAs of the grid.  One stream alone on an SM is decoded 2.5 times as fast as three side by side, so
@@ -332,6 +403,7 @@ extern "C" codag_status codag_batch_plan(const codag_chunk_desc* h_descs, uint64
   }
   const uint64_t need = p->n_team + (n - p->n_team + kWarps - 1) / kWarps;
   p->grid = static_cast<int>(std::min<uint64_t>(need, grid_cap(static_cast<uint64_t>(cap), longest, total)));
+  p->mixed_grid = cap;
   *plan = p;
   return CODAG_OK;
 }
@@ -343,7 +415,7 @@ extern "C" codag_status codag_batch_run(codag_plan* p, const uint8_t* d_comp, ui
   const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   const BatchArgs args{p->d_descs, p->d_order, d_comp, comp_bytes, d_out, out_bytes, d_status};
   if (!use_graph) {
-    batch_enqueue(args, p->n, p->n_team, p->d_queue, p->grid, s);
+    plan_enqueue(*p, args, s);
     return finish_launch();
   }
   const bool same = p->exec && p->g_comp == d_comp && p->g_out == d_out && p->g_status == d_status &&
@@ -358,7 +430,7 @@ extern "C" codag_status codag_batch_run(codag_plan* p, const uint8_t* d_comp, ui
     cudaGraph_t g = nullptr;
     cudaError_t err = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
     if (err == cudaSuccess) {
-      batch_enqueue(args, p->n, p->n_team, p->d_queue, p->grid, cap);
+      plan_enqueue(*p, args, cap);
       err = cudaStreamEndCapture(cap, &g);
     }
     if (err == cudaSuccess) err = cudaGraphInstantiate(&p->exec, g, 0);
@@ -410,7 +482,6 @@ codag_status cached_grid_cap(int* cap) {
 }
 }  // namespace
 
-// The host does not know the codecs here, so teams take every entry.
 extern "C" codag_status codag_batch_launch(const codag_chunk_desc* d_descs, const uint32_t* d_order, uint64_t n,
                                            uint32_t* d_queue, const codag_tune* tune, const uint8_t* d_comp,
                                            uint64_t comp_bytes, uint8_t* d_out, uint64_t out_bytes,
@@ -423,7 +494,6 @@ extern "C" codag_status codag_batch_launch(const codag_chunk_desc* d_descs, cons
   const codag_status st = cached_grid_cap(&cap);
   if (st != CODAG_OK) return st;
   const BatchArgs args{d_descs, d_order, d_comp, comp_bytes, d_out, out_bytes, d_status};
-  batch_enqueue(args, n, n, d_queue, static_cast<int>(std::min<uint64_t>(n, static_cast<uint64_t>(cap))),
-                reinterpret_cast<cudaStream_t>(stream));
+  mixed_enqueue(args, n, d_queue, static_cast<uint64_t>(cap), reinterpret_cast<cudaStream_t>(stream));
   return finish_launch();
 }

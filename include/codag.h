@@ -240,9 +240,9 @@ codag_status codag_batch_destroy(codag_plan *plan);
  * that rebuild the chunk list for every launch (continuous batching).  d_order (n u32,
  * may be NULL = descriptor order) is the order the warps take chunks in; d_queue is 4 bytes
  * of device memory that this call resets on `stream`; d_status has n entries (may be NULL)
- * and entry i reports descriptor i.  tune may be NULL (8 warps per CTA, 4 ring slots, 10-bit
- * tables, as codag_batch_plan).  Allocates
- * nothing; the launch shape of each tune is measured once per device and cached. */
+ * and entry i reports descriptor i.  Streams have six warps or one as in a plan, which a small
+ * kernel before the launch finds out.  tune may be NULL; it is checked and changes nothing.
+ * Allocates nothing; the number of CTAs that the device holds is looked up once and cached. */
 codag_status codag_batch_launch(const codag_chunk_desc *d_descs, const uint32_t *d_order, uint64_t n,
                                 uint32_t *d_queue, const codag_tune *tune, const uint8_t *d_comp,
                                 uint64_t comp_bytes, uint8_t *d_out, uint64_t out_bytes,
