@@ -271,14 +271,22 @@ codag_status launch_rle_team(const uint8_t* comp, uint64_t comp_bytes, const uin
   return finish_launch();
 }
 
-// Up to how many chunks a team each is faster than a warp each (measured, us, team | warp):
-//   RLE v1, 64-bit values: 33 chunks 49 | 214, 2048 187 | 273, 8192 656 | 722; 32 bits: 33 83 | 468,
-//   8192 1249 | 1601; 8 bits: 33 356 | 1830, 2048 1376 | 2211: at every count
+// Whether a team for each chunk is faster than a warp for each (measured, us, team | warp).
+//   RLE v1: up to about two chunks for each resident CTA, always (700 chunks: 17 | 20 at 6 bytes of stream each, 168 |
+//   715 at 152 KiB).  With more, a chunk also costs 2 us of a CTA's place, which the length of the streams has to
+//   earn back: 64-bit values, 2048 chunks: 25 | 20 at 6 bytes, 31 | 27 at 780, 49 | 51 at 3000, 187 | 272 at
+//   24 KiB; 8192 chunks: 51 | 21, 76 | 45, 144 | 110, 374 | 373 at 12 KiB, 458 | 704 at 38 KiB; 8 and 32 bits the
+//   same within a fifth.  The mean stream is taken from comp_bytes (too
+//   long for a part of a file, too short where chunks share a stream).
 //   RLE v2 (the look-ahead reads every byte as a header, which pays while SMs have room for it): 64-bit
 //   values: 32 chunks 80 | 138, 400 146 | 157, 640 204 | 175; 16 bits: 32 168 | 424, 400 370 | 479,
 //   640 527 | 484; 8 bits: 640 808 | 825, 1280 1389 | 884
 template <int CODEC>
-constexpr uint64_t kTeamChunks = CODEC == CODAG_CODEC_RLEV2 ? 3 * kSms : ~0ull;
+bool team_pays(uint64_t n, uint64_t comp_bytes) {
+  if (CODEC == CODAG_CODEC_RLEV2) return n <= 3 * kSms;
+  constexpr uint64_t kFree = 900, kAll = 8900;
+  return n <= kFree || comp_bytes / n * 4 >= 5 * ((n < kAll ? n : kAll) - kFree);
+}
 
 // Values go straight to global memory when the output is element aligned (DirectOut),
 // through the shared-memory ring otherwise; with cta_per_chunk (and no workspace) a whole
@@ -289,7 +297,7 @@ codag_status launch_rle(const codag_tune& t, const uint8_t* comp, uint64_t comp_
                         int32_t* status, void* ws, uint64_t ws_bytes, cudaStream_t s) {
   // direct stores write whole elements: the output and out_bytes must be element aligned
   const bool direct = (reinterpret_cast<uintptr_t>(out) % E) == 0 && out_bytes % E == 0;
-  if (direct && !ws && (t.cta_per_chunk || n <= kTeamChunks<CODEC>))
+  if (direct && !ws && (t.cta_per_chunk || team_pays<CODEC>(n, comp_bytes)))
     return launch_rle_team<CODEC, E>(comp, comp_bytes, blk_off, col_len, n, chunk_bytes, out, out_bytes, status, s);
   if (direct)
     return launch_rle_out<NSLOT, CODEC, E, true>(t, comp, comp_bytes, blk_off, col_len, n, chunk_bytes, out,

@@ -170,13 +170,14 @@ codag_status codag_compress_rlev2(const uint8_t *d_in, uint64_t in_bytes, uint64
 
 /* --- launch tuning --------------------------------------------------------------------
  * Process-wide launch shape for the per-file calls above, per codec.  It applies to the RLE
- * kernels that give each chunk one warp: RLE v2 with more than 444 chunks, calls with a
- * workspace, and outputs that are not element aligned.  warps_per_cta is the number of chunks
- * one CTA decodes (1..8); ring_slots the depth of the TMA input ring (2, 4 or 8 slots of 1 KiB;
- * the RLE codecs need at least 4 because an RLE v2 header with its data spans up to 2060 bytes).
- * cta_per_chunk = 1 gives each RLE v2 chunk a whole CTA whatever their number (fewer chunks, and
- * RLE v1 chunks, have one without being asked; it applies without a workspace, when the output
- * and out_bytes are element aligned).  Deflate chunks are always decoded by a team of six warps
+ * kernels that give each chunk one warp: RLE v2 with more than 444 chunks, RLE v1 with more than
+ * 900 chunks whose streams are short for their number, calls with a workspace, and outputs that
+ * are not element aligned.  warps_per_cta is the number of chunks one CTA decodes (1..8);
+ * ring_slots the depth of the TMA input ring (2, 4 or 8 slots of 1 KiB; the RLE codecs need at
+ * least 4 because an RLE v2 header with its data spans up to 2060 bytes).
+ * cta_per_chunk = 1 gives each RLE chunk a whole CTA whatever their number (without it, those not
+ * named above have one; it applies without a workspace, when the output and out_bytes are element
+ * aligned).  Deflate chunks are always decoded by a team of six warps
  * each: their shape, and lut_bits (9, 10 or 11), are checked and kept, and change nothing.
  * Values outside the supported sets return CODAG_EINVAL. */
 typedef struct {
