@@ -118,15 +118,19 @@ __host__ __device__ __forceinline__ uint32_t shifts_below(uint32_t out_len) {  /
   while (out_len > static_cast<uint64_t>(kWarpBytes) << j) j++;
   return j;
 }
-// long_v2[j]: RLE v2 files with shifts_below of j; the result: those with more than it gives get a CTA
+// long_v2[j]: RLE v2 files for teams with shifts_below of j; the result: those with more than it gives get a CTA
 __host__ __device__ __forceinline__ uint32_t v2_shift(const uint32_t* long_v2, uint64_t resident) {
   uint64_t longer = 0;
   uint32_t s = kShifts - 1;
   while (s > 0 && (longer += long_v2[s]) <= resident) s--;
   return s;
 }
-__host__ __device__ __forceinline__ bool rle_team_size(const codag_chunk_desc& d, uint32_t shift) {
-  return d.out_len > kWarpBytes && (d.codec == CODAG_CODEC_RLEV1 || shifts_below(d.out_len) > shift);
+__host__ __device__ __forceinline__ bool rle_team_pays(const codag_chunk_desc& d, uint32_t shift) {
+  if (d.out_len <= kWarpBytes || d.comp_len <= kTeamMinBytes) return false;  // (3000 of 40 KB in 120 bytes each: 112 us | 97)
+  if (d.codec == CODAG_CODEC_RLEV1) return true;
+  // mostly DIRECT groups, if it is that long: see rlev2_alone
+  const bool direct = d.comp_len > (2u + d.elem_bytes / 4u) * static_cast<uint64_t>(d.out_len / d.elem_bytes);
+  return shifts_below(d.out_len) > shift && !direct;
 }
 
 // Without a plan the host does not know the files.  k_classify writes to *queue what k_batch has to know of
@@ -135,7 +139,7 @@ __host__ __device__ __forceinline__ bool rle_team_size(const codag_chunk_desc& d
 constexpr uint32_t kCountBits = 26, kAnyTeam = 1u << 31;
 constexpr uint64_t kMaxMixed = (1u << (kCountBits - 1)) - 65536u;  // counts to twice that, and once more per warp
 __device__ __forceinline__ bool wants_team(const BatchArgs& a, const codag_chunk_desc& d, uint32_t shift) {
-  return d.codec == CODAG_CODEC_DEFLATE || (rle_team_size(d, shift) && rle_team_takes(a, d));
+  return d.codec == CODAG_CODEC_DEFLATE || (rle_team_takes(a, d) && rle_team_pays(d, shift));
 }
 __global__ void __launch_bounds__(1024) k_classify(BatchArgs a, uint32_t n, uint32_t resident, uint32_t* __restrict__ queue) {
   __shared__ uint32_t long_v2[kShifts];
@@ -145,8 +149,9 @@ __global__ void __launch_bounds__(1024) k_classify(BatchArgs a, uint32_t n, uint
 #pragma unroll 4
   for (uint32_t i = threadIdx.x; i < n; i += 1024) {
     const codag_chunk_desc& d = a.descs[i];
-    if (d.codec == CODAG_CODEC_RLEV2 && d.out_len > kWarpBytes) atomicAdd(&long_v2[shifts_below(d.out_len)], 1u);
-    else any |= wants_team(a, d, 0);
+    const bool wants = wants_team(a, d, 0);
+    if (d.codec != CODAG_CODEC_RLEV2) any |= wants;
+    else if (wants) atomicAdd(&long_v2[shifts_below(d.out_len)], 1u);
   }
   any = __syncthreads_or(any);
   if (threadIdx.x != 0) return;
@@ -376,11 +381,11 @@ extern "C" codag_status codag_batch_plan(const codag_chunk_desc* h_descs, uint64
   }
   uint32_t long_v2[kShifts] = {};
   for (uint64_t i = 0; i < n; i++)
-    if (h_descs[i].codec == CODAG_CODEC_RLEV2) long_v2[shifts_below(h_descs[i].out_len)]++;
+    if (h_descs[i].codec == CODAG_CODEC_RLEV2 && rle_team_pays(h_descs[i], 0)) long_v2[shifts_below(h_descs[i].out_len)]++;
   const uint32_t shift = v2_shift(long_v2, static_cast<uint64_t>(cap));
   const auto team = [&](uint32_t i) {
     const codag_chunk_desc& d = h_descs[i];
-    return d.codec == CODAG_CODEC_DEFLATE || (rle_team_size(d, shift) && d.out_off % d.elem_bytes == 0);
+    return d.codec == CODAG_CODEC_DEFLATE || (rle_team_pays(d, shift) && d.out_off % d.elem_bytes == 0);
   };
   uint64_t longest = 0, total = 0;
   for (uint64_t i = 0; i < n; i++) {

@@ -141,11 +141,17 @@ __global__ void __launch_bounds__(32 * kTeamWarpsOf<CODEC>)
     if (status && threadIdx.x == 0) status[chunk] = CODAG_ECORRUPT;
     return;
   }
-  if (warp == 1) init_ring_barriers<16>(sh.tb.bar, lane);
-  if (threadIdx.x == 0) sh.tb.phase = 0;
-  __syncthreads();
-  const uint32_t state = rle_team<CODEC, E, kTeamWarpsOf<CODEC>>(sh.team, sh.tb, comp + off, static_cast<uint32_t>(len),
-                                                                 out + cbase, store, cap, wait_cycles);
+  const bool alone = CODEC == CODAG_CODEC_RLEV2 && rlev2_alone(comp + off, static_cast<uint32_t>(len), cap);
+  if (alone && warp != 0) return;
+  if (!alone) {
+    if (warp == 1) init_ring_barriers<16>(sh.tb.bar, lane);
+    if (threadIdx.x == 0) sh.tb.phase = 0;
+    __syncthreads();
+  }
+  uint32_t state = kTeamFallback;
+  if (!alone)
+    state = rle_team<CODEC, E, kTeamWarpsOf<CODEC>>(sh.team, sh.tb, comp + off, static_cast<uint32_t>(len), out + cbase, store,
+                                                    cap, wait_cycles);
   if (warp != 0) return;
   int st = state == kTeamTimeout ? CODAG_ETIMEOUT : state == kTeamShort ? CODAG_ECORRUPT : CODAG_OK;
   if (state == kTeamFallback) {  // in one pass, from the start
@@ -280,12 +286,15 @@ codag_status launch_rle_team(const uint8_t* comp, uint64_t comp_bytes, const uin
 //   long for a part of a file, too short where chunks share a stream).
 //   RLE v2 (the look-ahead reads every byte as a header, which pays while SMs have room for it): 64-bit
 //   values: 32 chunks 80 | 138, 400 146 | 157, 640 204 | 175; 16 bits: 32 168 | 424, 400 370 | 479,
-//   640 527 | 484; 8 bits: 640 808 | 825, 1280 1389 | 884
+//   640 527 | 484; 8 bits: 640 808 | 825, 1280 1389 | 884.  Not for short streams (64-bit values, 8 chunks: 20 | 17 at
+//   144 bytes), nor where chunks are small and their streams are those that a team leaves to one of its warps
+//   (64-bit values, 32 chunks of 2 KiB: 19 | 16).
 template <int CODEC>
-bool team_pays(uint64_t n, uint64_t comp_bytes) {
-  if (CODEC == CODAG_CODEC_RLEV2) return n <= 3 * kSms;
+bool team_pays(uint64_t n, uint64_t comp_bytes, uint64_t values) {
+  const uint64_t mean = comp_bytes / n;
+  if (CODEC == CODAG_CODEC_RLEV2) return n <= 3 * kSms && mean > kTeamMinBytes && (values > 1024 || mean <= 2 * values);
   constexpr uint64_t kFree = 900, kAll = 8900;
-  return n <= kFree || comp_bytes / n * 4 >= 5 * ((n < kAll ? n : kAll) - kFree);
+  return n <= kFree || mean * 4 >= 5 * ((n < kAll ? n : kAll) - kFree);
 }
 
 // Values go straight to global memory when the output is element aligned (DirectOut),
@@ -297,7 +306,7 @@ codag_status launch_rle(const codag_tune& t, const uint8_t* comp, uint64_t comp_
                         int32_t* status, void* ws, uint64_t ws_bytes, cudaStream_t s) {
   // direct stores write whole elements: the output and out_bytes must be element aligned
   const bool direct = (reinterpret_cast<uintptr_t>(out) % E) == 0 && out_bytes % E == 0;
-  if (direct && !ws && (t.cta_per_chunk || team_pays<CODEC>(n, comp_bytes)))
+  if (direct && !ws && (t.cta_per_chunk || team_pays<CODEC>(n, comp_bytes, chunk_bytes / E)))
     return launch_rle_team<CODEC, E>(comp, comp_bytes, blk_off, col_len, n, chunk_bytes, out, out_bytes, status, s);
   if (direct)
     return launch_rle_out<NSLOT, CODEC, E, true>(t, comp, comp_bytes, blk_off, col_len, n, chunk_bytes, out,

@@ -44,6 +44,7 @@ struct __align__(16) TeamItem {
 };
 constexpr uint32_t kRunItem = 0xffffff00u;
 
+constexpr uint32_t kTeamMinBytes = 256;  // a shorter stream is over before a team's stages are under way
 constexpr uint32_t kBlockBytes = 2048;  // the look-ahead's step: two slots of the ring
 constexpr uint32_t kBlocks = 4;         // blocks whose look-ahead is kept
 
@@ -266,6 +267,22 @@ __device__ __forceinline__ void walk_v2(const TeamRing& in, TeamV2<AHEAD>& sm, T
   }
   b.items = items;
   if (state != kTeamGo) atomicMax(&sm.state, state);
+}
+
+// Whether one warp decodes an RLE v2 stream faster.  A team reads every byte as a header, 2.1 us per KiB; a warp
+// expands DIRECT groups in some 3 us per 1024 values and 0.6 per KiB, but takes longer over other headers.  So
+// streams of more than two bytes a value that begin with DIRECT groups are left to a warp (128 KiB of random 64-bit
+// values: 284 us by a team | 138, of 32-bit values 286 | 186, of 16-bit values, 2.02 bytes each, 343 | 292).
+// (Finding out in the walk, header by header, made it 5 to 17% slower for all.)
+__device__ __forceinline__ bool rlev2_alone(const uint8_t* src, uint32_t len, uint32_t values) {
+  if (len <= 2ull * values) return false;
+  uint32_t p = 0;
+  for (uint32_t h = 0; h < 8 && p + 2u <= len; h++) {
+    const uint32_t first = __ldg(src + p), len8 = ((((first & 1u) << 8) | __ldg(src + p + 1u)) + 1u) & 0xffu;
+    if (first >> 6 != 1u) return false;
+    p += 2u + (len8 * v2_width((first >> 1) & 0x1fu) + 7u) / 8u;
+  }
+  return true;
 }
 
 // The stream src[0, len) by all WARPS warps of the CTA: warp 0 walks, the next kAhead look ahead (the
