@@ -231,7 +231,7 @@ __device__ __forceinline__ bool team_jobs(const BatchArgs& a, uint64_t n, bool m
       inflate_place(sm, d.out_len, lane);
     } else {
       o.begin(a.out + d.out_off, d.out_len);
-      const int st = inflate_copy(sm, o, lane);
+      const int st = inflate_copy(sm, o, a.comp + d.comp_off, d.comp_len, lane);
       if (lane == 0) {
         if (a.status) a.status[i] = st;
         sh.st = sm.dead || sm.status == CODAG_ETIMEOUT ? static_cast<int>(CODAG_ETIMEOUT) : st;

@@ -22,6 +22,9 @@
 //     shared-memory window (the largest distance Deflate has, so no source is ever read back from
 //     global memory).  A source inside the same 32 bytes is followed lane to lane.
 //
+// Stored blocks pass the stages in between by: the copy warp takes their bytes from the stream, and the
+// input rings go on behind them (128 KiB of stored blocks: 226 us as tokens, 71 now; 512 chunks 461 | 154).
+//
 // The stages run as a pipeline, handing over in buffers guarded by named barriers, so no warp spins.
 // Each stage is one or two warps' chain of dependent instructions, about six cycles each, which is
 // why the work is spread over as many warps as it is.
@@ -243,11 +246,12 @@ constexpr uint32_t kRange = 3072;  // output bytes of one token batch
 struct TokenBatch {
   uint32_t starts[kRange / 32];  // bit b: a token starts at byte b of the range
   uint32_t list;    // which of the token warp's lists
-  uint32_t before;  // its tokens that start before the range
+  uint32_t before;  // its tokens that start before the range; kStored: where the bytes are in the stream
   uint32_t bytes;   // bytes of the range
-  uint32_t what;    // kMore: another range of the same list follows; kLast: the chunk's last batch
+  uint32_t what;    // kMore: another range of the same list follows; kLast: the chunk's last batch;
+                    // kStored: no tokens, but bytes of a stored block
 };
-enum : uint32_t { kMore = 1, kLast = 2 };
+enum : uint32_t { kMore = 1, kLast = 2, kStored = 4 };
 
 // 256 output bytes: word 32 i + l is the low half of byte 32 i + l's token.
 constexpr uint32_t kSteps = 8;
@@ -255,10 +259,11 @@ struct ByteBatch {
   uint16_t word[32 * kSteps];
   uint32_t bytes;
   uint32_t near;  // 0: every source lies before the batch; else one more than the bytes before the
-                  // first token that starts in the batch
+                  // first token that starts in the batch; or kStoredBytes
+  uint32_t from;  // kStoredBytes: where they are in the stream
   uint32_t last;  // the chunk's last batch; kBadChunk with it if the tokens were not sound
 };
-constexpr uint32_t kBadChunk = 2;
+constexpr uint32_t kBadChunk = 2, kStoredBytes = 0xffffffffu;
 
 using InflateRing = InRing<8>;   // the scan's input
 using TokenRing = InRing<2>;     // a token warp's, which lags by up to two stretches
@@ -545,7 +550,7 @@ struct InflateScan {
     }
   }
 
-  // Stored block: the token warps read its bytes themselves.
+  // Stored block: the copy warp reads its bytes itself, and the ring goes on behind it.
   __device__ __forceinline__ int stored() {
     pos = (pos + 7u) & ~7u;
     int st = need(64);
@@ -556,15 +561,11 @@ struct InflateScan {
     if (len != (~(v >> 16) & 0xffffu)) return CODAG_ECORRUPT;
     if ((pos >> 3) + len > in.hi) return CODAG_ECORRUPT;
     if (len && !handoff(kBatchStored, pos >> 3, len, CODAG_OK)) return CODAG_ECORRUPT;
-    // the ring goes on in steps it can hold
-    for (uint32_t left = len * 8u; left;) {
-      const uint32_t step = left < 4096u * 8u ? left : 4096u * 8u;
-      st = need(step);
-      if (st) return st;
-      pos += step;
-      left -= step;
-    }
-    return CODAG_OK;
+    pos += len * 8u;
+    scan_barrier();
+    if (warp == 0 && !in.skip(pos >> 3) && lane == 0) sm.scan_st = CODAG_ETIMEOUT;
+    scan_barrier();
+    return sm.scan_st;
   }
 
   // Code lengths and tables of a dynamic block (zlib.h:607-707); both warps read the code lengths,
@@ -732,7 +733,7 @@ __device__ __forceinline__ void inflate_scan(InflateRing& in, InflateTeam& sm, u
 // ---------------------------------------------------------------------------------------
 // token warps
 // ---------------------------------------------------------------------------------------
-// Token warps (2 and 3 of the team: `me` 0 and 1), taking turns at 32 cells or kTokens stored bytes; `in`
+// Token warps (2 and 3 of the team: `me` 0 and 1), taking turns at 32 cells or a stored block; `in`
 // is bound to the stream.  Every turn ends in a batch, an empty one when no more are wanted, so the
 // place warp knows whose turn it is.
 __device__ __forceinline__ void inflate_tokens(TokenRing& in, InflateTeam& sm, uint32_t me, uint32_t lane) {
@@ -761,7 +762,7 @@ __device__ __forceinline__ void inflate_tokens(TokenRing& in, InflateTeam& sm, u
   };
   // bytes [at, end) resident
   const auto need = [&](uint32_t at, uint32_t end) {
-    const bool ok = in.release(at) && in.ensure(end < in.hi ? end : in.hi) == CODAG_OK;
+    const bool ok = in.skip(at) && in.release(at) && in.ensure(end < in.hi ? end : in.hi) == CODAG_OK;
     if (!ok && lane == 0) sm.dead = 1;
     return ok;
   };
@@ -787,18 +788,10 @@ __device__ __forceinline__ void inflate_tokens(TokenRing& in, InflateTeam& sm, u
       return;
     }
     if (kind == kBatchStored) {
-      const uint32_t at = b.base, len = b.size;
-      for (uint32_t i = 0; i < len; i += kTokens, turn++) {
-        if ((turn & 1u) != me) continue;
-        const uint32_t n = len - i < kTokens ? len - i : kTokens;
+      if ((turn++ & 1u) == me) {
         reuse();
-        if (stopped() || !need(at + i, at + i + n)) {
-          handoff(0, 0, 0);
-          continue;
-        }
-        for (uint32_t q = lane; q < n; q += 32) sm.tok[me][list][q] = kLiteralToken | in.rd8(at + i + q);
-        if (32u * lane < n) sm.out[me][k].starts[lane] = n - 32u * lane >= 32u ? FULL : (1u << (n - 32u * lane)) - 1u;
-        handoff(0, n, 0);
+        const bool drop = stopped();
+        handoff(b.base, drop ? 0u : b.size, drop ? 0u : static_cast<uint32_t>(kStored));
       }
       continue;
     }
@@ -924,8 +917,13 @@ __device__ __forceinline__ void inflate_place(InflateTeam& sm, uint64_t chunk_by
     const TokenBatch& b = sm.out[me][buf];
     const uint32_t bytes = b.bytes, what = b.what, s_tok = smem_u32(sm.tok[me][b.list]);
     if (bytes > cap - op) ok = false;
+    if (ok && (what & kStored)) {
+      if (handed >= 2u) team_wait<64>(kBytesFree + k);
+      if (lane == 0) sm.place[k].from = b.before;
+      handoff(bytes, kStoredBytes, 0);
+    }
     uint32_t count = b.before;  // tokens that start before the 1 KiB at c
-    for (uint32_t c = 0; ok && c < bytes; c += 1024) {
+    for (uint32_t c = what & kStored ? bytes : 0u; ok && c < bytes; c += 1024) {
       // lane l: the starts in the 32 bytes at c + 32 l, and how many tokens start before them
       const uint32_t word = c + 32u * lane < bytes ? b.starts[c / 32u + lane] : 0u;
       const uint32_t upto = warp_scan_add(__popc(word), lane) + count, pre = upto - __popc(word);
@@ -1005,16 +1003,60 @@ __device__ __forceinline__ void inflate_place(InflateTeam& sm, uint64_t chunk_by
 // ---------------------------------------------------------------------------------------
 // copy warp
 // ---------------------------------------------------------------------------------------
-// Warp 5 of the team: writes the bytes through `out` and returns the chunk's status.
+// n bytes of the stream (`g`, which ends at `hi`) from `from` on to output position op, 2 KiB at a time: words that lie
+// whole in the stream, put together to words of the window, and single bytes around them.  The result: out.flushed.
 template <class OUT>
-__device__ __forceinline__ int inflate_copy(InflateTeam& sm, OUT& out, uint32_t lane) {
+__device__ __noinline__ uint32_t copy_stored(OUT out, uint32_t op, uint32_t n, const uint8_t* __restrict__ g, uint32_t from,
+                                         uint32_t hi, uint32_t lane) {
+  while (n) {
+    const uint32_t room = OUT::kFlush - (op & (OUT::kFlush - 1u)), m = n < room ? n : room;
+    const uint32_t ahead = from + 4u * OUT::kFlush + 64u * lane;
+    if (ahead < hi) asm volatile("prefetch.global.L2 [%0];" ::"l"(g + ahead));
+    const uint32_t head = (0u - op) & 3u, h = head < m ? head : m;
+    const uint32_t a0 = (from + h) & ~3u, sh = 8u * ((from + h) & 3u);
+    const uint32_t in_stream = a0 + 8u <= hi ? (hi - 8u - a0) / 4u + 1u : 0u;
+    const uint32_t words = (m - h) / 4u < in_stream ? (m - h) / 4u : in_stream;
+    constexpr uint32_t kEach = 8;
+#pragma unroll 1
+    for (uint32_t w0 = 0; w0 < words; w0 += 32u * kEach) {
+      uint32_t x[kEach], y[kEach];
+#pragma unroll
+      for (uint32_t i = 0; i < kEach; i++) {
+        const uint32_t w = w0 + 32u * i + lane;
+        const uint32_t* p = reinterpret_cast<const uint32_t*>(g + a0) + (w < words ? w : words - 1u);
+        x[i] = __ldg(p);
+        y[i] = __ldg(p + 1);
+      }
+#pragma unroll
+      for (uint32_t i = 0; i < kEach; i++) {
+        const uint32_t w = w0 + 32u * i + lane;
+        if (w < words) st_s32(out.sbuf + ((op + h + 4u * w) & OUT::kMask), __funnelshift_r(x[i], y[i], sh));
+      }
+    }
+    if (lane < h) out.put8(op + lane, __ldg(g + from + lane));
+    for (uint32_t b = h + 4u * words + lane; b < m; b += 32) out.put8(op + b, __ldg(g + from + b));
+    __syncwarp();
+    op += m;
+    from += m;
+    n -= m;
+    out.flush_to(op);
+  }
+  return out.flushed;
+}
+
+// Warp 5 of the team: writes the bytes through `out` and returns the chunk's status.  `src`: the stream.
+template <class OUT>
+__device__ __forceinline__ int inflate_copy(InflateTeam& sm, OUT& out, const uint8_t* src, uint32_t len, uint32_t lane) {
+  const uint32_t lo = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(src) & 15u);  // as in the rings
   uint32_t op = 0, k = 0, last;
   do {
     team_wait<64>(kBytesFull + k);
     const ByteBatch& b = sm.place[k];
     const uint32_t n = b.bytes, near = b.near;
     last = b.last;
-    if (!near) {  // every source lies before the batch: all bytes at once
+    if (near == kStoredBytes) {
+      out.flushed = copy_stored(out, op, n, src - lo, b.from, lo + len, lane);
+    } else if (!near) {  // every source lies before the batch: all bytes at once
       uint32_t v[kSteps];
 #pragma unroll
       for (uint32_t i = 0; i < kSteps; i++) v[i] = b.word[32u * i + lane];

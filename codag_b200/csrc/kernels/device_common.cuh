@@ -287,6 +287,18 @@ struct InRing {
     return true;
   }
 
+  // Goes on at byte `pos`, without the slots before it that were not asked for yet.
+  __device__ __forceinline__ bool skip(uint32_t pos) {
+    uint32_t s = pos >> kSlotLog2;
+    if (s > nslots) s = nslots;
+    if (s <= issued) return true;
+    if (!drain()) return false;
+    issued = waited = s;
+    ready = waited << kSlotLog2;
+    release_at = 0;
+    return true;
+  }
+
   // Makes bytes [.., end) readable.  Returns CODAG_OK, CODAG_ECORRUPT (beyond the window)
   // or CODAG_ETIMEOUT.
   __device__ __forceinline__ int ensure(uint32_t end) {

@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(32 * kTeamWarps, 3)
     InflateWin o;
     inflate_window(o, sm, lane);
     o.begin(out + base, store_bytes(base, chunk_bytes, out_bytes));
-    const int st = inflate_copy(sm, o, lane);
+    const int st = inflate_copy(sm, o, comp + off, static_cast<uint32_t>(next - off), lane);
     if (status && lane == 0) status[chunk] = st;
   }
 }
