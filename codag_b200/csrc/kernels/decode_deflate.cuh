@@ -23,7 +23,9 @@
 //     global memory).  A source inside the same 32 bytes is followed lane to lane.
 //
 // Stored blocks pass the stages in between by: the copy warp takes their bytes from the stream, and the
-// input rings go on behind them (128 KiB of stored blocks: 226 us as tokens, 71 now; 512 chunks 461 | 154).
+// input rings go on behind them (128 KiB of stored blocks: 226 us as tokens, 71 now; 512 chunks 461 | 154).  So do
+// long matches that follow one another at one distance, as in runs of a byte or of a record: the copy warp
+// repeats it over all of them (128 KiB of zeros: 602 us byte by byte, 147 now).
 //
 // The stages run as a pipeline, handing over in buffers guarded by named barriers, so no warp spins.
 // Each stage is one or two warps' chain of dependent instructions, about six cycles each, which is
@@ -220,9 +222,10 @@ constexpr uint32_t kCells = 13;        // noted starts of one piece: an odd row 
 // long, so that 64 pieces fit the 7 KiB of the input ring that are resident behind any read position.
 // (Longer pieces, in a ring of twice the size, warm up less often but lose more where a block ends in
 // the stretch: as many turns on text, a fifth more on columns.)  Spans are odd numbers of words: the
-// lanes' first words lie in different banks.
+// lanes' first words lie in different banks.  What is left of a short stream is cut into pieces of kMinSpan
+// (chunks of 1 KiB of text 416 us, 462 with 13; a chunk of zeros, where 13 words overfill a row, 147 | 170).
 constexpr uint32_t kPieceTokens = 90;
-constexpr uint32_t kMinSpan = 13, kMaxSpan = 27;
+constexpr uint32_t kMinSpan = 5, kMaxSpan = 27;
 constexpr uint32_t kWarmBits = 640;
 
 enum : uint32_t { kBatchTokens = 0, kBatchStored = 1, kBatchDone = 2 };
@@ -246,12 +249,13 @@ constexpr uint32_t kRange = 3072;  // output bytes of one token batch
 struct TokenBatch {
   uint32_t starts[kRange / 32];  // bit b: a token starts at byte b of the range
   uint32_t list;    // which of the token warp's lists
-  uint32_t before;  // its tokens that start before the range; kStored: where the bytes are in the stream
+  uint32_t before;  // its tokens that start before the range; kStored: where the bytes are in the
+                    // stream; kRepeat: the distance
   uint32_t bytes;   // bytes of the range
   uint32_t what;    // kMore: another range of the same list follows; kLast: the chunk's last batch;
-                    // kStored: no tokens, but bytes of a stored block
+                    // kStored: no tokens, but bytes of a stored block; kRepeat: all bytes from one distance
 };
-enum : uint32_t { kMore = 1, kLast = 2, kStored = 4 };
+enum : uint32_t { kMore = 1, kLast = 2, kStored = 4, kRepeat = 8 };
 
 // 256 output bytes: word 32 i + l is the low half of byte 32 i + l's token.
 constexpr uint32_t kSteps = 8;
@@ -259,11 +263,11 @@ struct ByteBatch {
   uint16_t word[32 * kSteps];
   uint32_t bytes;
   uint32_t near;  // 0: every source lies before the batch; else one more than the bytes before the
-                  // first token that starts in the batch; or kStoredBytes
-  uint32_t from;  // kStoredBytes: where they are in the stream
+                  // first token that starts in the batch; or kStoredBytes, kRepeatedBytes
+  uint32_t from;  // kStoredBytes: where they are in the stream; kRepeatedBytes: the distance
   uint32_t last;  // the chunk's last batch; kBadChunk with it if the tokens were not sound
 };
-constexpr uint32_t kBadChunk = 2, kStoredBytes = 0xffffffffu;
+constexpr uint32_t kBadChunk = 2, kStoredBytes = 0xffffffffu, kRepeatedBytes = 0xfffffffeu;
 
 using InflateRing = InRing<8>;   // the scan's input
 using TokenRing = InRing<2>;     // a token warp's, which lags by up to two stretches
@@ -487,15 +491,17 @@ struct InflateScan {
     const uint32_t s_lit = smem_u32(sm.tab[tab].lit_lut), s_dist = smem_u32(sm.tab[tab].dist_lut);
     for (;;) {
       // no longer than the rest of the stream needs, so that short streams use all lanes
-      const uint32_t rest = (hi8 - pos) / (32u * kPieces);
-      const uint32_t words = (span < rest ? span : rest > kMinSpan ? rest : kMinSpan) | 1u;
+      const uint32_t rest = (hi8 - pos) / (32u * kPieces), most = rest > kMinSpan ? rest : kMinSpan;
+      const uint32_t words = (span < most ? span : most) | 1u;
       const uint32_t bits = words * 32u;
       int st = need(kPieces * bits + 64u);
       if (st) return st;
+      // no more symbols than a piece aims at, where they are short
+      const uint32_t warm = 32u * span < kWarmBits ? 32u * span : kWarmBits;
       const uint32_t from = pos + id * bits, end = from + bits;
       uint16_t* row = sm.batch[k].row + id * kCells;
       const bool inside = from < hi8;
-      uint32_t start = warm_up(id * bits > kWarmBits ? from - kWarmBits : pos, from, inside && id, s_lit, s_dist);
+      uint32_t start = warm_up(id * bits > warm ? from - warm : pos, from, inside && id, s_lit, s_dist);
       if (!inside) start = from;
       bool redo = start < hi8;
       uint32_t last = start, cnt = 0, how = redo ? kRun : kBad;
@@ -860,9 +866,8 @@ __device__ __forceinline__ void inflate_tokens(TokenRing& in, InflateTeam& sm, u
         handoff(0, 0, 0);
         continue;
       }
-      // the tokens' bytes in ranges the bit map covers: one, unless there are long matches
-      for (uint32_t r = 0; r < total; r += kRange) {
-        if (r) reuse();
+      // bytes [r, r + bytes) of the list: a mark where each token starts
+      const auto mark = [&](uint32_t r, uint32_t bytes) {
         uint32_t* starts = sm.out[me][k].starts;
         for (uint32_t i = lane; i < kRange / 32u; i += 32) starts[i] = 0;
         __syncwarp();
@@ -878,13 +883,44 @@ __device__ __forceinline__ void inflate_tokens(TokenRing& in, InflateTeam& sm, u
           for (uint32_t i = 0; i < n; i++) {
             const uint32_t tok = dst[i];
             if (s < r) before++;
-            else if (s - r < kRange) atomicOr(&starts[(s - r) >> 5], 1u << (s & 31u));
+            else if (s - r < bytes) atomicOr(&starts[(s - r) >> 5], 1u << ((s - r) & 31u));
             s += tok >> 16;
           }
           before = __reduce_add_sync(FULL, before);
         }
-        const bool more = total - r > kRange;
-        handoff(before, more ? kRange : total - r, more ? kMore : 0u);
+        handoff(before, bytes, r + bytes < total ? kMore : 0u);
+      };
+      if (total <= kRange) {
+        mark(0, total);
+        continue;
+      }
+      // Long matches: lanes whose tokens all have one distance, and neighbours at the same, go as one batch; the
+      // bytes of the others in ranges the bit map covers.
+      constexpr uint32_t kRepeatMin = 512;  // bytes of a lane's tokens
+      uint32_t dist = n && len >= kRepeatMin ? dst[0] & 0xffffu : kLiteral;
+      if (!(dist >> 15))
+        for (uint32_t i = 1; i < n; i++)
+          if ((dst[i] & 0xffffu) != dist) dist = kLiteral;
+      if (dist >> 15) dist = kLiteral;
+      const uint32_t below = __shfl_up_sync(FULL, dist, 1);
+      uint32_t cuts = __ballot_sync(FULL, lane == 0 || dist != below);
+      bool again = false;
+      while (cuts) {
+        const uint32_t a = __ffs(cuts) - 1u;
+        cuts &= cuts - 1u;
+        const uint32_t x = __shfl_sync(FULL, s0, a), d = __shfl_sync(FULL, dist, a);
+        const uint32_t next = __shfl_sync(FULL, s0, cuts ? __ffs(cuts) - 1 : 0), y = cuts ? next : total;
+        if (d == kLiteral) {
+          for (uint32_t r = x; r < y; r += kRange) {
+            if (again) reuse();
+            again = true;
+            mark(r, y - r < kRange ? y - r : kRange);
+          }
+        } else {
+          if (again) reuse();
+          again = true;
+          handoff(d + 1u, y - x, kRepeat | (y < total ? kMore : 0u));
+        }
       }
     }
   }
@@ -917,13 +953,15 @@ __device__ __forceinline__ void inflate_place(InflateTeam& sm, uint64_t chunk_by
     const TokenBatch& b = sm.out[me][buf];
     const uint32_t bytes = b.bytes, what = b.what, s_tok = smem_u32(sm.tok[me][b.list]);
     if (bytes > cap - op) ok = false;
-    if (ok && (what & kStored)) {
+    constexpr uint32_t kWhole = kStored | kRepeat;
+    if ((what & kRepeat) && b.before > op) ok = false;
+    if (ok && (what & kWhole)) {
       if (handed >= 2u) team_wait<64>(kBytesFree + k);
       if (lane == 0) sm.place[k].from = b.before;
-      handoff(bytes, kStoredBytes, 0);
+      handoff(bytes, what & kStored ? kStoredBytes : kRepeatedBytes, 0);
     }
     uint32_t count = b.before;  // tokens that start before the 1 KiB at c
-    for (uint32_t c = what & kStored ? bytes : 0u; ok && c < bytes; c += 1024) {
+    for (uint32_t c = what & kWhole ? bytes : 0u; ok && c < bytes; c += 1024) {
       // lane l: the starts in the 32 bytes at c + 32 l, and how many tokens start before them
       const uint32_t word = c + 32u * lane < bytes ? b.starts[c / 32u + lane] : 0u;
       const uint32_t upto = warp_scan_add(__popc(word), lane) + count, pre = upto - __popc(word);
@@ -1044,6 +1082,52 @@ __device__ __noinline__ uint32_t copy_stored(OUT out, uint32_t op, uint32_t n, c
   return out.flushed;
 }
 
+// n bytes at distance d from output position op on, 2 KiB at a time: single bytes from the d before them, and 16 at
+// once from a multiple of d and of 16 further back as soon as the repetition reaches that far (zeros: 128 KiB a
+// byte a lane 105 us, 16 bytes a lane 20).
+template <class OUT>
+__device__ __noinline__ uint32_t copy_repeated(OUT out, uint32_t op, uint32_t n, uint32_t d, uint32_t lane) {
+  const uint32_t step = 32u % d, far = 16u * d * ((512u + 16u * d - 1u) / (16u * d));
+  const auto bytes = [&](uint32_t count) {  // from op on
+    uint32_t r = lane % d;
+    for (uint32_t at = lane; at - lane < count; at += 128) {
+      uint32_t v[4];
+#pragma unroll
+      for (uint32_t i = 0; i < 4; i++) {
+        v[i] = out.get8(op - d + r);
+        r += step;
+        if (r >= d) r -= d;
+      }
+      __syncwarp();  // a far source's place is that of a byte written here
+#pragma unroll
+      for (uint32_t i = 0; i < 4; i++)
+        if (at + 32u * i < count) out.put8(op + at + 32u * i, v[i]);
+      __syncwarp();
+    }
+    op += count;
+    n -= count;
+  };
+  const uint32_t start = op - d;  // the repetition goes back to here
+  while (n) {
+    const uint32_t room = OUT::kFlush - (op & (OUT::kFlush - 1u)), m = n < room ? n : room;
+    const uint32_t head = (0u - op) & 15u, body = m > head ? (m - head) & ~15u : 0u;
+    if (body && far <= OUT::kBytes / 2 && op + head - start >= far) {
+      if (head) bytes(head);
+      for (uint32_t w = 16u * lane; w - 16u * lane < body; w += 512) {  // far is at least 512: sources lie before the step
+        if (w < body) st_s128(out.sbuf + ((op + w) & OUT::kMask), ld_s128(out.sbuf + ((op + w - far) & OUT::kMask)));
+        __syncwarp();
+      }
+      op += body;
+      n -= body;
+      if (m - head - body) bytes(m - head - body);
+    } else {
+      bytes(m);
+    }
+    out.flush_to(op);
+  }
+  return out.flushed;
+}
+
 // Warp 5 of the team: writes the bytes through `out` and returns the chunk's status.  `src`: the stream.
 template <class OUT>
 __device__ __forceinline__ int inflate_copy(InflateTeam& sm, OUT& out, const uint8_t* src, uint32_t len, uint32_t lane) {
@@ -1056,6 +1140,8 @@ __device__ __forceinline__ int inflate_copy(InflateTeam& sm, OUT& out, const uin
     last = b.last;
     if (near == kStoredBytes) {
       out.flushed = copy_stored(out, op, n, src - lo, b.from, lo + len, lane);
+    } else if (near == kRepeatedBytes) {
+      out.flushed = copy_repeated(out, op, n, b.from, lane);
     } else if (!near) {  // every source lies before the batch: all bytes at once
       uint32_t v[kSteps];
 #pragma unroll
