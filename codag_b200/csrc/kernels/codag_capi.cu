@@ -125,8 +125,29 @@ struct TeamShared {
   uint64_t bar4[4];
 };
 
+// The chunk by one warp, from the start, through the first part of the team's ring.
 template <int CODEC, int E>
-__global__ void __launch_bounds__(32 * kTeamWarpsOf<CODEC>)
+__device__ __noinline__ int decode_alone(uint8_t* ring, uint64_t* bar, const uint8_t* src, uint32_t len, uint8_t* dst, uint32_t store,
+                                         uint32_t cap, uint64_t wait_cycles, uint32_t lane) {
+  DirectOut o;
+  o.lane = lane;
+  o.begin(dst, store);
+  InRing<4> one;
+  one.buf = ring;
+  one.sbuf = smem_u32(ring);
+  one.bar = bar;
+  one.phase = 0;
+  one.wait_cycles = wait_cycles;
+  one.lane = lane;
+  init_ring_barriers<4>(one.bar, lane);
+  fence_proxy_async_smem();
+  one.begin(src, len);
+  return CODEC == CODAG_CODEC_RLEV1 ? decode_rlev1_chunk<4, E>(one, o, cap) : decode_rlev2_chunk<4, E>(one, o, cap);
+}
+
+// RLE v2: two CTAs a SM, as the compiler spills to fit three otherwise (3 MB of 16-bit values 179 us | 164)
+template <int CODEC, int E>
+__global__ void __launch_bounds__(32 * kTeamWarpsOf<CODEC>, CODEC == CODAG_CODEC_RLEV2 ? 2 : 6)
     k_rle_team(const uint8_t* __restrict__ comp, uint64_t comp_bytes, const uint64_t* __restrict__ blk_off,
                const uint64_t* __restrict__ col_len, uint64_t chunk_bytes, uint8_t* __restrict__ out, uint64_t out_bytes,
                int32_t* __restrict__ status, uint64_t wait_cycles) {
@@ -141,35 +162,19 @@ __global__ void __launch_bounds__(32 * kTeamWarpsOf<CODEC>)
     if (status && threadIdx.x == 0) status[chunk] = CODAG_ECORRUPT;
     return;
   }
-  const bool alone = CODEC == CODAG_CODEC_RLEV2 && rlev2_alone(comp + off, static_cast<uint32_t>(len), cap);
-  if (alone && warp != 0) return;
-  if (!alone) {
+  uint32_t state = kTeamFallback;
+  if (CODEC == CODAG_CODEC_RLEV1 || !rlev2_alone(comp + off, static_cast<uint32_t>(len), cap)) {
     if (warp == 1) init_ring_barriers<16>(sh.tb.bar, lane);
     if (threadIdx.x == 0) sh.tb.phase = 0;
     __syncthreads();
-  }
-  uint32_t state = kTeamFallback;
-  if (!alone)
     state = rle_team<CODEC, E, kTeamWarpsOf<CODEC>>(sh.team, sh.tb, comp + off, static_cast<uint32_t>(len), out + cbase, store,
                                                     cap, wait_cycles);
+  }
   if (warp != 0) return;
   int st = state == kTeamTimeout ? CODAG_ETIMEOUT : state == kTeamShort ? CODAG_ECORRUPT : CODAG_OK;
-  if (state == kTeamFallback) {  // in one pass, from the start
-    DirectOut o;
-    o.lane = lane;
-    o.begin(out + cbase, store);
-    InRing<4> one;
-    one.buf = sh.team.ring;
-    one.sbuf = smem_u32(sh.team.ring);
-    one.bar = sh.bar4;
-    one.phase = 0;
-    one.wait_cycles = wait_cycles;
-    one.lane = lane;
-    init_ring_barriers<4>(one.bar, lane);
-    fence_proxy_async_smem();
-    one.begin(comp + off, static_cast<uint32_t>(len));
-    st = CODEC == CODAG_CODEC_RLEV1 ? decode_rlev1_chunk<4, E>(one, o, cap) : decode_rlev2_chunk<4, E>(one, o, cap);
-  }
+  if (state == kTeamFallback)
+    st = decode_alone<CODEC, E>(sh.team.ring, sh.bar4, comp + off, static_cast<uint32_t>(len), out + cbase, store, cap, wait_cycles,
+                                lane);
   if (status && lane == 0) status[chunk] = st;
 }
 
