@@ -161,10 +161,11 @@ __global__ void __launch_bounds__(1024) k_classify(BatchArgs a, uint32_t n, uint
 }
 
 // Entries [0, n) of the order, each taken by the CTA's warps together, an RLE stream that a team cannot take by
-// the first alone; `mixed`: those for a team, the others are passed over.  False after a timeout; else sh.job is
+// the first alone; MIXED: those for a team, the others are passed over.  False after a timeout; else sh.job is
 // what the queue gave after the last entry.
-__device__ __forceinline__ bool team_jobs(const BatchArgs& a, uint64_t n, bool mixed, uint32_t* queue, BatchShared& sh,
-                                          uint64_t wait_cycles, uint32_t warp, uint32_t lane, RleRing& rle) {
+template <bool MIXED>
+__device__ __forceinline__ bool team_jobs(const BatchArgs& a, uint64_t n, uint32_t* queue, BatchShared& sh, uint64_t wait_cycles,
+                                          uint32_t warp, uint32_t lane, RleRing& rle) {
   InflateTeam& sm = sh.inflate;
   InflateRing in;
   TokenRing tin;
@@ -181,11 +182,11 @@ __device__ __forceinline__ bool team_jobs(const BatchArgs& a, uint64_t n, bool m
       sm.stop = sm.dead = 0;
     }
     __syncthreads();
-    const uint32_t job = sh.job, k = mixed ? job & ((1u << kCountBits) - 1u) : job;
-    if (k >= n || (mixed && !(job & kAnyTeam))) return true;
+    const uint32_t job = sh.job, k = MIXED ? job & ((1u << kCountBits) - 1u) : job;
+    if (k >= n || (MIXED && !(job & kAnyTeam))) return true;
     const uint32_t i = a.order ? a.order[k] : k;
     const codag_chunk_desc d = a.descs[i];
-    if (mixed) {
+    if constexpr (MIXED) {
       const uint32_t shift = (job & ~kAnyTeam) >> kCountBits;
       if (!wants_team(a, d, shift)) {  // on to the next entry for a team, if it is among those the threads look at
         constexpr uint32_t kLook = 8;
@@ -245,26 +246,27 @@ __device__ __forceinline__ bool team_jobs(const BatchArgs& a, uint64_t n, bool m
   }
 }
 
-// RLE entries [n0, n) of the order, one per warp; `mixed`: those not for a team, the first warp beginning with
+// RLE entries [n0, n) of the order, one per warp; MIXED: those not for a team, the first warp beginning with
 // `job`, which its CTA has taken already.
-__device__ __forceinline__ void rle_jobs(const BatchArgs& a, uint64_t n0, uint64_t n, bool mixed, uint32_t job, uint32_t* queue,
-                                         uint32_t warp, uint32_t lane, RleRing& in) {
+template <bool MIXED>
+__device__ __forceinline__ void rle_jobs(const BatchArgs& a, uint64_t n0, uint64_t n, uint32_t job, uint32_t* queue, uint32_t warp,
+                                         uint32_t lane, RleRing& in) {
   // a list of fewer than the grid's warps, and none for teams: the CTAs share it evenly (600 of 128 KiB: 217 us | 185)
-  if (mixed && !(job & kAnyTeam) && warp * gridDim.x >= n) return;
-  bool have = mixed && warp == 0;
+  if (MIXED && !(job & kAnyTeam) && warp * gridDim.x >= n) return;
+  bool have = MIXED && warp == 0;
   for (;;) {
     if (!have && lane == 0) job = atomicAdd(queue, 1u);
     have = false;
     job = __shfl_sync(FULL, job, 0);
     uint32_t k = job;
-    if (mixed) {
+    if (MIXED) {
       k &= (1u << kCountBits) - 1u;
       if (job & kAnyTeam) k -= static_cast<uint32_t>(n);  // the list's second time
     }
     if (k >= n - n0) break;
     const uint32_t i = a.order ? a.order[n0 + k] : static_cast<uint32_t>(n0) + k;
     const codag_chunk_desc& d = a.descs[i];
-    if (mixed && (job & kAnyTeam) && wants_team(a, d, (job & ~kAnyTeam) >> kCountBits)) continue;
+    if (MIXED && (job & kAnyTeam) && wants_team(a, d, (job & ~kAnyTeam) >> kCountBits)) continue;
     const int st = rle_job(a, d, in, lane);
     if (a.status && lane == 0) a.status[i] = st;
     if (st == CODAG_ETIMEOUT) break;  // ring state unknown: this warp stops pulling work
@@ -273,18 +275,19 @@ __device__ __forceinline__ void rle_jobs(const BatchArgs& a, uint64_t n0, uint64
 
 // Persistent grid, three CTAs per SM.  The first n_team entries of the order are taken by CTAs
 // (queue[0]), longest first; the others, a plan's short RLE files, by single warps (queue[1]), which
-// fills the SMs while the last of the CTAs' streams are decoded.  `mixed`: the list is in no such order, and
+// fills the SMs while the last of the CTAs' streams are decoded.  MIXED: the list is in no such order, and
 // n_team is n.
+template <bool MIXED>
 __global__ void __launch_bounds__(32 * kWarps, 3)
-    k_batch(BatchArgs a, uint64_t n, uint64_t n_team, bool mixed, uint32_t* __restrict__ queue, uint64_t wait_cycles) {
+    k_batch(BatchArgs a, uint64_t n, uint64_t n_team, uint32_t* __restrict__ queue, uint64_t wait_cycles) {
   extern __shared__ __align__(128) uint8_t smem[];
   BatchShared& sh = *reinterpret_cast<BatchShared*>(smem);
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   RleRing rle;
   rle_ring(rle, sh, wait_cycles, warp, lane);
-  if (n_team && !team_jobs(a, n_team, mixed, queue, sh, wait_cycles, warp, lane, rle)) return;
-  if (mixed) rle_jobs(a, 0, n, true, sh.job, queue, warp, lane, rle);
-  else if (n_team < n) rle_jobs(a, n_team, n, false, 0, queue + 1, warp, lane, rle);
+  if (n_team && !team_jobs<MIXED>(a, n_team, queue, sh, wait_cycles, warp, lane, rle)) return;
+  if (MIXED) rle_jobs<true>(a, 0, n, sh.job, queue, warp, lane, rle);
+  else if (n_team < n) rle_jobs<false>(a, n_team, n, 0, queue + 1, warp, lane, rle);
 }
 
 }  // namespace
@@ -308,11 +311,12 @@ namespace {
 
 // CTAs of the persistent grid on the current device: as many as are resident at once
 codag_status batch_grid_cap(int* cap) {
-  if (allow_smem(k_batch, sizeof(BatchShared)) != cudaSuccess) return CODAG_ECUDA;
+  if (allow_smem(k_batch<false>, sizeof(BatchShared)) != cudaSuccess || allow_smem(k_batch<true>, sizeof(BatchShared)) != cudaSuccess)
+    return CODAG_ECUDA;
   int dev = 0, sms = 0, per_sm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return CODAG_ECUDA;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch, 32 * kWarps, sizeof(BatchShared)) != cudaSuccess)
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch<false>, 32 * kWarps, sizeof(BatchShared)) != cudaSuccess)
     return CODAG_ECUDA;
   *cap = sms * std::max(per_sm, 1);
   return CODAG_OK;
@@ -320,13 +324,13 @@ codag_status batch_grid_cap(int* cap) {
 
 void batch_enqueue(const BatchArgs& a, uint64_t n, uint64_t n_team, uint32_t* queue, int grid, cudaStream_t s) {
   cudaMemsetAsync(queue, 0, (n_team < n ? 2 : 1) * sizeof(uint32_t), s);
-  k_batch<<<grid, 32 * kWarps, sizeof(BatchShared), s>>>(a, n, n_team, false, queue, wait_of());
+  k_batch<false><<<grid, 32 * kWarps, sizeof(BatchShared), s>>>(a, n, n_team, queue, wait_of());
 }
 void mixed_enqueue(const BatchArgs& a, uint64_t n, uint32_t* queue, uint64_t resident, cudaStream_t s) {
   const int grid = static_cast<int>(std::min(n, resident));
   if (n > kMaxMixed) return batch_enqueue(a, n, n, queue, grid, s);
   k_classify<<<1, 1024, 0, s>>>(a, static_cast<uint32_t>(n), static_cast<uint32_t>(resident), queue);
-  k_batch<<<grid, 32 * kWarps, sizeof(BatchShared), s>>>(a, n, n, true, queue, wait_of());
+  k_batch<true><<<grid, 32 * kWarps, sizeof(BatchShared), s>>>(a, n, n, queue, wait_of());
 }
 // CTAs decode RLE files whose output is element aligned; a plan checks the offsets, so the base has to be, too
 void plan_enqueue(const codag_plan& p, const BatchArgs& a, cudaStream_t s) {

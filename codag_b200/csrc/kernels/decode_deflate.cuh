@@ -768,7 +768,7 @@ __device__ __forceinline__ void inflate_tokens(TokenRing& in, InflateTeam& sm, u
   };
   // bytes [at, end) resident
   const auto need = [&](uint32_t at, uint32_t end) {
-    const bool ok = in.skip(at) && in.release(at) && in.ensure(end < in.hi ? end : in.hi) == CODAG_OK;
+    const bool ok = in.release(at) && in.ensure(end < in.hi ? end : in.hi) == CODAG_OK;
     if (!ok && lane == 0) sm.dead = 1;
     return ok;
   };
@@ -799,6 +799,7 @@ __device__ __forceinline__ void inflate_tokens(TokenRing& in, InflateTeam& sm, u
         const bool drop = stopped();
         handoff(b.base, drop ? 0u : b.size, drop ? 0u : static_cast<uint32_t>(kStored));
       }
+      if (!in.skip(b.base + b.size) && lane == 0) sm.dead = 1;
       continue;
     }
     // cells of the pieces, as running totals
@@ -1138,11 +1139,7 @@ __device__ __forceinline__ int inflate_copy(InflateTeam& sm, OUT& out, const uin
     const ByteBatch& b = sm.place[k];
     const uint32_t n = b.bytes, near = b.near;
     last = b.last;
-    if (near == kStoredBytes) {
-      out.flushed = copy_stored(out, op, n, src - lo, b.from, lo + len, lane);
-    } else if (near == kRepeatedBytes) {
-      out.flushed = copy_repeated(out, op, n, b.from, lane);
-    } else if (!near) {  // every source lies before the batch: all bytes at once
+    if (!near) {  // every source lies before the batch: all bytes at once
       uint32_t v[kSteps];
 #pragma unroll
       for (uint32_t i = 0; i < kSteps; i++) v[i] = b.word[32u * i + lane];
@@ -1154,6 +1151,9 @@ __device__ __forceinline__ int inflate_copy(InflateTeam& sm, OUT& out, const uin
       for (uint32_t i = 0; i < kSteps; i++)
         if (32u * i + lane < n) out.put8(op + 32u * i + lane, v[i]);
       __syncwarp();
+    } else if (near >= kRepeatedBytes) {
+      out.flushed = near == kStoredBytes ? copy_stored(out, op, n, src - lo, b.from, lo + len, lane)
+                                         : copy_repeated(out, op, n, b.from, lane);
     } else if (near > n) {  // one match, repeating itself
       const uint32_t d = b.word[0] + 1u, step = 32u % d;
       uint32_t r = lane % d;
