@@ -177,8 +177,9 @@ codag_status codag_compress_rlev2(const uint8_t *d_in, uint64_t in_bytes, uint64
  * least 4 because an RLE v2 header with its data spans up to 2060 bytes).
  * cta_per_chunk = 1 gives each RLE chunk a whole CTA whatever their number (without it, those not
  * named above have one; it applies without a workspace, when the output and out_bytes are element
- * aligned).  Deflate chunks are always decoded by a team of six warps
- * each: their shape, and lut_bits (9, 10 or 11), are checked and kept, and change nothing.
+ * aligned).  Deflate chunks are decoded by a team of six warps each, or by one where many small
+ * ones, or long runs or stored bytes, make that faster: their shape, and lut_bits (9, 10 or 11), are
+ * checked and kept, and change nothing.
  * Values outside the supported sets return CODAG_EINVAL. */
 typedef struct {
     int32_t warps_per_cta;

@@ -1,0 +1,107 @@
+"""Deflate chunks of which each has a single warp, as there are many and they are small, or nearly all runs or stored
+bytes: the contents and sizes of the team decoder's tests, text whose matches reach past the warp's window of 1 KiB,
+damaged streams, and what they cost, as a multiple of a device copy of as many bytes."""
+import zlib
+
+import numpy as np
+import pytest
+
+from tests.test_deflate_team_edges import KINDS, _stream
+
+
+def _decode(cuda, parts, size, n, total):
+    """Streams `parts` in turn as n chunks of `size` bytes: (output with its guard, statuses)."""
+    from codag_b200 import api
+    blob = b"".join(parts)
+    comp = np.frombuffer(blob * -(-n // len(parts)), np.uint8).copy()
+    lens = np.array([len(p) for p in parts])
+    rel = np.concatenate([[0], np.cumsum(np.resize(lens, n))]).astype(np.int64)
+    comp = comp[:rel[-1]]
+    out = cuda.full((total + 64,), 0xA5, dtype=cuda.uint8, device="cuda")
+    st = cuda.full((n,), -1, dtype=cuda.int32, device="cuda")
+    api.decompress_deflate(cuda.from_numpy(comp).to("cuda"), cuda.from_numpy(rel).to("cuda"), size, out, 2, total, st)
+    return out.cpu().numpy(), st.cpu().numpy()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("size", [1, 31, 256, 257, 511, 1023, 1024, 1025, 2048, 5000, 16384])
+@pytest.mark.parametrize("kind", sorted(KINDS))
+def test_kinds(cuda, kind, size):
+    data = KINDS[kind](np.random.default_rng(size), size).tobytes()[:size]
+    parts = [_stream(data, level, strategy, every)
+             for level, strategy in ((0, 0), (1, 0), (9, 0), (6, zlib.Z_FIXED), (6, zlib.Z_HUFFMAN_ONLY))
+             for every in (0, max(size // 7, 1), max(size // 2 - 1, 1))]
+    n = 6000
+    total = n * size - size // 3
+    for group in (parts, parts[:3], parts[6:9]):  # all; stored blocks; level 9
+        got, st = _decode(cuda, group, size, n, total)
+        assert not st.any()
+        assert np.all(got[total:] == 0xA5), "wrote past out_bytes"
+        assert np.array_equal(got[:total], np.resize(np.frombuffer(data, np.uint8), total))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("size,n", [(1024, 4096), (2048, 9000), (3000, 9000)])
+def test_text(cuda, native, size, n):
+    raw = native.gen_text(64 * size, size)
+    parts = [zlib.compress(raw[i * size:(i + 1) * size].tobytes(), 1 + i % 9) for i in range(64)]
+    got, st = _decode(cuda, parts, size, n, n * size)
+    assert not st.any()
+    assert np.array_equal(got[:n * size], np.resize(raw, n * size))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("size", [700, 2000])
+def test_damaged(cuda, native, oracle, size):
+    """Bytes flipped: what zlib takes is taken and gives the same bytes."""
+    rng = np.random.default_rng(size)
+    raw = native.gen_text(400 * size, 5)
+    parts = []
+    for i in range(400):
+        s = bytearray(zlib.compress(raw[i * size:(i + 1) * size].tobytes(), int(rng.integers(0, 10))))
+        for p in rng.integers(2, len(s), int(rng.integers(0, 4))):
+            s[p] ^= int(rng.integers(1, 256))
+        parts.append(bytes(s))
+    got, st = _decode(cuda, parts, size, 8000, 8000 * size)
+    seen = set()
+    for i, p in enumerate(parts):
+        d = zlib.decompressobj(-15)
+        try:
+            ref = d.decompress(p[2:], size + 1)
+            ok = d.eof and len(ref) == size
+        except zlib.error:
+            ok = False
+        seen.add(ok)
+        assert len(set(st[i::400])) == 1
+        if ok:
+            assert st[i] == 0 and np.array_equal(got[i * size:(i + 1) * size], np.frombuffer(ref, np.uint8)), i
+        else:
+            assert st[i] in (0, 2)  # incomplete codes, which zlib refuses, are accepted
+    assert seen == {True, False}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind,chunk,most", [("text", 1024, 150), ("zeros", 4096, 20), ("noise", 4096, 5)])
+def test_cost(cuda, native, kind, chunk, most):
+    """64 MiB; teams take 220, 50 and 7.7 times as long as a device copy."""
+    from codag_b200 import api
+    size = 64 << 20
+    raw = {"text": lambda: native.gen_text(size, 3), "zeros": lambda: np.zeros(size, np.uint8),
+           "noise": lambda: np.random.default_rng(2).integers(0, 256, size, dtype=np.uint8)}[kind]()
+    comp, blk, _ = native.encode_deflate(raw, chunk, 6, require_no_stored=False)
+    d, o = cuda.from_numpy(comp).to("cuda"), cuda.from_numpy(blk[1:].view(np.int64)).to("cuda")
+    out, src = cuda.zeros(size, dtype=cuda.uint8, device="cuda"), cuda.from_numpy(raw).to("cuda")
+    st = cuda.full((blk.size - 2,), -1, dtype=cuda.int32, device="cuda")
+    best = [1e9, 1e9]
+    for r in range(10):
+        for i, fn in enumerate((lambda: api.decompress_deflate(d, o, chunk, out, 2, None, st), lambda: out.copy_(src))):
+            a, b = cuda.cuda.Event(enable_timing=True), cuda.cuda.Event(enable_timing=True)
+            a.record()
+            fn()
+            b.record()
+            cuda.cuda.synchronize()
+            if r >= 2:
+                best[i] = min(best[i], a.elapsed_time(b))
+            if r == 0 and i == 0:
+                assert not st.cpu().numpy().any() and np.array_equal(out.cpu().numpy(), raw)
+    assert best[0] < most * best[1], best
