@@ -8,7 +8,7 @@
 #include <vector>
 
 #include "capi_common.cuh"
-#include "decode_deflate.cuh"
+#include "decode_deflate_warp.cuh"
 #include "decode_rle_team.cuh"
 
 using namespace codag_dev;
@@ -19,12 +19,17 @@ namespace {
 constexpr uint32_t kWarps = kTeamWarps;  // warps per CTA (eight, for RLE files, cost Deflate 7% in registers)
 using RleRing = InRing<4>;
 using BatchV2 = TeamV2<3>;
+struct OneWarp {  // a stream on one warp
+  alignas(128) uint8_t ring[align_up(RleRing::kAlloc, 128)];
+  alignas(16) uint8_t win[InflateWarpWin::kBytes];  // Deflate
+  InflateWarp tables;
+};
 struct BatchShared {
   union {
     InflateTeam inflate;
     TeamV1 v1;
     BatchV2 v2;
-    alignas(128) uint8_t ring[kWarps][align_up(RleRing::kAlloc, 128)];
+    OneWarp one[kWarps];
   };
   TeamBars tb;
   uint64_t bar[kWarps][4];  // of the warps' own rings
@@ -33,7 +38,7 @@ struct BatchShared {
   int32_t st;
 };
 static_assert(sizeof(TeamV1) <= offsetof(InflateTeam, bar) && sizeof(BatchV2) <= offsetof(InflateTeam, bar) &&
-                  kWarps * align_up(RleRing::kAlloc, 128) <= offsetof(InflateTeam, bar),
+                  kWarps * sizeof(OneWarp) <= offsetof(InflateTeam, bar),
               "the Deflate team's barriers keep their place");
 static_assert(sizeof(BatchShared) <= 76800, "three CTAs per SM");
 
@@ -52,10 +57,27 @@ __device__ __forceinline__ bool job_in_bounds(const BatchArgs& a, const codag_ch
          stream_in_bounds(d.comp_off, d.comp_len, a.comp_bytes);
 }
 
-// An RLE stream on one warp.  Values go straight to global memory: element by element when the
+// A Deflate stream on one warp
+__device__ __noinline__ int inflate_job(const uint8_t* src, uint32_t len, uint8_t* dst, uint32_t out_len, uint32_t wrapper,
+                                        RleRing& ring, OneWarp& sh, uint32_t lane) {
+  RleRing in = ring;
+  in.begin(src, len);
+  InflateWarpWin o;
+  o.buf = sh.win;
+  o.sbuf = smem_u32(sh.win);
+  o.lane = lane;
+  o.begin(dst, out_len);
+  const int st = inflate_warp(in, o, sh.tables, out_len, wrapper, lane);
+  ring = in;
+  return st;
+}
+
+// A stream on one warp.  RLE values go straight to global memory: element by element when the
 // output is element aligned, byte by byte otherwise.
-__device__ __forceinline__ int rle_job(const BatchArgs& a, const codag_chunk_desc& d, RleRing& in, uint32_t lane) {
+__device__ __forceinline__ int warp_job(const BatchArgs& a, const codag_chunk_desc& d, RleRing& in, OneWarp& sh, uint32_t lane) {
   if (!job_in_bounds(a, d)) return CODAG_ECORRUPT;
+  if (d.codec == CODAG_CODEC_DEFLATE)
+    return inflate_job(a.comp + d.comp_off, d.comp_len, a.out + d.out_off, d.out_len, d.wrapper_bytes, in, sh, lane);
   if (d.codec != CODAG_CODEC_RLEV1 && d.codec != CODAG_CODEC_RLEV2) return CODAG_EINVAL;
   in.begin(a.comp + d.comp_off, d.comp_len);
   const uint32_t e = d.elem_bytes;
@@ -71,11 +93,10 @@ __device__ __forceinline__ int rle_job(const BatchArgs& a, const codag_chunk_des
   return decode_rle_any(d.codec, in, ob, d.out_len, static_cast<int>(e));
 }
 
-__device__ __forceinline__ void rle_ring(RleRing& in, BatchShared& sh, uint64_t wait_cycles, uint32_t warp,
-                                         uint32_t lane) {
-  in.buf = sh.ring[warp];
+__device__ __forceinline__ void rle_ring(RleRing& in, OneWarp& sh, uint64_t* bar, uint64_t wait_cycles, uint32_t lane) {
+  in.buf = sh.ring;
   in.sbuf = smem_u32(in.buf);
-  in.bar = sh.bar[warp];
+  in.bar = bar;
   in.phase = 0;
   in.wait_cycles = wait_cycles;
   in.lane = lane;
@@ -133,31 +154,66 @@ __host__ __device__ __forceinline__ bool rle_team_pays(const codag_chunk_desc& d
   return shifts_below(d.out_len) > shift && !direct;
 }
 
+// Deflate files that warps (18 a SM) get through faster than teams (three a SM).  Teams take them all the same where
+// these are done before the longest of them is on a warp.
+struct InflateJob {
+  InflateCost c;
+  __host__ __device__ __forceinline__ explicit InflateJob(const codag_chunk_desc& d) : c(inflate_cost(d.out_len, d.comp_len)) {}
+  __host__ __device__ __forceinline__ bool small() const { return 15.f * c.team > 4.f * c.warp; }
+};
+struct SmallInflates {
+  float team = 0, longest = 0;
+  __host__ __device__ __forceinline__ void add(const InflateJob& j) {
+    if (!j.small()) return;
+    team += j.c.team;
+    longest = longest > j.c.warp ? longest : j.c.warp;
+  }
+  __host__ __device__ __forceinline__ bool by_warps(uint64_t resident) const { return team > longest * static_cast<float>(resident); }
+};
+
 // Without a plan the host does not know the files.  k_classify writes to *queue what k_batch has to know of
 // them; k_batch counts its entries in the low bits.  It goes over the list twice: CTAs take the files for
 // teams, then single warps the others, which is how a plan sorts them.
-constexpr uint32_t kCountBits = 26, kAnyTeam = 1u << 31;
+constexpr uint32_t kCountBits = 25, kAnyTeam = 1u << 31, kInflateWarps = 1u << kCountBits, kShiftAt = kCountBits + 1;
 constexpr uint64_t kMaxMixed = (1u << (kCountBits - 1)) - 65536u;  // counts to twice that, and once more per warp
-__device__ __forceinline__ bool wants_team(const BatchArgs& a, const codag_chunk_desc& d, uint32_t shift) {
-  return d.codec == CODAG_CODEC_DEFLATE || (rle_team_takes(a, d) && rle_team_pays(d, shift));
+__device__ __forceinline__ bool wants_team(const BatchArgs& a, const codag_chunk_desc& d, uint32_t flags) {
+  if (d.codec == CODAG_CODEC_DEFLATE) return !(flags & kInflateWarps) || !InflateJob(d).small();
+  return d.out_len > kWarpBytes && rle_team_takes(a, d) && rle_team_pays(d, (flags & ~kAnyTeam) >> kShiftAt);
 }
 __global__ void __launch_bounds__(1024) k_classify(BatchArgs a, uint32_t n, uint32_t resident, uint32_t* __restrict__ queue) {
   __shared__ uint32_t long_v2[kShifts];
+  __shared__ float small_team;
+  __shared__ int small_longest;  // a float's bits, which compare as it does
   if (threadIdx.x < kShifts) long_v2[threadIdx.x] = 0;
+  if (threadIdx.x == 0) small_team = small_longest = 0;
   __syncthreads();
-  bool any = false;
+  bool any = false, large = false;  // there are files for teams; Deflate files among them that warps do not take
+  SmallInflates mine;
 #pragma unroll 4
   for (uint32_t i = threadIdx.x; i < n; i += 1024) {
-    const codag_chunk_desc& d = a.descs[i];
-    const bool wants = wants_team(a, d, 0);
-    if (d.codec != CODAG_CODEC_RLEV2) any |= wants;
-    else if (wants) atomicAdd(&long_v2[shifts_below(d.out_len)], 1u);
+    const codag_chunk_desc d = a.descs[i];
+    if (d.codec == CODAG_CODEC_DEFLATE) {
+      const InflateJob j(d);
+      mine.add(j);
+      large |= !j.small();
+    } else if (wants_team(a, d, 0)) {
+      if (d.codec != CODAG_CODEC_RLEV2) any = true;
+      else atomicAdd(&long_v2[shifts_below(d.out_len)], 1u);
+    }
   }
-  any = __syncthreads_or(any);
+  if (mine.team > 0) {
+    atomicAdd(&small_team, mine.team);
+    atomicMax(&small_longest, __float_as_int(mine.longest));
+  }
+  any = __syncthreads_or(any || large);
   if (threadIdx.x != 0) return;
+  mine.team = small_team;
+  mine.longest = __int_as_float(small_longest);
+  const bool warps = mine.by_warps(resident);
+  any |= mine.team > 0 && !warps;
   const uint32_t shift = v2_shift(long_v2, resident);
   for (uint32_t j = shift + 1; j < kShifts; j++) any |= long_v2[j] != 0;
-  *queue = (any ? kAnyTeam : 0u) | (shift << kCountBits);
+  *queue = (any ? kAnyTeam : 0u) | (warps ? kInflateWarps : 0u) | (shift << kShiftAt);
 }
 
 // Entries [0, n) of the order, each taken by the CTA's warps together, an RLE stream that a team cannot take by
@@ -187,15 +243,14 @@ __device__ __forceinline__ bool team_jobs(const BatchArgs& a, uint64_t n, uint32
     const uint32_t i = a.order ? a.order[k] : k;
     const codag_chunk_desc d = a.descs[i];
     if constexpr (MIXED) {
-      const uint32_t shift = (job & ~kAnyTeam) >> kCountBits;
-      if (!wants_team(a, d, shift)) {  // on to the next entry for a team, if it is among those the threads look at
+      if (!wants_team(a, d, job)) {  // on to the next entry for a team, if it is among those the threads look at
         constexpr uint32_t kLook = 8;
         uint32_t far = k + 1u + kLook * 32u * kWarps;
         if (far > n) far = static_cast<uint32_t>(n);
 #pragma unroll
         for (uint32_t q = 0; q < kLook; q++) {
           const uint32_t e = k + 1u + q * 32u * kWarps + threadIdx.x;
-          if (e < far && wants_team(a, a.descs[a.order ? a.order[e] : e], shift)) far = e;
+          if (e < far && wants_team(a, a.descs[a.order ? a.order[e] : e], job)) far = e;
         }
         far = __reduce_min_sync(FULL, far);
         if (lane == 0) atomicMin(&sh.ahead, far);
@@ -213,7 +268,7 @@ __device__ __forceinline__ bool team_jobs(const BatchArgs& a, uint64_t n, uint32
         int st = state == kTeamTimeout ? CODAG_ETIMEOUT : state == kTeamShort ? CODAG_ECORRUPT : CODAG_OK;
         if (state == kTeamFallback) {
           fence_proxy_async_smem();
-          st = rle_job(a, d, rle, lane);
+          st = warp_job(a, d, rle, sh.one[0], lane);
         }
         if (lane == 0) {
           if (a.status) a.status[i] = st;
@@ -246,11 +301,11 @@ __device__ __forceinline__ bool team_jobs(const BatchArgs& a, uint64_t n, uint32
   }
 }
 
-// RLE entries [n0, n) of the order, one per warp; MIXED: those not for a team, the first warp beginning with
+// Entries [n0, n) of the order, one per warp; MIXED: those not for a team, the first warp beginning with
 // `job`, which its CTA has taken already.
 template <bool MIXED>
-__device__ __forceinline__ void rle_jobs(const BatchArgs& a, uint64_t n0, uint64_t n, uint32_t job, uint32_t* queue, uint32_t warp,
-                                         uint32_t lane, RleRing& in) {
+__device__ __forceinline__ void warp_jobs(const BatchArgs& a, uint64_t n0, uint64_t n, uint32_t job, uint32_t* queue, uint32_t warp,
+                                          uint32_t lane, RleRing& in, OneWarp& sh) {
   // a list of fewer than the grid's warps, and none for teams: the CTAs share it evenly (600 of 128 KiB: 217 us | 185)
   if (MIXED && !(job & kAnyTeam) && warp * gridDim.x >= n) return;
   bool have = MIXED && warp == 0;
@@ -266,8 +321,8 @@ __device__ __forceinline__ void rle_jobs(const BatchArgs& a, uint64_t n0, uint64
     if (k >= n - n0) break;
     const uint32_t i = a.order ? a.order[n0 + k] : static_cast<uint32_t>(n0) + k;
     const codag_chunk_desc& d = a.descs[i];
-    if (MIXED && (job & kAnyTeam) && wants_team(a, d, (job & ~kAnyTeam) >> kCountBits)) continue;
-    const int st = rle_job(a, d, in, lane);
+    if (MIXED && (job & kAnyTeam) && wants_team(a, d, job)) continue;
+    const int st = warp_job(a, d, in, sh, lane);
     if (a.status && lane == 0) a.status[i] = st;
     if (st == CODAG_ETIMEOUT) break;  // ring state unknown: this warp stops pulling work
   }
@@ -284,10 +339,22 @@ __global__ void __launch_bounds__(32 * kWarps, 3)
   BatchShared& sh = *reinterpret_cast<BatchShared*>(smem);
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   RleRing rle;
-  rle_ring(rle, sh, wait_cycles, warp, lane);
+  rle_ring(rle, sh.one[warp], sh.bar[warp], wait_cycles, lane);
   if (n_team && !team_jobs<MIXED>(a, n_team, queue, sh, wait_cycles, warp, lane, rle)) return;
-  if (MIXED) rle_jobs<true>(a, 0, n, sh.job, queue, warp, lane, rle);
-  else if (n_team < n) rle_jobs<false>(a, n_team, n, 0, queue + 1, warp, lane, rle);
+  if (MIXED) warp_jobs<true>(a, 0, n, sh.job, queue, warp, lane, rle, sh.one[warp]);
+  else if (n_team < n) warp_jobs<false>(a, n_team, n, 0, queue + 1, warp, lane, rle, sh.one[warp]);
+}
+
+// A plan without files for teams: as many warps as an SM has registers for.
+constexpr uint32_t kFew = 2, kFewCtas = 12;
+__global__ void __launch_bounds__(32 * kFew, kFewCtas)
+    k_batch_warps(BatchArgs a, uint64_t n, uint32_t* __restrict__ queue, uint64_t wait_cycles) {
+  __shared__ OneWarp one[kFew];
+  __shared__ uint64_t bar[kFew][4];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  RleRing rle;
+  rle_ring(rle, one[warp], bar[warp], wait_cycles, lane);
+  warp_jobs<false>(a, 0, n, 0, queue, warp, lane, rle, one[warp]);
 }
 
 }  // namespace
@@ -324,7 +391,8 @@ codag_status batch_grid_cap(int* cap) {
 
 void batch_enqueue(const BatchArgs& a, uint64_t n, uint64_t n_team, uint32_t* queue, int grid, cudaStream_t s) {
   cudaMemsetAsync(queue, 0, (n_team < n ? 2 : 1) * sizeof(uint32_t), s);
-  k_batch<false><<<grid, 32 * kWarps, sizeof(BatchShared), s>>>(a, n, n_team, queue, wait_of());
+  if (n_team == 0) k_batch_warps<<<grid, 32 * kFew, 0, s>>>(a, n, queue, wait_of());
+  else k_batch<false><<<grid, 32 * kWarps, sizeof(BatchShared), s>>>(a, n, n_team, queue, wait_of());
 }
 void mixed_enqueue(const BatchArgs& a, uint64_t n, uint32_t* queue, uint64_t resident, cudaStream_t s) {
   const int grid = static_cast<int>(std::min(n, resident));
@@ -387,9 +455,14 @@ extern "C" codag_status codag_batch_plan(const codag_chunk_desc* h_descs, uint64
   for (uint64_t i = 0; i < n; i++)
     if (h_descs[i].codec == CODAG_CODEC_RLEV2 && rle_team_pays(h_descs[i], 0)) long_v2[shifts_below(h_descs[i].out_len)]++;
   const uint32_t shift = v2_shift(long_v2, static_cast<uint64_t>(cap));
+  SmallInflates small;
+  for (uint64_t i = 0; i < n; i++)
+    if (h_descs[i].codec == CODAG_CODEC_DEFLATE) small.add(InflateJob(h_descs[i]));
+  const bool inflate_warps = small.by_warps(static_cast<uint64_t>(cap));
   const auto team = [&](uint32_t i) {
     const codag_chunk_desc& d = h_descs[i];
-    return d.codec == CODAG_CODEC_DEFLATE || (rle_team_pays(d, shift) && d.out_off % d.elem_bytes == 0);
+    if (d.codec == CODAG_CODEC_DEFLATE) return !inflate_warps || !InflateJob(d).small();
+    return (rle_team_pays(d, shift) && d.out_off % d.elem_bytes == 0);
   };
   uint64_t longest = 0, total = 0;
   for (uint64_t i = 0; i < n; i++) {
@@ -413,6 +486,7 @@ extern "C" codag_status codag_batch_plan(const codag_chunk_desc* h_descs, uint64
   const uint64_t need = p->n_team + (n - p->n_team + kWarps - 1) / kWarps;
   p->grid = static_cast<int>(std::min<uint64_t>(need, grid_cap(static_cast<uint64_t>(cap), longest, total)));
   p->mixed_grid = cap;
+  if (p->n_team == 0) p->grid = static_cast<int>(std::min<uint64_t>((n + kFew - 1) / kFew, static_cast<uint64_t>(cap) / 3 * kFewCtas));
   *plan = p;
   return CODAG_OK;
 }

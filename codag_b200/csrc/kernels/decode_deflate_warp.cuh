@@ -264,12 +264,13 @@ struct WarpInflater {
 // What a chunk takes, in ns: a team's place (three a SM), or one warp, of which 32 a SM take 1.6 times as long; fitted
 // to text, columns, zeros and random bytes in chunks of 1 to 128 KiB (64 MiB of each, and few chunks).
 struct InflateCost {
-  uint64_t team, warp;
+  float team, warp;
 };
 __host__ __device__ __forceinline__ InflateCost inflate_cost(uint64_t out_bytes, uint64_t stream) {
+  const float o = static_cast<float>(out_bytes), s = static_cast<float>(stream);
   if (stream >= out_bytes && stream <= out_bytes + out_bytes / 64u + 64u)  // stored blocks
-    return {4000u + out_bytes * 6u / 10u, 4000u + out_bytes * 19u / 10u};
-  return {34000u + out_bytes * 15u / 10u + stream * 14u, 15000u + out_bytes * 31u / 10u + stream * 270u};
+    return {4000.f + 0.6f * o, 4000.f + 1.9f * o};
+  return {34000.f + 1.5f * o + 14.f * s, 15000.f + 3.1f * o + 270.f * s};
 }
 
 // The chunk's status; `in` is bound to its stream, `out` to its output.

@@ -92,11 +92,10 @@ codag_status launch_warp(const uint8_t* comp, uint64_t comp_bytes, const uint64_
 // 57 | 152, 4096 415 | 220, 1024 of 4 KiB 175 | 480, 16384 2063 | 2433; zeros: 1024 of 4 KiB 122 | 42, of 64 KiB
 // 329 | 210, 512 of 128 KiB 283 | 370; random bytes: 1024 of 4 KiB 31 | 23, 512 of 128 KiB 155 | 263.
 bool warp_pays(uint64_t n, uint64_t chunk_bytes, uint64_t comp_bytes) {
-  constexpr double kSms = 148;
+  constexpr float kSms = 148;
   const InflateCost c = inflate_cost(chunk_bytes, comp_bytes / n);
-  const double count = static_cast<double>(n), teams = count / (3 * kSms), warps = 1.6 * count / (32 * kSms);
-  const double team = 4000.0 + static_cast<double>(c.team) * (teams > 1 ? teams : 1);
-  return static_cast<double>(c.warp) * (warps > 1 ? warps : 1) < team;
+  const float count = static_cast<float>(n), teams = count / (3 * kSms), warps = 1.6f * count / (32 * kSms);
+  return c.warp * (warps > 1 ? warps : 1) < 4000.f + c.team * (teams > 1 ? teams : 1);
 }
 
 }  // namespace

@@ -1,4 +1,4 @@
-"""Which RLE streams of a batch have a whole CTA and which a single warp, planned or not: lists in which the two
+"""Which streams of a batch have a whole CTA and which a single warp, planned or not: lists in which the two
 kinds alternate, stand apart or leave one kind out, in both orders; and the cost of a choice that does not look at
 the list, as a ratio of two times taken in turn."""
 import numpy as np
@@ -54,6 +54,9 @@ LISTS = {
     "a team at the start": [(DEF, 1, 5000)] + [(V2, 8, 256)] * 5000,
     "far apart": ([(DEF, 1, 2000)] + [(V1, 2, 512)] * 1600) * 3,
     "in turn": [(DEF, 1, 2000), (V2, 8, 512), (V1, 4, 33000), (V2, 2, 40000)] * 120,
+    "small deflate": [(DEF, 1, 700)] * 9000,
+    "small deflate and others": [(DEF, 1, 700)] * 9000 + [(V2, 8, 512), (DEF, 1, 70000), (V1, 4, 33000), (V2, 8, 40000)] * 30,
+    "small deflate, too few": [(DEF, 1, 700)] * 100 + [(V1, 8, 512)] * 100,
     "many long v2, one longest": [(V2, 8, 40000)] * 460 + [(V2, 8, 800000)],
 }
 

@@ -63,6 +63,8 @@ def test_damaged(cuda, native, oracle, size):
             s[p] ^= int(rng.integers(1, 256))
         parts.append(bytes(s))
     got, st = _decode(cuda, parts, size, 8000, 8000 * size)
+    _, in_batch = _batch(cuda, native, parts, size, 8000)
+    assert np.array_equal(st, in_batch)
     seen = set()
     for i, p in enumerate(parts):
         d = zlib.decompressobj(-15)
@@ -78,6 +80,33 @@ def test_damaged(cuda, native, oracle, size):
         else:
             assert st[i] in (0, 2)  # incomplete codes, which zlib refuses, are accepted
     assert seen == {True, False}
+
+
+def _batch(cuda, native, parts, size, n):
+    """The same as files of one plan."""
+    from codag_b200 import api
+    cs = api.pack_chunks([np.frombuffer(parts[i % len(parts)], np.uint8) for i in range(n)], [native.DEFLATE] * n, [1] * n,
+                         [size] * n)
+    out = cuda.zeros(cs.out_bytes, dtype=cuda.uint8, device="cuda")
+    st = cuda.full((n,), -1, dtype=cuda.int32, device="cuda")
+    plan = api.BatchPlan(cs.descs)
+    plan.run(cuda.from_numpy(cs.comp).to("cuda"), out, st)
+    got = out.cpu().numpy()
+    plan.close()
+    step = int(cs.descs[1]["out_off"])
+    return got.reshape(n, step)[:, :size], st.cpu().numpy()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("size", [1, 600, 1100, 4096, 16384])
+@pytest.mark.parametrize("kind", sorted(KINDS))
+def test_files(cuda, native, kind, size):
+    data = KINDS[kind](np.random.default_rng(size), size).tobytes()[:size]
+    parts = [_stream(data, level, strategy, 0) for level, strategy in ((0, 0), (1, 0), (9, 0), (6, zlib.Z_FIXED))]
+    for group in (parts, parts[:1], parts[2:3]):
+        got, st = _batch(cuda, native, group, size, 5000)
+        assert not st.any()
+        assert np.all(got == np.frombuffer(data, np.uint8))
 
 
 @pytest.mark.gpu
@@ -105,3 +134,27 @@ def test_cost(cuda, native, kind, chunk, most):
             if r == 0 and i == 0:
                 assert not st.cpu().numpy().any() and np.array_equal(out.cpu().numpy(), raw)
     assert best[0] < most * best[1], best
+
+
+@pytest.mark.gpu
+def test_cost_of_files(cuda, native):
+    """20000 files of 4 KiB of random bytes in one plan: teams take 18 times as long as a device copy."""
+    from codag_b200 import api
+    n, size = 20000, 4096
+    raw = np.random.default_rng(3).integers(0, 256, size, dtype=np.uint8).tobytes()
+    cs = api.pack_chunks([np.frombuffer(zlib.compress(raw, 6), np.uint8)] * n, [native.DEFLATE] * n, [1] * n, [size] * n)
+    comp = cuda.from_numpy(cs.comp).to("cuda")
+    out, src = (cuda.zeros(cs.out_bytes, dtype=cuda.uint8, device="cuda") for _ in range(2))
+    plan = api.BatchPlan(cs.descs)
+    best = [1e9, 1e9]
+    for r in range(10):
+        for i, fn in enumerate((lambda: plan.run(comp, out, None), lambda: out.copy_(src))):
+            a, b = cuda.cuda.Event(enable_timing=True), cuda.cuda.Event(enable_timing=True)
+            a.record()
+            fn()
+            b.record()
+            cuda.cuda.synchronize()
+            if r >= 2:
+                best[i] = min(best[i], a.elapsed_time(b))
+    plan.close()
+    assert best[0] < 8 * best[1], best
