@@ -74,14 +74,34 @@ struct Wide<uint32_t> { using T = unsigned int; };
 template <>
 struct Wide<uint64_t> { using T = unsigned long long; };
 
-constexpr uint32_t kTile = 3072;  // values whose items are found at a time (2048: 1 to 8% slower; 4000: one CTA per SM)
-constexpr uint32_t kAhead = 160;                 // values of an item beyond them (at most 129)
-constexpr uint32_t kMaskWords = (kTile + kAhead) / 32;
-constexpr uint32_t kItems = kTile / 2 + 64;      // a literal between runs of three: two items per four values
+// How a chunk is encoded: TILE values whose items are found at a time, by FRONT warps, and BACK warps that encode them
+// meanwhile; FRONT = 0: one warp that does one after the other.
+template <uint32_t TILE, uint32_t FRONT, uint32_t BACK, uint32_t CTAS>
+struct Shape {
+  static constexpr bool kAlone = FRONT == 0;
+  static constexpr uint32_t kTile = TILE, kFront = kAlone ? 1 : FRONT, kBack = BACK, kCtas = CTAS;
+  static constexpr uint32_t kThreads = 32 * (FRONT + BACK);
+  static constexpr uint32_t kAhead = 160;  // values of an item beyond the tile (at most 129)
+  static constexpr uint32_t kMaskWords = (TILE + kAhead) / 32;
+  static constexpr uint32_t kItems = TILE / 2 + 64;  // a literal between runs of three: two items per four values
+};
+using BigV1 = Shape<3072, 8, 8, 2>;   // tiles of 2048: 1 to 8% slower; of 4000: one CTA per SM
+using BigV2 = Shape<3072, 5, 11, 2>;
+using Small = Shape<256, 0, 1, 24>;   // tiles of 128 and 32 CTAs: 10% faster up to 128 values, slower above
+
+// A big CTA is busy 7 us with the smallest chunk, and two fit an SM.  So many small chunks have a CTA of one warp each, which
+// takes longer over long ones, the more so for RLE v2, whose items cost more.  Measured, us, big | small, 64-bit values,
+// RLE v1: 65536 chunks of 64 values 1420 - 1690 | 290 - 340, 16384 of 256 380 - 520 | 94 - 145, 4096 of 1024
+// 114 - 196 | 67 - 115; RLE v2: 2070 - 2470 | 316 - 447, 670 - 700 | 132 - 249, 200 - 240 | 112 - 359.
+template <bool V1>
+bool small_pays(uint64_t n, uint64_t values) {
+  return n > 2 * 148 && values <= 2048 && n >= (V1 ? 1 : 6) * values;
+}
 
 // one tile: its values, comparisons and items
-template <typename T>
+template <typename T, class S>
 struct EncodeTile {
+  static constexpr uint32_t kTile = S::kTile, kAhead = S::kAhead, kMaskWords = S::kMaskWords, kItems = S::kItems;
   T val[kTile + kAhead];
   uint32_t a[kMaskWords];  // RLE v1: a run starts here; RLE v2: the third of three equal values
   uint32_t b[kMaskWords];  // RLE v1: the step to the next value equals the one after; RLE v2: equals the value before
@@ -91,10 +111,12 @@ struct EncodeTile {
   uint64_t next;           // first value of the tile after
 };
 
-template <typename T, uint32_t FRONT, uint32_t BACK, bool V1>
+template <typename T, class S, bool V1>
 struct EncodeShared {
-  static constexpr uint32_t kFront = FRONT, kBack = BACK;
-  EncodeTile<T> tile[2];
+  static constexpr bool kAlone = S::kAlone;
+  static constexpr uint32_t kFront = S::kFront, kBack = S::kBack, kCtas = S::kCtas, kItems = S::kItems, BACK = kBack;
+  static constexpr uint32_t kThreads = S::kThreads;
+  EncodeTile<T, S> tile[kAlone ? 1 : 2];
   uint32_t off[kItems];           // size of each item
   uint32_t end[V1 ? 1 : kItems];  // RLE v2: where it ends in the tile's bytes
   uint32_t how[V1 ? 1 : kItems];  // RLE v2: see ItemV2::pack
@@ -167,9 +189,10 @@ __device__ __forceinline__ uint32_t varint_byte(uint64_t v, uint32_t k, uint32_t
 }
 
 // --- RLE v1 items ---------------------------------------------------------------------------------
-template <typename T>
+template <typename T, class S>
 struct ItemV1 {
-  using Shared = EncodeShared<T, 8, 8, true>;
+  using Shared = EncodeShared<T, S, true>;
+  using Tile = EncodeTile<T, S>;
 
   static __device__ __forceinline__ uint32_t measure(const T* v, uint32_t n, bool run, Shared&, uint32_t, uint32_t,
                                                      uint32_t lane) {
@@ -210,9 +233,10 @@ struct ItemV1 {
 };
 
 // --- RLE v2 items (the choices are those of RleV2Writer, ../rle_writers.h) ------------------------------
-template <typename T>
+template <typename T, class S>
 struct ItemV2 {
-  using Shared = EncodeShared<T, 5, 11, false>;
+  using Shared = EncodeShared<T, S, false>;
+  using Tile = EncodeTile<T, S>;
   enum : uint32_t { kShortRepeat, kDirect, kDeltaFixed, kDelta, kPatched };
   uint64_t v[4];   // value 32 q + lane
   uint64_t first, second, lmin;
@@ -508,9 +532,10 @@ struct ItemV2 {
 };
 
 // Front warps: the tile whose first value is t0.
-template <bool V1, typename T, uint32_t FRONT, class Get>
-__device__ __forceinline__ void prepare_tile(EncodeTile<T>& t, const Get& get, uint64_t t0, uint64_t n, uint32_t warp,
+template <bool V1, typename T, class S, class Get>
+__device__ __forceinline__ void prepare_tile(EncodeTile<T, S>& t, const Get& get, uint64_t t0, uint64_t n, uint32_t warp,
                                              uint32_t lane) {
+  constexpr uint32_t kTile = S::kTile, kAhead = S::kAhead, kMaskWords = S::kMaskWords, FRONT = S::kFront;
   const uint32_t end = static_cast<uint32_t>(n - t0 < kTile + kAhead ? n - t0 : kTile + kAhead);
   constexpr uint32_t kStep = 32 * FRONT;
   for (uint32_t i = 32u * warp + lane; i < end; i += 8 * kStep) {
@@ -573,16 +598,18 @@ __device__ __forceinline__ void prepare_tile(EncodeTile<T>& t, const Get& get, u
   t.next = t0 + p;
 }
 
-// One CTA per chunk.  Bound by the latency of the front's walk and of the back's longest items.
+// One CTA per chunk.  Bound by the latency of the front's walk and of the back's longest items, with small chunks by
+// how many fit the GPU at once.
 template <class Item, typename T, bool V1>
-__global__ void __launch_bounds__(32 * (Item::Shared::kFront + Item::Shared::kBack), 2)
+__global__ void __launch_bounds__(Item::Shared::kThreads, Item::Shared::kCtas)
     k_encode(const uint8_t* __restrict__ in, uint64_t in_bytes, uint64_t chunk_bytes, uint8_t* __restrict__ scratch,
              uint64_t slot, uint64_t* __restrict__ lens) {
-  constexpr uint32_t kFront = Item::Shared::kFront, kBack = Item::Shared::kBack;
+  constexpr bool kAlone = Item::Shared::kAlone;
+  constexpr uint32_t kFront = kAlone ? 0 : Item::Shared::kFront, kBack = Item::Shared::kBack;
   extern __shared__ __align__(16) uint8_t smem[];
   auto& sh = *reinterpret_cast<typename Item::Shared*>(smem);
   const uint32_t lane = threadIdx.x & 31u;
-  const bool front = threadIdx.x < 32u * kFront;
+  const bool front = threadIdx.x < 32u * kFront;  // none where one warp does all
   const uint32_t warp = (threadIdx.x >> 5) - (front ? 0u : kFront);
   const uint64_t chunk = blockIdx.x;
   const uint64_t n = chunk_bytes / sizeof(T);
@@ -594,10 +621,12 @@ __global__ void __launch_bounds__(32 * (Item::Shared::kFront + Item::Shared::kBa
   if (threadIdx.x < 4) sh.taken[threadIdx.x >> 1][threadIdx.x & 1u] = 0;
   __syncthreads();
   for (uint32_t c = 0; ready < n || have; c ^= 1u) {
-    if (front) {
-      if (ready < n) prepare_tile<V1, T, kFront>(sh.tile[c], get, ready, n, warp, lane);
-    } else if (have) {
-      const EncodeTile<T>& t = sh.tile[c ^ 1u];
+    if (front || kAlone) {
+      if (ready < n) prepare_tile<V1, T>(sh.tile[kAlone ? 0 : c], get, ready, n, warp, lane);
+      __syncwarp();
+    }
+    if (kAlone || (!front && have)) {
+      const typename Item::Tile& t = sh.tile[kAlone ? 0 : c ^ 1u];
       const uint32_t items = t.items;
       // RLE v2 items take from 50 to some 600 instructions, so the warps take them as they come (1064 us with
       // every kBack-th for each warp, 1032 with the measuring as they come, 932 with the writing, too); RLE v1
@@ -650,8 +679,9 @@ __global__ void __launch_bounds__(32 * (Item::Shared::kFront + Item::Shared::kBa
       base += total;
     }
     __syncthreads();
-    have = ready < n;
-    if (have) ready = sh.tile[c].next;
+    have = ready < n && !kAlone;
+    if (ready < n) ready = sh.tile[kAlone ? 0 : c].next;
+    if (kAlone) __syncwarp();
   }
   if (threadIdx.x == 32u * kFront) lens[chunk] = base > slot ? kOverflow : base;
 }
@@ -739,16 +769,24 @@ uint64_t slot_of(int codec, uint64_t chunk_bytes, int e) {
   return (b + 15u) / 16u * 16u;
 }
 
+template <class Item, typename T, bool V1>
+bool launch_shape(const uint8_t* in, uint64_t in_bytes, uint64_t chunk, uint64_t n, uint8_t* scratch, uint64_t slot,
+                  uint64_t* lens, cudaStream_t s) {
+  auto kern = k_encode<Item, T, V1>;
+  constexpr uint32_t bytes = sizeof(typename Item::Shared);
+  if (codag_capi::allow_smem(kern, bytes) != cudaSuccess) return false;
+  kern<<<static_cast<unsigned>(n), Item::Shared::kThreads, bytes, s>>>(in, in_bytes, chunk, scratch, slot, lens);
+  return true;
+}
+
 template <int CODEC, typename T>
 bool launch_encode(const uint8_t* in, uint64_t in_bytes, uint64_t chunk, uint64_t n, uint8_t* scratch, uint64_t slot,
                    uint64_t* lens, cudaStream_t s) {
   constexpr bool V1 = CODEC == CODAG_CODEC_RLEV1;
-  using Item = std::conditional_t<V1, ItemV1<T>, ItemV2<T>>;
-  auto kern = k_encode<Item, T, V1>;
-  constexpr uint32_t bytes = sizeof(typename Item::Shared);
-  if (codag_capi::allow_smem(kern, bytes) != cudaSuccess) return false;
-  kern<<<static_cast<unsigned>(n), 32 * (Item::Shared::kFront + Item::Shared::kBack), bytes, s>>>(in, in_bytes, chunk, scratch, slot, lens);
-  return true;
+  using Big = std::conditional_t<V1, ItemV1<T, BigV1>, ItemV2<T, BigV2>>;
+  using One = std::conditional_t<V1, ItemV1<T, Small>, ItemV2<T, Small>>;
+  const auto launch = small_pays<V1>(n, chunk / sizeof(T)) ? launch_shape<One, T, V1> : launch_shape<Big, T, V1>;
+  return launch(in, in_bytes, chunk, n, scratch, slot, lens, s);
 }
 
 template <int CODEC>
