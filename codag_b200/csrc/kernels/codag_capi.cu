@@ -247,10 +247,10 @@ codag_status launch_rle_out(const codag_tune& t, const uint8_t* comp, uint64_t c
                             const uint64_t* col_len, uint64_t n, uint64_t chunk_bytes, uint8_t* out,
                             uint64_t out_bytes, int32_t* status, void* ws, uint64_t ws_bytes, cudaStream_t s) {
   using L = std::conditional_t<DIRECT, RleDirectLayout<NSLOT>, RleLayout<NSLOT>>;
-  // With more chunks than warps are resident (32 per SM), CTAs of at most four warps: a slot is taken again
-  // as soon as its four are done (RLE v2, 1 GiB of 64-bit values 438 us with eight, 428 with four, 700 MB of 32-bit
-  // values 615 | 595; 256 MiB, all resident at once, 190 | 191).
-  const int warps = n > 32 * kSms && t.warps_per_cta > 4 ? 4 : t.warps_per_cta;
+  // With more chunks than warps are resident (32 per SM), CTAs of four warps in the place of the default's eight: a slot is
+  // taken again as soon as its four are done (RLE v2, 1 GiB of 64-bit values 438 us with eight, 428 with four, 700 MB
+  // of 32-bit values 615 | 595; 256 MiB, all resident at once, 190 | 191; not measured with a workspace or the ring).
+  const int warps = DIRECT && !ws && n > 32 * kSms && t.warps_per_cta == 8 ? 4 : t.warps_per_cta;
   const uint32_t smem = L::kPerWarp * warps;
   auto kern = k_rle_plain<NSLOT, CODEC, E, DIRECT>;
   if (allow_smem(kern, smem) != cudaSuccess) return CODAG_ECUDA;
@@ -441,7 +441,7 @@ extern "C" codag_status codag_set_tune(int codec, const codag_tune* tune) {
   if (codec != CODAG_CODEC_DEFLATE && tune->ring_slots < 4) return CODAG_EINVAL;
   if (tune->cta_per_chunk != 0 && tune->cta_per_chunk != 1) return CODAG_EINVAL;
   if (tune->table_global != 0) return CODAG_EINVAL;  // per-file calls: tables in shared memory (no workspace)
-  // a Deflate chunk per CTA takes a decoder and an expander warp: an even count, up to 4 pairs
+  // refused since a Deflate chunk per CTA meant pairs of warps
   if (codec == CODAG_CODEC_DEFLATE && tune->cta_per_chunk && (tune->warps_per_cta & 1)) return CODAG_EINVAL;
   std::lock_guard<std::mutex> g(g_mu);
   g_tune[codec] = *tune;

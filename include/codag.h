@@ -172,14 +172,15 @@ codag_status codag_compress_rlev2(const uint8_t *d_in, uint64_t in_bytes, uint64
  * Process-wide launch shape for the per-file calls above, per codec.  It applies to the RLE
  * kernels that give each chunk one warp: RLE v2 with more than 444 chunks or streams of some
  * hundred bytes, RLE v1 with more than 900 chunks whose streams are short for their number, calls
- * with a workspace, and outputs that are not element aligned.  warps_per_cta is the number of chunks one CTA decodes (1..8);
- * ring_slots the depth of the TMA input ring (2, 4 or 8 slots of 1 KiB; the RLE codecs need at
- * least 4 because an RLE v2 header with its data spans up to 2060 bytes).
- * cta_per_chunk = 1 gives each RLE chunk a whole CTA whatever their number (without it, those not
- * named above have one; it applies without a workspace, when the output and out_bytes are element
- * aligned).  Deflate chunks are decoded by a team of six warps each, or by one where many small
- * ones, or long runs or stored bytes, make that faster: their shape, and lut_bits (9, 10 or 11), are
- * checked and kept, and change nothing.
+ * with a workspace, and outputs that are not element aligned.  warps_per_cta is the number of
+ * chunks one CTA decodes (1..8; 8, the default, becomes 4 for more than 4736 chunks with an
+ * aligned output and no workspace); ring_slots the depth of the TMA input ring (2, 4 or 8 slots of
+ * 1 KiB; the RLE codecs need at least 4 because an RLE v2 header with its data spans up to 2060
+ * bytes).  cta_per_chunk = 1 gives each RLE chunk a whole CTA whatever their number (without it,
+ * those not named above have one; it applies without a workspace, when the output and out_bytes
+ * are element aligned).  Deflate chunks are decoded by a team of six warps each, or by one warp
+ * where many small ones, or long runs or stored bytes, make that faster: their shape, and lut_bits
+ * (9, 10 or 11), are checked and kept, and change nothing.
  * Values outside the supported sets return CODAG_EINVAL. */
 typedef struct {
     int32_t warps_per_cta;
