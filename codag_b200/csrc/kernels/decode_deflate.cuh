@@ -1151,20 +1151,23 @@ __device__ __forceinline__ int inflate_copy(InflateTeam& sm, OUT& out, const uin
       for (uint32_t i = 0; i < kSteps; i++)
         if (32u * i + lane < n) out.put8(op + 32u * i + lane, v[i]);
       __syncwarp();
-    } else if (near >= kRepeatedBytes) {
-      out.flushed = near == kStoredBytes ? copy_stored(out, op, n, src - lo, b.from, lo + len, lane)
-                                         : copy_repeated(out, op, n, b.from, lane);
-    } else if (near > n) {  // one match, repeating itself
-      const uint32_t d = b.word[0] + 1u, step = 32u % d;
-      uint32_t r = lane % d;
+    } else if (near > n) {
+      if (near == kStoredBytes) {
+        out.flushed = copy_stored(out, op, n, src - lo, b.from, lo + len, lane);
+      } else if (near == kRepeatedBytes) {
+        out.flushed = copy_repeated(out, op, n, b.from, lane);
+      } else {  // one match, repeating itself
+        const uint32_t d = b.word[0] + 1u, step = 32u % d;
+        uint32_t r = lane % d;
 #pragma unroll 4
-      for (uint32_t at = lane; at - lane < n; at += 32) {
-        const uint32_t v = out.get8(op - d + r);
-        if (at < n) out.put8(op + at, v);
-        r += step;
-        if (r >= d) r -= d;
+        for (uint32_t at = lane; at - lane < n; at += 32) {
+          const uint32_t v = out.get8(op - d + r);
+          if (at < n) out.put8(op + at, v);
+          r += step;
+          if (r >= d) r -= d;
+        }
+        __syncwarp();
       }
-      __syncwarp();
     } else {
 #pragma unroll 1
       for (uint32_t h = 0; h < n; h += 128) {
