@@ -49,8 +49,8 @@ enum { CODAG_CODEC_RLEV1 = 0, CODAG_CODEC_RLEV2 = 1, CODAG_CODEC_DEFLATE = 2 };
  *   elem_bytes  1, 2, 4 or 8 (the DATA_TYPE template argument)
  *   d_workspace optional scratch of codag_workspace_bytes(codec, n_chunks) bytes, 256-byte
  *               aligned; with it the headers are walked one thread per chunk before the
- *               warp-per-chunk expansion; NULL decodes each chunk in a single warp pass,
- *               which measures faster on B200 (the walk is bound by dependent global loads)
+ *               warp-per-chunk expansion; NULL decodes each chunk in one pass, by a CTA or a
+ *               warp, which measures faster on B200 (the walk is bound by dependent global loads)
  */
 codag_status codag_decompress_rlev1(const uint8_t *d_comp, uint64_t comp_bytes,
                                     const uint64_t *d_blk_off, const uint64_t *d_col_len,
@@ -244,7 +244,7 @@ codag_status codag_batch_destroy(codag_plan *plan);
  * may be NULL = descriptor order) is the order the warps take chunks in; d_queue is 4 bytes
  * of device memory that this call resets on `stream`; d_status has n entries (may be NULL)
  * and entry i reports descriptor i.  Streams have six warps or one as in a plan, which a small
- * kernel before the launch finds out.  tune may be NULL; it is checked and changes nothing.
+ * kernel before the launch finds out, and six where the GPU holds as many for each.  tune may be NULL; it is checked and changes nothing.
  * Allocates nothing; the number of CTAs that the device holds is looked up once and cached. */
 codag_status codag_batch_launch(const codag_chunk_desc *d_descs, const uint32_t *d_order, uint64_t n,
                                 uint32_t *d_queue, const codag_tune *tune, const uint8_t *d_comp,
