@@ -53,7 +53,7 @@ WORKLOADS = {
     "rlev1x128": dict(codec=0, n=134_217_728, elem=8, desc="ORC RLE v1, 134,217,728 uint64 (1 GiB), 8192 x 128 KiB chunks"),
     "deflate": dict(codec=2, n=1 << 30, elem=1, desc="Deflate (zlib level 6), 1 GiB Zipf text, 8192 x 128 KiB chunks"),
 }
-TEAM_CHUNKS = 444  # up to this many RLE v2 chunks have a CTA each, RLE v1 chunks at any count
+TEAM_CHUNKS = 444  # up to this many RLE v2 chunks of these workloads have a CTA each, the RLE v1 chunks all
 
 
 def _kernel_name(codec: int, t, n: int, two_pass: bool) -> str:
@@ -375,7 +375,7 @@ def measure_encode(workload: str, local: int, steps: int = 5) -> dict:
     torch.cuda.empty_cache()
     return {"workload": "GPU encode of " + w["desc"], "value": round(f["col"].size / dt / 1e9, 2), "unit": "GB/s",
             "ms_per_step": round(dt * 1e3, 3), "bit_exact_vs_host_producer": ok,
-            "how": f"codag_compress_rlev{codec + 1}: one warp per chunk, scan, gather; input bytes per second"}
+            "how": f"codag_compress_rlev{codec + 1}: one CTA per chunk, scan, gather; input bytes per second"}
 
 
 def measure_transposed(local: int, steps: int = 10, read_unit: int = 1) -> dict:

@@ -6,10 +6,10 @@ u32 or u64 (50/50); about 3.8 GB decompressed.  Seeded per rank (weak scaling).
 
 Two ways of decoding the same resident set are timed:
   batched   one persistent launch over all files (codag_batch_run, replayed from a CUDA
-            graph), launch shape from the autotuner;
+            graph), whose shape the plan picks by the files;
   per-file  one C-ABI call per file, in order on one stream -- the only way CODAG's kernels,
             which take one uniform chunk size per launch, can decode such a set.  Its full
-            run takes minutes (each Deflate file is decoded by one warp), so it is timed on a
+            run takes minutes (20,000 launches with an SM or two at work), so it is timed on a
             stratified sample of the files; its GB/s is the sample's bytes over its time.
 Both outputs are checked byte for byte against the source slices.
 """
@@ -116,7 +116,7 @@ def main(args, rank: int, world: int, local: int):
     d_st = torch.zeros(ms.n, dtype=torch.int32, device=dev)
     want = torch.from_numpy(ms.expected()).to(dev)
 
-    # launch shape: autotuner over (warps_per_cta, ring_slots, lut_bits), cached per GPU
+    # launch shape: the tune fields, which a plan checks and does not use
     shape = None
     if args.tune:
         shape = tuple(int(x) for x in args.tune.split(","))

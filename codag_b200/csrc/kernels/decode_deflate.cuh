@@ -32,8 +32,8 @@
 // why the work is spread over as many warps as it is.
 //
 // Text in 128 KiB chunks (zlib level 6), one symbol at a time on one or two warps | by teams:
-// 256 MiB 8.6 ms | 2.4, 8 MiB 6.8 ms | 0.39, 200 KB 6.6 ms | 0.46; a 40 MB column in 64 KiB chunks of
-// level 9 6.3 ms | 0.85.  A lone chunk takes 0.37 ms: the scan's chain of table look-ups, some 310 cycles
+// 256 MiB 8.6 ms | 2.3, 8 MiB 6.8 ms | 0.40, 200 KB 6.6 ms | 0.39; a 40 MB column in 64 KiB chunks of
+// level 9 6.3 ms | 0.84.  (Many small chunks are left to single warps, decode_deflate_warp.cuh.)  A lone chunk takes 0.37 ms: the scan's chain of table look-ups, some 310 cycles
 // a symbol for 64 lanes (warm-up 30%, pieces 45%, headers and tables 9%).  With three teams on every SM
 // all stages slow down together, a third of the issue slots used and a third of the stalls waiting for
 // instructions: seven different loops compete for the instruction cache, so what makes them longer

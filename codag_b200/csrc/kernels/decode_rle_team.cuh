@@ -17,8 +17,8 @@
 // that may be longer than kLongestLiteral, a stream that ends early) is left to the one-warp decoder, which
 // starts the chunk over and reports the exact error.
 //
-// One warp per chunk | a team: RLE v1, 8 MiB of 64-bit values 214 us | 46, 256 MiB of 32-bit values
-// 577 | 335 (8 warps; 6, 10 or 12 gain nothing); RLE v2, 3 MB of 16-bit values 434 | 165 (16 warps; 24 or
+// One warp per chunk | a team: RLE v1, 8 MiB of 64-bit values 214 us | 43, 256 MiB of 32-bit values
+// 577 | 321 (8 warps; 6, 10 or 12 gain nothing); RLE v2, 3 MB of 16-bit values 434 | 160 (16 warps; 24 or
 // 32 are slower from 256 chunks on).  Alone, a chunk waits for the walk (some 60 cycles a header) and the
 // barriers between steps; many keep the issue slots 70% busy, mostly with literals' varints.
 #pragma once

@@ -1,17 +1,17 @@
 // Device building blocks shared by the chunk decoders (sm_100a).
 //
 //   InRing   the compressed stream of one chunk, staged into a shared-memory ring of 1 KiB
-//            slots by TMA bulk copies (cp.async.bulk ... mbarrier::complete_tx).  The warp
-//            that decodes the chunk is both producer and consumer: it issues the copies
-//            for the slots ahead of its read position and waits on each slot's mbarrier
-//            (bounded, see wait_slot) before reading it.  This replaces CODAG's
+//            slots by TMA bulk copies (cp.async.bulk ... mbarrier::complete_tx).  One warp
+//            issues the copies for the slots ahead of its read position and waits on each
+//            slot's mbarrier (bounded, see wait_slot) before it reads the slot; in a team the
+//            other warps read what that warp has waited for, after a barrier of theirs.  This replaces CODAG's
 //            warp-cooperative refill (include/common_warp.h:730-950) and its spin queues
 //            (common_warp.h:72-372).  Every copy is a plain single-CTA bulk copy.
 //   OutRing  a shared-memory staging ring for decoded bytes, drained to global memory in
 //            fixed-size pieces with coalesced 16-byte vector stores.
 //
-// Conventions: one warp decodes one chunk; every lane keeps an identical copy of the
-// decoder state (control flow is warp-uniform); lane 0 issues the TMA copies.
+// Conventions: the lanes of a warp keep identical copies of the state of the rings they use, whether the warp
+// decodes a chunk alone or as one of a team; lane 0 issues the TMA copies.
 #pragma once
 #include <cstdint>
 

@@ -19,7 +19,7 @@
 //     literals, in groups of 127.
 //   RLE v2: from p, the first three equal values in a row within 128 values start a fixed run, which
 //     goes on for at most 128 values; what lies before them, else 128 values, is a variable group.
-// So a CTA's front warps take kTile values at a time into shared memory and write their comparisons as
+// So a CTA's front warps take a tile of 3072 values at a time into shared memory and write their comparisons as
 // bit masks, then the length that an item starting at each of the values would have, all in parallel;
 // one lane follows the lengths from item to item (searching the masks there instead took 480 cycles
 // an item).  Meanwhile
@@ -27,7 +27,8 @@
 // the items' bytes.  With one warp per chunk running the state machine, an item cost about 9000 warp
 // instructions and a chunk had one warp to wait for.
 //
-// RLE v2, 256 MiB of 64-bit values: 3.75 ms with a warp per chunk, 0.91 now (2 CTAs of 16 warps per SM,
+// Many small chunks have a CTA of one warp each (Small).
+// RLE v2, 256 MiB of 64-bit values: 3.75 ms with a warp per chunk, 0.90 now (2 CTAs of 16 warps per SM,
 // which registers allow; 3 or 4 with fewer registers each: 1.26, 1.40; three, four, six, eight
 // front warps instead of five: 0.99, 0.93, 0.93, 0.99).  RLE v1,
 // 20 MB of 32-bit values: 1.60 ms, 0.12 now.

@@ -174,7 +174,7 @@ SERVE_SHAPES = [(8, 4, 10, 0)]
 
 def tune_server(srv: "Server", n_requests: int = 96, seed: int = 7, use_cache: bool = True):
     """Times a burst of n_requests requests that all arrive at once (the loop saturated) for each
-    shape of SERVE_SHAPES, installs the fastest on `srv` and returns it; the result is cached per
+    shape of SERVE_SHAPES if there is a choice, installs the fastest on `srv` and returns it; the result is cached per
     GPU model next to the decoders' (codag_b200.tuning)."""
     from . import tuning
     hit = tuning.load_cached(-1, "serve") if use_cache else None
@@ -184,7 +184,7 @@ def tune_server(srv: "Server", n_requests: int = 96, seed: int = 7, use_cache: b
     rng = np.random.default_rng(seed)
     burst = [(0.0, int(f)) for f in rng.integers(0, len(srv.pool.files), n_requests)]
     best, best_t = None, None
-    for shape in SERVE_SHAPES:
+    for shape in SERVE_SHAPES if len(SERVE_SHAPES) > 1 else ():
         srv.tune = native.Tune(*shape, 0)
         t0 = time.perf_counter()
         reqs = srv.run(burst)
@@ -193,6 +193,7 @@ def tune_server(srv: "Server", n_requests: int = 96, seed: int = 7, use_cache: b
             raise RuntimeError(f"serving shape {shape}: a request did not decode exactly")
         if best_t is None or t < best_t:
             best, best_t = shape, t
+    best = best or SERVE_SHAPES[0]
     srv.tune = native.Tune(*best, 0)
     tuning.store_cached(-1, "serve", best)
     return best

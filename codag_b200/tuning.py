@@ -3,7 +3,7 @@
 Per codec it times every supported combination of
   warps_per_cta  chunks decoded by one CTA (one warp per chunk): 1, 2, 4, 8
   ring_slots     depth of the TMA input ring in 1 KiB slots: 4, 8
-  cta_per_chunk  RLE v2: a whole CTA per chunk instead of one warp, whatever their number
+  cta_per_chunk  RLE: a whole CTA per chunk instead of one warp, whatever their number
 on a resident sample of the caller's chunks, installs with codag_set_tune the fastest if it is faster
 than the library's own shape by more than such times differ from one another (else that one), and caches it in
 a JSON file keyed by GPU name and codec, so later runs on the same kind of GPU skip the search.
