@@ -110,6 +110,20 @@ def test_files(cuda, native, kind, size):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("size", [1, 31, 33, 256, 511, 513, 3073, 8192])
+@pytest.mark.parametrize("kind", sorted(KINDS))
+def test_few_files(cuda, native, kind, size):
+    """Few files have teams, however small they are."""
+    data = KINDS[kind](np.random.default_rng(size), size).tobytes()[:size]
+    parts = [_stream(data, level, strategy, every)
+             for level, strategy in ((0, 0), (1, 0), (9, 0), (6, zlib.Z_FIXED), (6, zlib.Z_HUFFMAN_ONLY))
+             for every in (0, max(size // 7, 1), max(size // 2 - 1, 1))]
+    got, st = _batch(cuda, native, parts, size, len(parts))
+    assert not st.any()
+    assert np.all(got == np.frombuffer(data, np.uint8))
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("kind,chunk,most", [("text", 1024, 150), ("zeros", 4096, 20), ("noise", 4096, 5)])
 def test_cost(cuda, native, kind, chunk, most):
     """64 MiB; teams take 220, 50 and 7.7 times as long as a device copy."""
