@@ -128,7 +128,8 @@ __device__ __forceinline__ bool rle_team_takes(const BatchArgs& a, const codag_c
          (d.comp_len | d.out_len) < 0x80000000u;
 }
 
-// RLE files of up to this size are taken by a warp each.  So are longer RLE v2 files where there are more of them
+// RLE files below this size, and RLE v2 files of it, are taken by a warp each (3000 RLE v1 files of 32 KiB without a
+// plan: 179 us by warps | 143).  So are longer RLE v2 files where there are more of them
 // than CTAs are resident (as in codag_decompress_rlev2; 2048 of 128 KiB: 257 us | 581 by CTAs), but for the
 // longest: those above the smallest power of two that no more than the resident CTAs exceed, so that a few
 // long files among many are not left to single warps (450 of 40 KB and one of 8 MiB: 7.1 ms by warps | 5.3).
@@ -147,7 +148,7 @@ __host__ __device__ __forceinline__ uint32_t v2_shift(const uint32_t* long_v2, u
   return s;
 }
 __host__ __device__ __forceinline__ bool rle_team_pays(const codag_chunk_desc& d, uint32_t shift) {
-  if (d.out_len <= kWarpBytes || d.comp_len <= kTeamMinBytes) return false;  // (3000 of 40 KB in 120 bytes each: 112 us | 97)
+  if (d.out_len < kWarpBytes || d.comp_len <= kTeamMinBytes) return false;  // (3000 of 40 KB in 120 bytes each: 112 us | 97)
   if (d.codec == CODAG_CODEC_RLEV1) return true;
   // mostly DIRECT groups, if it is that long: see rlev2_alone
   const bool direct = d.comp_len > (2u + d.elem_bytes / 4u) * static_cast<uint64_t>(d.out_len / d.elem_bytes);
@@ -178,7 +179,7 @@ constexpr uint32_t kCountBits = 25, kAnyTeam = 1u << 31, kInflateWarps = 1u << k
 constexpr uint64_t kMaxMixed = (1u << (kCountBits - 1)) - 65536u;  // counts to twice that, and once more per warp
 __device__ __forceinline__ bool wants_team(const BatchArgs& a, const codag_chunk_desc& d, uint32_t flags) {
   if (d.codec == CODAG_CODEC_DEFLATE) return !(flags & kInflateWarps) || !InflateJob(d).small();
-  return d.out_len > kWarpBytes && rle_team_takes(a, d) && rle_team_pays(d, (flags & ~kAnyTeam) >> kShiftAt);
+  return d.out_len >= kWarpBytes && rle_team_takes(a, d) && rle_team_pays(d, (flags & ~kAnyTeam) >> kShiftAt);
 }
 __global__ void __launch_bounds__(1024) k_classify(BatchArgs a, uint32_t n, uint32_t resident, uint32_t* __restrict__ queue) {
   __shared__ uint32_t long_v2[kShifts];

@@ -223,8 +223,8 @@ typedef struct {
 typedef struct codag_plan codag_plan;
 
 /* Copies the descriptors to the device (the only allocating call), orders the queue and
- * picks the launch shape by their sizes: Deflate streams, and RLE streams of more than 32 KiB
- * whose output is element aligned, are decoded by six warps together, longest first, other RLE
+ * picks the launch shape by their sizes: Deflate streams, and RLE v1 streams of at least and RLE v2
+ * streams of more than 32 KiB whose output is element aligned, are decoded by six warps together, longest first, other RLE
  * streams, and Deflate streams where many are small, by a warp each.  So are longer RLE v2 streams where more than fill the GPU with six
  * warps each: then only those of at least 64 KiB (128 KiB, 256 KiB, ... as long as they are still
  * too many) have six warps.  tune (may be NULL) is checked (cta_per_chunk 0..4, with an even

@@ -146,3 +146,29 @@ def test_a_long_file_among_many(cuda, native):
     for p in plans:
         p.close()
     assert among < 1.2 * alone, (alone, among)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("planned", [True, False])
+def test_rlev1_files_of_32_kib(cuda, native, planned):
+    """3000 RLE v1 files of exactly 32 KiB take what as many of 33 KiB take; with a warp each, 1.6 times as long."""
+    from codag_b200 import api
+    calls, keep = [], []
+    for size in (32 * KIB, 33 * KIB):
+        col = native.gen_rlev1_column(size, 3, 1)
+        blob, _, ln = native.encode_rlev1(col, size, 1)
+        cs = api.pack_chunks([blob[8:8 + int(ln[0])]] * 3000, [V1] * 3000, [1] * 3000, [size] * 3000)
+        comp, out = cuda.from_numpy(cs.comp).to("cuda"), cuda.zeros(cs.out_bytes, dtype=cuda.uint8, device="cuda")
+        st = cuda.full((3000,), -1, dtype=cuda.int32, device="cuda")
+        if planned:
+            plan = api.BatchPlan(cs.descs)
+            keep.append(plan)
+            calls.append(lambda plan=plan, comp=comp, out=out, st=st: plan.run(comp, out, st))
+        else:
+            calls.append(_launch(native, cuda, cs.descs, None, comp, out, st))
+        calls[-1]()
+        assert not st.cpu().numpy().any() and np.array_equal(out.cpu().numpy()[:size], col)
+    at, above = _us(cuda, *calls)
+    for plan in keep:
+        plan.close()
+    assert at < 1.2 * above, (at, above)
